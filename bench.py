@@ -39,15 +39,14 @@ UNIT = "rays/s"
 FALLBACK_HBM_GBS = 6800.0
 L2_FLUSH_BYTES = 256 << 20
 PCL_POINT_BYTES = 16
-STATUS_BYTES = 80  # device status block (DevStatus) read back by every call
+STATUS_BYTES = 88  # device status block (DevStatus) read back by every call
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch of
 # each kernel on a steady-state dense scan, from one ncu capture of the
 # default workload's launch list (the last of three inserts; prep = k_prep +
 # k_scatter). Only meaningful for the dense workload; other workloads report
 # None.
-NCU_TRAFFIC_BYTES = {"k_dda_mark": 429.4e6, "k_apply_runs": 804.0e6, "k_sweep": 1986.8e6,
-                     "prep (k_prep+k_scan+k_scatter)": 8.4e6}
+NCU_TRAFFIC_BYTES = {}
 
 
 def parse_args():
@@ -479,14 +478,13 @@ def run_ours(args):
     #     read once per touched leaf), over the whole insertion's kernels;
     #   atomics of the marking = V (one visited-bit OR per DDA visit and one
     #     hit-bit OR per unclipped ray, before any merging), over the marking
-    #     kernels (k_mark_hits, k_dda_mark, k_apply_runs), against the L2
+    #     kernels (k_mark_hits, k_march), against the L2
     #     atomic rate measured on this GPU (vdbg_l2_atomic_rate).
-    # Intermediates this design chose (ray records, the DDA run buffer) are
+    # Intermediates this design chose (ray records) are
     # not algorithmic: they show up in `traffic` (ncu DRAM bytes).
     hbm_peak, peak_kind = measured_peaks()
     mean = lambda key: statistics.mean(p[key] for p in phases)  # noqa: E731
     dda = mean("dda_ms")
-    apply_ms = mean("apply_ms")
     sweep = mean("sweep_ms")
     prep = mean("prep_ms")
     mean_u = statistics.mean(s["updates"] for s in stats)
@@ -508,16 +506,16 @@ def run_ours(args):
         atomic = {"achieved": a_achieved, "peak": atomic_rate["random"] / 1e9, "unit": "G atomics/s",
                   "frac": a_achieved / (atomic_rate["random"] / 1e9), "peak_kind": "measured (vdbg_l2_atomic_rate)",
                   "peak_coalesced": atomic_rate["coalesced"] / 1e9, "algorithmic_atomics_per_launch": mean_v,
-                  "launch_ms": dda, "scope": "the marking (k_mark_hits, k_dda_mark, k_apply_runs)",
-                  "note": "the marking merges visits into z-plane runs and leaf masks before its ORs reach L2, so "
-                          "it issues far fewer atomics than V"}
+                  "launch_ms": dda, "scope": "the marking (k_mark_hits, k_march)",
+                  "note": "the marking merges visits into z-plane runs before its ORs reach L2, so it issues far "
+                          "fewer atomics than V"}
     top = atomic if atomic and atomic["frac"] > hbm["frac"] else hbm
     per_kernel = {
         "prep (k_prep+k_scan+k_scatter)": {"ms": prep, "algorithmic_bytes": 12.0 * n_pts,
                                            "traffic": traffic.get("prep (k_prep+k_scan+k_scatter)")},
-        "marking (k_mark_hits+k_dda_mark+k_apply_runs)": {
+        "marking (k_mark_hits+k_march)": {
             "ms": dda, "algorithmic_atomics": mean_v,
-            "traffic": (traffic["k_dda_mark"] + traffic["k_apply_runs"]) if traffic else None},
+            "traffic": traffic.get("k_march")},
         "sweep (k_compact+k_sweep)": {"ms": sweep, "algorithmic_bytes": 8.25 * mean_u + 128.0 * mean_lt,
                                       "GBps": (8.25 * mean_u + 128.0 * mean_lt) / (sweep / 1000.0) / 1e9,
                                       "traffic": traffic.get("k_sweep")},
@@ -532,14 +530,14 @@ def run_ours(args):
         "voxel_updates_per_s": updates / total_s,
         "latency_ms": {"p50": float(np.percentile(step_ms, 50)), "p99": float(np.percentile(step_ms, 99)),
                        "max": max(step_ms)},
-        "phases_ms": {"prep": prep, "traversal (k_mark_hits+k_dda_mark)": dda - apply_ms, "k_apply_runs": apply_ms,
+        "phases_ms": {"prep": prep, "marking (k_mark_hits+k_march)": dda,
                       "sweep (k_compact+k_sweep)": sweep, "kernels_total": mean_total_ms},
         "per_scan": {"rays": n_pts, "visits": statistics.mean(s["visits"] for s in stats),
                      "runs": mean_runs, "updates": mean_u, "touched_leaves": mean_lt,
                      "new_leaves": statistics.mean(s["new_leaves"] for s in stats),
                      "dda_passes": [p["passes"] for p in phases], "warmup_dda_passes": warmup_passes},
         "roofline": {"bound": "l2_atomic" if top is atomic else "hbm",
-                     "kernel": "marking (k_mark_hits+k_dda_mark+k_apply_runs)" if top is atomic else
+                     "kernel": "marking (k_mark_hits+k_march)" if top is atomic else
                                "the whole insertion",
                      "achieved": top["achieved"], "peak": top["peak"], "unit": top["unit"], "frac": top["frac"],
                      "traffic": hbm["traffic"], "hbm": hbm, "atomic": atomic, "per_kernel": per_kernel},

@@ -156,9 +156,9 @@ typedef struct vdbg_timings
   uint64_t launches;       /* kernels launched by the call */
   uint64_t launches_total; /* kernels launched by this map since creation */
   uint64_t retries;        /* re-marking passes after a pool or hash growth */
-  double apply_ms;         /* the run-merging kernel (k_apply_runs) alone, all passes (part of dda_ms) */
-  uint64_t runs;           /* slab runs the traversal wrote (the merging kernel's input) */
-  uint64_t passes;         /* DDA passes of the call (more than one when the run buffer filled) */
+  double apply_ms;         /* 0: the traversal applies its runs itself (part of dda_ms) */
+  uint64_t runs;           /* z-plane runs the traversal applied to the update masks */
+  uint64_t passes;         /* 1 when rays were traversed voxel by voxel, else 0 */
 } vdbg_timings;
 
 int vdbg_get_timings(const vdbg_map* map, vdbg_timings* out);
@@ -242,11 +242,11 @@ int vdbg_export_changes(vdbg_map* map, int map_index, int64_t capacity, int32_t*
  * on a sample of the caller's scans. */
 typedef struct vdbg_tuning
 {
-  int32_t rays_per_take;     /* rays a DDA warp takes from the sorted order at a time (1-1024; 32) */
-  int32_t apply_chunk_runs;  /* DDA runs an apply block stages and merges at a time (256-4096, a multiple of 256; 2048) */
-  int32_t length_edges[3];   /* L1 lengths (voxels) starting the sort's length classes, descending (2048, 1024, 512) */
+  int32_t rays_per_take;     /* an eighth of it: chunks of 32 rays a warp takes at a time, at most (1-1024; 32) */
+  int32_t apply_chunk_runs;  /* checked (256-4096, a multiple of 256; 2048), steers nothing */
+  int32_t length_edges[3];   /* checked (positive, descending; 2048, 1024, 512), steers nothing */
   float hash_load;           /* block-hash load factor (0.05-0.9; 0.5); a change rebuilds the hash */
-  int32_t dda_warps_per_sm;  /* resident DDA warps per SM (2-20, even; 16) */
+  int32_t dda_warps_per_sm;  /* resident traversal warps per SM in sixteenths of what fits (2-20, even; 16) */
   int32_t sweep_kernel;      /* 0 (default): one z-plane per lane, or for a batch of maps eight lanes
                                 per z-plane when its previous sweep updated 16-30 voxels per touched
                                 leaf; 1: one z-plane per lane; 2: eight lanes per z-plane */
@@ -263,8 +263,7 @@ int vdbg_get_tuning(const vdbg_map* map, vdbg_tuning* out);
  * vdbg_insert_point_cloud, but the per-scan scratch lives in one fixed
  * VDBG_NOALLOC_SCRATCH_BYTES device array inside the library (held by every
  * GPU that loads it, until the process exits) instead of buffers the map
- * grows on demand. It also runs its ray traversal on fewer warps, in as many
- * passes as the scan needs, so it is slower than the regular call. Limits:
+ * grows on demand. Limits:
  * n <= VDBG_NOALLOC_MAX_POINTS and, for host input,
  * stride_bytes <= 16; larger inputs return VDBG_ERR_SIZE_LIMIT. The map's leaf
  * pool is not grown: when it is full the call returns VDBG_ERR_OUT_OF_MEMORY,
@@ -275,8 +274,6 @@ int vdbg_get_tuning(const vdbg_map* map, vdbg_tuning* out);
  * so calls that overlap on the GPU (other threads, other streams, other maps)
  * race: serialise them. */
 #define VDBG_NOALLOC_MAX_POINTS 262144
-#define VDBG_NOALLOC_DDA_WARPS 256
-#define VDBG_NOALLOC_RUN_SEGMENT 4096
 #define VDBG_NOALLOC_SCRATCH_BYTES (28u << 20)
 int vdbg_insert_point_cloud_noalloc(vdbg_map* map, const float* xyz, int64_t n, int64_t stride_bytes,
                                     const double origin[3], const char* source_id, uint32_t flags,
@@ -409,11 +406,10 @@ int vdbg_raytrace(vdbg_map* map, int map_index, int64_t n, const double* origins
 
 /* CUDA-graph replay of vdbg_batch_insert (batches of two or more maps; on by
  * default). The step is captured once per buffer layout and replayed as one
- * graph launch: prep, endpoint hits, the first DDA pass with its apply,
- * compact, sweep. It is captured again after a pool, scratch or run-buffer
- * reallocation or a tuning change (the input's address and point counts
- * reach the graph through device memory). When a step
- * needs a second DDA pass or a pool to grow, the graph's compact and sweep
+ * graph launch: prep, endpoint hits beside the traversal, compact, sweep. It
+ * is captured again after a pool or scratch reallocation or a tuning change
+ * (the input's address and point counts reach the graph through device
+ * memory). When a step needs a pool to grow, the graph's compact and sweep
  * skip themselves on the device and the call finishes the step with separate
  * launches. Off, or with change tracking on, every step uses separate
  * launches; the results are the same either way. vdbg_graph_stats reports

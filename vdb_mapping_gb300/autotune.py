@@ -1,9 +1,9 @@
 """Autotuner of the insertion kernels' launch and layout parameters.
 
-The parameters (``vdbg_tuning``: resident DDA warps per SM, rays a DDA warp
-takes from the sorted order at a time, runs an apply block merges at a time,
-the L1 edges of the sort's length classes, the block-hash load factor) change
-speed only, never the map.
+The parameters (``vdbg_tuning``: resident traversal warps per SM, chunks of
+rays a warp takes at a time, the block-hash load factor) change speed only,
+never the map. ``apply_chunk_runs`` and ``length_edges`` are accepted and steer
+nothing, so they have one candidate.
 ``tune`` times candidates on a sample of the caller's own scans, each on a
 fresh map (or batch) so the timed inserts see the same map states, and keeps
 the fastest by coordinate descent: one parameter at a time, starting from the
@@ -18,10 +18,10 @@ DEFAULT = {"rays_per_take": 32, "apply_chunk_runs": 2048, "length_edges": (2048,
 
 CANDIDATES = {
     "rays_per_take": (8, 16, 32),
-    "apply_chunk_runs": (1024, 2048, 4096),
-    "length_edges": ((512, 256, 128), (1024, 512, 256), (2048, 1024, 512), (2048, 768, 256)),
+    "apply_chunk_runs": (2048,),
+    "length_edges": ((2048, 1024, 512),),
     "hash_load": (0.25, 0.5),
-    "dda_warps_per_sm": (6, 8, 12, 16, 20),
+    "dda_warps_per_sm": (8, 12, 16),
 }
 
 

@@ -78,10 +78,10 @@ constexpr uint32_t kMetaL1Mask   = (1u << 29) - 1;
 constexpr uint32_t kMetaClipped  = 1u << 29;
 constexpr uint32_t kMetaValid    = 1u << 30;
 
-// Counting-sort buckets of the DDA order: 8 length classes x scans x 1014
+// Counting-sort buckets of the ray order: 11 length classes x scans x 1014
 // direction cells (see ray_bucket).
 constexpr int kDirCells    = 1014;
-constexpr int kLenClasses  = 8;
+constexpr int kLenClasses  = 11;
 constexpr int kBucketsPerScan = kLenClasses * kDirCells;
 
 struct DevStatus
@@ -95,11 +95,12 @@ struct DevStatus
   unsigned long long hits;
   unsigned long long updates;
   unsigned long long nonfinite;
-  uint32_t ray_cursor;  // next position in the ray order handed to a DDA warp
+  uint32_t max_l1;      // longest ray, when in the first length class (else 0)
   uint32_t n_blocks;    // block bump allocator
-  uint32_t inflight;    // lanes that ended a DDA pass with a ray in flight
   uint32_t windows;     // update-grid windows closed by k_finish_window
-  unsigned long long runs;  // plane runs written by the traversal (all passes)
+  uint32_t pad;
+  unsigned long long runs;         // plane runs merged by k_march
+  unsigned long long item_cursor;  // next work item of k_march
 };
 
 struct LogOdds
@@ -137,7 +138,7 @@ struct ScanTable
   const uint32_t* first;    // [n + 1] (n > 1)
   const uint16_t* ray_scan; // [rays] scan of each ray (n > 1)
   int n;
-  uint32_t edge[3];         // L1 lengths that start the length classes 0, 1, 2 (descending)
+  int clog;                 // log2 of the most steps of a chunk of k_march
 };
 
 __device__ __forceinline__ int scan_of_point(const ScanTable& t, uint32_t i)
@@ -176,43 +177,6 @@ struct MapView
   int4* origin;
   uint32_t capacity;
   DevStatus* st;
-};
-
-// Plane runs of one DDA pass: a run is the set of voxels one ray visits in one
-// z-plane (64 voxels, one mask word) of one leaf. Warp w of the pass writes its
-// runs to its own segment [w * seg, w * seg + count[w]).
-struct RunBuffer
-{
-  unsigned long long* key;   // leaf key
-  unsigned long long* bits;  // visited voxels of the plane, bit (y & 7) << 3 | (x & 7)
-  unsigned char* slab;       // z & 7 (the mask word)
-  uint32_t* count;           // runs per warp segment
-  uint32_t seg;              // segment capacity (runs)
-  uint32_t warps;            // segments
-  uint32_t take;             // rays a DDA warp takes from the order at a time
-  uint32_t apply_chunk;      // runs an apply block merges at a time
-  uint32_t* chunk_prefix;    // [warps + 1] apply chunks of the segments before each (k_apply_prefix)
-  uint32_t* ticket;          // next apply chunk to hand out
-};
-
-// DDA state of a lane whose ray was still in flight when its warp's segment
-// filled; the next pass resumes from it.
-struct LaneState
-{
-  long long nx, ny, nz;
-  double dx, dy, dz;
-  unsigned long long run;
-  int vx, vy, vz;
-  int rx, ry, rz;
-  int sx, sy, sz;
-  uint32_t budget;
-  uint32_t flags;  // bit 0: has_ray, bit 1: run_open
-  uint32_t map;
-};
-
-struct WarpState
-{
-  uint32_t chunk_next, chunk_end, drained, pad;
 };
 
 struct ChannelView
@@ -274,6 +238,18 @@ __device__ __forceinline__ uint32_t ld_ca_u32(const uint32_t* p)
   asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ ulonglong2 ld_ca_u64x2(const unsigned long long* p)
+{
+  ulonglong2 v;
+  asm volatile("ld.global.ca.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int2 ld_ca_s32x2(const int* p)
+{
+  int2 v;
+  asm volatile("ld.global.ca.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
 // Relaxed (coherent, unordered) load and store at device scope: for a value
 // that is itself the whole message, with nothing else to order behind it.
 // The pools publish slots this way: within a kernel the threads that wait
@@ -291,56 +267,6 @@ __device__ __forceinline__ void st_relaxed_s32(int* p, int v)
   asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// ---- bulk asynchronous copies (global -> shared) completed on an mbarrier ----
-__device__ __forceinline__ uint32_t smem_u32(const void* p)
-{
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, uint32_t count)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-// Orders this thread's earlier shared-memory accesses (and an mbarrier
-// initialisation) before later asynchronous-proxy accesses to shared memory.
-__device__ __forceinline__ void fence_proxy_async_smem()
-{
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, uint32_t bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-// `bytes` from global `src` to shared `dst`; both 16-byte aligned, bytes a
-// multiple of 16. Completion is counted on `bar`.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, unsigned long long* bar)
-{
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                 smem_u32(dst)),
-               "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, uint32_t parity)
-{
-  uint32_t ok;
-  asm volatile(
-    "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-    : "=r"(ok)
-    : "r"(smem_u32(bar)), "r"(parity)
-    : "memory");
-  return ok != 0u;
-}
-// Bounded wait for phase `parity` of `bar`; false when it gave up.
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, uint32_t parity)
-{
-  for (uint32_t i = 0; i < kSpinLimit; ++i)
-  {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (i > 64) __nanosleep(128);
-  }
-  return false;
-}
-
 // Murmur3 64-bit finaliser (published mixing function).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long k)
 {
@@ -350,6 +276,25 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long k)
   k *= 0xc4ceb9fe1a85ec53ull;
   k ^= k >> 33;
   return k;
+}
+
+// Home of a block key in the block hash: a 32-bit multiply-xor mix of its
+// halves (every run that k_march applies takes one). Homes are even, so that a
+// probe's first two entries are one aligned pair.
+__device__ __forceinline__ uint32_t block_home(unsigned long long key, uint32_t mask)
+{
+  uint32_t h = static_cast<uint32_t>(key) * 0x9E3779B1u ^ static_cast<uint32_t>(key >> 32) * 0x85EBCA77u;
+  h ^= h >> 15;
+  h *= 0xC2B2AE3Du;
+  h ^= h >> 13;
+  return h & mask & ~1u;
+}
+
+// Sets an error bit; one that is set already is left alone (a pool that ran
+// out is met by every later allocation).
+__device__ __forceinline__ void set_error(DevStatus* st, uint32_t bit)
+{
+  if (!(ld_ca_u32(&st->error) & bit)) atomicOr(&st->error, bit);
 }
 
 __device__ __forceinline__ int unpack_leaf_coord(unsigned long long key, int field)
@@ -373,13 +318,9 @@ __device__ __forceinline__ unsigned long long pack_leaf_key(int map, int lx, int
 
 // Appends block `b` to the channel's touched-block list the first time it is
 // seen in the current integration window.
-// True when this call's marking is complete and free of errors (every ray
-// cast, none left in flight), so its update grids may be integrated.
-__device__ __forceinline__ bool marking_complete(const DevStatus* st)
-{
-  return ld_relaxed_u32(&st->error) == 0u && ld_relaxed_u32(&st->inflight) == 0u &&
-         ld_relaxed_u32(&st->ray_cursor) >= ld_relaxed_u32(&st->n_valid);
-}
+// True when this call's marking is free of errors (k_march casts every ray),
+// so its update grids may be integrated.
+__device__ __forceinline__ bool marking_complete(const DevStatus* st) { return ld_relaxed_u32(&st->error) == 0u; }
 
 __device__ __forceinline__ void touch_block(const ChannelView& c, int b)
 {
@@ -404,7 +345,7 @@ __device__ __forceinline__ void touch_block(const ChannelView& c, int b)
 __device__ __forceinline__ int find_or_insert_block(const MapView& m, int map, int bx, int by, int bz)
 {
   const unsigned long long key = pack_leaf_key(map, bx, by, bz);
-  uint32_t h                   = static_cast<uint32_t>(mix64(key)) & m.bhmask;
+  uint32_t h                   = block_home(key, m.bhmask);
   for (uint32_t probe = 0; probe < kMaxProbes; ++probe)
   {
     unsigned long long k = ld_ca_u64(m.bkeys + h);
@@ -417,7 +358,7 @@ __device__ __forceinline__ int find_or_insert_block(const MapView& m, int map, i
         int slot;
         if (s >= m.bcapacity)
         {
-          atomicOr(&m.st->error, kErrBlockFull);
+          set_error(m.st, kErrBlockFull);
           slot = kSlotFailed;
         }
         else
@@ -440,7 +381,7 @@ __device__ __forceinline__ int find_or_insert_block(const MapView& m, int map, i
         // (a wait that another thread already gave up on ends here too)
         if (++spins > kSpinLimit || ((spins & 1023u) == 0u && (ld_relaxed_u32(&m.st->error) & kErrSpin)))
         {
-          atomicOr(&m.st->error, kErrSpin);
+          set_error(m.st, kErrSpin);
           return kSlotFailed;
         }
         __nanosleep(64);
@@ -449,14 +390,16 @@ __device__ __forceinline__ int find_or_insert_block(const MapView& m, int map, i
       if (s < 0)
       {
         // An allocation that failed earlier: the host has to grow and retry.
-        atomicOr(&m.st->error, kErrBlockFull);
+        set_error(m.st, kErrBlockFull);
         return kSlotFailed;
       }
       return s;
     }
+    // (a hash another thread found full: the call is repeated anyway)
+    if ((probe & 63u) == 63u && (ld_relaxed_u32(&m.st->error) & kErrHashFull)) return kSlotFailed;
     h = (h + 1) & m.bhmask;
   }
-  atomicOr(&m.st->error, kErrHashFull);
+  set_error(m.st, kErrHashFull);
   return kSlotFailed;
 }
 
@@ -477,7 +420,7 @@ __device__ __forceinline__ int find_or_insert_leaf(const MapView& m, int b, int 
       const uint32_t t = atomicAdd(&m.st->n_leaves, 1u);
       if (t >= m.capacity)
       {
-        atomicOr(&m.st->error, kErrPoolFull);
+        set_error(m.st, kErrPoolFull);
         st_relaxed_s32(e, kLeafFailed);
         return kSlotFailed;
       }
@@ -493,7 +436,7 @@ __device__ __forceinline__ int find_or_insert_leaf(const MapView& m, int b, int 
     // (a wait that another thread already gave up on ends here too)
     if (++spins > kSpinLimit || ((spins & 1023u) == 0u && (ld_relaxed_u32(&m.st->error) & kErrSpin)))
     {
-      atomicOr(&m.st->error, kErrSpin);
+      set_error(m.st, kErrSpin);
       return kSlotFailed;
     }
     __nanosleep(64);
@@ -502,7 +445,7 @@ __device__ __forceinline__ int find_or_insert_leaf(const MapView& m, int b, int 
   if (s < 0)
   {
     // An allocation that failed earlier: the host has to grow and retry.
-    atomicOr(&m.st->error, kErrPoolFull);
+    set_error(m.st, kErrPoolFull);
     return kSlotFailed;
   }
   return s;

@@ -6,11 +6,9 @@
 //   k_scan     (none)                   exclusive scan of the bin histogram
 //   k_scatter  (none)                   counting-sort scatter of ray ids (rays
 //                                       grouped by direction)
-//   k_dda_mark VDBMapping.hpp:550-566    FP64 DDA from the sensor voxel to the
-//                                       endpoint voxel; writes the visited
-//                                       voxels as z-plane runs
-//   k_apply_runs VDBMapping.hpp:563     merges the runs, ORs them into the
-//                                       per-leaf update masks
+//   k_march    VDBMapping.hpp:550-566   DDA from the sensor voxel to the endpoint
+//                                       voxel, in chunks; ORs the visited voxels
+//                                       into the per-leaf update masks
 //   k_mark_hits VDBMapping.hpp:533-536  hit bits of unclipped endpoints
 //   k_compact  (none)                   touched blocks -> flat touched-leaf list
 //   k_sweep    VDBMapping.hpp:731-792 + per touched leaf: FP32 log-odds update,
@@ -31,18 +29,34 @@
 
 #include "device_common.cuh"
 #include "hdda.cuh"
+#include "march.cuh"
 #include "morph.cuh"
 
 namespace vdbg {
 
+// Length classes of the sort, longest first: rays of 2^9 chunks and more
+// (march.cuh), one class per number of chunks down to two, and those of one
+// chunk by halves of a chunk. The rays of a class have the same number of
+// chunks (the first class up to the scan's longest ray), so the lanes of a
+// ray group walk equally far.
+__device__ __forceinline__ int ray_class(uint32_t l1, int clog)
+{
+  const int p = march::chunk_log2(l1, clog);
+  return p > 0 ? max(9 - p, 0) : (l1 > (1u << (clog - 1)) ? 9 : 10);
+}
+// log2 of the chunks of class k's rays, at most.
+__device__ __forceinline__ int class_log2(int k, uint32_t max_l1, int clog)
+{
+  return k == 0 ? max(9, march::chunk_log2(max_l1, clog)) : max(9 - k, 0);
+}
+static_assert(kLenClasses == 11, "length classes");
+
 // Sort bucket of a ray of scan s (voxel offset d from the sensor voxel, L1
-// length l1): eight length classes, longest first, so long rays start early
-// and do not extend the tail; within a class the scan, then the cube-map face
-// of the dominant axis and a 13 x 13 cell on it (6 * 169 = 1014 direction
-// cells). Rays of one bucket are angular neighbours of similar length in one
-// map; the DDA hands warps short runs of this order so their lanes walk
-// through the same leaves and their leaf records merge. Order only; the map
-// does not depend on it.
+// length l1): its length class, then the scan, then the cube-map face of the
+// dominant axis and a 13 x 13 cell on it (6 * 169 = 1014 direction cells).
+// Rays of one bucket are angular neighbours of similar length in one map; a
+// warp walks 32 consecutive rays of this order, so its lanes go through the
+// same leaves and their runs merge. Order only; the map does not depend on it.
 __device__ __forceinline__ int ray_bucket(int dx, int dy, int dz, uint32_t l1, int s, const ScanTable& t)
 {
   const int n_scans = t.n;
@@ -69,20 +83,7 @@ __device__ __forceinline__ int ray_bucket(int dx, int dy, int dz, uint32_t l1, i
     v    = dy;
     mx   = az;
   }
-  // Three tuned edges, then halvings of the last edge (four at most), so the
-  // shortest rays come last and the end of a pass waits on short rays only.
-  int cls;
-  if (l1 >= t.edge[0])
-    cls = 0;
-  else if (l1 >= t.edge[1])
-    cls = 1;
-  else if (l1 >= t.edge[2])
-    cls = 2;
-  else
-  {
-    const int halvings = (31 - __clz(static_cast<int>(t.edge[2]))) - (31 - __clz(static_cast<int>(max(l1, 1u)))) - 1;
-    cls                = 3 + min(max(halvings, 0), kLenClasses - 4);
-  }
+  const int cls  = ray_class(l1, t.clog);
   const int base = (cls * n_scans + s) * kDirCells;
   if (mx == 0) return base;
   const int iu = static_cast<int>((static_cast<long long>(u + mx) * 13) / (2 * mx + 1));
@@ -177,8 +178,11 @@ __global__ void __launch_bounds__(256) k_prep(const char* __restrict__ pts, cons
     sr += __shfl_xor_sync(0xffffffffu, sr, off);
     sn += __shfl_xor_sync(0xffffffffu, sn, off);
   }
+  const uint32_t longest = __reduce_max_sync(0xffffffffu, meta & kMetaL1Mask);
   if ((threadIdx.x & 31) == 0)
   {
+    // (only the first length class needs the longest ray's length)
+    if (ray_class(longest, t.clog) == 0) atomicMax(&st->max_l1, longest);
     if (sv) atomicAdd(&st->visits, sv);
     if (sh) atomicAdd(&st->hits, sh);
     if (sr) atomicAdd(&st->rays, sr);
@@ -362,45 +366,6 @@ __global__ void __launch_bounds__(256) k_scatter(const int4* __restrict__ rays, 
   order[base + rank] = static_cast<int>(i);
 }
 
-// ---------------------------------------------------------------------------
-// k_dda_mark: warp-cooperative traversal, writing plane runs.
-//
-// Each lane walks one ray at a time with the FP64 DDA of OpenVDB's
-// DDA<Ray<double>,0> as driven by castRayIntoGrid (eye = origin voxel + 0.5,
-// dir = end - origin, t in [0,1]). The positive tMax values are compared as
-// int64 bit patterns, which order like the doubles, so the only FP64 operation
-// per step is the sequential tMax += tDelta of the stepped axis; the step is
-// branch-free so the 32 lanes stay converged.
-//
-// A ray is monotone in every axis, so it visits each z-plane of each 8^3 leaf
-// (64 voxels, one mask word) in a single contiguous run; a near-horizontal
-// ray (LiDAR, depth cameras) stays in one plane for its whole crossing of a
-// leaf. The lane keeps the
-// bits of the current run in a register; a run is emitted at the first step
-// that leaves it (or after the ray's last voxel). Each step the warp ranks
-// its emitting lanes with one ballot and appends their runs to the warp's
-// record list in shared memory, packed in step order; every kDdaSteps steps
-// the list is copied to the warp's segment of the run buffer with plain
-// coalesced stores, and k_apply_runs merges and applies the segments. Rays
-// come from the length-then-direction order in short runs per warp
-// (ray_bucket), so a segment holds runs of neighbouring rays.
-//
-// A pass ends for a warp when its segment cannot take another round: the
-// lanes' DDA state and the warp's ray run are saved and the next pass
-// (resume != 0) continues from them, after k_apply_runs emptied the buffer.
-// ---------------------------------------------------------------------------
-constexpr int kDdaWarps      = 2;                // warps per block
-constexpr int kDdaSteps      = 16;               // DDA steps between ring copies
-constexpr int kDdaRing       = kDdaSteps + 1;    // emissions per lane per round: one per step + the flush
-constexpr uint32_t kDdaRound = 32u * kDdaRing;   // most runs a warp writes per round
-
-struct DdaWarpSmem
-{
-  unsigned long long keys[kDdaRound];  // leaf key of the run
-  unsigned long long bits[kDdaRound];  // visited voxels of the plane
-  unsigned char slab[kDdaRound];       // z & 7 of the plane (its mask word)
-};
-
 __device__ __forceinline__ uint32_t lanemask_lt()
 {
   uint32_t m;
@@ -408,28 +373,9 @@ __device__ __forceinline__ uint32_t lanemask_lt()
   return m;
 }
 
-// Emits the lane's open run when `close` (ranked among the warp's emitting
-// lanes by one ballot) at position *n of the warp's record list.
-__device__ __forceinline__ void dda_emit(DdaWarpSmem& q, bool close, uint32_t lt, int map, int rx, int ry, int rz,
-                                         unsigned long long& run, bool& run_open, uint32_t& n)
-{
-  const unsigned em = __ballot_sync(0xffffffffu, close);
-  if (close)
-  {
-    const uint32_t p = n + static_cast<uint32_t>(__popc(em & lt));
-    q.keys[p]        = pack_leaf_key(map, rx, ry, rz >> 3);
-    q.bits[p]        = run;
-    q.slab[p]        = static_cast<unsigned char>(rz & 7);
-    run              = 0ull;
-    run_open         = false;
-  }
-  n += static_cast<uint32_t>(__popc(em));
-}
-
-// OpenVDB's DDA<Ray<double>,0> (VDBMapping.hpp:554-558) for one ray from
-// the origin voxel o to the end voxel e: eye = o + 0.5, dir = e - o, t in
-// [0, 1]. tMax is kept as the bit pattern of a non-negative double, so the
-// argmin is an integer compare.
+// OpenVDB's DDA<Ray<double>,0> on integer-keyed state: tMax is kept as the bit
+// pattern of a non-negative double, so the argmin is an integer compare (fast
+// mode's span walk; the insertion's walk is march.cuh).
 struct DdaRay
 {
   int vx, vy, vz;        // current voxel
@@ -438,53 +384,8 @@ struct DdaRay
   double dx, dy, dz;     // tDelta
 };
 
-constexpr long long kDdaOne = 0x3ff0000000000000ll;  // bits of 1.0
-constexpr long long kDdaMax = 0x7fefffffffffffffll;  // bits of DBL_MAX
-
-__device__ __forceinline__ void dda_setup(const int o[3], const int e[3], DdaRay& r)
-{
-  int vox[3], stp[3];
-  long long nxt[3];
-  double dlt[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-  {
-    const double eye = __dadd_rn(static_cast<double>(o[a]), 0.5);
-    const double dir = __dsub_rn(static_cast<double>(e[a]), static_cast<double>(o[a]));
-    const double pos = __dadd_rn(eye, __dmul_rn(dir, 0.0));
-    vox[a]           = static_cast<int>(floor(pos));
-    if (dir == 0.0)
-    {
-      stp[a] = 0;
-      nxt[a] = kDdaMax;
-      dlt[a] = 1.7976931348623157e308;
-    }
-    else
-    {
-      const double inv = __ddiv_rn(1.0, dir);
-      if (inv > 0.0)
-      {
-        stp[a] = 1;
-        nxt[a] = __double_as_longlong(
-          __dadd_rn(0.0, __dmul_rn(__dsub_rn(static_cast<double>(vox[a] + 1), pos), inv)));
-      }
-      else
-      {
-        stp[a] = -1;
-        nxt[a] = __double_as_longlong(__dadd_rn(0.0, __dmul_rn(__dsub_rn(static_cast<double>(vox[a]), pos), inv)));
-      }
-      dlt[a] = __dmul_rn(static_cast<double>(stp[a]), inv);
-    }
-  }
-  r.vx = vox[0]; r.vy = vox[1]; r.vz = vox[2];
-  r.sx = stp[0]; r.sy = stp[1]; r.sz = stp[2];
-  r.nx = nxt[0]; r.ny = nxt[1]; r.nz = nxt[2];
-  r.dx = dlt[0]; r.dy = dlt[1]; r.dz = dlt[2];
-}
-
 // DDA::step(): argmin of tMax with ties to the higher axis, branch-free; the
-// sequential tMax += tDelta in FP64. Returns the bits of the t it stepped at
-// (the ray goes on while that is <= 1.0).
+// sequential tMax += tDelta in FP64. Returns the bits of the t it stepped at.
 __device__ __forceinline__ long long dda_advance(DdaRay& r)
 {
   const bool ax      = (r.nx < r.ny) && (r.nx < r.nz);
@@ -501,487 +402,450 @@ __device__ __forceinline__ long long dda_advance(DdaRay& r)
   return t0;
 }
 
-__global__ void __launch_bounds__(kDdaWarps * 32, 10) k_dda_mark(const int4* __restrict__ rays,
-                                                               const int* __restrict__ order, ScanTable t,
-                                                               MapView m, RunBuffer rb,
-                                                               LaneState* __restrict__ lstate,
-                                                               WarpState* __restrict__ wstate, int resume)
-{
-  __shared__ DdaWarpSmem smem[kDdaWarps];
-  const int lane    = static_cast<int>(threadIdx.x & 31);
-  const uint32_t lt = lanemask_lt();
-  const uint32_t gw = blockIdx.x * kDdaWarps + (threadIdx.x >> 5);
-  DdaWarpSmem& q    = smem[threadIdx.x >> 5];
-  const uint32_t nv = m.st->n_valid;
-  const size_t seg0 = static_cast<size_t>(gw) * rb.seg;
-  uint32_t count    = 0;  // runs this warp wrote in this pass
-
-  bool drained        = false;
-  uint32_t chunk_next = 0, chunk_end = 0;  // the warp's current run of rays
-  // Per-lane ray state.
-  bool has_ray = false, run_open = false;
-  int vx = 0, vy = 0, vz = 0, sx = 0, sy = 0, sz = 0;
-  long long nx = 0, ny = 0, nz = 0;
-  double dx = 0.0, dy = 0.0, dz = 0.0;
-  int rx = 0, ry = 0, rz = 0;  // current run: leaf x, leaf y, exact z
-  int map = 0;                 // map of the lane's ray
-  unsigned long long run = 0ull;
-  uint32_t budget = 0;
-  if (resume)
-  {
-    const WarpState w = wstate[gw];
-    chunk_next        = w.chunk_next;
-    chunk_end         = w.chunk_end;
-    drained           = w.drained != 0u;
-    const LaneState l = lstate[gw * 32 + lane];
-    has_ray           = (l.flags & 1u) != 0u;
-    run_open          = (l.flags & 2u) != 0u;
-    nx = l.nx; ny = l.ny; nz = l.nz;
-    dx = l.dx; dy = l.dy; dz = l.dz;
-    run = l.run;
-    vx = l.vx; vy = l.vy; vz = l.vz;
-    rx = l.rx; ry = l.ry; rz = l.rz;
-    sx = l.sx; sy = l.sy; sz = l.sz;
-    budget = l.budget;
-    map    = static_cast<int>(l.map);
-  }
-  const long long kOne = kDdaOne;
-  bool paused          = false;
-
-  for (;;)
-  {
-    // ---- hand out rays to idle lanes ------------------------------------------
-    // (The traversal allocates nothing, so it ignores the error word: pool
-    // overflows come from k_apply_runs and k_mark_hits, which the host re-runs.)
-    unsigned need = drained ? 0u : __ballot_sync(0xffffffffu, !has_ray);
-    while (need)
-    {
-      // Idle lanes take the next rays of the warp's run of the binned order.
-      if (chunk_next >= chunk_end)
-      {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(&m.st->ray_cursor, rb.take);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= nv)
-        {
-          drained = true;
-          break;
-        }
-        chunk_next = base;
-        chunk_end  = min(base + rb.take, nv);
-      }
-      const uint32_t avail = chunk_end - chunk_next;
-      const uint32_t rank  = static_cast<uint32_t>(__popc(need & lt));
-      const bool take      = ((need >> lane) & 1u) && rank < avail;
-      const uint32_t idx   = chunk_next + rank;
-      const unsigned took  = __ballot_sync(0xffffffffu, take);
-      chunk_next += static_cast<uint32_t>(__popc(took));
-      need &= ~took;
-      if (take)
-      {
-        const int ri      = order[idx];
-        const int4 r      = rays[ri];
-        const uint32_t l1 = static_cast<uint32_t>(r.w) & kMetaL1Mask;
-        if (l1 > 0)
-        {
-          // (An endpoint in the sensor voxel is only a hit; k_mark_hits does it.)
-          const ScanGeom& g = scan_geom(t, scan_of_ray(t, static_cast<uint32_t>(ri)));
-          map               = g.map;
-          const int o[3]    = {g.ovx, g.ovy, g.ovz};
-          const int e[3]    = {r.x, r.y, r.z};
-          DdaRay d;
-          dda_setup(o, e, d);
-          vx = d.vx; vy = d.vy; vz = d.vz;
-          sx = d.sx; sy = d.sy; sz = d.sz;
-          nx = d.nx; ny = d.ny; nz = d.nz;
-          dx = d.dx; dy = d.dy; dz = d.dz;
-          budget   = l1 + 1;
-          has_ray  = true;
-          run_open = false;
-        }
-      }
-    }
-    if (__ballot_sync(0xffffffffu, has_ray) == 0u && drained) break;
-    if (count + kDdaRound > rb.seg)
-    {
-      paused = true;  // the segment cannot take another round
-      break;
-    }
-
-    // ---- DDA steps ----------------------------------------------------------------
-    uint32_t n_rec = 0;  // records of this round in the warp's list
-#pragma unroll 4
-    for (int s = 0; s < kDdaSteps; ++s)
-    {
-      // setActiveState(voxel) on the update grid, one z-plane run at a time:
-      // the run of the previous step ends when the voxel leaves it or the ray
-      // ended.
-      const int lx = vx >> 3, ly = vy >> 3;
-      dda_emit(q, run_open && (!has_ray || vz != rz || lx != rx || ly != ry), lt, map, rx, ry, rz, run, run_open,
-               n_rec);
-      if (has_ray)
-      {
-        rx       = lx;
-        ry       = ly;
-        rz       = vz;
-        run_open = true;
-        run |= 1ull << (((vy & 7) << 3) | (vx & 7));
-        DdaRay d{vx, vy, vz, sx, sy, sz, nx, ny, nz, dx, dy, dz};
-        const long long t0 = dda_advance(d);
-        vx = d.vx; vy = d.vy; vz = d.vz;
-        nx = d.nx; ny = d.ny; nz = d.nz;
-        budget -= 1;
-        bool fin = t0 > kOne;
-        if (!fin && budget == 0)
-        {
-          // More than L1 + 1 visits: cannot happen for integer rays.
-          atomicOr(&m.st->error, kErrStepBound);
-          fin = true;
-        }
-        if (fin) has_ray = false;  // its last run is emitted next step
-      }
-    }
-    // Runs of rays that ended in the last step (a refill must not find them open).
-    dda_emit(q, run_open && !has_ray, lt, map, rx, ry, rz, run, run_open, n_rec);
-
-    // ---- copy the list to the warp's segment -------------------------------------
-    __syncwarp();
-    const size_t pos = seg0 + count;
-    for (uint32_t j = static_cast<uint32_t>(lane); j < n_rec; j += 32)
-    {
-      rb.key[pos + j]  = q.keys[j];
-      rb.bits[pos + j] = q.bits[j];
-      rb.slab[pos + j] = q.slab[j];
-    }
-    __syncwarp();
-    count += n_rec;
-  }
-
-  // ---- end of the pass: record the segment and what is left in flight ------------
-  if (lane == 0)
-  {
-    rb.count[gw] = count;
-    if (count) atomicAdd(&m.st->runs, static_cast<unsigned long long>(count));
-    WarpState w;
-    w.chunk_next = chunk_next;
-    w.chunk_end  = chunk_end;
-    w.drained    = drained ? 1u : 0u;
-    w.pad        = 0u;
-    wstate[gw]   = w;
-  }
-  const unsigned live = __ballot_sync(0xffffffffu, has_ray);
-  if (lane == 0 && paused)
-  {
-    const uint32_t left = static_cast<uint32_t>(__popc(live)) + (chunk_end > chunk_next ? chunk_end - chunk_next : 0u);
-    if (left) atomicAdd(&m.st->inflight, left);
-  }
-  LaneState l;
-  l.nx = nx; l.ny = ny; l.nz = nz;
-  l.dx = dx; l.dy = dy; l.dz = dz;
-  l.run = run;
-  l.vx = vx; l.vy = vy; l.vz = vz;
-  l.rx = rx; l.ry = ry; l.rz = rz;
-  l.sx = sx; l.sy = sy; l.sz = sz;
-  l.budget = budget;
-  l.flags  = (has_ray ? 1u : 0u) | (run_open ? 2u : 0u);
-  l.map    = static_cast<uint32_t>(map);
-  lstate[gw * 32 + lane] = l;
-}
-
 // ---------------------------------------------------------------------------
-// k_apply_runs: merges the scan's plane runs and ORs them into the update masks.
+// k_march: castRayIntoGrid for every ray (VDBMapping.hpp:550-566) into the
+// update grid's visited masks.
 //
-// Persistent blocks take chunks of rb.apply_chunk runs of one warp segment
-// (written together by a warp walking neighbouring rays, so a chunk repeats
-// few leaves). A chunk is staged in shared memory by bulk asynchronous copies
-// (three: keys, bits, slab indices) completed on an mbarrier; the copy of a
-// block's next chunk is issued as soon as the current one has been read, so
-// it overlaps the drain. Each thread ORs its runs into the block's leaf table
-// in shared memory (lanes of a warp holding the same leaf probe it once,
-// through their leader); the first insertion of a leaf appends it to the
-// table's list. The block then drains the list in two steps: one thread per
-// listed leaf resolves its slot through the block index (allocating leaves
-// and blocks as needed) and marks it touched, then eight threads per leaf OR
-// its eight mask words into the update masks, so the words of one leaf go
-// out as one coalesced atomic request. A run that finds the table full is
-// applied directly.
+// The rays are walked in chunks of 32 to 128 voxel steps (march.cuh). A work
+// item is chunk i of 32 rays that follow one another in the sorted order; they
+// share a length class, so all of them have 2^p chunks of similar length and
+// the lanes of a warp finish together (8-24% of the step slots are idle). Items are numbered class by class,
+// ray group by ray group, chunk by chunk, and persistent warps take short runs
+// of them from a device cursor: neither a long ray nor a small scan leaves
+// most of the device waiting, and the lanes of an item walk neighbouring rays
+// through the same leaves.
+//
+// A ray is monotone in every axis, so it visits each z-plane of each 8^3 leaf
+// (64 voxels, one mask word) in a single contiguous run. A lane keeps the bits
+// of its current run in a register; a run that ends is appended to the warp's
+// record list in shared memory, ranked among the warp's lanes by one ballot.
+// Records are applied 32 at a time, with every lane busy: a lane finds its
+// run's leaf through the block index (allocating leaves and blocks as needed),
+// marks it touched and ORs the run into the leaf's mask word.
+//
+// A leaf or block pool that runs out sets the error word; the walk goes on, so the
+// allocation counters tell the whole demand (a full block hash, which cannot
+// count, ends it), and the host grows the pools and runs the marking again
+// (the ORs are idempotent).
+//
+// It is bound by the ALU pipe and instruction issue: a step of a warp takes
+// about 48 instructions, 28 of them on the ALU pipe, which takes one every two
+// cycles; applying 32 runs takes about 120. Measured on one GB300 against one
+// FP64 walk per ray with a run buffer and a merging kernel behind it (marking
+// alone, hits included): 262,144-point street scan 0.55 ms (1.10), 307,200-point
+// depth image 0.45 (0.78), 65,536-point room scan 0.097 (0.23), 16,381 random
+// rays of 2,490 steps 0.62 (4.0), 2,048 points 0.027 (0.10).
+// Merging the runs per leaf in shared memory before they reach L2 was slower
+// (0.66-0.73 ms on the street scan): neighbouring rays share too few leaves for
+// the 150 instructions a merge of 32 runs takes, and the tables cost warps.
 // ---------------------------------------------------------------------------
-// Two block shapes: 256 threads with a 512-entry table for chunks of 1280
-// runs and more (3 blocks per SM at 2048), 128 threads with a 256-entry table
-// for chunks of up to 1024 (6 blocks per SM): fewer threads wait at each
-// barrier and more chunks are in flight per SM.
-constexpr uint32_t kApplyMaxChunk   = 4096;  // runs staged at a time, at most
-constexpr uint32_t kApplySmallChunk = 1024;  // largest chunk of the small shape
+constexpr int kMarchWarps          = 2;    // per block (each works by itself)
+constexpr int kMarchBlocks         = 14;   // per SM (72 registers; 12 and 16 were 1-4% slower)
+constexpr int kMarchSteps          = 4;    // steps between looks at the ends and the record list
+constexpr uint32_t kMarchRecords   = 32u * (kMarchSteps + 2);  // a remainder below 32, 8 steps, the last runs
+constexpr uint32_t kMarchMaxRounds = 96;   // far above a chunk's rounds (one more per cut)
 
-template <int kTable>
-struct ApplySmem
+// The axis entries of march.cuh for all n below kAxisTableN in the binades
+// [2^-(j + 1), 2^-j), j < kAxisTableJ, n fastest: with chunks of 64 steps all
+// that rays with L1 up to 65,536 need. Other entries are computed when a chunk
+// begins.
+constexpr uint32_t kAxisTableN   = 16384;
+constexpr int kAxisTableJ        = 10;
+constexpr size_t kAxisTableBytes = size_t(kAxisTableN) * kAxisTableJ * (sizeof(ulonglong2) + sizeof(int2)) +
+                                   size_t(kAxisTableN) * sizeof(double);
+
+struct AxisTable
 {
-  unsigned long long key[kTable];
-  unsigned int words[kTable][16];  // 8 mask words as lo/hi halves
-  int slot[kTable];                // resolved leaf slot of a listed entry
-  unsigned short list[kTable];     // entries in use
-  unsigned long long bar;          // completion of the staged chunk's copies
-  unsigned int count;
-  unsigned int next;               // the block's next chunk ticket
-  unsigned int next_sg, next_start, next_end;  // and its segment and runs
-  unsigned int failed;
+  ulonglong2* td;  // [kAxisTableJ][kAxisTableN] t1, d
+  int2* kf;        // [kAxisTableJ][kAxisTableN] k1, df
+  double* delta;   // [kAxisTableN] 1 / n (DBL_MAX for 0)
 };
 
-// Dynamic shared memory of k_apply_runs for chunks of `chunk` runs.
-__host__ __device__ constexpr size_t apply_stage_bytes(uint32_t chunk)
+__device__ __noinline__ march::Axis axis_entry_far(uint32_t n, int j) { return march::axis_entry(n, j); }
+
+__device__ __forceinline__ march::Axis axis_at(const AxisTable& at, uint32_t n, int j)
 {
-  return static_cast<size_t>(chunk) * 17 + 16;
+  if (n < kAxisTableN && j < kAxisTableJ)
+  {
+    const ulonglong2 td = __ldg(at.td + static_cast<size_t>(j) * kAxisTableN + n);
+    const int2 kf       = __ldg(at.kf + static_cast<size_t>(j) * kAxisTableN + n);
+    return march::Axis{td.x, td.y, static_cast<uint32_t>(kf.x), kf.y};
+  }
+  return n == 0u ? march::axis_never() : axis_entry_far(n, j);
 }
 
-// Table slot of `key` (Fibonacci hashing to log2(kTable) bits).
-template <int kTable>
-__device__ __forceinline__ uint32_t apply_hash(unsigned long long key)
+__device__ __forceinline__ double axis_delta_at(const AxisTable& at, uint32_t n)
 {
-  constexpr int kBits = kTable == 512 ? 9 : 8;
-  static_assert((1 << kBits) == kTable, "table of 256 or 512 entries");
-  return static_cast<uint32_t>((key * 0x9E3779B97F4A7C15ull) >> (64 - kBits));
+  return n < kAxisTableN ? __ldg(at.delta + n) : march::axis_delta(n);
 }
 
-// Slab of leaf `key` in the update masks: resolves (and allocates) the leaf
-// and marks it touched in its block. Returns the leaf slot or kSlotFailed.
-// The common case (block and leaf exist) costs two dependent load pairs: the
-// hash key with its slot, then the leaf cell with the block's epoch; anything
-// else takes the general find-or-insert paths.
-__device__ __forceinline__ int apply_resolve(const MapView& m, const ChannelView& c, unsigned long long key)
+// One thread per entry (a new map).
+__global__ void __launch_bounds__(256) k_axis_table(AxisTable at)
 {
-  const int lx = unpack_leaf_coord(key, 0), ly = unpack_leaf_coord(key, 1), lz = unpack_leaf_coord(key, 2);
-  const int mp = unpack_map(key);
+  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= kAxisTableN * kAxisTableJ) return;
+  const uint32_t n    = x % kAxisTableN;
+  const int j         = static_cast<int>(x / kAxisTableN);
+  const march::Axis a = n == 0u ? march::axis_never() : march::axis_entry(n, j);
+  at.td[x]            = make_ulonglong2(a.t1, a.d);
+  at.kf[x]            = make_int2(static_cast<int>(a.k1), a.df);
+  if (j == 0) at.delta[n] = n == 0u ? hdda::kDblMax : march::axis_delta(n);
+}
+
+// A ray as the walk takes it: origin voxel, signed voxel counts, p (its 2^p
+// chunks; negative: nothing to walk) and map.
+struct MarchRay
+{
+  int ox, oy, oz;
+  int nx, ny, nz;
+  int p;
+  int map;
+};
+
+__device__ __forceinline__ int sign_of(int x) { return (x > 0) - (x < 0); }
+
+// Begins chunk i of ray r: the walk (its `end` possibly cut, see march::Cuts)
+// and the origin leaf (bx, by, bz) its positions are relative to. Returns the
+// chunk's end.
+__device__ __forceinline__ uint32_t march_begin(const AxisTable& at, const MarchRay& r, uint32_t i, march::Walk& w,
+                                                march::Cuts& cuts, int& bx, int& by, int& bz)
+{
+  const uint32_t nx = static_cast<uint32_t>(abs(r.nx)), ny = static_cast<uint32_t>(abs(r.ny)),
+                 nz = static_cast<uint32_t>(abs(r.nz));
+  const int sx = sign_of(r.nx), sy = sign_of(r.ny), sz = sign_of(r.nz);
+  w.px         = sx;
+  w.py         = sy * (1 << march::kPosBits);
+  w.pz         = sz * (1 << (2 * march::kPosBits));
+  int vx = r.ox, vy = r.oy, vz = r.oz;
+  cuts.f[0] = cuts.f[1] = cuts.f[2] = 0;
+  const uint32_t end = march::chunk_end(i, r.p);
+  if (i == 0u)
+  {
+    march::begin_head(w, axis_delta_at(at, nx), axis_delta_at(at, ny), axis_delta_at(at, nz), r.p);
+  }
+  else
+  {
+    const uint64_t tau   = march::threshold_bits(i, r.p);
+    const int j          = r.p - 1 - march::log2_floor(i);
+    const march::Axis ax = axis_at(at, nx, j), ay = axis_at(at, ny, j), az = axis_at(at, nz, j);
+    const march::Start x = march::start_axis(ax, nx, i, r.p, tau);
+    const march::Start y = march::start_axis(ay, ny, i, r.p, tau);
+    const march::Start z = march::start_axis(az, nz, i, r.p, tau);
+    w.tx = x.t;
+    w.ty = y.t;
+    w.tz = z.t;
+    w.dx = x.d;
+    w.dy = y.d;
+    w.dz = z.d;
+    vx += sx * static_cast<int>(x.k);
+    vy += sy * static_cast<int>(y.k);
+    vz += sz * static_cast<int>(z.k);
+    cuts.f[0] = static_cast<int8_t>(x.df);
+    cuts.f[1] = static_cast<int8_t>(y.df);
+    cuts.f[2] = static_cast<int8_t>(z.df);
+    march::cut_end(w, cuts, end);
+  }
+  w.pos = march::first_pos(vx, vy, vz);
+  bx    = march::base_leaf(vx);
+  by    = march::base_leaf(vy);
+  bz    = march::base_leaf(vz);
+  return end;
+}
+
+__device__ __forceinline__ MarchRay march_ray(const int4& r, const ScanGeom& g, int clog)
+{
+  MarchRay q;
+  q.ox              = g.ovx;
+  q.oy              = g.ovy;
+  q.oz              = g.ovz;
+  q.nx              = r.x - g.ovx;
+  q.ny              = r.y - g.ovy;
+  q.nz              = r.z - g.ovz;
+  const uint32_t l1 = static_cast<uint32_t>(r.w) & kMetaL1Mask;
+  // (an endpoint in the sensor voxel is only a hit; k_mark_hits does it)
+  q.p   = l1 == 0u ? -1 : march::chunk_log2(l1, clog);
+  q.map = g.map;
+  return q;
+}
+
+// Sets the position's voxel in the run: its bit is the low six bits of
+// (pos & 7) | (pos >> 6 & ~7).
+__device__ __forceinline__ void march_mark(uint32_t pos, uint32_t& lo, uint32_t& hi)
+{
+  const uint32_t s = (pos & 7u) | ((pos >> (march::kPosBits - 3)) & ~7u);
+  asm("{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b32 b, t;\n\t"
+      "shf.l.wrap.b32 b, 0, 1, %2;\n\t"
+      "and.b32 t, %2, 32;\n\t"
+      "setp.ne.u32 p, t, 0;\n\t"
+      "@p or.b32 %1, %1, b;\n\t"
+      "@!p or.b32 %0, %0, b;\n\t"
+      "}"
+      : "+r"(lo), "+r"(hi)
+      : "r"(s));
+}
+
+struct MarchWarp
+{
+  unsigned long long bits[kMarchRecords];  // a run: its visited voxels,
+  uint32_t pos[kMarchRecords];             // its position (march::Walk), the lane above it
+};
+
+// ORs records [at, at + n) (n <= 32) into the update masks, one lane per run.
+// Finding the word (block and leaf exist) costs three dependent loads: the
+// hash bucket of the block with its slots, the leaf cell, the word itself.
+// Anything else takes the general find-or-insert paths. A word that already
+// holds the bits is left alone: the leaves around the sensor lie on every ray,
+// and their words would otherwise take an atomic from each (an SM's own
+// atomics drop the line from its L1, so a set bit is seen by the next load; a
+// stale line only costs another atomic). A word without a bit may be its
+// leaf's first of the window, which marks the leaf touched in its block.
+__device__ __forceinline__ void march_apply(const MarchWarp& q, uint32_t at, uint32_t n, int bx, int by, int bz, int map,
+                                            const MapView& m, const ChannelView& c, int lane)
+{
+  const bool have     = static_cast<uint32_t>(lane) < n;
+  const uint32_t pos  = have ? q.pos[at + lane] : 0u;
+  const int src       = static_cast<int>(pos >> (3 * march::kPosBits));
+  constexpr int kLeaf = static_cast<int>(march::kPosMask >> 3);
+  const int lx = __shfl_sync(0xffffffffu, bx, src) + (static_cast<int>(pos >> 3) & kLeaf);
+  const int ly = __shfl_sync(0xffffffffu, by, src) + (static_cast<int>(pos >> (march::kPosBits + 3)) & kLeaf);
+  const int lz = __shfl_sync(0xffffffffu, bz, src) + (static_cast<int>(pos >> (2 * march::kPosBits + 3)) & kLeaf);
+  const int mp = __shfl_sync(0xffffffffu, map, src);
+  if (!have) return;
+  const unsigned long long bits = q.bits[at + lane];
   const unsigned long long bkey = pack_leaf_key(mp, lx >> 3, ly >> 3, lz >> 3);
-  const uint32_t h0             = static_cast<uint32_t>(mix64(bkey)) & m.bhmask;
-  const unsigned long long k0   = ld_ca_u64(m.bkeys + h0);
-  const int s0                  = ld_ca_s32(m.bslots + h0);
-  const int b = (k0 == bkey && s0 >= 0) ? s0 : find_or_insert_block(m, mp, lx >> 3, ly >> 3, lz >> 3);
-  if (b < 0) return kSlotFailed;
+  const uint32_t h              = block_home(bkey, m.bhmask);
+  const ulonglong2 k2           = ld_ca_u64x2(m.bkeys + h);
+  const int2 s2                 = ld_ca_s32x2(m.bslots + h);
+  int b                         = k2.x == bkey ? s2.x : k2.y == bkey ? s2.y : -1;
+  if (b < 0) b = find_or_insert_block(m, mp, lx >> 3, ly >> 3, lz >> 3);
+  if (b < 0) return;
   const int cell = ((lx & 7) << 6) | ((ly & 7) << 3) | (lz & 7);
-  const int c0   = ld_ca_s32(m.bleaf + static_cast<size_t>(b) * 512 + cell);
-  const uint32_t ep = ld_ca_u32(c.bepoch + b);
-  if (ep != c.cur_epoch) touch_block(c, b);
-  const int slot = c0 >= 0 ? c0 : find_or_insert_leaf(m, b, cell, mp, lx, ly, lz);
-  if (slot >= 0) atomicOr(c.btouched + static_cast<size_t>(b) * 8 + (cell >> 6), 1ull << (cell & 63));
-  return slot;
-}
-
-// Apply chunks of the segments, for k_apply_runs' tickets: chunk_prefix[w] =
-// chunks of the segments before w, chunk_prefix[warps] = all of them; resets
-// the ticket counter. One block of 1024 threads, run after the DDA pass.
-__global__ void __launch_bounds__(1024) k_apply_prefix(RunBuffer rb)
-{
-  uint32_t carry = 0;
-  for (uint32_t base = 0; base < rb.warps; base += 1024u)
+  int slot       = ld_ca_s32(m.bleaf + static_cast<size_t>(b) * 512 + cell);
+  if (slot < 0) slot = find_or_insert_leaf(m, b, cell, mp, lx, ly, lz);
+  if (slot < 0) return;
+  unsigned long long* const u  = c.upd + static_cast<size_t>(slot) * 16 + march::plane_of(pos);
+  const unsigned long long old = ld_ca_u64(u);
+  if (bits & ~old) atomicOr(u, bits);
+  if (old == 0ull)
   {
-    const uint32_t w = base + threadIdx.x;
-    const uint32_t n = w < rb.warps ? (rb.count[w] + rb.apply_chunk - 1u) / rb.apply_chunk : 0u;
-    uint32_t total   = 0;
-    const uint32_t e = block_scan_exclusive(n, &total);
-    if (w < rb.warps) rb.chunk_prefix[w] = carry + e;
-    carry += total;
-  }
-  if (threadIdx.x == 0)
-  {
-    rb.chunk_prefix[rb.warps] = carry;
-    *rb.ticket                = 0u;
+    touch_block(c, b);
+    atomicOr(c.btouched + static_cast<size_t>(b) * 8 + (cell >> 6), 1ull << (cell & 63));
   }
 }
 
-// Segment and runs [start, end) of apply chunk `item` (< all chunks): the
-// segment is the last one whose first chunk is at or before `item`.
-__device__ __forceinline__ void apply_item_range(const RunBuffer& rb, uint32_t item, uint32_t& sg, uint32_t& start,
-                                                 uint32_t& end)
+// How a chunk is walked: chunk 0 with FP64 additions, the others with integer
+// ones, with or without a look at the chunk's end at every step.
+enum MarchMode : int
 {
-  uint32_t lo = 0, hi = rb.warps;  // chunk_prefix[lo] <= item < chunk_prefix[hi]
-  while (hi - lo > 1u)
-  {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (rb.chunk_prefix[mid] <= item)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  sg    = lo;
-  start = (item - rb.chunk_prefix[lo]) * rb.apply_chunk;
-  end   = min(start + rb.apply_chunk, rb.count[lo]);
-}
+  kMarchFp64,
+  kMarchChecked,
+  kMarchFree,
+};
 
-// Stages runs [start, end) of segment `sg` (thread 0 only). Segments start on
-// 16-run boundaries and chunks are multiples of 256 runs, so every copy starts
-// 16-byte aligned; lengths are rounded up to 16 bytes, which stays inside the
-// segment.
-template <int kTable>
-__device__ __forceinline__ void apply_stage(const RunBuffer& rb, uint32_t sg, uint32_t start, uint32_t end,
-                                            ApplySmem<kTable>& t, unsigned long long* s_key,
-                                            unsigned long long* s_bits, unsigned char* s_slab)
+// kMarchSteps steps: marks every voxel in the open run (lo, hi) before it is
+// left, and appends the runs that end to the list. Returns whether the last
+// step moved.
+template <int kMode>
+__device__ __forceinline__ bool march_steps(MarchWarp& q, march::Walk& w, uint32_t& lo, uint32_t& hi, uint32_t& n,
+                                            uint32_t lt)
 {
-  const size_t base  = static_cast<size_t>(sg) * rb.seg + start;
-  const uint32_t n   = end - start;
-  const uint32_t b8  = (n * 8u + 15u) & ~15u;
-  const uint32_t b1  = (n + 15u) & ~15u;
-  mbar_arrive_expect_tx(&t.bar, 2u * b8 + b1);
-  bulk_copy_g2s(s_key, rb.key + base, b8, &t.bar);
-  bulk_copy_g2s(s_bits, rb.bits + base, b8, &t.bar);
-  bulk_copy_g2s(s_slab, rb.slab + base, b1, &t.bar);
-}
-
-// Takes the block's next chunk ticket (thread 0 only) and stages its runs.
-template <int kTable>
-__device__ __forceinline__ void apply_take(const RunBuffer& rb, uint32_t items, ApplySmem<kTable>& t,
-                                           unsigned long long* s_key, unsigned long long* s_bits,
-                                           unsigned char* s_slab)
-{
-  const uint32_t item = atomicAdd(rb.ticket, 1u);
-  t.next              = min(item, items);
-  if (item >= items) return;
-  uint32_t sg, start, end;
-  apply_item_range(rb, item, sg, start, end);
-  t.next_sg    = sg;
-  t.next_start = start;
-  t.next_end   = end;
-  apply_stage(rb, sg, start, end, t, s_key, s_bits, s_slab);
-}
-
-template <int kApplyThreads, int kApplyTable>
-__global__ void __launch_bounds__(kApplyThreads) k_apply_runs(RunBuffer rb, MapView m, ChannelView c)
-{
-  c.cur_epoch = *c.epoch;
-  __shared__ ApplySmem<kApplyTable> t;
-  extern __shared__ __align__(16) unsigned char stage[];
-  unsigned long long* s_key  = reinterpret_cast<unsigned long long*>(stage);
-  unsigned long long* s_bits = s_key + rb.apply_chunk;
-  unsigned char* s_slab      = reinterpret_cast<unsigned char*>(s_bits + rb.apply_chunk);
-  const uint32_t items       = rb.chunk_prefix[rb.warps];  // chunks of the pass
-  // The error word can be set by other blocks while this one starts: read it
-  // once for the whole block, so that either every thread returns or none
-  // does (the barriers below need all of them).
-  if (threadIdx.x == 0)
-  {
-    t.failed = ld_relaxed_u32(&m.st->error);
-    t.count  = 0u;
-    t.next   = items;
-    if (t.failed == 0u)
-    {
-      mbar_init(&t.bar, 1);
-      fence_proxy_async_smem();
-      apply_take(rb, items, t, s_key, s_bits, s_slab);
-    }
-  }
-  for (int e = threadIdx.x; e < kApplyTable; e += kApplyThreads)
-  {
-    t.key[e] = kEmptyKey;
+  uint32_t before = 0u;
 #pragma unroll
-    for (int w = 0; w < 16; ++w) t.words[e][w] = 0u;
-  }
-  __syncthreads();
-  if (t.failed != 0u) return;
-  const int lane  = static_cast<int>(threadIdx.x & 31);
-  uint32_t parity = 0;
-  for (uint32_t item = t.next; item < items;)
+  for (int s = 0; s < kMarchSteps; ++s)
   {
-    const uint32_t start = t.next_start, end = t.next_end;
-    const bool staged = mbar_wait_bounded(&t.bar, parity);
-    parity ^= 1u;
-    if (__syncthreads_or(!staged))
+    march_mark(w.pos, lo, hi);
+    before = w.pos;
+    if (kMode == kMarchFp64)
+      march::step<true>(w);
+    else if (kMode == kMarchChecked)
+      march::step<false>(w);
+    else
+      march::step_free(w);
+    // The run ends when the voxel leaves its plane or leaf.
+    const bool ends   = ((w.pos ^ before) & march::kCrossing) != 0u;
+    const unsigned em = __ballot_sync(0xffffffffu, ends);
+    if (ends)
     {
-      // The copy did not complete in time: report, and wait (bounded) once
-      // more so no copy is left writing into this block's shared memory.
-      if (threadIdx.x == 0)
-      {
-        atomicOr(&m.st->error, kErrSpin);
-        mbar_wait_bounded(&t.bar, parity ^ 1u);
-      }
-      __syncthreads();
-      return;
+      const uint32_t p = n + static_cast<uint32_t>(__popc(em & lt));
+      q.bits[p]        = (static_cast<unsigned long long>(hi) << 32) | lo;
+      q.pos[p]         = before;
+      lo = hi = 0u;
     }
-    // Whole warps walk the chunk (tail lanes idle) so the match below sees full warps.
-    for (uint32_t i0 = start + (threadIdx.x & ~31u); i0 < end; i0 += kApplyThreads)
+    n += static_cast<uint32_t>(__popc(em));
+  }
+  return w.pos != before;
+}
+
+// Walks one chunk on every `live` lane and applies its runs. The chunk's first
+// voxel is marked too: it is the sensor voxel, or the last of the chunk before.
+// Returns the number of runs.
+__device__ __forceinline__ uint32_t march_chunk(MarchWarp& q, int mode, march::Walk& w, march::Cuts& cuts, uint32_t end,
+                                                bool live, int bx, int by, int bz, int map, const MapView& m,
+                                                const ChannelView& c, int lane, uint32_t lt)
+{
+  const uint32_t first = w.pos;
+  uint32_t n = 0, runs = 0;  // records in the list; all of the chunk's
+  uint32_t lo = 0, hi = 0;   // the open run
+  unsigned walking = 0xffffffffu;
+  for (uint32_t round = 0;; ++round)
+  {
+    bool go;
+    if (mode == kMarchFree)
     {
-      const uint32_t i              = i0 + static_cast<uint32_t>(lane);
-      const bool have               = i < end;
-      const uint32_t k              = i - start;
-      const unsigned long long key  = have ? s_key[k] : kEmptyKey;
-      const unsigned long long bits = have ? s_bits[k] : 0ull;
-      const int w                   = have ? s_slab[k] : 0;
-      const unsigned peers          = __match_any_sync(0xffffffffu, key);
-      const int leader              = __ffs(peers) - 1;
-      int h                         = -1;
-      if (have && lane == leader)
+      march_steps<kMarchFree>(q, w, lo, hi, n, lt);
+      go                   = march::has_step(w);
+      const unsigned going = __ballot_sync(0xffffffffu, go);
+      if (going != walking)
       {
-        uint32_t p = apply_hash<kApplyTable>(key);
-        for (int probe = 0; probe < 16; ++probe)
+        // (a lane that has passed its end stays where it is)
+        walking = going;
+        if (!go)
         {
-          unsigned long long kk = t.key[p];
-          if (kk == kEmptyKey)
-          {
-            const unsigned long long prev = atomicCAS(&t.key[p], kEmptyKey, key);
-            if (prev == kEmptyKey)
-            {
-              t.list[atomicAdd(&t.count, 1u)] = static_cast<unsigned short>(p);
-              kk                               = key;
-            }
-            else
-            {
-              kk = prev;
-            }
-          }
-          if (kk == key)
-          {
-            h = static_cast<int>(p);
-            break;
-          }
-          p = (p + 1) & (kApplyTable - 1);
+          w.dx = w.dy = w.dz = 0ull;
+          w.px = w.py = w.pz = 0;
         }
       }
-      h = __shfl_sync(0xffffffffu, h, leader);
-      if (!have) continue;
-      if (h >= 0)
+    }
+    else if (mode == kMarchChecked)
+    {
+      go = march_steps<kMarchChecked>(q, w, lo, hi, n, lt);
+      if (!go && w.end != end)
       {
-        const unsigned int lo = static_cast<unsigned int>(bits), hi = static_cast<unsigned int>(bits >> 32);
-        if (lo) atomicOr(&t.words[h][2 * w], lo);
-        if (hi) atomicOr(&t.words[h][2 * w + 1], hi);
-      }
-      else
-      {
-        // Table crowded: apply this run directly.
-        const int slot = apply_resolve(m, c, key);
-        if (slot >= 0) atomicOr(c.upd + static_cast<size_t>(slot) * 16 + w, bits);
+        march::resume(w, cuts, first, end);
+        go = true;
       }
     }
-    __syncthreads();
-    // The staging buffer is free: start copying the block's next chunk. The
-    // last thread takes the ticket: it has the fewest (mostly no) leaves to
-    // resolve below, so the ticket's round trips stay off the slowest path.
-    if (threadIdx.x == kApplyThreads - 1)
+    else
     {
-      fence_proxy_async_smem();
-      apply_take(rb, items, t, s_key, s_bits, s_slab);
+      go = march_steps<kMarchFp64>(q, w, lo, hi, n, lt);
     }
-    const uint32_t n_used = t.count;
-    for (uint32_t k = threadIdx.x; k < n_used; k += kApplyThreads)
+    bool more = __any_sync(0xffffffffu, go);
+    if (more && round >= kMarchMaxRounds)
     {
-      const int e = t.list[k];
-      t.slot[e]   = apply_resolve(m, c, t.key[e]);
+      // More than L1 + 1 visits: cannot happen for integer rays.
+      if (lane == 0) atomicOr(&m.st->error, kErrStepBound);
+      more = false;
     }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < n_used * 8u; k += kApplyThreads)
+    if (!more)
     {
-      const int e    = t.list[k >> 3];
-      const int w    = static_cast<int>(k & 7u);
-      const int slot = t.slot[e];
-      const unsigned long long b =
-        (static_cast<unsigned long long>(t.words[e][2 * w + 1]) << 32) | t.words[e][2 * w];
-      if (slot >= 0 && b) atomicOr(c.upd + static_cast<size_t>(slot) * 16 + w, b);
-      t.words[e][2 * w]     = 0u;
-      t.words[e][2 * w + 1] = 0u;
-      if (w == 0) t.key[e] = kEmptyKey;
+      march_mark(w.pos, lo, hi);
+      const unsigned em = __ballot_sync(0xffffffffu, live);
+      if (live)
+      {
+        const uint32_t p = n + static_cast<uint32_t>(__popc(em & lt));
+        q.bits[p]        = (static_cast<unsigned long long>(hi) << 32) | lo;
+        q.pos[p]         = w.pos;
+      }
+      n += static_cast<uint32_t>(__popc(em));
     }
-    __syncthreads();
-    item = t.next;
-    if (threadIdx.x == 0) t.count = 0u;
-    __syncthreads();
+    __syncwarp();
+    while (n >= 32u || (!more && n > 0u))
+    {
+      const uint32_t take = min(n, 32u);
+      n -= take;
+      runs += take;
+      march_apply(q, n, take, bx, by, bz, map, m, c, lane);
+    }
+    if (!more) break;
   }
+  return runs;
+}
+
+// `cursor`: the sort's bucket cursors after k_scatter (each holds its
+// bucket's end). `max_take`: items a warp takes at a time, at most. `one`: 1, as
+// a value the compiler does not know (march::step).
+__global__ void __launch_bounds__(kMarchWarps * 32, kMarchBlocks)
+  k_march(const int4* __restrict__ rays, const int* __restrict__ order, const uint32_t* __restrict__ cursor,
+          ScanTable t, MapView m, ChannelView c, AxisTable at, uint32_t max_take, uint32_t one)
+{
+  __shared__ MarchWarp warps[kMarchWarps];
+  __shared__ uint32_t s_end[kLenClasses];             // rays of the classes up to each
+  __shared__ unsigned long long s_items[kLenClasses];  // items of the classes up to each
+  __shared__ int s_log2[kLenClasses];                  // log2 of a group's items, by class
+  __shared__ uint32_t s_error;
+  const int lane    = static_cast<int>(threadIdx.x & 31);
+  const uint32_t lt = lanemask_lt();
+  MarchWarp& q      = warps[threadIdx.x >> 5];
+  c.cur_epoch       = *c.epoch;
+  if (threadIdx.x < kLenClasses)
+    s_end[threadIdx.x] = cursor[(threadIdx.x + 1u) * static_cast<uint32_t>(t.n) * kDirCells - 1u];
+  __syncthreads();
+  if (threadIdx.x == 0)
+  {
+    unsigned long long items = 0ull;
+    uint32_t from            = 0u;
+    for (int k = 0; k < kLenClasses; ++k)
+    {
+      const int l = class_log2(k, m.st->max_l1, t.clog);
+      items += static_cast<unsigned long long>((s_end[k] - from + 31u) >> 5) << l;
+      from       = s_end[k];
+      s_items[k] = items;
+      s_log2[k]  = l;
+    }
+    // A scan with a voxel index out of range is not cast at all (the prep
+    // stage flagged it). Other errors of this call do not stop the walk.
+    s_error = ld_relaxed_u32(&m.st->error) & kErrCoordRange;
+  }
+  __syncthreads();
+  if (s_error != 0u) return;
+  const unsigned long long total = s_items[kLenClasses - 1];
+  // Several items at a time (their chunks follow one another and share
+  // leaves), but no fewer than four turns for every warp.
+  const unsigned long long share = total / (static_cast<unsigned long long>(gridDim.x) * kMarchWarps * 4ull);
+  const uint32_t take = share < 1ull ? 1u : share > max_take ? max_take : static_cast<uint32_t>(share);
+
+  unsigned long long it = 0ull, it_end = 0ull, runs = 0ull;
+  uint32_t loaded = 0xffffffffu;  // first ray of the group held in `r`
+  MarchRay r{0, 0, 0, 0, 0, 0, -1, 0};
+  for (;;)
+  {
+    if (it == it_end)
+    {
+      // (a full block hash can count no demand: the walk ends, the host grows
+      // it and marks again)
+      if (lane == 0)
+        it = (ld_relaxed_u32(&m.st->error) & kErrHashFull)
+               ? total
+               : atomicAdd(&m.st->item_cursor, static_cast<unsigned long long>(take));
+      it = __shfl_sync(0xffffffffu, it, 0);
+      if (it >= total) break;
+      it_end = min(it + take, total);
+    }
+    int k = 0;
+    while (it >= s_items[k]) ++k;
+    const unsigned long long local = it - (k ? s_items[k - 1] : 0ull);
+    const int l                    = s_log2[k];
+    const uint32_t i               = static_cast<uint32_t>(local) & ((1u << l) - 1u);
+    const uint32_t ray0            = (k ? s_end[k - 1] : 0u) + (static_cast<uint32_t>(local >> l) << 5);
+    ++it;
+    if (ray0 != loaded)
+    {
+      loaded             = ray0;
+      const uint32_t idx = ray0 + static_cast<uint32_t>(lane);
+      r.p                = -1;
+      if (idx < s_end[k])
+      {
+        const int ri = order[idx];
+        r            = march_ray(rays[ri], scan_geom(t, scan_of_ray(t, static_cast<uint32_t>(ri))), t.clog);
+      }
+    }
+    const bool live = r.p >= 0 && (i >> r.p) == 0u;
+    if (!__any_sync(0xffffffffu, live)) continue;
+    march::Walk w{march::kNever, march::kNever, march::kNever, 0ull, 0ull, 0ull, 0u, 0u, 0, 0, 0, one};
+    march::Cuts cuts{{0, 0, 0}};
+    int bx = 0, by = 0, bz = 0;
+    uint32_t end = 0u;
+    if (live) end = march_begin(at, r, i, w, cuts, bx, by, bz);
+    w.pos |= static_cast<uint32_t>(lane) << (3 * march::kPosBits);
+    const bool cut = live && w.end != end;
+    const int mode = i == 0u                                                            ? kMarchFp64
+                     : march::chunk_is_free(i) && !__any_sync(0xffffffffu, cut) ? kMarchFree
+                                                                                        : kMarchChecked;
+    runs += march_chunk(q, mode, w, cuts, end, live, bx, by, bz, r.map, m, c, lane, lt);
+  }
+  if (lane == 0 && runs) atomicAdd(&m.st->runs, runs);
 }
 
 // Endpoint hits (setValueOn(end, true), VDBMapping.hpp:533-536): one thread
@@ -1426,7 +1290,7 @@ __global__ void k_window_init(ChannelView c)
 // the window is left to the host's continuation of the step.
 // A step whose rays were prepared ahead on another stream into their own
 // status block: its counters and the quantiser's error bit join the call's
-// status before the marking reads them (k_dda_mark reads n_valid).
+// status before the marking reads them.
 __global__ void k_absorb_prep(DevStatus* st, const DevStatus* __restrict__ prep)
 {
   st->rays += prep->rays;
@@ -1434,6 +1298,7 @@ __global__ void k_absorb_prep(DevStatus* st, const DevStatus* __restrict__ prep)
   st->hits += prep->hits;
   st->nonfinite += prep->nonfinite;
   st->n_valid = prep->n_valid;
+  st->max_l1  = prep->max_l1;
   st->error |= prep->error;
 }
 
@@ -1454,7 +1319,7 @@ __global__ void k_rehash(MapView m, uint32_t n)
   if (s >= n) return;
   const int4 o                 = m.borigin[s];
   const unsigned long long key = pack_leaf_key(o.w, o.x, o.y, o.z);
-  uint32_t h                   = static_cast<uint32_t>(mix64(key)) & m.bhmask;
+  uint32_t h                   = block_home(key, m.bhmask);
   for (uint32_t probe = 0; probe <= m.bhmask; ++probe)
   {
     if (atomicCAS(m.bkeys + h, kEmptyKey, key) == kEmptyKey)
@@ -1491,7 +1356,7 @@ __global__ void k_release_leaves(MapView m, uint32_t from, uint32_t to, uint32_t
   const int4 o = m.origin[slot];
   const int lx = o.x >> 3, ly = o.y >> 3, lz = o.z >> 3;
   const unsigned long long key = pack_leaf_key(o.w, lx >> 3, ly >> 3, lz >> 3);
-  uint32_t h = static_cast<uint32_t>(mix64(key)) & m.bhmask;
+  uint32_t h = block_home(key, m.bhmask);
   for (uint32_t probe = 0; probe <= m.bhmask; ++probe)
   {
     const unsigned long long k = m.bkeys[h];
@@ -1531,7 +1396,7 @@ __global__ void k_reset_failed_leaves(int* __restrict__ bleaf, size_t cells)
 __device__ __forceinline__ int find_leaf(const MapView& m, int map, int lx, int ly, int lz)
 {
   const unsigned long long bkey = pack_leaf_key(map, lx >> 3, ly >> 3, lz >> 3);
-  uint32_t h                    = static_cast<uint32_t>(mix64(bkey)) & m.bhmask;
+  uint32_t h                    = block_home(bkey, m.bhmask);
   for (uint32_t probe = 0; probe < kMaxProbes; ++probe)
   {
     const unsigned long long k = m.bkeys[h];
@@ -1843,7 +1708,7 @@ __device__ __forceinline__ bool voxel_in_map_range(const int v[3])
 __device__ __forceinline__ int find_block(const MapView& m, int map, int bx, int by, int bz)
 {
   const unsigned long long bkey = pack_leaf_key(map, bx, by, bz);
-  uint32_t h                    = static_cast<uint32_t>(mix64(bkey)) & m.bhmask;
+  uint32_t h                    = block_home(bkey, m.bhmask);
   for (uint32_t probe = 0; probe < kMaxProbes; ++probe)
   {
     const unsigned long long k = m.bkeys[h];
@@ -2605,40 +2470,55 @@ __device__ __forceinline__ unsigned long long digest_key(int x, int y, int z)
          static_cast<unsigned long long>(static_cast<uint32_t>(z)) * 0x165667B19E3779F9ull;
 }
 
-// One thread per ray record (k_prep's output, point order): the DDA of
-// k_dda_mark (dda_setup / dda_advance) walked alone, hashed as above.
+// One thread per ray record (k_prep's output, point order): the walk of
+// k_march (march_begin, march::step), chunk after chunk, hashed as above.
 __global__ void __launch_bounds__(256) k_ray_digest(const int4* __restrict__ rays, int64_t n, ScanTable t,
-                                                    unsigned long long* __restrict__ out, DevStatus* st)
+                                                    AxisTable at, unsigned long long* __restrict__ out, DevStatus* st)
 {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int4 r            = rays[i];
-  const uint32_t meta     = static_cast<uint32_t>(r.w);
+  const int4 rec          = rays[i];
+  const uint32_t meta     = static_cast<uint32_t>(rec.w);
   const bool valid        = (meta & kMetaValid) != 0u;
   const bool clipped      = (meta & kMetaClipped) != 0u;
-  const uint32_t l1       = meta & kMetaL1Mask;
   unsigned long long h    = 0x243F6A8885A308D3ull;
   unsigned long long cnt  = 0;
-  if (valid && l1 > 0)
+  const MarchRay r = march_ray(valid ? rec : make_int4(0, 0, 0, 0), scan_geom(t, scan_of_point(t, static_cast<uint32_t>(i))),
+                               t.clog);
+  for (uint32_t k = 0; valid && r.p >= 0 && (k >> r.p) == 0u; ++k)
   {
-    const ScanGeom& g = scan_geom(t, scan_of_point(t, static_cast<uint32_t>(i)));
-    const int o[3]    = {g.ovx, g.ovy, g.ovz};
-    const int e[3]    = {r.x, r.y, r.z};
-    DdaRay d;
-    dda_setup(o, e, d);
-    for (uint32_t budget = l1 + 1;; --budget)
-    {
-      h = mix64(h ^ digest_key(d.vx, d.vy, d.vz));
+    march::Walk w;
+    w.one = 1u;
+    march::Cuts cuts;
+    int bx, by, bz;
+    const uint32_t end   = march_begin(at, r, k, w, cuts, bx, by, bz);
+    const uint32_t first = w.pos;
+    auto visit = [&]() {
+      h = mix64(h ^ digest_key(bx * 8 + static_cast<int>(march::pos_field(w.pos, 0)),
+                               by * 8 + static_cast<int>(march::pos_field(w.pos, 1)),
+                               bz * 8 + static_cast<int>(march::pos_field(w.pos, 2))));
       ++cnt;
-      if (dda_advance(d) > kDdaOne) break;
-      if (budget == 1u)
+    };
+    if (k == 0u) visit();
+    uint32_t steps = 0;
+    for (;;)
+    {
+      if (march::has_step(w))
       {
+        if (k == 0u)
+          march::step<true>(w);
+        else
+          march::step<false>(w);
+        visit();
+        if (++steps <= march::kMaxSteps) continue;
         atomicOr(&st->error, kErrStepBound);
         break;
       }
+      if (k == 0u || w.end == end) break;
+      march::resume(w, cuts, first, end);
     }
   }
-  if (valid) h = mix64(h ^ digest_key(r.x, r.y, r.z) ^ 0x5851F42D4C957F2Dull);
+  if (valid) h = mix64(h ^ digest_key(rec.x, rec.y, rec.z) ^ 0x5851F42D4C957F2Dull);
   out[2 * i]     = cnt | (clipped ? 1ull << 40 : 0ull) | (valid ? 1ull << 41 : 0ull);
   out[2 * i + 1] = valid ? h : 0ull;
 }

@@ -304,7 +304,7 @@ int queue_prep(vdbg_map* m, PrepSet& p, const std::vector<ServerRequest>& step, 
     t.first    = p.first;
     t.ray_scan = p.ray_scan;
   }
-  set_edges(m, t);
+  t.clog  = chunk_log2_for(p.total);
   p.table = t;
   if (p.status != VDBG_OK || p.total == 0) return VDBG_OK;
   for (const ServerRequest& r : step)
@@ -337,22 +337,12 @@ int run_prepped(vdbg_map* m, PrepSet& p, vdbg_scan_stats* stats)
   VDBG_TRY(begin_call(m, s));
   const uint32_t leaves_before = m->n_leaves;
   if (p.total == 0) return VDBG_OK;
-  uint32_t seg = std::max<uint32_t>(m->run_seg, kMinRunSeg);
-  if (m->passes_last > 1)
-  {
-    const uint64_t want  = static_cast<uint64_t>(m->run_seg) * m->passes_last * 2;
-    const uint64_t limit = m->run_budget / (17ull * m->dda_warps);
-    seg                  = static_cast<uint32_t>(std::min<uint64_t>(want, limit));
-  }
-  VDBG_TRY(ensure_runs(m, seg));
-  const RunBuffer rb =
-    run_buffer(m, m->run_key, m->run_bits, m->run_slab, m->run_count, m->run_prefix, m->run_seg, m->dda_warps);
   VDBG_CUDA(cudaStreamWaitEvent(s, p.ready, 0));
   k_absorb_prep<<<1, 1, 0, s>>>(m->d_status, p.st);
   VDBG_CUDA(cudaGetLastError());
   c.pending  = true;
   bool swept = false;
-  int d = run_dda_passes(m, c, p.rays, p.order, p.total, p.table, rb, m->lstate, m->wstate, true, s, true, &swept);
+  int d = run_marking(m, c, p.rays, p.order, p.cursor, p.total, p.table, true, s, true, &swept);
   int call_status = VDBG_OK;
   if (d == VDBG_OK && swept)
   {

@@ -77,9 +77,8 @@ struct vdbg_map
 
   cudaStream_t stream   = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  cudaEvent_t ev_prep = nullptr, ev_dda = nullptr;  // after k_scatter, after k_dda_mark
-  cudaEvent_t ev_a0 = nullptr, ev_a1 = nullptr;     // around each k_apply_runs launch
-  cudaStream_t side     = nullptr;  // k_mark_hits beside the first DDA pass
+  cudaEvent_t ev_prep = nullptr, ev_dda = nullptr;  // after k_scatter, after k_march
+  cudaStream_t side     = nullptr;  // k_mark_hits beside k_march
   cudaEvent_t ev_fork = nullptr, ev_hits = nullptr;
   bool timed_prep       = false;
   vdbg_timings timings{};
@@ -148,24 +147,13 @@ struct vdbg_map
   uint32_t* d_hist      = nullptr;  // [buckets]
   uint32_t* d_cursor    = nullptr;
   uint32_t buckets      = 0;
-  // DDA run buffer (one segment per DDA warp) and resumable lane/warp state.
-  uint32_t dda_warps    = 0;
-  uint32_t run_seg      = 0;
-  unsigned long long* run_key  = nullptr;
-  unsigned long long* run_bits = nullptr;
-  unsigned char* run_slab      = nullptr;
-  uint32_t* run_count   = nullptr;
-  uint32_t* run_prefix  = nullptr;  // [dda_warps + 2]: apply chunk prefix, then the ticket
-  LaneState* lstate     = nullptr;
-  WarpState* wstate     = nullptr;
-  uint32_t passes_last  = 0;
+  // Crossing-time table of k_march (march.cuh), built when the map is created.
+  char* axis_mem        = nullptr;  // [kAxisTableBytes]
+  AxisTable axis{};
 
   int64_t bytes         = 0;
-  uint64_t run_budget   = 2ull << 30;  // run buffer bytes the map may grow to
   int num_sms           = 152;
   vdbg_tuning tuning{32, 2048, {2048, 1024, 512}, 0.5f, 16, 0};
-  uint32_t apply_grid_chunk = 0;   // apply_chunk the cached grid size is for
-  unsigned apply_grid_blocks = 0;
   // Change set of the last integration (vdbg_track_changes).
   bool track_changes               = false;
   uint32_t chg_cap                 = 0;  // leaf slots the arrays cover (cap_ready while tracking)
@@ -175,7 +163,7 @@ struct vdbg_map
   uint32_t* chg_epoch              = nullptr;
   uint32_t* chg_count              = nullptr;
   uint32_t chg_cur                 = 0;
-  // Captured batched step: prep, endpoint hits, one DDA pass and its apply,
+  // Captured batched step: prep, endpoint hits beside the walk,
   // compact, sweep, window end. Replayed while nothing it names has moved.
   uint64_t layout                  = 0;  // bumped by every device (re)allocation and tuning change
   bool use_graph                   = true;
@@ -233,8 +221,6 @@ constexpr uint32_t kDefaultCapacity = 1u << 16;
 constexpr uint32_t kMinBlocks       = 1u << 10;
 constexpr int kSweepBlocks          = 152 * 8;
 constexpr int kSweepThreads         = 256;
-constexpr uint32_t kMinRunSeg       = 2048;   // runs per DDA warp segment, at least
-constexpr uint64_t kMaxRunBytes     = 8ull << 30;  // run buffer growth budget, at most 1/32 of the device
 
 uint32_t next_pow2(uint64_t v)
 {
@@ -774,10 +760,14 @@ bool scan_geom_for(const vdbg_map* m, int map, const double origin[3], double ra
   return true;
 }
 
-void set_edges(const vdbg_map* m, ScanTable& t)
-{
-  for (int k = 0; k < 3; ++k) t.edge[k] = static_cast<uint32_t>(m->tuning.length_edges[k]);
-}
+// log2 of the most steps of k_march's chunks, by the points of the call. A
+// chunk costs about 400 instructions to begin, a step of a warp about 55, so
+// long chunks are cheaper; a small scan needs short ones to keep the device
+// busy. Marking times on one GB300 with chunks of 32 / 64 / 128 steps: 2,048
+// points of a room (99 steps a ray) 27 / 35 / 55 us, 16,381 random rays of
+// 2,490 steps 774 / 618 / 733 us, 65,536 points (197) 101 / 97 / 115 us, 262,144
+// (478) 633 / 584 / 552 us, 307,200 of a depth camera (346) 520 / 475 / 453 us.
+int chunk_log2_for(int64_t n) { return n >= 100000 ? 7 : n >= 8192 ? 6 : 5; }
 
 ScanTable single_table(const ScanGeom& g)
 {
@@ -787,6 +777,7 @@ ScanTable single_table(const ScanGeom& g)
   t.first    = nullptr;
   t.ray_scan = nullptr;
   t.n        = 1;
+  t.clog     = march::kMaxChunkLog2;
   return t;
 }
 
@@ -832,65 +823,6 @@ int launch_prep(vdbg_map* m, Channel& c, const float* xyz, int64_t n, int64_t st
   return VDBG_OK;
 }
 
-// Allocates (or grows) the DDA run buffer: dda_warps segments of `seg` runs,
-// plus the per-lane and per-warp resume state.
-// Persistent grid of k_apply_runs: as many blocks as fit on the device with
-// the staging buffer of `chunk` runs.
-unsigned apply_grid(vdbg_map* m, uint32_t chunk)
-{
-  if (m->apply_grid_chunk != chunk)
-  {
-    int per_sm = 0;
-    const bool small = chunk <= kApplySmallChunk;
-    const cudaError_t e =
-      small ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_apply_runs<128, 256>, 128, apply_stage_bytes(chunk))
-            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_apply_runs<256, 512>, 256, apply_stage_bytes(chunk));
-    if (e != cudaSuccess ||
-        per_sm < 1)
-      per_sm = 1;
-    m->apply_grid_chunk  = chunk;
-    m->apply_grid_blocks = static_cast<unsigned>(m->num_sms * per_sm);
-  }
-  return m->apply_grid_blocks;
-}
-
-int ensure_runs(vdbg_map* m, uint32_t seg)
-{
-  seg = (seg + 15u) & ~15u;  // segments start on 16-run boundaries (bulk copies)
-  if (m->run_key && seg <= m->run_seg) return VDBG_OK;
-  const size_t W = m->dda_warps;
-  dev_free(m, m->run_key, W * m->run_seg);
-  dev_free(m, m->run_bits, W * m->run_seg);
-  dev_free(m, m->run_slab, W * m->run_seg);
-  m->run_seg = 0;
-  VDBG_TRY(dev_alloc(m, &m->run_key, W * seg));
-  VDBG_TRY(dev_alloc(m, &m->run_bits, W * seg));
-  VDBG_TRY(dev_alloc(m, &m->run_slab, W * seg));
-  if (!m->run_count) VDBG_TRY(dev_alloc(m, &m->run_count, W));
-  if (!m->run_prefix) VDBG_TRY(dev_alloc(m, &m->run_prefix, W + 2));
-  if (!m->lstate) VDBG_TRY(dev_alloc(m, &m->lstate, W * 32));
-  if (!m->wstate) VDBG_TRY(dev_alloc(m, &m->wstate, W));
-  m->run_seg = seg;
-  return VDBG_OK;
-}
-
-RunBuffer run_buffer(const vdbg_map* m, unsigned long long* key, unsigned long long* bits, unsigned char* slab,
-                     uint32_t* count, uint32_t* prefix, uint32_t seg, uint32_t warps)
-{
-  RunBuffer rb;
-  rb.chunk_prefix = prefix;
-  rb.ticket       = prefix + warps + 1;
-  rb.take        = static_cast<uint32_t>(m->tuning.rays_per_take);
-  rb.apply_chunk = static_cast<uint32_t>(m->tuning.apply_chunk_runs);
-  rb.key   = key;
-  rb.bits  = bits;
-  rb.slab  = slab;
-  rb.count = count;
-  rb.seg   = seg;
-  rb.warps = warps;
-  return rb;
-}
-
 void clear_error_keep_counters(vdbg_map* m)
 {
   m->h_status->error    = 0;
@@ -903,32 +835,9 @@ int grow_for(vdbg_map* m, uint64_t requested);
 int grow_blocks_for(vdbg_map* m, uint64_t requested);
 int rebuild_hash(vdbg_map* m, uint32_t hsize, uint32_t n);
 
-// Adds the last k_apply_runs launch's duration (its events are complete after
-// a status fetch).
-void add_apply_time(vdbg_map* m)
-{
-  float ms = 0.f;
-  if (cudaEventElapsedTime(&ms, m->ev_a0, m->ev_a1) == cudaSuccess) m->timings.apply_ms += ms;
-}
-
-// Queues k_apply_runs in the block shape of the run chunk.
-void launch_apply(vdbg_map* m, Channel& c, const RunBuffer& rb, cudaStream_t s)
-{
-  const unsigned grid = apply_grid(m, rb.apply_chunk);
-  const size_t smem   = apply_stage_bytes(rb.apply_chunk);
-  k_apply_prefix<<<1, 1024, 0, s>>>(rb);
-  if (rb.apply_chunk <= kApplySmallChunk)
-    k_apply_runs<128, 256><<<grid, 128, smem, s>>>(rb, map_view(m), channel_view(c));
-  else
-    k_apply_runs<256, 512><<<grid, 256, smem, s>>>(rb, map_view(m), channel_view(c));
-}
-
-// Queues one DDA pass (a fresh one, or `resume` of the rays left in flight)
-// and its k_apply_runs.
 // The endpoint hits (k_mark_hits) on the map's side stream, forked from `s`:
-// they read the sorted rays and write hit bits and leaves, the first DDA
-// pass only reads the rays, so the two run side by side; the pass's apply
-// joins them (join_hits of launch_dda_pass).
+// both read the sorted rays, allocate leaves and OR into the update masks, so
+// the two run side by side; launch_march joins them.
 int launch_hits_forked(vdbg_map* m, Channel& c, const int4* rays, const int* order, const ScanTable& t,
                        unsigned blocks, cudaStream_t s)
 {
@@ -941,110 +850,94 @@ int launch_hits_forked(vdbg_map* m, Channel& c, const int4* rays, const int* ord
   return VDBG_OK;
 }
 
-int launch_dda_pass(vdbg_map* m, Channel& c, const int4* rays, const int* order, const ScanTable& t,
-                    const RunBuffer& rb, LaneState* ls, WarpState* ws, bool resume, cudaStream_t s,
-                    unsigned event_flags = cudaEventRecordDefault, bool join_hits = false)
+// Queues k_march on `s`. The tuning's dda_warps_per_sm scales the resident
+// warps (16: as many as fit), rays_per_take the items a warp takes at a time.
+int launch_march(vdbg_map* m, Channel& c, const int4* rays, const int* order, const uint32_t* cursor,
+                 const ScanTable& t, cudaStream_t s)
 {
-  VDBG_CUDA(cudaMemsetAsync(&m->d_status->inflight, 0, sizeof(uint32_t), s));
-  k_dda_mark<<<rb.warps / kDdaWarps, kDdaWarps * 32, 0, s>>>(rays, order, t, map_view(m), rb, ls, ws,
-                                                            resume ? 1 : 0);
-  if (join_hits) VDBG_CUDA(cudaStreamWaitEvent(s, m->ev_hits, 0));
-  VDBG_CUDA(cudaEventRecordWithFlags(m->ev_a0, s, event_flags));
-  launch_apply(m, c, rb, s);
-  VDBG_CUDA(cudaEventRecordWithFlags(m->ev_a1, s, event_flags));
+  const unsigned per_sm = std::max(1u, kMarchBlocks * std::min(16u, static_cast<unsigned>(m->tuning.dda_warps_per_sm)) / 16u);
+  k_march<<<static_cast<unsigned>(m->num_sms) * per_sm, kMarchWarps * 32, 0, s>>>(
+    rays, order, cursor, t, map_view(m), channel_view(c), m->axis,
+    std::max(1u, static_cast<uint32_t>(m->tuning.rays_per_take) / 8u), 1u);
   VDBG_CUDA(cudaGetLastError());
-  m->timings.launches += 3;  // k_dda_mark, k_apply_prefix, k_apply_runs
+  m->timings.launches += 1;
   return VDBG_OK;
 }
 
-// After `passes` DDA passes whose status has been fetched: handles a pool or
-// hash that ran out (grow what ran out, let the failed leaf cells be
-// allocated again, apply the hits and the pass's runs again, both
-// idempotent; OUT_OF_MEMORY when the pools may not grow) and queues resume
-// passes, one status fetch each, until no ray is left in flight.
-int settle_dda_passes(vdbg_map* m, Channel& c, const int4* rays, const int* order, int64_t n, const ScanTable& t,
-                      const RunBuffer& rb, LaneState* ls, WarpState* ws, bool may_grow, cudaStream_t s,
-                      uint32_t passes)
+// The walk and the endpoint hits beside it, joined on `s`.
+int launch_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, const uint32_t* cursor, int64_t n,
+                   const ScanTable& t, cudaStream_t s)
 {
-  const unsigned hit_blocks = static_cast<unsigned>((n + 255) / 256);
-  for (;;)
+  VDBG_TRY(launch_hits_forked(m, c, rays, order, t, static_cast<unsigned>((n + 255) / 256), s));
+  VDBG_TRY(launch_march(m, c, rays, order, cursor, t, s));
+  VDBG_CUDA(cudaStreamWaitEvent(s, m->ev_hits, 0));
+  return VDBG_OK;
+}
+
+// After a marking whose status has been fetched: handles a pool or hash that
+// ran out (grow what ran out, let the failed leaf cells be allocated again,
+// mark again, which is idempotent; OUT_OF_MEMORY when the pools may not grow).
+int settle_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, const uint32_t* cursor, int64_t n,
+                   const ScanTable& t, bool may_grow, cudaStream_t s)
+{
+  for (int attempt = 0; m->h_status->error != 0u; ++attempt)
   {
-    for (int attempt = 0; m->h_status->error != 0u; ++attempt)
+    const uint32_t err = m->h_status->error;
+    m->n_leaves        = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
+    m->n_blocks        = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
+    if (err & kErrCoordRange)
     {
-      const uint32_t err = m->h_status->error;
-      m->n_leaves        = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
-      m->n_blocks        = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
-      if (err & kErrCoordRange)
-      {
-        // Nothing of the cloud was cast (the prep stage flagged it).
-        clear_error_keep_counters(m);
-        VDBG_CUDA(cudaMemcpyAsync(m->d_status, m->h_status, sizeof(DevStatus), cudaMemcpyHostToDevice, s));
-        VDBG_CUDA(cudaEventRecord(m->ev_dda, s));
-        VDBG_CUDA(cudaStreamSynchronize(s));
-        m->passes_last    = passes;
-        m->timings.passes = passes;
-        return VDBG_ERR_COORD_RANGE;
-      }
-      if (err & (kErrSpin | kErrStepBound)) return map_error(err);
-      if (!may_grow || attempt >= 40) return oom("settle_dda_passes", attempt, err);
-      if (err & kErrPoolFull) VDBG_TRY(grow_for(m, m->h_status->n_leaves));
-      if (err & kErrBlockFull) VDBG_TRY(grow_blocks_for(m, m->h_status->n_blocks));
-      if ((err & kErrHashFull) && !(err & kErrBlockFull))
-        VDBG_TRY(rebuild_hash(m, m->bhash_size * 2, m->n_blocks));
-      if (m->n_blocks > 0)
-      {
-        k_reset_failed_leaves<<<m->num_sms * 4, 256, 0, m->stream>>>(m->bleaf,
-                                                                     static_cast<size_t>(m->n_blocks) * 512);
-        VDBG_CUDA(cudaGetLastError());
-      }
-      VDBG_CUDA(cudaStreamSynchronize(m->stream));
+      // Nothing of the cloud was cast (the prep stage flagged it).
       clear_error_keep_counters(m);
       VDBG_CUDA(cudaMemcpyAsync(m->d_status, m->h_status, sizeof(DevStatus), cudaMemcpyHostToDevice, s));
-      k_mark_hits<<<hit_blocks, 256, 0, s>>>(rays, order, t, map_view(m), channel_view(c));
-      VDBG_CUDA(cudaEventRecord(m->ev_a0, s));
-      launch_apply(m, c, rb, s);
-      VDBG_CUDA(cudaEventRecord(m->ev_a1, s));
-      VDBG_CUDA(cudaGetLastError());
-      m->timings.launches += 3;  // k_mark_hits, k_apply_prefix, k_apply_runs
-      m->timings.retries += 1;
-      VDBG_TRY(fetch_status(m, s));
-      add_apply_time(m);
+      VDBG_CUDA(cudaEventRecord(m->ev_dda, s));
+      VDBG_CUDA(cudaStreamSynchronize(s));
+      m->timings.passes = 1;
+      return VDBG_ERR_COORD_RANGE;
     }
-    m->n_leaves = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
-    m->n_blocks = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
-    if (m->h_status->inflight == 0u && m->h_status->ray_cursor >= m->h_status->n_valid) break;
-    // Every pass completes at least one round per warp, so this bound is
-    // never reached by a working device; it turns a logic error into a status.
-    if (passes > (1u << 20)) return VDBG_ERR_TIMEOUT;
-    VDBG_TRY(launch_dda_pass(m, c, rays, order, t, rb, ls, ws, true, s));
-    ++passes;
+    if (err & (kErrSpin | kErrStepBound)) return map_error(err);
+    if (!may_grow || attempt >= 40) return oom("settle_marking", attempt, err);
+    if (err & kErrPoolFull) VDBG_TRY(grow_for(m, m->h_status->n_leaves));
+    if (err & kErrBlockFull) VDBG_TRY(grow_blocks_for(m, m->h_status->n_blocks));
+    if ((err & kErrHashFull) && !(err & kErrBlockFull))
+      VDBG_TRY(rebuild_hash(m, m->bhash_size * 2, m->n_blocks));
+    if (m->n_blocks > 0)
+    {
+      k_reset_failed_leaves<<<m->num_sms * 4, 256, 0, m->stream>>>(m->bleaf,
+                                                                   static_cast<size_t>(m->n_blocks) * 512);
+      VDBG_CUDA(cudaGetLastError());
+    }
+    VDBG_CUDA(cudaStreamSynchronize(m->stream));
+    clear_error_keep_counters(m);
+    m->h_status->item_cursor = 0;
+    m->h_status->runs        = 0;
+    VDBG_CUDA(cudaMemcpyAsync(m->d_status, m->h_status, sizeof(DevStatus), cudaMemcpyHostToDevice, s));
+    VDBG_TRY(launch_marking(m, c, rays, order, cursor, n, t, s));
+    m->timings.retries += 1;
     VDBG_TRY(fetch_status(m, s));
-    add_apply_time(m);
   }
+  m->n_leaves = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
+  m->n_blocks = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
   VDBG_CUDA(cudaEventRecord(m->ev_dda, s));
-  m->passes_last    = passes;
-  m->timings.passes = passes;
+  m->timings.passes = 1;
   return VDBG_OK;
 }
 
 // castRayIntoGrid for every ray (VDBMapping.hpp:550-566) and the endpoint
-// hits (VDBMapping.hpp:533-536), into channel `c`: endpoint hits once, then
-// DDA passes, each followed by k_apply_runs, until no ray is left in flight.
-// One status fetch per pass.
+// hits (VDBMapping.hpp:533-536), into channel `c`, with one status fetch
+// (more after a pool or hash that ran out).
 int reset_changes(vdbg_map* m, cudaStream_t s);
 int launch_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated);
 
 // `eager`: the channel's window is the only one the call integrates, so its
-// compact, sweep and window end go out right behind the first pass, gated on
-// the device on a complete marking (no host round trip in between); *swept
-// tells whether they ran. Otherwise the caller sweeps after the passes.
-int run_dda_passes(vdbg_map* m, Channel& c, const int4* rays, const int* order, int64_t n, const ScanTable& t,
-                   const RunBuffer& rb, LaneState* ls, WarpState* ws, bool may_grow, cudaStream_t s,
-                   bool eager = false, bool* swept = nullptr)
+// compact, sweep and window end go out right behind the marking, gated on
+// the device on a marking without errors (no host round trip in between);
+// *swept tells whether they ran. Otherwise the caller sweeps.
+int run_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, const uint32_t* cursor, int64_t n,
+                const ScanTable& t, bool may_grow, cudaStream_t s, bool eager = false, bool* swept = nullptr)
 {
   if (swept) *swept = false;
-  VDBG_TRY(launch_hits_forked(m, c, rays, order, t, static_cast<unsigned>((n + 255) / 256), s));
-  VDBG_TRY(launch_dda_pass(m, c, rays, order, t, rb, ls, ws, false, s, cudaEventRecordDefault, true));
+  VDBG_TRY(launch_marking(m, c, rays, order, cursor, n, t, s));
   if (eager)
   {
     VDBG_CUDA(cudaEventRecord(m->ev_dda, s));
@@ -1055,18 +948,16 @@ int run_dda_passes(vdbg_map* m, Channel& c, const int4* rays, const int* order, 
     m->timings.launches += 1;
   }
   VDBG_TRY(fetch_status(m, s));
-  add_apply_time(m);
   if (eager && m->h_status->windows > 0u)
   {
     m->n_leaves       = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
     m->n_blocks       = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
-    m->passes_last    = 1;
     m->timings.passes = 1;
     c.pending         = false;
     *swept            = true;
     return VDBG_OK;
   }
-  return settle_dda_passes(m, c, rays, order, n, t, rb, ls, ws, may_grow, s, 1);
+  return settle_marking(m, c, rays, order, cursor, n, t, may_grow, s);
 }
 
 // Integration of one update grid: compact its touched blocks into the list
@@ -1315,8 +1206,8 @@ bool bad_points(const float* xyz, int64_t n, int64_t stride)
 }
 
 // accumulate (optional) + integration of the listed channels. The marking
-// fetches the status once per DDA pass (normally one); pool and hash
-// exhaustion are handled inside run_dda_passes. A voxel index out of range
+// fetches the status once; pool and hash exhaustion are handled inside
+// run_marking. A voxel index out of range
 // skips the whole cloud (nothing of it is marked) and the other pending
 // update grids are still integrated.
 // After a marking that had to give up (a pool that may not grow, a bounded
@@ -1537,13 +1428,12 @@ CastPlan plan_single(const vdbg_map* m, int64_t n, const double origin[3], doubl
 }
 
 // Kernel launches of one captured step (memsets excluded).
-constexpr uint32_t kGraphKernels = 10;
+constexpr uint32_t kGraphKernels = 8;
 
 // Queues one batched step for capture: the point count is read on the device
 // from t.first[t.n], the grids cover the scratch capacity `cap`, and every
-// kernel after the DDA pass skips itself unless the marking completed.
-int queue_step(vdbg_map* m, Channel& c, int64_t cap, int64_t stride, const ScanTable& t, const RunBuffer& rb,
-               cudaStream_t s)
+// kernel after the marking skips itself unless it completed.
+int queue_step(vdbg_map* m, Channel& c, int64_t cap, int64_t stride, const ScanTable& t, cudaStream_t s)
 {
   const unsigned blocks = static_cast<unsigned>((cap + 255) / 256);
   k_prep<<<blocks, 256, 0, s>>>(nullptr, m->d_pts_ref, cap, stride, t, m->d_rays, m->d_ray_scan, m->d_hist,
@@ -1551,9 +1441,7 @@ int queue_step(vdbg_map* m, Channel& c, int64_t cap, int64_t stride, const ScanT
   launch_scan(m->d_hist, m->d_cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), m->d_status, s);
   k_scatter<<<blocks, 256, 0, s>>>(m->d_rays, cap, t, m->d_cursor, m->d_order);
   VDBG_CUDA(cudaEventRecordWithFlags(m->ev_prep, s, cudaEventRecordExternal));
-  VDBG_TRY(launch_hits_forked(m, c, m->d_rays, m->d_order, t, blocks, s));
-  VDBG_TRY(launch_dda_pass(m, c, m->d_rays, m->d_order, t, rb, m->lstate, m->wstate, false, s,
-                           cudaEventRecordExternal, true));
+  VDBG_TRY(launch_marking(m, c, m->d_rays, m->d_order, m->d_cursor, cap, t, s));
   VDBG_CUDA(cudaEventRecordWithFlags(m->ev_dda, s, cudaEventRecordExternal));
   VDBG_TRY(launch_sweep(m, c, s, true));
   k_finish_window<<<1, 1, 0, s>>>(channel_view(c), m->d_status, 1);
@@ -1563,13 +1451,12 @@ int queue_step(vdbg_map* m, Channel& c, int64_t cap, int64_t stride, const ScanT
 
 // Captures the step for the current layout into m->graph (updating the
 // executable graph in place when its topology allows).
-int capture_step(vdbg_map* m, Channel& c, int64_t stride, const ScanTable& t, const RunBuffer& rb, cudaStream_t s)
+int capture_step(vdbg_map* m, Channel& c, int64_t stride, const ScanTable& t, cudaStream_t s)
 {
-  apply_grid(m, rb.apply_chunk);  // (an occupancy query: not inside the capture)
   const uint32_t launches = m->timings.launches;
   cudaGraph_t g           = nullptr;
   VDBG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  const int q          = queue_step(m, c, static_cast<int64_t>(m->ray_cap), stride, t, rb, s);
+  const int q          = queue_step(m, c, static_cast<int64_t>(m->ray_cap), stride, t, s);
   const cudaError_t ec = cudaStreamEndCapture(s, &g);
   m->timings.launches  = launches;
   if (q != VDBG_OK || ec != cudaSuccess)
@@ -1605,10 +1492,10 @@ int capture_step(vdbg_map* m, Channel& c, int64_t stride, const ScanTable& t, co
 
 // One batched step through the captured graph: the points' copy, the graph,
 // one status fetch. *swept when the graph integrated the window (the marking
-// completed in its one DDA pass); otherwise the step goes on as the launch
-// loop does (pool growth, resume passes) and the caller sweeps.
+// completed); otherwise the step goes on as the launch loop does (pool
+// growth, marking again) and the caller sweeps.
 int graph_step(vdbg_map* m, Channel& c, const float* xyz, int64_t n, int64_t stride, const ScanTable& t,
-               uint32_t flags, const RunBuffer& rb, cudaStream_t s, bool* swept)
+               uint32_t flags, cudaStream_t s, bool* swept)
 {
   *swept          = false;
   const char* pts = reinterpret_cast<const char*>(xyz);
@@ -1624,24 +1511,22 @@ int graph_step(vdbg_map* m, Channel& c, const float* xyz, int64_t n, int64_t str
   VDBG_CUDA(cudaMemcpyAsync(m->d_pts_ref, m->h_pts_ref, sizeof(const char*), cudaMemcpyHostToDevice, s));
   c.pending = true;
   if (!m->graph || m->graph_layout != m->layout || m->graph_stride != stride || m->graph_grouped != use_grouped_sweep(m))
-    VDBG_TRY(capture_step(m, c, stride, t, rb, s));
+    VDBG_TRY(capture_step(m, c, stride, t, s));
   VDBG_CUDA(cudaGraphLaunch(m->graph, s));
   m->graph_replays += 1;
   m->timed_prep = true;
   m->timings.launches += kGraphKernels;
   VDBG_TRY(fetch_status(m, s));
-  add_apply_time(m);
   if (m->h_status->windows > 0u)
   {
     m->n_leaves    = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
     m->n_blocks    = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
-    m->passes_last    = 1;
     m->timings.passes = 1;
     c.pending         = false;
     *swept         = true;
     return VDBG_OK;
   }
-  return settle_dda_passes(m, c, m->d_rays, m->d_order, n, t, rb, m->lstate, m->wstate, true, s, 1);
+  return settle_marking(m, c, m->d_rays, m->d_order, m->d_cursor, n, t, true, s);
 }
 
 template <class F>
@@ -1676,19 +1561,8 @@ int accumulate_and_integrate(vdbg_map* m, const float* xyz, int64_t n, int64_t s
   {
     const bool host_input = (flags & VDBG_POINTS_DEVICE) == 0;
     VDBG_TRY(ensure_scratch(m, n, stride, host_input));
-    // One pass for a scan like the last one: segments sized from the previous
-    // call's pass count, with room to spare (a warp's runs vary from call to
-    // call with the long rays it takes), bounded by the run-buffer budget.
-    uint32_t seg = std::max<uint32_t>(m->run_seg, kMinRunSeg);
-    if (m->passes_last > 1)
-    {
-      const uint64_t want  = static_cast<uint64_t>(m->run_seg) * m->passes_last * 2;
-      const uint64_t limit = m->run_budget / (17ull * m->dda_warps);
-      seg                  = static_cast<uint32_t>(std::min<uint64_t>(want, limit));
-    }
-    VDBG_TRY(ensure_runs(m, seg));
     ScanTable t = plan.table;
-    set_edges(m, t);
+    t.clog      = chunk_log2_for(n);
     if (t.n > 1)
     {
       // Scan table to the device (from pinned staging, so the copy is async).
@@ -1700,16 +1574,16 @@ int accumulate_and_integrate(vdbg_map* m, const float* xyz, int64_t n, int64_t s
       t.first    = m->d_first;
       t.ray_scan = m->d_ray_scan;
     }
-    const RunBuffer rb =
-      run_buffer(m, m->run_key, m->run_bits, m->run_slab, m->run_count, m->run_prefix, m->run_seg, m->dda_warps);
     const bool fast    = !m->batch && m->conf[0].fast_mode;
     const bool graphed = !fast && m->use_graph && m->batch && t.n > 1 && !m->track_changes && integrate_all &&
                          m->channels.size() == 1 && src == &m->channels[0];
     int d = VDBG_OK;
     if (graphed)
     {
+      // (fixed by the layout, so that steps of any size replay one graph)
+      t.clog     = chunk_log2_for(static_cast<int64_t>(m->ray_cap));
       bool swept = false;
-      d          = graph_step(m, *src, xyz, n, stride, t, flags, rb, s, &swept);
+      d          = graph_step(m, *src, xyz, n, stride, t, flags, s, &swept);
       if (d == VDBG_OK && swept)
       {
         record_timings(m);
@@ -1735,7 +1609,7 @@ int accumulate_and_integrate(vdbg_map* m, const float* xyz, int64_t n, int64_t s
         for (const Channel& c : m->channels)
           if (&c != src && c.pending) eager = false;
       bool swept = false;
-      d = run_dda_passes(m, *src, m->d_rays, m->d_order, n, t, rb, m->lstate, m->wstate, true, s, eager, &swept);
+      d = run_marking(m, *src, m->d_rays, m->d_order, m->d_cursor, n, t, true, s, eager, &swept);
       if (d == VDBG_OK && swept)
       {
         record_timings(m);
@@ -1912,17 +1786,6 @@ int create_impl(int n_maps, const double* resolutions, const vdbg_options* optio
   if (cudaSetDevice(m->device) != cudaSuccess) return fail(VDBG_ERR_CUDA);
   if (cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, m->device) != cudaSuccess)
     return fail(VDBG_ERR_CUDA);
-  {
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return fail(VDBG_ERR_CUDA);
-    m->run_budget = std::min<uint64_t>(kMaxRunBytes, total_b / 32);
-  }
-  m->dda_warps = static_cast<uint32_t>(m->num_sms) * static_cast<uint32_t>(m->tuning.dda_warps_per_sm);
-  if (cudaFuncSetAttribute(k_apply_runs<256, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(apply_stage_bytes(kApplyMaxChunk))) != cudaSuccess ||
-      cudaFuncSetAttribute(k_apply_runs<128, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(apply_stage_bytes(kApplySmallChunk))) != cudaSuccess)
-    return fail(VDBG_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&m->grow, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1931,8 +1794,7 @@ int create_impl(int n_maps, const double* resolutions, const vdbg_options* optio
       cudaEventCreateWithFlags(&m->ev_hits, cudaEventDisableTiming) != cudaSuccess)
     return fail(VDBG_ERR_CUDA);
   if (cudaEventCreate(&m->ev0) != cudaSuccess || cudaEventCreate(&m->ev1) != cudaSuccess ||
-      cudaEventCreate(&m->ev_prep) != cudaSuccess || cudaEventCreate(&m->ev_dda) != cudaSuccess ||
-      cudaEventCreate(&m->ev_a0) != cudaSuccess || cudaEventCreate(&m->ev_a1) != cudaSuccess)
+      cudaEventCreate(&m->ev_prep) != cudaSuccess || cudaEventCreate(&m->ev_dda) != cudaSuccess)
     return fail(VDBG_ERR_CUDA);
   if (cudaMallocHost(reinterpret_cast<void**>(&m->h_status), sizeof(DevStatus)) != cudaSuccess)
     return fail(VDBG_ERR_OUT_OF_MEMORY);
@@ -1949,6 +1811,13 @@ int create_impl(int n_maps, const double* resolutions, const vdbg_options* optio
   if (s != VDBG_OK) return fail(s);
   if (cudaMemsetAsync(m->d_hist, 0, m->buckets * sizeof(uint32_t), m->stream) != cudaSuccess)
     return fail(VDBG_ERR_CUDA);
+  s = dev_alloc(m, &m->axis_mem, kAxisTableBytes);
+  if (s != VDBG_OK) return fail(s);
+  m->axis.td    = reinterpret_cast<ulonglong2*>(m->axis_mem);
+  m->axis.kf    = reinterpret_cast<int2*>(m->axis.td + kAxisTableN * kAxisTableJ);
+  m->axis.delta = reinterpret_cast<double*>(m->axis.kf + kAxisTableN * kAxisTableJ);
+  k_axis_table<<<(kAxisTableN * kAxisTableJ + 255) / 256, 256, 0, m->stream>>>(m->axis);
+  if (cudaGetLastError() != cudaSuccess) return fail(VDBG_ERR_CUDA);
   if (batch)
   {
     m->batch = true;
@@ -2123,13 +1992,7 @@ int vdbg_destroy(vdbg_map* m)
   dev_free(m, m->d_pts, m->pts_cap);
   dev_free(m, m->d_rays, m->ray_cap);
   dev_free(m, m->d_order, m->ray_cap);
-  dev_free(m, m->run_key, static_cast<size_t>(m->dda_warps) * m->run_seg);
-  dev_free(m, m->run_bits, static_cast<size_t>(m->dda_warps) * m->run_seg);
-  dev_free(m, m->run_slab, static_cast<size_t>(m->dda_warps) * m->run_seg);
-  dev_free(m, m->run_count, m->dda_warps);
-  dev_free(m, m->run_prefix, static_cast<size_t>(m->dda_warps) + 2);
-  dev_free(m, m->lstate, static_cast<size_t>(m->dda_warps) * 32);
-  dev_free(m, m->wstate, m->dda_warps);
+  dev_free(m, m->axis_mem, kAxisTableBytes);
   dev_free(m, m->topo_keys, 2 * static_cast<size_t>(m->topo_cap));
   dev_free(m, m->topo_box, 8);
   dev_free(m, m->d_trace, m->trace_bytes);
@@ -2144,8 +2007,6 @@ int vdbg_destroy(vdbg_map* m)
   if (m->ev1) cudaEventDestroy(m->ev1);
   if (m->ev_prep) cudaEventDestroy(m->ev_prep);
   if (m->ev_dda) cudaEventDestroy(m->ev_dda);
-  if (m->ev_a0) cudaEventDestroy(m->ev_a0);
-  if (m->ev_a1) cudaEventDestroy(m->ev_a1);
   if (m->ev_fork) cudaEventDestroy(m->ev_fork);
   if (m->ev_hits) cudaEventDestroy(m->ev_hits);
   if (m->ev_grow) cudaEventDestroy(m->ev_grow);
@@ -2335,7 +2196,7 @@ int vdbg_ray_digests(vdbg_map* m, const float* xyz, int64_t n, int64_t stride, c
   CastPlan plan = plan_single(m, n, origin, raycast_range);
   if (plan.status != VDBG_OK) return plan.status;
   if (!plan.any) return VDBG_OK;  // a NaN origin: nothing is cast
-  set_edges(m, plan.table);
+  plan.table.clog = chunk_log2_for(n);
   const bool host_input = (flags & VDBG_POINTS_DEVICE) == 0;
   VDBG_TRY(ensure_scratch(m, n, stride, host_input));
   const char* pts = reinterpret_cast<const char*>(xyz);
@@ -2349,7 +2210,7 @@ int vdbg_ray_digests(vdbg_map* m, const float* xyz, int64_t n, int64_t stride, c
   VDBG_TRY(dev_alloc(m, &d_out, static_cast<size_t>(n) * 2));
   const unsigned blocks = static_cast<unsigned>((n + 255) / 256);
   k_prep<<<blocks, 256, 0, s>>>(pts, nullptr, n, stride, plan.table, m->d_rays, nullptr, m->d_hist, m->d_status);
-  k_ray_digest<<<blocks, 256, 0, s>>>(m->d_rays, n, plan.table, d_out, m->d_status);
+  k_ray_digest<<<blocks, 256, 0, s>>>(m->d_rays, n, plan.table, m->axis, d_out, m->d_status);
   int st = cudaGetLastError() == cudaSuccess ? VDBG_OK : VDBG_ERR_CUDA;
   // (k_prep counted the rays into the sort histogram, which must start the
   // next insertion at zero)
@@ -2452,36 +2313,21 @@ int vdbg_set_tuning(vdbg_map* m, const vdbg_tuning* t)
 {
   if (!m || !t) return VDBG_ERR_INVALID_ARGUMENT;
   if (t->rays_per_take < 1 || t->rays_per_take > 1024) return VDBG_ERR_INVALID_ARGUMENT;
-  if (t->apply_chunk_runs < 256 || t->apply_chunk_runs > static_cast<int32_t>(kApplyMaxChunk) ||
-      (t->apply_chunk_runs % 256) != 0)
+  // (apply_chunk_runs and length_edges steer nothing any more; their ranges
+  // are checked as before)
+  if (t->apply_chunk_runs < 256 || t->apply_chunk_runs > 4096 || (t->apply_chunk_runs % 256) != 0)
     return VDBG_ERR_INVALID_ARGUMENT;
   if (!(t->length_edges[0] > t->length_edges[1] && t->length_edges[1] > t->length_edges[2] &&
         t->length_edges[2] > 0))
     return VDBG_ERR_INVALID_ARGUMENT;
   if (!(t->hash_load > 0.05f && t->hash_load <= 0.9f)) return VDBG_ERR_INVALID_ARGUMENT;
-  if (t->dda_warps_per_sm < kDdaWarps || t->dda_warps_per_sm > 10 * kDdaWarps || (t->dda_warps_per_sm % kDdaWarps))
+  if (t->dda_warps_per_sm < 2 || t->dda_warps_per_sm > 20 || (t->dda_warps_per_sm % 2))
     return VDBG_ERR_INVALID_ARGUMENT;
   if (t->sweep_kernel < 0 || t->sweep_kernel > 2) return VDBG_ERR_INVALID_ARGUMENT;
   VDBG_TRY(set_device(m));
   VDBG_CUDA(cudaStreamSynchronize(m->stream));
   VDBG_TRY(publish_growth(m, m->stream));
   const bool rehash = t->hash_load != m->tuning.hash_load;
-  if (t->dda_warps_per_sm != m->tuning.dda_warps_per_sm)
-  {
-    // The run buffer and the DDA resume state are per warp: drop them, the
-    // next insertion sizes them for the new warp count.
-    const size_t W = m->dda_warps;
-    dev_free(m, m->run_key, W * m->run_seg);
-    dev_free(m, m->run_bits, W * m->run_seg);
-    dev_free(m, m->run_slab, W * m->run_seg);
-    dev_free(m, m->run_count, W);
-    dev_free(m, m->run_prefix, W + 2);
-    dev_free(m, m->lstate, W * 32);
-    dev_free(m, m->wstate, W);
-    m->run_seg     = 0;
-    m->passes_last = 0;
-    m->dda_warps   = static_cast<uint32_t>(m->num_sms) * static_cast<uint32_t>(t->dda_warps_per_sm);
-  }
   m->tuning = *t;
   m->layout += 1;  // kernel parameters of a captured step change
   if (rehash)
@@ -3476,36 +3322,21 @@ int vdbg_apply_section_values(vdbg_map* m, int map, int64_t n, const int32_t* or
 // Insertion without device allocation (vdbg_insert_point_cloud_noalloc).
 //
 // The per-scan scratch of the regular path (host points staged on the device,
-// ray records, the DDA order, the bucket histogram/cursor, the DDA run buffer
-// and the DDA resume state) is carved out of one file-scope device array
-// instead of map-owned buffers that grow on demand; the DDA runs on a fixed
-// number of warps with small run segments, in as many passes as the scan
-// needs. The map's leaf pool and block index are used as created and never
+// ray records, the ray order and the bucket histogram/cursor) is carved out of
+// one file-scope device array instead of map-owned buffers that grow on
+// demand. The map's leaf pool and block index are used as created and never
 // grown.
 // ---------------------------------------------------------------------------
 namespace {
 
 constexpr int64_t kNoAllocMaxPoints = VDBG_NOALLOC_MAX_POINTS;
-constexpr uint32_t kNoAllocWarps    = VDBG_NOALLOC_DDA_WARPS;
-constexpr uint32_t kNoAllocSeg      = VDBG_NOALLOC_RUN_SEGMENT;
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kNoAllocPtsBytes   = align256(static_cast<size_t>(kNoAllocMaxPoints) * 16);
 constexpr size_t kNoAllocRaysBytes  = align256(static_cast<size_t>(kNoAllocMaxPoints) * sizeof(int4));
 constexpr size_t kNoAllocOrderBytes = align256(static_cast<size_t>(kNoAllocMaxPoints) * sizeof(int));
 constexpr size_t kNoAllocHistBytes  = align256(static_cast<size_t>(kBucketsPerScan) * sizeof(uint32_t));
-constexpr size_t kNoAllocRunN       = static_cast<size_t>(kNoAllocWarps) * kNoAllocSeg;
-constexpr size_t kNoAllocKeyBytes   = align256(kNoAllocRunN * sizeof(unsigned long long));
-constexpr size_t kNoAllocSlabBytes  = align256(kNoAllocRunN);
-constexpr size_t kNoAllocCountBytes = align256(static_cast<size_t>(kNoAllocWarps) * sizeof(uint32_t));
-constexpr size_t kNoAllocPrefixBytes = align256((static_cast<size_t>(kNoAllocWarps) + 2) * sizeof(uint32_t));
-constexpr size_t kNoAllocLaneBytes  = align256(static_cast<size_t>(kNoAllocWarps) * 32 * sizeof(LaneState));
-constexpr size_t kNoAllocWarpBytes  = align256(static_cast<size_t>(kNoAllocWarps) * sizeof(WarpState));
-constexpr size_t kNoAllocBytes = kNoAllocPtsBytes + kNoAllocRaysBytes + kNoAllocOrderBytes + 2 * kNoAllocHistBytes +
-                                 2 * kNoAllocKeyBytes + kNoAllocSlabBytes + kNoAllocCountBytes + kNoAllocPrefixBytes +
-                                 kNoAllocLaneBytes +
-                                 kNoAllocWarpBytes;
+constexpr size_t kNoAllocBytes = kNoAllocPtsBytes + kNoAllocRaysBytes + kNoAllocOrderBytes + 2 * kNoAllocHistBytes;
 static_assert(kNoAllocBytes <= static_cast<size_t>(VDBG_NOALLOC_SCRATCH_BYTES), "scratch size and header disagree");
-static_assert(kNoAllocWarps % kDdaWarps == 0, "DDA warps per block");
 
 constexpr int kNoAllocMaxDevices = 64;
 
@@ -3581,21 +3412,7 @@ extern "C" int vdbg_insert_point_cloud_noalloc(vdbg_map* m, const float* xyz, in
   uint32_t* d_hist   = reinterpret_cast<uint32_t*>(p);
   p += kNoAllocHistBytes;
   uint32_t* d_cursor = reinterpret_cast<uint32_t*>(p);
-  p += kNoAllocHistBytes;
-  unsigned long long* r_key  = reinterpret_cast<unsigned long long*>(p);
-  p += kNoAllocKeyBytes;
-  unsigned long long* r_bits = reinterpret_cast<unsigned long long*>(p);
-  p += kNoAllocKeyBytes;
-  unsigned char* r_slab      = reinterpret_cast<unsigned char*>(p);
-  p += kNoAllocSlabBytes;
-  uint32_t* r_count          = reinterpret_cast<uint32_t*>(p);
-  p += kNoAllocCountBytes;
-  uint32_t* r_prefix         = reinterpret_cast<uint32_t*>(p);
-  p += kNoAllocPrefixBytes;
-  LaneState* ls              = reinterpret_cast<LaneState*>(p);
-  p += kNoAllocLaneBytes;
-  WarpState* ws              = reinterpret_cast<WarpState*>(p);
-  cudaStream_t s             = pick_stream(m, stream);
+  cudaStream_t s     = pick_stream(m, stream);
 
   Channel* src = find_channel(m, id);
   int pre      = VDBG_OK;
@@ -3614,14 +3431,13 @@ extern "C" int vdbg_insert_point_cloud_noalloc(vdbg_map* m, const float* xyz, in
     // The histogram must start at zero; the previous call's contents remain.
     VDBG_CUDA(cudaMemsetAsync(d_hist, 0, kNoAllocHistBytes, s));
     CastPlan plan = plan_single(m, n, origin, src->max_range);
-    set_edges(m, plan.table);
+    plan.table.clog = chunk_log2_for(n);
     if (plan.status != VDBG_OK) result = plan.status;
     if (plan.any)
     {
       VDBG_TRY(launch_prep(m, *src, xyz, n, stride, plan.table, flags, s, d_pts, d_rays, nullptr, d_order, d_hist,
                            d_cursor));
-      const RunBuffer rb = run_buffer(m, r_key, r_bits, r_slab, r_count, r_prefix, kNoAllocSeg, kNoAllocWarps);
-      dda                = run_dda_passes(m, *src, d_rays, d_order, n, plan.table, rb, ls, ws, false, s);
+      dda = run_marking(m, *src, d_rays, d_order, d_cursor, n, plan.table, false, s);
       if (dda == VDBG_ERR_COORD_RANGE)
       {
         result = dda;
