@@ -54,6 +54,20 @@ def test_section_extraction_matches_oracle(vdbg, oracle, full):
         same_section(g.getMapSection(lo, hi, full), o.getMapSection(lo, hi, full), f"box {lo} {hi}")
 
 
+@pytest.mark.parametrize("lo, hi", [
+    ((-512, -512, -256), (511, 511, 255)),  # 2^20 leaf cells: looked up cell by cell
+    ((-513, -512, -256), (511, 511, 255)),  # a row more: the map's leaves listed and sorted
+    ((-(1 << 31), -3, 0), ((1 << 31) - 1, 4, 17)),  # past the index range on one axis
+    ((2000000, -40, -40), (2100000, 40, 40)),  # nothing there, partly out of range
+    ((3, 4, 5), (2, 4, 5)),  # empty
+    ((-8, 0, 7), (7, 15, 8)),  # whole leaf cells and halves
+])
+def test_section_box_limits(vdbg, oracle, lo, hi):
+    g, o = built_pair(vdbg, oracle)
+    for full in (True, False):
+        same_section(g.getMapSection(lo, hi, full), o.getMapSection(lo, hi, full), f"box {lo} {hi}")
+
+
 def test_apply_section_states_matches_oracle(vdbg, oracle):
     g, o = built_pair(vdbg, oracle)
     src_g, src_o = built_pair(vdbg, oracle)

@@ -151,6 +151,13 @@ struct vdbg_map
   char* axis_mem        = nullptr;  // [kAxisTableBytes]
   AxisTable axis{};
 
+  // Device workspaces of the section calls, kept between calls up to
+  // kWorkKept bytes. The mutex is held by the call that uses them (readers of
+  // one map may come from several threads).
+  std::mutex work_mutex;
+  char* work[2]         = {nullptr, nullptr};
+  size_t work_bytes[2]  = {0, 0};
+
   int64_t bytes         = 0;
   int num_sms           = 152;
   vdbg_tuning tuning{32, 2048, {2048, 1024, 512}, 0.5f, 16, 0};
@@ -221,6 +228,8 @@ constexpr uint32_t kDefaultCapacity = 1u << 16;
 constexpr uint32_t kMinBlocks       = 1u << 10;
 constexpr int kSweepBlocks          = 152 * 8;
 constexpr int kSweepThreads         = 256;
+constexpr size_t kWorkKept          = size_t(64) << 20;
+constexpr int64_t kSectionCells     = int64_t(1) << 20;  // boxes of more leaf cells list the map's leaves
 
 uint32_t next_pow2(uint64_t v)
 {
@@ -284,6 +293,29 @@ void dev_free(vdbg_map* m, T*& p, size_t count)
     const int s_ = (expr);    \
     if (s_ != VDBG_OK) return s_; \
   } while (0)
+
+// Workspace `k` with at least `bytes` (its contents are lost when it grows).
+int work_ensure(vdbg_map* m, int k, size_t bytes)
+{
+  if (bytes <= m->work_bytes[k]) return VDBG_OK;
+  dev_free(m, m->work[k], m->work_bytes[k]);
+  m->work_bytes[k] = 0;
+  const size_t want = (bytes + bytes / 4 + 0xfffff) & ~size_t(0xfffff);
+  VDBG_TRY(dev_alloc(m, &m->work[k], want));
+  m->work_bytes[k] = want;
+  return VDBG_OK;
+}
+
+// The end of a call that used the workspaces: large ones are given back.
+void work_done(vdbg_map* m, size_t keep = kWorkKept)
+{
+  for (int k = 0; k < 2; ++k)
+    if (m->work_bytes[k] > keep)
+    {
+      dev_free(m, m->work[k], m->work_bytes[k]);
+      m->work_bytes[k] = 0;
+    }
+}
 
 MapView map_view(const vdbg_map* m)
 {
@@ -1542,8 +1574,8 @@ int reactivate_artificial(vdbg_map* m, Channel& c, cudaStream_t s)
   VDBG_CUDA(cudaStreamSynchronize(s));
   if (touched == 0u) return VDBG_OK;
   return run_allocating(m, [&]() -> int {
-    k_section_set_states<<<(m->art_n + 255) / 256, 256, 0, s>>>(map_view(m), m->d_art_o, m->d_art_m, m->art_n, 0,
-                                                                m->flags, m->active);
+    k_section_set_states<false><<<(m->art_n + 255) / 256, 256, 0, s>>>(map_view(m), m->d_art_o, m->d_art_m, m->art_n,
+                                                                       0, m->flags, m->active);
     VDBG_CUDA(cudaGetLastError());
     m->timings.launches += 1;
     return VDBG_OK;
@@ -1879,25 +1911,16 @@ void values_to_vdb(const float* in, float* out)
   for (int o = 0; o < 512; ++o) out[swap_xz(o)] = in[leaf_float(o)];
 }
 
-// The same from plain z-major order (offset z << 6 | y << 3 | x), the order
-// the section extraction writes.
-void zmajor_to_vdb(const float* in, float* out)
-{
-  for (int o = 0; o < 512; ++o) out[swap_xz(o)] = in[o];
-}
-
-// One leaf's 8-word voxel mask into OpenVDB's order.
+// One leaf's 8-word voxel mask into OpenVDB's order (or back).
 void mask_to_vdb(const unsigned long long* in, uint64_t* out)
 {
-  for (int w = 0; w < 8; ++w) out[w] = 0;
+  uint64_t swapped[8];
   for (int w = 0; w < 8; ++w)
   {
-    for (unsigned long long b = in[w]; b; b &= b - 1)
-    {
-      const int o = swap_xz(w * 64 + __builtin_ctzll(b));
-      out[o >> 6] |= 1ull << (o & 63);
-    }
+    swapped[w] = 0;
+    for (int k = 0; k < 8; ++k) swapped[w] |= ((in[k] >> w) & 0x0101010101010101ull) << k;
   }
+  std::memcpy(out, swapped, sizeof(swapped));
 }
 
 int export_impl(vdbg_map* m, int map, int64_t capacity, int32_t* origins, float* values, uint64_t* masks,
@@ -1993,6 +2016,7 @@ int vdbg_destroy(vdbg_map* m)
   dev_free(m, m->d_rays, m->ray_cap);
   dev_free(m, m->d_order, m->ray_cap);
   dev_free(m, m->axis_mem, kAxisTableBytes);
+  work_done(m, 0);
   dev_free(m, m->topo_keys, 2 * static_cast<size_t>(m->topo_cap));
   dev_free(m, m->topo_box, 8);
   dev_free(m, m->d_trace, m->trace_bytes);
@@ -2546,22 +2570,106 @@ bool leaf_origin_ok(const int32_t* o)
   return true;
 }
 
-// Device list of the map's leaves overlapping [lo, hi] (slots), its length on
-// the host. The caller frees list and count.
-int section_list(vdbg_map* m, int mp, int3 lo, int3 hi, uint32_t** list, uint32_t** count, uint32_t* n_host)
+// A section box's corner, brought to just outside the index range (differences
+// with voxel indices stay within int).
+int3 box_corner(const int32_t v[3])
 {
-  *list = nullptr;
-  *count = nullptr;
-  *n_host = 0;
+  auto c = [](int32_t x) { return std::min(std::max(x, -(1 << 22)), 1 << 22); };
+  return make_int3(c(v[0]), c(v[1]), c(v[2]));
+}
+
+// Candidate slots of the box [lo, hi] of map `mp` in the order of their
+// origins, into workspace 0 (from its start). *cand null: none.
+int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, int** cand, uint32_t* n_out)
+{
+  *cand  = nullptr;
+  *n_out = 0;
+  cudaStream_t s   = m->stream;
   const uint32_t n = std::min(m->n_leaves, m->capacity);
-  VDBG_TRY(dev_alloc(m, count, 1));
-  if (n == 0) return VDBG_OK;
-  VDBG_TRY(dev_alloc(m, list, n));
-  cudaStream_t s = m->stream;
-  VDBG_CUDA(cudaMemsetAsync(*count, 0, sizeof(uint32_t), s));
-  k_section_leaves<<<(n + 255) / 256, 256, 0, s>>>(m->origin, m->flags, n, mp, lo, hi, *list, *count);
+  if (n == 0 || lo.x > hi.x || lo.y > hi.y || lo.z > hi.z) return VDBG_OK;
+  // Leaf cells of the box within the map's range.
+  const int kLo = static_cast<int>(kVoxelMin) >> 3, kHi = (static_cast<int>(kVoxelMaxExcl) >> 3) - 1;
+  const int3 first = make_int3(std::max(lo.x >> 3, kLo), std::max(lo.y >> 3, kLo), std::max(lo.z >> 3, kLo));
+  const int3 last  = make_int3(std::min(hi.x >> 3, kHi), std::min(hi.y >> 3, kHi), std::min(hi.z >> 3, kHi));
+  if (first.x > last.x || first.y > last.y || first.z > last.z) return VDBG_OK;
+  const int3 dims = make_int3(last.x - first.x + 1, last.y - first.y + 1, last.z - first.z + 1);
+  // (each at most 2^19)
+  const int64_t plane = static_cast<int64_t>(dims.x) * dims.y;
+  if (plane <= kSectionCells && plane * dims.z <= kSectionCells)
+  {
+    const uint32_t cells = static_cast<uint32_t>(plane * dims.z);
+    VDBG_TRY(work_ensure(m, 0, static_cast<size_t>(cells) * 3 * sizeof(uint32_t) + 256));
+    *cand  = reinterpret_cast<int*>(m->work[0]);
+    *n_out = cells;
+    k_section_cells<<<(cells + 255) / 256, 256, 0, s>>>(map_view(m), mp, m->flags, first, dims, cells, *cand);
+    VDBG_CUDA(cudaGetLastError());
+    return VDBG_OK;
+  }
+  VDBG_TRY(work_ensure(m, 1, static_cast<size_t>(n) * sizeof(uint32_t) + 256));
+  uint32_t* count = reinterpret_cast<uint32_t*>(m->work[1]);
+  uint32_t* list  = count + 64;
+  uint32_t c      = 0;
+  VDBG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
+  k_section_leaves<<<(n + 255) / 256, 256, 0, s>>>(m->origin, m->flags, n, mp, lo, hi, list, count);
   VDBG_CUDA(cudaGetLastError());
-  VDBG_CUDA(cudaMemcpyAsync(n_host, *count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaMemcpyAsync(&c, count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaStreamSynchronize(s));
+  if (c == 0) return VDBG_OK;
+  VDBG_TRY(work_ensure(m, 0, static_cast<size_t>(c) * std::max(3 * sizeof(uint32_t), sizeof(int4)) + 256));
+  std::vector<int4> ho(c);
+  std::vector<uint32_t> hl(c), idx(c);
+  int4* d_o = reinterpret_cast<int4*>(m->work[0]);
+  k_section_origins<<<(c + 255) / 256, 256, 0, s>>>(list, c, m->origin, d_o);
+  VDBG_CUDA(cudaGetLastError());
+  VDBG_CUDA(cudaMemcpyAsync(ho.data(), d_o, c * sizeof(int4), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaMemcpyAsync(hl.data(), list, c * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaStreamSynchronize(s));
+  std::iota(idx.begin(), idx.end(), 0u);
+  std::sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) {
+    if (ho[a].x != ho[b].x) return ho[a].x < ho[b].x;
+    if (ho[a].y != ho[b].y) return ho[a].y < ho[b].y;
+    return ho[a].z < ho[b].z;
+  });
+  for (uint32_t& i : idx) i = hl[i];
+  VDBG_CUDA(cudaMemcpyAsync(m->work[0], idx.data(), c * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  VDBG_CUDA(cudaStreamSynchronize(s));  // (idx goes out of scope)
+  *cand  = reinterpret_cast<int*>(m->work[0]);
+  *n_out = c;
+  return VDBG_OK;
+}
+
+// getMapSection into host arrays (any of them may be null).
+int section_export(vdbg_map* m, int mp, int3 lo, int3 hi, int full, int64_t capacity, int32_t* origins, float* values,
+                   uint64_t* masks, int64_t* n_out)
+{
+  cudaStream_t s = m->stream;
+  int* cand      = nullptr;
+  uint32_t n = 0, kept = 0;
+  VDBG_TRY(section_candidates(m, mp, lo, hi, &cand, &n));
+  if (n == 0) return VDBG_OK;
+  uint32_t* keep  = reinterpret_cast<uint32_t*>(cand) + n;
+  uint32_t* pos   = keep + n;
+  uint32_t* total = pos + n;
+  k_section_keep<<<static_cast<unsigned>((static_cast<uint64_t>(n) * 8 + 255) / 256), 256, 0, s>>>(
+    cand, n, m->origin, m->values, m->active, lo, hi, full, keep);
+  k_section_scan<<<1, 1024, 0, s>>>(keep, n, pos, total);
+  VDBG_CUDA(cudaGetLastError());
+  VDBG_CUDA(cudaMemcpyAsync(&kept, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaStreamSynchronize(s));
+  *n_out = kept;
+  if (static_cast<int64_t>(kept) > capacity) return VDBG_ERR_BUFFER_TOO_SMALL;
+  if (kept == 0 || (!origins && !values && !masks)) return VDBG_OK;
+  const size_t k = kept;
+  VDBG_TRY(work_ensure(m, 1, k * (512 * sizeof(float) + 8 * sizeof(uint64_t) + 3 * sizeof(int32_t))));
+  float* d_v              = reinterpret_cast<float*>(m->work[1]);
+  unsigned long long* d_m = reinterpret_cast<unsigned long long*>(d_v + k * 512);
+  int* d_o                = reinterpret_cast<int*>(d_m + k * 8);
+  k_section_write<<<static_cast<unsigned>((static_cast<uint64_t>(n) * 32 + 255) / 256), 256, 0, s>>>(
+    cand, n, keep, pos, m->origin, m->values, m->active, lo, hi, full, d_o, values ? d_v : nullptr, d_m);
+  VDBG_CUDA(cudaGetLastError());
+  if (values) VDBG_CUDA(cudaMemcpyAsync(values, d_v, k * 512 * sizeof(float), cudaMemcpyDeviceToHost, s));
+  if (masks) VDBG_CUDA(cudaMemcpyAsync(masks, d_m, k * 8 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  if (origins) VDBG_CUDA(cudaMemcpyAsync(origins, d_o, k * 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   VDBG_CUDA(cudaStreamSynchronize(s));
   return VDBG_OK;
 }
@@ -2898,8 +3006,8 @@ int vdbg_restore_map_integrity(vdbg_map* m)
     // background 0 exceeds the threshold; then its leaf is created first.
     if (0.0f > thres_max)
       VDBG_TRY(run_allocating(m, [&]() -> int {
-        k_section_set_states<<<(m->art_n + 255) / 256, 256, 0, s>>>(map_view(m), m->d_art_o, m->d_art_m, m->art_n,
-                                                                    0, m->flags, m->active);
+        k_section_set_states<false><<<(m->art_n + 255) / 256, 256, 0, s>>>(map_view(m), m->d_art_o, m->d_art_m,
+                                                                           m->art_n, 0, m->flags, m->active);
         VDBG_CUDA(cudaGetLastError());
         return VDBG_OK;
       }));
@@ -3054,73 +3162,11 @@ int vdbg_export_section(vdbg_map* m, int map, const int32_t lo[3], const int32_t
   *n_out = 0;
   VDBG_TRY(set_device(m));
   VDBG_CUDA(cudaStreamSynchronize(m->stream));
-  const int3 blo = make_int3(lo[0], lo[1], lo[2]), bhi = make_int3(hi[0], hi[1], hi[2]);
-  uint32_t *list = nullptr, *count = nullptr, *keep = nullptr;
-  int4* out_o      = nullptr;
-  float* out_v     = nullptr;
-  unsigned long long* out_m = nullptr;
-  uint32_t c = 0;
-  std::vector<int4> ho;
-  std::vector<uint32_t> hk;
-  std::vector<float> hv;
-  std::vector<unsigned long long> hm;
-  int st = section_list(m, mp, blo, bhi, &list, &count, &c);
-  if (st == VDBG_OK && c > 0)
-  {
-    cudaStream_t s = m->stream;
-    st = dev_alloc(m, &out_o, c);
-    if (st == VDBG_OK) st = dev_alloc(m, &out_v, static_cast<size_t>(c) * 512);
-    if (st == VDBG_OK) st = dev_alloc(m, &out_m, static_cast<size_t>(c) * 8);
-    if (st == VDBG_OK) st = dev_alloc(m, &keep, c);
-    if (st == VDBG_OK)
-    {
-      k_section_extract<<<static_cast<unsigned>((static_cast<uint64_t>(c) * 32 + 255) / 256), 256, 0, s>>>(
-        list, count, m->origin, m->values, m->active, blo, bhi, full ? 1 : 0, out_o, out_v, out_m, keep);
-      ho.resize(c);
-      hk.resize(c);
-      if (values) hv.resize(static_cast<size_t>(c) * 512);
-      if (masks) hm.resize(static_cast<size_t>(c) * 8);
-      if (cudaGetLastError() != cudaSuccess ||
-          cudaMemcpyAsync(ho.data(), out_o, c * sizeof(int4), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-          cudaMemcpyAsync(hk.data(), keep, c * sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-          (values && cudaMemcpyAsync(hv.data(), out_v, hv.size() * sizeof(float), cudaMemcpyDeviceToHost, s) !=
-                       cudaSuccess) ||
-          (masks && cudaMemcpyAsync(hm.data(), out_m, hm.size() * sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
-          cudaStreamSynchronize(s) != cudaSuccess)
-        st = VDBG_ERR_CUDA;
-    }
-  }
-  dev_free(m, list, std::min(m->n_leaves, m->capacity));
-  dev_free(m, count, 1);
-  dev_free(m, out_o, c);
-  dev_free(m, out_v, static_cast<size_t>(c) * 512);
-  dev_free(m, out_m, static_cast<size_t>(c) * 8);
-  dev_free(m, keep, c);
-  if (st != VDBG_OK) return st;
-  std::vector<uint32_t> idx;
-  for (uint32_t j = 0; j < c; ++j)
-    if (hk[j]) idx.push_back(j);
-  std::sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) {
-    if (ho[a].x != ho[b].x) return ho[a].x < ho[b].x;
-    if (ho[a].y != ho[b].y) return ho[a].y < ho[b].y;
-    return ho[a].z < ho[b].z;
-  });
-  *n_out = static_cast<int64_t>(idx.size());
-  if (static_cast<int64_t>(idx.size()) > capacity) return VDBG_ERR_BUFFER_TOO_SMALL;
-  for (size_t k = 0; k < idx.size(); ++k)
-  {
-    const uint32_t j = idx[k];
-    if (origins)
-    {
-      origins[3 * k + 0] = ho[j].x;
-      origins[3 * k + 1] = ho[j].y;
-      origins[3 * k + 2] = ho[j].z;
-    }
-    if (values) zmajor_to_vdb(hv.data() + static_cast<size_t>(j) * 512, values + 512 * k);
-    if (masks) mask_to_vdb(hm.data() + static_cast<size_t>(j) * 8, masks + 8 * k);
-  }
-  return VDBG_OK;
+  std::lock_guard<std::mutex> lock(m->work_mutex);
+  const int st = section_export(m, mp, box_corner(lo), box_corner(hi), full ? 1 : 0, capacity, origins, values,
+                                masks, n_out);
+  work_done(m);
+  return st;
 }
 
 int vdbg_test_stall_leaf(vdbg_map* m, int map, int32_t lx, int32_t ly, int32_t lz)
@@ -3167,31 +3213,25 @@ int vdbg_apply_section_states(vdbg_map* m, int map, const int32_t lo[3], const i
   VDBG_CUDA(cudaStreamSynchronize(m->stream));
   VDBG_TRY(reserve_for(m, n));
   cudaStream_t s = m->stream;
-  const int3 blo = make_int3(lo[0], lo[1], lo[2]), bhi = make_int3(hi[0], hi[1], hi[2]);
+  const int3 blo = box_corner(lo), bhi = box_corner(hi);
   std::vector<int4> ho(static_cast<size_t>(n));
-  std::vector<unsigned long long> hm(static_cast<size_t>(n) * 8);
-  for (int64_t i = 0; i < n; ++i)
-  {
-    ho[i] = make_int4(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2], mp);
-    mask_to_vdb(reinterpret_cast<const unsigned long long*>(masks + 8 * i), reinterpret_cast<uint64_t*>(&hm[8 * i]));
-  }
-  uint32_t *list = nullptr, *count = nullptr;
-  int4* d_o      = nullptr;
-  unsigned long long* d_m = nullptr;
-  uint32_t c     = 0;
-  const uint32_t n_list = std::min(m->n_leaves, m->capacity);
-  int st = section_list(m, mp, blo, bhi, &list, &count, &c);
-  if (st == VDBG_OK && n > 0) st = dev_alloc(m, &d_o, static_cast<size_t>(n));
-  if (st == VDBG_OK && n > 0) st = dev_alloc(m, &d_m, static_cast<size_t>(n) * 8);
+  for (int64_t i = 0; i < n; ++i) ho[i] = make_int4(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2], mp);
+  std::lock_guard<std::mutex> lock(m->work_mutex);
+  int* cand  = nullptr;
+  uint32_t c = 0;
+  const size_t k = static_cast<size_t>(n);
+  int st         = section_candidates(m, mp, blo, bhi, &cand, &c);
+  if (st == VDBG_OK) st = work_ensure(m, 1, k * (sizeof(int4) + 8 * sizeof(uint64_t)) + 16);
+  int4* d_o               = reinterpret_cast<int4*>(m->work[1]);
+  unsigned long long* d_m = reinterpret_cast<unsigned long long*>(d_o + k);
   if (st == VDBG_OK && n > 0 &&
-      (cudaMemcpyAsync(d_o, ho.data(), ho.size() * sizeof(int4), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-       cudaMemcpyAsync(d_m, hm.data(), hm.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, s) !=
-         cudaSuccess))
+      (cudaMemcpyAsync(d_o, ho.data(), k * sizeof(int4), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+       cudaMemcpyAsync(d_m, masks, k * 8 * sizeof(uint64_t), cudaMemcpyHostToDevice, s) != cudaSuccess))
     st = VDBG_ERR_CUDA;
   if (st == VDBG_OK) st = begin_call(m, s);
   if (st == VDBG_OK && c > 0)
   {
-    k_section_clear<<<(c * 8 + 255) / 256, 256, 0, s>>>(list, count, m->origin, m->active, blo, bhi);
+    k_section_clear<<<(c * 8 + 255) / 256, 256, 0, s>>>(cand, c, m->origin, m->active, blo, bhi);
     if (cudaGetLastError() != cudaSuccess) st = VDBG_ERR_CUDA;
   }
   if (st == VDBG_OK)
@@ -3199,17 +3239,14 @@ int vdbg_apply_section_states(vdbg_map* m, int map, const int32_t lo[3], const i
     st = run_allocating(m, [&]() -> int {
       if (n > 0)
       {
-        k_section_set_states<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(
+        k_section_set_states<true><<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(
           map_view(m), d_o, d_m, static_cast<uint32_t>(n), mp, m->flags, m->active);
         VDBG_CUDA(cudaGetLastError());
       }
       return VDBG_OK;
     });
   }
-  dev_free(m, list, n_list);
-  dev_free(m, count, 1);
-  dev_free(m, d_o, static_cast<size_t>(n));
-  dev_free(m, d_m, static_cast<size_t>(n) * 8);
+  work_done(m);
   if (st != VDBG_OK) return st;
   return end_call(m, s);
 }

@@ -183,11 +183,16 @@ def _section_export(lib, h, map_index, lo, hi, full, check):
     lo = np.ascontiguousarray(lo, np.int32)
     hi = np.ascontiguousarray(hi, np.int32)
     n = C.c_int64()
-    cap = 0
+    # Room for every leaf cell of the box (one call), unless it is large: then
+    # the first call counts. (Only the rows returned are ever written.)
+    cells = 1
+    for a, b in zip(lo.tolist(), hi.tolist()):
+        cells *= max(0, (b >> 3) - (a >> 3) + 1)
+    cap = cells if cells <= 16384 else 0
     while True:
-        origins = np.zeros((cap, 3), np.int32)
-        values = np.zeros((cap, 512), np.float32)
-        masks = np.zeros((cap, 8), np.uint64)
+        origins = np.empty((cap, 3), np.int32)
+        values = np.empty((cap, 512), np.float32)
+        masks = np.empty((cap, 8), np.uint64)
         s = lib.vdbg_export_section(h, int(map_index), lo.ctypes.data, hi.ctypes.data, 1 if full else 0, cap,
                                     origins.ctypes.data, values.ctypes.data, masks.ctypes.data, C.byref(n))
         if s == _lib.STATUS_CODE["VDBG_ERR_BUFFER_TOO_SMALL"]:
