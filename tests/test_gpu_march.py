@@ -38,3 +38,21 @@ def test_rays_beyond_the_table(vdbg, oracle, res):
                     [-20.1, -3.3, -0.4], [0.02, 16.384, 0.0], [1.0, 3.0, 0.2]], np.float32)
     compare(g, o, pts, (0.0, 0.0, 0.0))
     assert g.mapDigest() == o.mapDigest()
+
+
+@pytest.mark.parametrize("spread, n", [(0.02, 1), (0.5, 40), (60.0, 40), (60.0, 4000)])
+@pytest.mark.parametrize("prob", [(0.7, 0.4, 0.12, 0.97), (0.9, 0.1, 0.49, 0.51), (0.6, 0.45, 0.001, 0.999)])
+def test_sweep_of_few_and_many_leaves(vdbg, oracle, spread, n, prob):
+    """One leaf, few leaves per warp, leaves spread over many blocks, full
+    planes; thresholds inside and outside the clamp limits; repeated scans, so
+    that voxels are clamped and states flip both ways (with the change set)."""
+    cfg = ref_config(max_range=80.0)
+    cfg.prob_hit, cfg.prob_miss, cfg.prob_thres_min, cfg.prob_thres_max = prob
+    g, o = pair(vdbg, oracle, 0.2, cfg)
+    g.trackChanges()
+    rng = np.random.default_rng(n)
+    base = (rng.normal(size=(n, 3)) * spread * [1.0, 1.0, 0.2]).astype(np.float32)
+    for k in range(14):
+        pts = base if k < 7 else base * np.float32(1.5)  # first hit, then passed through
+        compare(g, o, np.ascontiguousarray(pts), (0.05, 0.05, 0.05))
+    assert_same_map(g.exportLeaves(), o.exportLeaves(), f"{n} points, spread {spread}")

@@ -29,7 +29,7 @@
 //   btouched u64[PB][8]  leaf cells of the block touched in the current window
 //   bepoch   u32[PB]     window in which the block was last touched
 //   blist    i32[PB]     blocks touched in the current window (n_blist)
-//   touched  i32[P]      leaves touched in the window, compacted before the sweep
+//   touched  i32[P]      leaves touched in the window (listed when a marking is dropped)
 #pragma once
 
 #include <cstdint>
@@ -461,31 +461,6 @@ __device__ __forceinline__ bool world_to_index_axis(double w, const ScanGeom& g,
   if (!(f >= kVoxelMin && f < kVoxelMaxExcl)) return false;
   out = static_cast<int>(f);
   return true;
-}
-
-// OpenVDB log-odds node updates (OccupancyVDBMapping.hpp:92-117): FP32 add,
-// clamp only inside the threshold branch; a hit never deactivates, a miss
-// never activates.
-__device__ __forceinline__ void apply_update(float& v, bool& on, bool hit, const LogOdds& lo)
-{
-  if (hit)
-  {
-    v = __fadd_rn(v, lo.hit);
-    if (v > lo.thres_max)
-    {
-      on = true;
-      if (v > lo.max) v = lo.max;
-    }
-  }
-  else
-  {
-    v = __fadd_rn(v, lo.miss);
-    if (v < lo.thres_min)
-    {
-      on = false;
-      if (v < lo.min) v = lo.min;
-    }
-  }
 }
 
 } // namespace vdbg

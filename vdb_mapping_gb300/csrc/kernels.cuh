@@ -11,6 +11,7 @@
 //                                       into the per-leaf update masks
 //   k_mark_hits VDBMapping.hpp:533-536  hit bits of unclipped endpoints
 //   k_compact  (none)                   touched blocks -> flat touched-leaf list
+//                                       (a dropped marking)
 //   k_sweep    VDBMapping.hpp:731-792 + per touched leaf: FP32 log-odds update,
 //              OccupancyVDBMapping.hpp:92-117  thresholds, clamp, active mask;
 //                                       clears the update masks
@@ -878,332 +879,325 @@ __global__ void __launch_bounds__(256) k_mark_hits(const int4* __restrict__ rays
   atomicOr(c.upd + static_cast<size_t>(slot) * 16 + 8 + (off >> 6), 1ull << (off & 63));
 }
 
-// Persistent sweep over the touched leaves, in two stages per warp. Finding:
-// 8 lanes per leaf, lane w reading the update words of the z-plane w (voxel
-// offsets 64w..64w+63, one word of each mask) of four leaves at once; the
-// planes holding update bits go to the warp's queue in shared memory (most
-// planes of a touched leaf hold none). Applying: once 32 planes are queued,
-// each lane takes one, loads the float4 groups with update bits (all loads
-// issued before any use), applies the log-odds rules, stores them back and
-// clears the plane's update words; so every lane of the warp has a plane.
+// Persistent sweep over the window's touched leaves (VDBMapping.hpp:731-792,
+// OccupancyVDBMapping.hpp:92-117), each warp by itself, in three stages.
+// Leaves: a lane takes a byte of a block's touched cells (eight cells), which
+// gives leaf slots; neighbouring bytes go to different warps, and to as many
+// as there are, because the blocks around the sensor are full and most others
+// are not. Planes: up to eight leaves at a time, two
+// planes per lane; a leaf's update and active words are read side by side, its
+// update words cleared, and every 16-byte group of values (four voxels) with
+// an update bit goes to the warp's list. Values: one lane per group, four
+// groups per lane loaded before the first is used; the log-odds rules, the
+// store, and an atomic on the active word where a voxel's state flipped (few
+// do). So every lane has a group whatever the planes hold, and neighbouring
+// lanes take neighbouring groups of a plane.
+//
+// It is bound by the latency of its loads (DRAM is about half busy). Measured
+// on one GB300 against a compaction kernel and a sweep of one plane per lane
+// (eight lanes per plane for batches): street scan, 1.48M leaves with 42
+// updates each, 0.46 ms (0.53); 32 maps, 6.3M leaves with 51, 1.9 ms (2.8);
+// random long rays, 4.5M leaves with 9, 1.23 ms (1.46); 2,048 points, 3,400
+// leaves, 0.016 ms (0.030).
+//
 // kPerMap: the pool holds a batch of maps, each leaf takes its map's log-odds
-// constants (else the one map's, kept in registers). kChanges: record the
-// change set (every touched word, and the leaves with a flip).
-struct SweepTask
+// constants. kChanges: record the change set (every touched word, and the
+// leaves with a flip).
+constexpr int kSweepWarps  = 4;                // per block
+constexpr int kSweepBlocks = 7;                // per SM (70 registers; 6 and 8 were 0-4% slower)
+constexpr int kSweepLeaves = 8;                // leaves whose planes are handled together
+constexpr int kSweepQueue  = 32 * 8 + kSweepLeaves;
+constexpr int kSweepAhead  = 4;                // groups a lane loads ahead (2: 1% slower, 8: 15%)
+
+struct SweepWarp
 {
-  unsigned long long actw, hitw;  // visited-or-hit and hit bits of the plane
-  int slot;                       // leaf slot
-  short w;                        // plane
-  short map;                      // the leaf's map (a pool of several maps)
+  unsigned long long act[kSweepLeaves * 8];  // visited-or-hit bits of a plane
+  unsigned long long hit[kSweepLeaves * 8];
+  unsigned long long on[kSweepLeaves * 8];   // active word before the sweep
+  int leaves[kSweepQueue];                   // leaf slots found
+  int slot[kSweepLeaves];                    // the leaves in hand
+  int map[kSweepLeaves];
+  unsigned short groups[kSweepLeaves * 128];  // plane << 4 | quad
 };
-constexpr int kSweepQueue = 64;  // per-warp ring: up to 31 left over + 32 found
 
-template <bool kPerMap, bool kChanges>
-__device__ __forceinline__ unsigned long long sweep_plane(const SweepTask& k, ChannelView& c, float* values,
-                                                          unsigned long long* active, const int4* origin,
-                                                          const LogOddsTable& lt, const ChangeView& ch)
+// Exclusive scan over the warp; *total receives the sum.
+__device__ __forceinline__ uint32_t warp_scan_exclusive(uint32_t v, int lane, uint32_t* total)
 {
-  const unsigned long long actw = k.actw, hitw = k.hitw;
-  const int slot = k.slot, w = k.w;
-  const LogOdds lo               = kPerMap ? lt.table[k.map] : lt.lo0;
-  unsigned long long* aw         = active + static_cast<size_t>(slot) * 8 + w;
-  const unsigned long long on_in = *aw;
-  unsigned long long on          = on_in;
-  float4* vp = reinterpret_cast<float4*>(values + static_cast<size_t>(slot) * 512 + w * 64);
+  uint32_t inc = v;
 #pragma unroll
-  for (int half = 0; half < 2; ++half)
+  for (int off = 1; off < 32; off <<= 1)
   {
-    float4 v[8];
-#pragma unroll
-    for (int k4 = 0; k4 < 8; ++k4)
-    {
-      const int qd = half * 8 + k4;
-      if ((actw >> (4 * qd)) & 0xfull) v[k4] = vp[plane_quad(qd)];
-    }
-#pragma unroll
-    for (int k4 = 0; k4 < 8; ++k4)
-    {
-      const int qd      = half * 8 + k4;
-      const uint32_t a4 = static_cast<uint32_t>(actw >> (4 * qd)) & 0xfu;
-      if (!a4) continue;
-      const uint32_t h4 = static_cast<uint32_t>(hitw >> (4 * qd)) & 0xfu;
-      float vv[4]       = {v[k4].x, v[k4].y, v[k4].z, v[k4].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-      {
-        if ((a4 >> j) & 1u)
-        {
-          const int bit = 4 * qd + j;
-          bool o        = (on >> bit) & 1ull;
-          apply_update(vv[j], o, (h4 >> j) & 1u, lo);
-          on = o ? (on | (1ull << bit)) : (on & ~(1ull << bit));
-        }
-      }
-      vp[plane_quad(qd)] = make_float4(vv[0], vv[1], vv[2], vv[3]);
-    }
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += y;
   }
-  if (on != on_in) *aw = on;
-  unsigned long long* u = c.upd + static_cast<size_t>(slot) * 16;
-  u[w]                  = 0ull;
-  if (hitw) u[8 + w] = 0ull;
-  if (kChanges)
-  {
-    // A hit only turns voxels on and a miss only off, so the flipped bits
-    // that are now on are the hits of VDBMapping.hpp:768-772.
-    const unsigned long long flip                   = on ^ on_in;
-    ch.words[static_cast<size_t>(slot) * 16 + w]     = flip;
-    ch.words[static_cast<size_t>(slot) * 16 + 8 + w] = flip & on;
-    if (flip && atomicExch(ch.epoch + slot, ch.cur) != ch.cur) ch.list[atomicAdd(ch.count, 1u)] = slot;
-  }
-  return static_cast<unsigned long long>(__popcll(actw));
+  *total = __shfl_sync(0xffffffffu, inc, 31);
+  return inc - v;
+}
+
+// The four bits of group `quad` in a plane's word held in shared memory.
+__device__ __forceinline__ uint32_t group_bits(const unsigned long long* word, int quad)
+{
+  const uint32_t half = reinterpret_cast<const uint32_t*>(word)[quad >> 3];
+  return (half >> (4 * (quad & 7))) & 0xfu;
+}
+
+// The log-odds node update (OccupancyVDBMapping.hpp:92-117) without branches:
+// FP32 add, clamp only past the threshold; a hit never deactivates, a miss
+// never activates. A value is clamped when it passes both the threshold and
+// the limit: `past_max` / `past_min` are the outer of the two.
+struct SweepOdds
+{
+  LogOdds lo;
+  float past_max, past_min;
+};
+
+__device__ __forceinline__ SweepOdds sweep_odds(const LogOdds& lo)
+{
+  // (a threshold that is NaN is never passed)
+  return SweepOdds{lo, lo.thres_max <= lo.max ? lo.max : lo.thres_max, lo.thres_min >= lo.min ? lo.min : lo.thres_min};
+}
+
+// One voxel: `act`, `hit` its update bits, `bit` its place in the group's
+// states `on`.
+__device__ __forceinline__ float update_voxel(float v, uint32_t act, uint32_t hit, uint32_t bit, const SweepOdds& o,
+                                              uint32_t& on)
+{
+  const float x = __fadd_rn(v, hit ? o.lo.hit : o.lo.miss);
+  if (act && (hit ? x > o.lo.thres_max : x < o.lo.thres_min)) on = hit ? on | bit : on & ~bit;
+  const bool clip = hit ? x > o.past_max : x < o.past_min;
+  return act ? (clip ? (hit ? o.lo.max : o.lo.min) : x) : v;
+}
+
+// The same for a miss.
+__device__ __forceinline__ float update_missed(float v, uint32_t act, uint32_t bit, const SweepOdds& o, uint32_t& on)
+{
+  const float x = __fadd_rn(v, o.lo.miss);
+  if (act && x < o.lo.thres_min) on &= ~bit;
+  return act ? (x < o.past_min ? o.lo.min : x) : v;
+}
+
+// Bit q set where nibble q of x holds a bit.
+__device__ __forceinline__ uint32_t nibbles(unsigned long long x)
+{
+  auto half = [](uint32_t y) {
+    y |= y >> 1;
+    y |= y >> 2;
+    y &= 0x11111111u;        // bits 0, 4, .., 28
+    y = (y | (y >> 3)) & 0x03030303u;
+    y = (y | (y >> 6)) & 0x000f000fu;
+    return (y | (y >> 12)) & 0xffu;
+  };
+  return half(static_cast<uint32_t>(x)) | (half(static_cast<uint32_t>(x >> 32)) << 8);
 }
 
 template <bool kPerMap, bool kChanges>
-__global__ void __launch_bounds__(256, 4) k_sweep(ChannelView c, float* __restrict__ values,
-                                                  unsigned long long* __restrict__ active,
-                                                  uint32_t* __restrict__ flags, const int4* __restrict__ origin,
-                                                  LogOddsTable lt, ChangeView ch, DevStatus* st, int gated)
+__global__ void __launch_bounds__(kSweepWarps * 32, kSweepBlocks)
+  k_sweep(MapView m, ChannelView c, float* __restrict__ values, unsigned long long* __restrict__ active,
+          uint32_t* __restrict__ flags, LogOddsTable lt, int n_maps, ChangeView ch, DevStatus* st, int gated)
 {
   if (gated ? !marking_complete(st) : ld_relaxed_u32(&st->error) != 0u) return;
-  __shared__ SweepTask queue[8][kSweepQueue];
-  SweepTask* q        = queue[threadIdx.x >> 5];
-  const uint32_t nt   = *c.n_touched;
+  __shared__ SweepWarp warps[kSweepWarps];
+  __shared__ SweepOdds odds[kPerMap ? kMaxMaps : 1];
+  SweepWarp& q        = warps[threadIdx.x >> 5];
   const int lane      = static_cast<int>(threadIdx.x & 31);
-  const uint32_t lt_m = lanemask_lt();
   const int w         = lane & 7;
   const uint32_t grp  = static_cast<uint32_t>(lane >> 3);
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw   = (gridDim.x * blockDim.x) >> 5;
-  unsigned long long n_upd = 0;
-  uint32_t head = 0, tail = 0;  // queued planes: [head, tail) modulo kSweepQueue
-  for (uint32_t base = warp * 4;; base += nw * 4)
+  if (kPerMap)
   {
-    const bool more = base < nt;  // warp-uniform
-    if (more)
-    {
-      const uint32_t i             = base + grp;
-      unsigned long long actw      = 0ull, hitw = 0ull;
-      int slot                     = 0;
-      int map                      = 0;
-      if (i < nt)
-      {
-        slot = c.touched[i];
-        if (kPerMap && w == 0) map = origin[slot].w;  // once per leaf
-        // Mark the leaf as part of the map the first time it is swept (every
-        // touched leaf carries at least one update bit).
-        if (w == 0 && ld_ca_u32(flags + slot) == 0u) flags[slot] = 1u;
-        const unsigned long long* u = c.upd + static_cast<size_t>(slot) * 16;
-        hitw                        = u[8 + w];
-        actw                        = u[w] | hitw;
-        if (kChanges && actw == 0ull)
-        {
-          ch.words[static_cast<size_t>(slot) * 16 + w]     = 0ull;
-          ch.words[static_cast<size_t>(slot) * 16 + 8 + w] = 0ull;
-        }
-      }
-      if (kPerMap) map = __shfl_sync(0xffffffffu, map, lane & ~7);
-      const bool act    = actw != 0ull;
-      const unsigned am = __ballot_sync(0xffffffffu, act);
-      if (act)
-      {
-        SweepTask& k = q[(tail + static_cast<uint32_t>(__popc(am & lt_m))) % kSweepQueue];
-        k.actw       = actw;
-        k.hitw       = hitw;
-        k.slot       = slot;
-        k.w          = static_cast<short>(w);
-        k.map        = static_cast<short>(map);
-      }
-      tail += static_cast<uint32_t>(__popc(am));
-      __syncwarp();
-    }
-    while (tail - head >= 32u || (!more && tail != head))
-    {
-      const uint32_t n = min(32u, tail - head);
-      if (static_cast<uint32_t>(lane) < n)
-      {
-        const SweepTask k = q[(head + static_cast<uint32_t>(lane)) % kSweepQueue];
-        n_upd += sweep_plane<kPerMap, kChanges>(k, c, values, active, origin, lt, ch);
-      }
-      head += n;
-      __syncwarp();
-    }
-    if (!more) break;
+    for (int i = static_cast<int>(threadIdx.x); i < n_maps; i += kSweepWarps * 32) odds[i] = sweep_odds(lt.table[i]);
+    __syncthreads();
   }
-  for (int off = 16; off > 0; off >>= 1) n_upd += __shfl_xor_sync(0xffffffffu, n_upd, off);
-  if (lane == 0 && n_upd) atomicAdd(&st->updates, n_upd);
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->touched, nt);
-}
-
-// Grouped sweep, for maps whose touched planes hold few updates: the same
-// finding stage and per-voxel rules as k_sweep, but eight lanes apply one
-// plane: lane `sub` of the group holds the 16-byte groups at positions sub
-// and sub + 8 of the plane (two planes per group at a time), so a warp's
-// loads and stores of four planes are four contiguous 128-byte runs
-// instead of 32 scattered groups. The new active word is the OR of the
-// group's lanes. On the batched workload's planes (about 20 updates per
-// touched leaf) it takes 10% less time than k_sweep; on dense planes (about
-// 40) k_sweep, which keeps twice the loads in flight, is faster, and on very
-// sparse ones (about 9, one update per plane) its per-plane overhead makes
-// it slower too. The host picks by the update density of the previous sweep.
-__device__ __forceinline__ int quad_at(int pos)  // inverse of plane_quad
-{
-  return (pos & 8) | (((pos >> 1) & 1) << 2) | ((pos & 1) << 1) | ((pos >> 2) & 1);
-}
-
-template <bool kPerMap, bool kChanges>
-__global__ void __launch_bounds__(256, 3) k_sweep_grouped(ChannelView c, float* __restrict__ values,
-                                                          unsigned long long* __restrict__ active,
-                                                          uint32_t* __restrict__ flags,
-                                                          const int4* __restrict__ origin, LogOddsTable lt,
-                                                          ChangeView ch, DevStatus* st, int gated)
-{
-  constexpr int kUnroll = 2;
-  if (gated ? !marking_complete(st) : ld_relaxed_u32(&st->error) != 0u) return;
-  __shared__ SweepTask queue[8][kSweepQueue];
-  SweepTask* q        = queue[threadIdx.x >> 5];
-  const uint32_t nt   = *c.n_touched;
-  const int lane      = static_cast<int>(threadIdx.x & 31);
-  const uint32_t lt_m = lanemask_lt();
-  const int w         = lane & 7;
-  const uint32_t grp  = static_cast<uint32_t>(lane >> 3);
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw   = (gridDim.x * blockDim.x) >> 5;
-  const int sub       = lane & 7;
-  const int qa = quad_at(sub), qb = quad_at(sub + 8);
-  constexpr uint32_t kTake = 4u * kUnroll;
+  const SweepOdds odds0 = sweep_odds(lt.lo0);
+  // Byte i of the window's touched cells goes to warp i % nw; a warp looks at
+  // `lanes` of its bytes at a time.
+  const uint64_t bytes = *c.n_blist * 64ull;
+  const uint32_t lanes = bytes >= 32ull * nw ? 32u : max(static_cast<uint32_t>(bytes) / nw, 1u);
+  uint64_t next        = warp;
+  uint32_t n = 0, head = 0;  // leaves found, and handled, of q.leaves
+  uint32_t n_touched = 0;
   unsigned long long n_upd = 0;
-  uint32_t head = 0, tail = 0;  // queued planes: [head, tail) modulo kSweepQueue
-  for (uint32_t base = warp * 4;; base += nw * 4)
-  {
-    const bool more = base < nt;  // warp-uniform
-    if (more)
+  // The words of the batch that follows the one in hand, loaded ahead of its
+  // values so that the two latencies overlap (lane: planes w of leaves grp and
+  // grp + 4).
+  unsigned long long vis[2], hit[2], on[2];
+  int slot[2], map[2];
+  uint32_t flag[2], take = 0;
+  auto load_batch = [&]() {
+    // ---- leaves ------------------------------------------------------------
+    while (n - head < static_cast<uint32_t>(kSweepLeaves) && next < bytes)
     {
-      const uint32_t i        = base + grp;
-      unsigned long long actw = 0ull, hitw = 0ull;
-      int slot                = 0;
-      int map                 = 0;
-      if (i < nt)
+      if (head > 0)
       {
-        slot = c.touched[i];
-        if (kPerMap && w == 0) map = origin[slot].w;  // once per leaf
-        if (w == 0 && ld_ca_u32(flags + slot) == 0u) flags[slot] = 1u;
-        const unsigned long long* u = c.upd + static_cast<size_t>(slot) * 16;
-        hitw                        = u[8 + w];
-        actw                        = u[w] | hitw;
-        if (kChanges && actw == 0ull)
+        // (fewer than eight are left: to the front)
+        const int keep = head + lane < n ? q.leaves[head + lane] : -1;
+        __syncwarp();
+        if (keep >= 0) q.leaves[lane] = keep;
+        n -= head;
+        head = 0;
+      }
+      const uint64_t t = next + static_cast<uint64_t>(lane) * nw;
+      next += static_cast<uint64_t>(lanes) * nw;
+      uint32_t bits = 0;
+      int4 s0{}, s1{};
+      if (static_cast<uint32_t>(lane) < lanes && t < bytes)
+      {
+        const int b         = c.blist[t >> 6];
+        const uint32_t i    = static_cast<uint32_t>(t) & 63u;  // cells 8i .. 8i + 7
+        unsigned char* mark = reinterpret_cast<unsigned char*>(c.btouched + static_cast<size_t>(b) * 8) + i;
+        bits                = *mark;
+        if (bits)
         {
-          ch.words[static_cast<size_t>(slot) * 16 + w]     = 0ull;
-          ch.words[static_cast<size_t>(slot) * 16 + 8 + w] = 0ull;
+          *mark             = 0;
+          const int4* cells = reinterpret_cast<const int4*>(m.bleaf + static_cast<size_t>(b) * 512 + i * 8u);
+          s0                = cells[0];
+          s1                = cells[1];
         }
       }
-      if (kPerMap) map = __shfl_sync(0xffffffffu, map, lane & ~7);
-      const bool act    = actw != 0ull;
-      const unsigned am = __ballot_sync(0xffffffffu, act);
-      if (act)
-      {
-        SweepTask& k = q[(tail + static_cast<uint32_t>(__popc(am & lt_m))) % kSweepQueue];
-        k.actw       = actw;
-        k.hitw       = hitw;
-        k.slot       = slot;
-        k.w          = static_cast<short>(w);
-        k.map        = static_cast<short>(map);
-      }
-      tail += static_cast<uint32_t>(__popc(am));
+      uint32_t found = 0;
+      uint32_t at    = n + warp_scan_exclusive(static_cast<uint32_t>(__popc(bits)), lane, &found);
+      const int s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if ((bits >> k) & 1u) q.leaves[at++] = s[k];
+      n += found;
+      n_touched += found;
       __syncwarp();
     }
-    while (tail - head >= kTake || (!more && tail != head))
-    {
-      const uint32_t n = min(kTake, tail - head);
-      SweepTask k[kUnroll];
-      float4 va[kUnroll], vb[kUnroll];
-      unsigned long long on_in[kUnroll];
+    take = min(n - head, static_cast<uint32_t>(kSweepLeaves));
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u)
+    for (int k = 0; k < 2; ++k)
+    {
+      const uint32_t i = static_cast<uint32_t>(k) * 4u + grp;
+      vis[k] = hit[k] = on[k] = 0ull;
+      slot[k]                 = -1;
+      if (i < take)
       {
-        const uint32_t idx = static_cast<uint32_t>(u) * 4u + grp;
-        if (idx < n)
+        slot[k]                     = q.leaves[head + i];
+        const unsigned long long* u = c.upd + static_cast<size_t>(slot[k]) * 16;
+        vis[k]                      = u[w];
+        hit[k]                      = u[8 + w];
+        on[k]                       = active[static_cast<size_t>(slot[k]) * 8 + w];
+        if (w == 0)
         {
-          k[u] = q[(head + idx) % kSweepQueue];
+          flag[k] = flags[slot[k]];
+          if (kPerMap) map[k] = m.origin[slot[k]].w;
+        }
+      }
+    }
+    head += take;
+  };
+  load_batch();
+  while (take)
+  {
+    // ---- planes ------------------------------------------------------------
+    uint32_t held = 0;  // groups with an update bit: 16 bits per plane
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      const uint32_t i             = static_cast<uint32_t>(k) * 4u + grp;
+      const uint32_t p             = i * 8u + static_cast<uint32_t>(w);
+      const unsigned long long act = vis[k] | hit[k];
+      if (slot[k] >= 0)
+      {
+        unsigned long long* u = c.upd + static_cast<size_t>(slot[k]) * 16;
+        q.act[p]              = act;
+        q.hit[p]              = hit[k];
+        q.on[p]               = on[k];
+        if (vis[k]) u[w] = 0ull;
+        if (hit[k]) u[8 + w] = 0ull;
+        if (kChanges)
+        {
+          ch.words[static_cast<size_t>(slot[k]) * 16 + w]     = 0ull;
+          ch.words[static_cast<size_t>(slot[k]) * 16 + 8 + w] = 0ull;
+        }
+        if (w == 0)
+        {
+          q.slot[i] = slot[k];
+          if (kPerMap) q.map[i] = map[k];
+          // Part of the map from the first time it is swept on (every touched
+          // leaf carries at least one update bit).
+          if (flag[k] == 0u) flags[slot[k]] = 1u;
+        }
+      }
+      n_upd += static_cast<uint32_t>(__popcll(act));
+      held |= nibbles(act) << (16 * k);
+    }
+    uint32_t n_groups = 0;
+    uint32_t at       = warp_scan_exclusive(static_cast<uint32_t>(__popc(held)), lane, &n_groups);
+    // (bit 16k + q of `held` is group q of plane 32k + lane)
+    for (uint32_t z = held; z; z &= z - 1u)
+    {
+      const uint32_t f = static_cast<uint32_t>(__ffs(static_cast<int>(z)) - 1);
+      q.groups[at++]   = static_cast<unsigned short>(((f & 16u) << 5) | (static_cast<uint32_t>(lane) << 4) | (f & 15u));
+    }
+    __syncwarp();
+    load_batch();
+    // ---- values ------------------------------------------------------------
+    for (uint32_t g0 = 0; g0 < n_groups; g0 += 32u * kSweepAhead)
+    {
+      float4 v[kSweepAhead];
+      uint32_t e[kSweepAhead];
+      auto at_group = [&](uint32_t x) {
+        const uint32_t p = x >> 4;
+        return reinterpret_cast<float4*>(values + static_cast<size_t>(q.slot[p >> 3]) * 512 + (p & 7u) * 64u) +
+               plane_quad(static_cast<int>(x & 15u));
+      };
+#pragma unroll
+      for (int k = 0; k < kSweepAhead; ++k)
+      {
+        const uint32_t g = g0 + static_cast<uint32_t>(k) * 32u + static_cast<uint32_t>(lane);
+        e[k]             = g < n_groups ? q.groups[g] : 0xffffffffu;
+        if (e[k] != 0xffffffffu) v[k] = *at_group(e[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < kSweepAhead; ++k)
+      {
+        if (e[k] == 0xffffffffu) continue;
+        const uint32_t p  = e[k] >> 4;
+        const int quad    = static_cast<int>(e[k] & 15u);
+        const SweepOdds& o = kPerMap ? odds[q.map[p >> 3]] : odds0;
+        const uint32_t a4 = group_bits(&q.act[p], quad), h4 = group_bits(&q.hit[p], quad), o4 = group_bits(&q.on[p], quad);
+        uint32_t n4       = o4;
+        if (h4)
+        {
+          v[k].x = update_voxel(v[k].x, a4 & 1u, h4 & 1u, 1u, o, n4);
+          v[k].y = update_voxel(v[k].y, a4 & 2u, h4 & 2u, 2u, o, n4);
+          v[k].z = update_voxel(v[k].z, a4 & 4u, h4 & 4u, 4u, o, n4);
+          v[k].w = update_voxel(v[k].w, a4 & 8u, h4 & 8u, 8u, o, n4);
         }
         else
         {
-          k[u].actw = 0ull;
-          k[u].hitw = 0ull;
-          k[u].slot = 0;
-          k[u].w    = 0;
-          k[u].map  = 0;
+          v[k].x = update_missed(v[k].x, a4 & 1u, 1u, o, n4);
+          v[k].y = update_missed(v[k].y, a4 & 2u, 2u, o, n4);
+          v[k].z = update_missed(v[k].z, a4 & 4u, 4u, o, n4);
+          v[k].w = update_missed(v[k].w, a4 & 8u, 8u, o, n4);
         }
-        const float4* vp =
-          reinterpret_cast<const float4*>(values + static_cast<size_t>(k[u].slot) * 512 + k[u].w * 64);
-        if ((k[u].actw >> (4 * qa)) & 0xfull) va[u] = vp[sub];
-        if ((k[u].actw >> (4 * qb)) & 0xfull) vb[u] = vp[sub + 8];
-        on_in[u] = idx < n ? active[static_cast<size_t>(k[u].slot) * 8 + k[u].w] : 0ull;
-      }
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u)
-      {
-        const uint32_t idx            = static_cast<uint32_t>(u) * 4u + grp;
-        const LogOdds lo              = kPerMap ? lt.table[k[u].map] : lt.lo0;
-        const unsigned long long actw = k[u].actw, hitw = k[u].hitw;
-        unsigned long long mine       = 0ull;
-        float4* vp = reinterpret_cast<float4*>(values + static_cast<size_t>(k[u].slot) * 512 + k[u].w * 64);
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
+        *at_group(e[k])   = v[k];
+        const uint32_t flip = n4 ^ o4;
+        if (flip)
         {
-          const int qd      = half ? qb : qa;
-          const uint32_t a4 = static_cast<uint32_t>(actw >> (4 * qd)) & 0xfu;
-          if (!a4) continue;
-          const uint32_t h4 = static_cast<uint32_t>(hitw >> (4 * qd)) & 0xfu;
-          const float4 v4   = half ? vb[u] : va[u];
-          float vv[4]       = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-          {
-            if ((a4 >> j) & 1u)
-            {
-              const int bit = 4 * qd + j;
-              bool o        = (on_in[u] >> bit) & 1ull;
-              apply_update(vv[j], o, (h4 >> j) & 1u, lo);
-              if (o) mine |= 1ull << bit;
-            }
-          }
-          vp[half ? sub + 8 : sub] = make_float4(vv[0], vv[1], vv[2], vv[3]);
-        }
-        // The group's new bits (each lane holds its own eight voxels).
-        uint32_t mlo = static_cast<uint32_t>(mine), mhi = static_cast<uint32_t>(mine >> 32);
-#pragma unroll
-        for (int off = 1; off < 8; off <<= 1)
-        {
-          mlo |= __shfl_xor_sync(0xffffffffu, mlo, off);
-          mhi |= __shfl_xor_sync(0xffffffffu, mhi, off);
-        }
-        if (sub == 0 && idx < n)
-        {
-          const int slot = k[u].slot, pw = k[u].w;
-          const unsigned long long on =
-            (on_in[u] & ~actw) | ((static_cast<unsigned long long>(mhi) << 32) | mlo);
-          if (on != on_in[u]) active[static_cast<size_t>(slot) * 8 + pw] = on;
-          unsigned long long* up = c.upd + static_cast<size_t>(slot) * 16;
-          up[pw]                 = 0ull;
-          if (hitw) up[8 + pw] = 0ull;
+          const int leaf = q.slot[p >> 3];
+          atomicXor(active + static_cast<size_t>(leaf) * 8 + (p & 7u), static_cast<unsigned long long>(flip) << (4 * quad));
           if (kChanges)
           {
-            const unsigned long long flip                    = on ^ on_in[u];
-            ch.words[static_cast<size_t>(slot) * 16 + pw]     = flip;
-            ch.words[static_cast<size_t>(slot) * 16 + 8 + pw] = flip & on;
-            if (flip && atomicExch(ch.epoch + slot, ch.cur) != ch.cur) ch.list[atomicAdd(ch.count, 1u)] = slot;
+            // A hit only turns voxels on and a miss only off, so the flipped
+            // bits that are now on are the hits of VDBMapping.hpp:768-772.
+            unsigned long long* cw = ch.words + static_cast<size_t>(leaf) * 16 + (p & 7u);
+            atomicOr(cw, static_cast<unsigned long long>(flip) << (4 * quad));
+            if (flip & n4) atomicOr(cw + 8, static_cast<unsigned long long>(flip & n4) << (4 * quad));
+            if (atomicExch(ch.epoch + leaf, ch.cur) != ch.cur) ch.list[atomicAdd(ch.count, 1u)] = leaf;
           }
-          n_upd += static_cast<unsigned long long>(__popcll(actw));
         }
       }
-      head += n;
-      __syncwarp();
     }
-    if (!more) break;
+    __syncwarp();
   }
   for (int off = 16; off > 0; off >>= 1) n_upd += __shfl_xor_sync(0xffffffffu, n_upd, off);
   if (lane == 0 && n_upd) atomicAdd(&st->updates, n_upd);
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->touched, nt);
+  if (lane == 0 && n_touched) atomicAdd(&st->touched, n_touched);
 }
 
 // Gathers the listed change leaves of map `map` (-1: all): origin and the 16
@@ -1222,16 +1216,12 @@ __global__ void k_gather_changes(ChangeView ch, const int4* __restrict__ origin,
   for (int w = 0; w < 16; ++w) out_w[static_cast<size_t>(j) * 16 + w] = ch.words[static_cast<size_t>(slot) * 16 + w];
 }
 
-// Turns the touched-block list of a window into the flat list of touched
-// leaves the sweep walks, clearing the blocks' touched bits. One warp per
-// block, one lane per 64-cell word. `force` runs it while an error is set
-// (to undo a partial marking).
-// `mode`: 0 skips on an error, 1 (a dropped marking) always runs, 2 (a
-// captured step) skips unless the marking is complete.
-__global__ void __launch_bounds__(256) k_compact(MapView m, ChannelView c, DevStatus* st, int mode)
+// Turns the touched-block list of a window into the flat list of its touched
+// leaves, clearing the blocks' touched bits (a marking that is dropped: the
+// sweep finds its leaves itself). One warp per block, one lane per 64-cell
+// word.
+__global__ void __launch_bounds__(256) k_compact(MapView m, ChannelView c)
 {
-  if (mode == 0 && ld_relaxed_u32(&st->error) != 0u) return;
-  if (mode == 2 && !marking_complete(st)) return;
   const uint32_t nb   = *c.n_blist;
   const int lane      = static_cast<int>(threadIdx.x & 31);
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1241,21 +1231,15 @@ __global__ void __launch_bounds__(256) k_compact(MapView m, ChannelView c, DevSt
     const int b                 = c.blist[i];
     unsigned long long* tw      = c.btouched + static_cast<size_t>(b) * 8;
     const unsigned long long w  = lane < 8 ? tw[lane] : 0ull;
-    const uint32_t cnt          = static_cast<uint32_t>(__popcll(w));
-    uint32_t incl               = cnt;
-    for (int off = 1; off < 8; off <<= 1)
-    {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += y;
-    }
-    uint32_t base = 0;
-    if (lane == 7) base = atomicAdd(c.n_touched, incl);
-    base = __shfl_sync(0xffffffffu, base, 7) + incl - cnt;
-    if (lane < 8 && w)
+    uint32_t total              = 0;
+    uint32_t at                 = warp_scan_exclusive(static_cast<uint32_t>(__popcll(w)), lane, &total);
+    uint32_t base               = 0;
+    if (lane == 0) base = atomicAdd(c.n_touched, total);
+    at += __shfl_sync(0xffffffffu, base, 0);
+    if (w)
     {
       const int* cells = m.bleaf + static_cast<size_t>(b) * 512 + lane * 64;
-      uint32_t k       = 0;
-      for (unsigned long long z = w; z; z &= z - 1) c.touched[base + k++] = cells[__ffsll(z) - 1];
+      for (unsigned long long z = w; z; z &= z - 1) c.touched[at++] = cells[__ffsll(z) - 1];
       tw[lane] = 0ull;
     }
   }

@@ -176,12 +176,6 @@ struct vdbg_map
   bool use_graph                   = true;
   cudaGraphExec_t graph            = nullptr;
   uint64_t graph_layout            = 0;
-  bool graph_grouped               = false;  // the sweep kernel the captured step holds
-  // Sweep kernel choice by the update density (updated voxels per touched
-  // leaf) of the previous sweep: k_sweep_grouped inside a band of medium
-  // densities, k_sweep outside it (the band's edges have gaps, so the
-  // choice does not flip between steps of similar scans).
-  bool sweep_grouped               = false;
   const char** d_pts_ref           = nullptr;  // the step's points address (batch), read by k_prep
   const char** h_pts_ref           = nullptr;  // pinned staging
   int64_t graph_stride             = 0;
@@ -226,8 +220,6 @@ namespace {
 
 constexpr uint32_t kDefaultCapacity = 1u << 16;
 constexpr uint32_t kMinBlocks       = 1u << 10;
-constexpr int kSweepBlocks          = 152 * 8;
-constexpr int kSweepThreads         = 256;
 constexpr size_t kWorkKept          = size_t(64) << 20;
 constexpr int64_t kSectionCells     = int64_t(1) << 20;  // boxes of more leaf cells list the map's leaves
 
@@ -711,39 +703,9 @@ void fill_stats(vdbg_map* m, uint32_t leaves_before, vdbg_scan_stats* st)
   st->device_ms = m->timings.total_ms;
 }
 
-// The sweep kernel of the map's next sweep (the tuning may fix it). By
-// default the grouped sweep is picked for batches of maps only, where it was
-// measured faster inside the density band; on single maps it was measured
-// slower at 26 updates per touched leaf (a dense street scan at a quarter of
-// its rays: 384 against 255 us under ncu), so updates per leaf do not
-// predict it there.
-bool use_grouped_sweep(const vdbg_map* m)
-{
-  if (m->tuning.sweep_kernel == 1) return false;
-  if (m->tuning.sweep_kernel == 2) return true;
-  return m->batch && m->sweep_grouped;
-}
-
-// The grouped sweep's band, in updated voxels per touched leaf. Measured on
-// one GB300: the grouped sweep takes 10% less time at 20-25 (the batched
-// workload's maps), 27% more at 42 (dense street scans) and also more at 9
-// (precision-stress scans into an empty map, about one update per plane,
-// where its per-plane overhead dominates). Entered inside [16, 30), left
-// outside [13, 36).
-constexpr double kGroupedEnterLo = 16.0;
-constexpr double kGroupedEnterHi = 30.0;
-constexpr double kGroupedLeaveLo = 13.0;
-constexpr double kGroupedLeaveHi = 36.0;
-
 void record_timings(vdbg_map* m)
 {
   m->timings.runs = m->h_status->runs;
-  if (m->h_status->touched > 0u && m->h_status->updates > 0u)
-  {
-    const double density = static_cast<double>(m->h_status->updates) / static_cast<double>(m->h_status->touched);
-    if (!m->sweep_grouped && density >= kGroupedEnterLo && density < kGroupedEnterHi) m->sweep_grouped = true;
-    if (m->sweep_grouped && (density < kGroupedLeaveLo || density > kGroupedLeaveHi)) m->sweep_grouped = false;
-  }
   float ms = 0.f;
   cudaEventElapsedTime(&ms, m->ev0, m->ev1);
   m->timings.total_ms = ms;
@@ -1049,7 +1011,6 @@ int reset_changes(vdbg_map* m, cudaStream_t s)
 int launch_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated = false)
 {
   const int g = gated ? 1 : 0;
-  k_compact<<<kSweepBlocks, kSweepThreads, 0, s>>>(map_view(m), channel_view(c), m->d_status, gated ? 2 : 0);
   LogOddsTable lt;
   lt.lo0   = m->conf[0].lo;
   lt.table = m->batch ? m->d_lo : nullptr;
@@ -1066,35 +1027,13 @@ int launch_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated = false)
     ch.cur   = m->chg_cur;
   }
   const ChannelView cv = channel_view(c);
-  if (use_grouped_sweep(m))
-  {
-    if (m->batch && m->track_changes)
-      k_sweep_grouped<true, true><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags,
-                                                                         m->origin, lt, ch, m->d_status, g);
-    else if (m->batch)
-      k_sweep_grouped<true, false><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags,
-                                                                          m->origin, lt, ch, m->d_status, g);
-    else if (m->track_changes)
-      k_sweep_grouped<false, true><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags,
-                                                                          m->origin, lt, ch, m->d_status, g);
-    else
-      k_sweep_grouped<false, false><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags,
-                                                                           m->origin, lt, ch, m->d_status, g);
-  }
-  else if (m->batch && m->track_changes)
-    k_sweep<true, true><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags, m->origin, lt, ch,
-                                                               m->d_status, g);
-  else if (m->batch)
-    k_sweep<true, false><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags, m->origin, lt,
-                                                                ch, m->d_status, g);
-  else if (m->track_changes)
-    k_sweep<false, true><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags, m->origin, lt,
-                                                                ch, m->d_status, g);
-  else
-    k_sweep<false, false><<<kSweepBlocks, kSweepThreads, 0, s>>>(cv, m->values, m->active, m->flags, m->origin, lt,
-                                                                 ch, m->d_status, g);
+  const int nm         = static_cast<int>(m->conf.size());
+  const unsigned grid  = static_cast<unsigned>(m->num_sms) * kSweepBlocks;
+  auto* kernel = m->batch ? (m->track_changes ? k_sweep<true, true> : k_sweep<true, false>)
+                          : (m->track_changes ? k_sweep<false, true> : k_sweep<false, false>);
+  kernel<<<grid, kSweepWarps * 32, 0, s>>>(map_view(m), cv, m->values, m->active, m->flags, lt, nm, ch, m->d_status, g);
   VDBG_CUDA(cudaGetLastError());
-  m->timings.launches += 2;
+  m->timings.launches += 1;
   return VDBG_OK;
 }
 
@@ -1251,7 +1190,7 @@ int discard_marking(vdbg_map* m, Channel& c, cudaStream_t s)
 {
   m->n_leaves = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
   m->n_blocks = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
-  k_compact<<<m->num_sms * 4, 256, 0, s>>>(map_view(m), channel_view(c), m->d_status, 1);
+  k_compact<<<m->num_sms * 4, 256, 0, s>>>(map_view(m), channel_view(c));
   k_clear_touched<<<m->num_sms * 4, 256, 0, s>>>(channel_view(c));
   VDBG_CUDA(cudaGetLastError());
   VDBG_TRY(finish_sweep(m, c, s));
@@ -1460,7 +1399,7 @@ CastPlan plan_single(const vdbg_map* m, int64_t n, const double origin[3], doubl
 }
 
 // Kernel launches of one captured step (memsets excluded).
-constexpr uint32_t kGraphKernels = 8;
+constexpr uint32_t kGraphKernels = 7;
 
 // Queues one batched step for capture: the point count is read on the device
 // from t.first[t.n], the grids cover the scratch capacity `cap`, and every
@@ -1516,7 +1455,6 @@ int capture_step(vdbg_map* m, Channel& c, int64_t stride, const ScanTable& t, cu
     return ei == cudaErrorMemoryAllocation ? oom("cudaGraphInstantiate") : VDBG_ERR_CUDA;
   }
   m->graph_layout  = m->layout;
-  m->graph_grouped = use_grouped_sweep(m);
   m->graph_stride = stride;
   m->graph_captures += 1;
   return VDBG_OK;
@@ -1542,7 +1480,7 @@ int graph_step(vdbg_map* m, Channel& c, const float* xyz, int64_t n, int64_t str
   *m->h_pts_ref = pts;
   VDBG_CUDA(cudaMemcpyAsync(m->d_pts_ref, m->h_pts_ref, sizeof(const char*), cudaMemcpyHostToDevice, s));
   c.pending = true;
-  if (!m->graph || m->graph_layout != m->layout || m->graph_stride != stride || m->graph_grouped != use_grouped_sweep(m))
+  if (!m->graph || m->graph_layout != m->layout || m->graph_stride != stride)
     VDBG_TRY(capture_step(m, c, stride, t, s));
   VDBG_CUDA(cudaGraphLaunch(m->graph, s));
   m->graph_replays += 1;
@@ -1569,8 +1507,8 @@ int run_allocating(vdbg_map* m, F&& launch);
 // the update grid was empty (updateMap returns before, VDBMapping.hpp:735-738).
 int reactivate_artificial(vdbg_map* m, Channel& c, cudaStream_t s)
 {
-  uint32_t touched = 0;
-  VDBG_CUDA(cudaMemcpyAsync(&touched, c.n_touched, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  uint32_t touched = 0;  // blocks
+  VDBG_CUDA(cudaMemcpyAsync(&touched, c.n_blist, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   VDBG_CUDA(cudaStreamSynchronize(s));
   if (touched == 0u) return VDBG_OK;
   return run_allocating(m, [&]() -> int {
