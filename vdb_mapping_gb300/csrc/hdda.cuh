@@ -213,26 +213,12 @@ struct Dda
 // the bit pattern read as an integer orders as the doubles do, once -0.0 is
 // folded onto +0.0 (they compare equal). Integer compares keep the walks off
 // the FP64 pipe, which is narrow on this GPU; the results are those of the
-// double compares.
+// double compares. Only a ray's t1 can be -0.0 (a product of its clip): t0 starts
+// at +0.0, and a sum t0 + x with t0 = +0.0 is never -0.0.
 VDBG_HD long long tkey(double t)
 {
-#ifdef __CUDA_ARCH__
-  const long long b = __double_as_longlong(t);
-#else
-  long long b;
-  std::memcpy(&b, &t, sizeof(b));
-#endif
+  const long long b = dbits(t);
   return b == static_cast<long long>(0x8000000000000000ull) ? 0ll : b;
-}
-
-// Index of the smallest of three values, ties to the higher index
-// (math::MinIndex). Constant indices only, so the DDA state stays in
-// registers.
-VDBG_HD int min_index(const double v[3])
-{
-  const long long a = tkey(v[0]), b = tkey(v[1]), c = tkey(v[2]);
-  if (a < b) return a < c ? 0 : 2;
-  return b < c ? 1 : 2;
 }
 
 // DDA::init(ray, t0, t1). The caller guarantees |ray(t0)| < 2^30 per axis.
@@ -270,41 +256,36 @@ VDBG_HD void dda_init(Dda& d, const Ray& r, double t0, double t1, int log2)
   }
 }
 
-// DDA::step(): enter the next cell; false once its entry time passes t1.
+// DDA::step(): enter the next cell; false once its entry time passes t1. The
+// axis is the smallest time's, ties to the higher index (math::MinIndex). Without
+// branches: the lanes of a warp step different axes, and three branches cost
+// three FP64 additions a step.
 VDBG_HD bool dda_step(Dda& d)
 {
-  // Constant indices only, so the state stays in registers.
-  const int a = min_index(d.next);
-  if (a == 0)
-  {
-    d.t0      = d.next[0];
-    d.next[0] = add(d.next[0], d.delta[0]);
-    d.voxel[0] += d.step[0];
-  }
-  else if (a == 1)
-  {
-    d.t0      = d.next[1];
-    d.next[1] = add(d.next[1], d.delta[1]);
-    d.voxel[1] += d.step[1];
-  }
-  else
-  {
-    d.t0      = d.next[2];
-    d.next[2] = add(d.next[2], d.delta[2]);
-    d.voxel[2] += d.step[2];
-  }
-  return tkey(d.t0) <= tkey(d.t1);
+  const long long n0 = dbits(d.next[0]), n1 = dbits(d.next[1]), n2 = dbits(d.next[2]);
+  const bool ax      = n0 < n1 && n0 < n2;
+  const bool ay      = !ax && n1 < n2;
+  const bool az      = !ax && !ay;
+  d.t0               = ax ? d.next[0] : (ay ? d.next[1] : d.next[2]);
+  const double t     = add(d.t0, ax ? d.delta[0] : (ay ? d.delta[1] : d.delta[2]));
+  d.next[0]          = ax ? t : d.next[0];
+  d.next[1]          = ay ? t : d.next[1];
+  d.next[2]          = az ? t : d.next[2];
+  d.voxel[0] += ax ? d.step[0] : 0;
+  d.voxel[1] += ay ? d.step[1] : 0;
+  d.voxel[2] += az ? d.step[2] : 0;
+  return dbits(d.t0) <= tkey(d.t1);
 }
 
 // A voxel-level DDA (log2 = 0) continued on integer-keyed state: the times
-// held as their order keys (tkey), the argmin with ties to the higher axis,
+// held as their bit patterns, the argmin with ties to the higher axis,
 // and the FP64 tMax += tDelta; fine_step enters the next voxel exactly as
 // dda_step does, with fewer instructions per step.
 struct FineDda
 {
   int voxel[3];
   int step[3];
-  long long next[3];  // tkey of the times
+  long long next[3];  // bits of the times
   double delta[3];
   long long t1;
 };
@@ -316,22 +297,11 @@ VDBG_HD FineDda fine_from(const Dda& d)
   {
     f.voxel[a] = d.voxel[a];
     f.step[a]  = d.step[a];
-    f.next[a]  = tkey(d.next[a]);
+    f.next[a]  = dbits(d.next[a]);
     f.delta[a] = d.delta[a];
   }
   f.t1 = tkey(d.t1);
   return f;
-}
-
-VDBG_HD double key_time(long long k)
-{
-#ifdef __CUDA_ARCH__
-  return __longlong_as_double(k);
-#else
-  double t;
-  std::memcpy(&t, &k, sizeof(t));
-  return t;
-#endif
 }
 
 VDBG_HD bool fine_step(FineDda& f)
@@ -340,7 +310,7 @@ VDBG_HD bool fine_step(FineDda& f)
   const bool ay      = !ax && (f.next[1] < f.next[2]);
   const long long t0 = ax ? f.next[0] : (ay ? f.next[1] : f.next[2]);
   const double d     = ax ? f.delta[0] : (ay ? f.delta[1] : f.delta[2]);
-  const long long tn = tkey(add(key_time(t0), d));
+  const long long tn = dbits(add(bits_double(t0), d));
   f.next[0]          = ax ? tn : f.next[0];
   f.next[1]          = ay ? tn : f.next[1];
   f.next[2]          = (!ax && !ay) ? tn : f.next[2];
@@ -355,7 +325,7 @@ VDBG_HD double dda_exit(const Dda& d)
 {
   double m = d.t1;
   for (int a = 0; a < 3; ++a)
-    if (tkey(d.next[a]) < tkey(m)) m = d.next[a];
+    if (dbits(d.next[a]) < tkey(m)) m = d.next[a];
   return m;
 }
 
@@ -377,22 +347,173 @@ enum Walk : int
   kWalkBound = 2,  // the step bound was reached
 };
 
+// Where a span's voxel walk can meet an active voxel: windows of time (lo, hi]
+// around the leaf cells with an active voxel, so that the walk can jump from one
+// to the next. The cells are those of the hierarchical walk; the voxel walk is a
+// DDA of its own, and each puts a leaf boundary of an axis at a time of its own.
+// The two differ by less than
+//   2^-50 (|eye| + |dir| + 1) |1 / dir|   (the rounding of the start position)
+//   + 2^-31 t                             (of at most 2^22 additions per axis)
+// = e. So at any time t the voxel walk is in a leaf cell that the hierarchical
+// walk visits within e of t, unless that walk crosses two axes within 2 e of
+// one another around t, in either order. Such a pair is told by the upper words
+// of the two times (at least 2^-21 t apart when they differ by two) once t is
+// past 2^23 times the first term, before which every crossing is taken for one
+// (`floor_hi`), and gets a window by itself. A ray whose first term reaches
+// 2^-26 (nearly parallel to a boundary, or starting far outside the map) is one
+// window from end to end.
+// A window is wider than its cells by three voxel steps of the ray (they come
+// |dir|_1 to a unit of time) and 2^-21 > 3 e (and the times' single precision):
+// at least one voxel boundary lies between its start and the cells, so that the
+// voxel the walk stands on at its start need not be looked at either.
+// `sink`: open(t0) at a span's first cell; window(lo, hi) in ascending order, without
+// overlap (the last one's hi may lie past the span's end).
+// A window that starts within kGapVoxels of the last one's end joins it: walking
+// the gap costs less than the jump over it, or a piece of its own.
+template <class Sink>
+struct RunTrack
+{
+  static constexpr float kGapVoxels = 24.0f;
+  Sink& sink;
+  float margin = 0.0f, gap = 0.0f, lo = 0.0f, hi = 0.0f;
+  int floor_hi = 0;
+  bool all = false, has = false, running = false, near = false;
+  VDBG_HD explicit RunTrack(Sink& s) : sink(s) {}
+  VDBG_HD void set_ray(const Ray& r)
+  {
+    constexpr float k2m50 = 9.3132257e-10f * 9.5367432e-7f;
+    float e = k2m50, l1 = 0.0f;
+    for (int a = 0; a < 3; ++a)
+    {
+      if (is_zero(r.dir[a])) continue;
+      const float d = fabsf(static_cast<float>(r.dir[a]));
+      const float w = (fabsf(static_cast<float>(r.eye[a])) + d + 1.0f) * fabsf(static_cast<float>(r.inv[a])) * k2m50;
+      e             = w > e || w != w ? w : e;
+      l1 += d;
+    }
+    all    = !(e < 1.4901161e-8f);  // 2^-26
+    margin = 3.0f / l1 + 4.7683716e-7f;
+    gap    = kGapVoxels / l1;
+    // Upper word of 2^23 e as a double, rounded up.
+    const float f = all ? 2.0f : e * 8388608.0f;
+    int b;
+#ifdef __CUDA_ARCH__
+    b = __float_as_int(f);
+#else
+    std::memcpy(&b, &f, sizeof(b));
+#endif
+    floor_hi = (b >> 3) + ((1023 - 127) << 20) + 1;
+  }
+  static VDBG_HD int upper(double t) { return static_cast<int>(dbits(t) >> 32); }
+  // Before a step of a DDA at any level: are its two next crossings too close?
+  VDBG_HD void crossing(const double next[3])
+  {
+    const int a = upper(next[0]), b = upper(next[1]), c = upper(next[2]);
+    const int low = a < b ? a : b, high = a < b ? b : a;
+    const int first = low < c ? low : c, rest = low < c ? c : low, second = rest < high ? rest : high;
+    near = near || second - first < 2 || first < floor_hi;
+  }
+  VDBG_HD void add_time(double t)
+  {
+    const float f = static_cast<float>(t);
+    if (has && (running || f - margin <= hi + gap))
+    {
+      hi = f + margin;
+      return;
+    }
+    if (has && !all) sink.window(lo, hi);
+    lo  = f - margin;
+    hi  = f + margin;
+    has = true;
+  }
+  // The span opens in the leaf cell `cell` of a ray at time t.
+  VDBG_HD void open(const Ray& r, double t, const int cell[3])
+  {
+    sink.open(t);
+    has     = false;
+    running = false;
+    near    = false;
+    for (int a = 0; a < 3; ++a)
+      near = near || (flr_int(add(r.eye[a], mul(r.dir[a], t))) & ~7) != cell[a];
+  }
+  VDBG_HD void enter(double t, bool active)
+  {
+    if (near || running || active) add_time(t);
+    running = active;
+    near    = false;
+  }
+  VDBG_HD void close(double t)
+  {
+    if (near || running) add_time(t);
+    if (all)
+      sink.window(-1.0f, 2.0f);
+    else if (has)
+      sink.window(lo, hi);
+    has     = false;
+    running = false;
+    near    = false;
+  }
+};
+
+// The windows of one span, kept (further ones are joined to the last).
+struct Runs
+{
+  static constexpr int kMax = 4;
+  float lo[kMax], hi[kMax];
+  int n = 0;
+  VDBG_HD void open(double) { n = 0; }
+  VDBG_HD void window(float a, float b)
+  {
+    for (int k = 0; k < kMax; ++k)  // (constant indices: the state stays in registers)
+    {
+      if (k == n) lo[k] = a;
+      if (k == n || (k == kMax - 1 && n == kMax)) hi[k] = b;
+    }
+    n += n < kMax ? 1 : 0;
+  }
+};
+
+// (a walk that needs no runs)
+struct NoTrack
+{
+  VDBG_HD void set_ray(const Ray&) {}
+  VDBG_HD void crossing(const double*) {}
+  VDBG_HD void open(const Ray&, double, const int*) {}
+  VDBG_HD void enter(double, bool) {}
+  VDBG_HD void close(double) {}
+};
+
+// Active bit of the leaf cell that has0 found, for a walk that asks for it.
+template <class Topo, class Sink>
+VDBG_HD bool cell_active(const Topo& topo, const RunTrack<Sink>&)
+{
+  return topo.active0();
+}
+template <class Topo>
+VDBG_HD bool cell_active(const Topo&, const NoTrack&)
+{
+  return false;
+}
+
 // VolumeHDDA<Tree, Ray, 2>::march / ::hits over `topo` (has2/has1/has0 of a
 // cell origin at that level). For every complete span, `on_span(span)` is
 // called; with `first_only` the walk stops at the first one (march). The open
 // span at the end (t1 = the end of the marched interval) is left in `t`, as
 // the reference leaves it for its caller. `steps` counts cells stepped.
-template <class Topo, class OnSpan>
-VDBG_HD int walk(Ray r, const Topo& topo, bool first_only, Span& t, uint32_t& steps, OnSpan&& on_span)
+// `track` (RunTrack) reports a span's windows before on_span reports the span.
+template <class Topo, class OnSpan, class Track>
+VDBG_HD int walk(Ray r, const Topo& topo, bool first_only, Span& t, uint32_t& steps, OnSpan&& on_span, Track& track)
 {
   // `open`: a span has started (t.t0 holds its start; closed spans are reset
   // to t = {-1, -1}). A span ends at a cell without a node: report it (march
   // stops there).
   bool open = t.t0 >= 0.0;
+  track.set_ray(r);
 #define VDBG_HDDA_CLOSE(time)                       \
   do                                                \
   {                                                 \
     t.t1 = (time);                                  \
+    track.close(t.t1);                              \
     if (span_valid(t, kSpanEps))                    \
     {                                               \
       on_span(t);                                   \
@@ -402,6 +523,7 @@ VDBG_HD int walk(Ray r, const Topo& topo, bool first_only, Span& t, uint32_t& st
     t.t1 = -1.0;                                    \
     open = false;                                   \
   } while (0)
+#define VDBG_HDDA_STEP(d) (track.crossing((d).next), dda_step(d))
 
   Dda d2;
   dda_init(d2, r, r.t0, r.t1, 12);
@@ -432,57 +554,128 @@ VDBG_HD int walk(Ray r, const Topo& topo, bool first_only, Span& t, uint32_t& st
               {
                 t.t0 = d0.t0;
                 open = true;
+                track.open(r, d0.t0, d0.voxel);
               }
+              track.enter(d0.t0, cell_active(topo, track));
             }
             else if (open)
             {
               VDBG_HDDA_CLOSE(d0.t0);
             }
-          } while (dda_step(d0));
+          } while (VDBG_HDDA_STEP(d0));
           if (open) t.t1 = d0.t1;
         }
         else if (open)
         {
           VDBG_HDDA_CLOSE(d1.t0);
         }
-      } while (dda_step(d1));
+      } while (VDBG_HDDA_STEP(d1));
       if (open) t.t1 = d1.t1;
     }
     else if (open)
     {
       VDBG_HDDA_CLOSE(d2.t0);
     }
-  } while (dda_step(d2));
-  if (open) t.t1 = d2.t1;
+  } while (VDBG_HDDA_STEP(d2));
+  if (open)
+  {
+    t.t1 = d2.t1;
+    track.close(t.t1);
+  }
   return kWalkDone;
 #undef VDBG_HDDA_CLOSE
+#undef VDBG_HDDA_STEP
 }
 
 // VolumeRayIntersector::march(t0, t1) after setIndexRay: the first span, valid
 // when longer than 0. `r` is the ray after the bounding-box clip.
-template <class Topo>
-VDBG_HD int march_first(const Ray& r, const Topo& topo, Span& out, bool& found, uint32_t& steps)
+template <class Topo, class Track>
+VDBG_HD int march_first(const Ray& r, const Topo& topo, Span& out, bool& found, uint32_t& steps, Track& track)
 {
   Span t{-1.0, -1.0};
   found = false;
   if (!(sub(r.t1, r.t0) > kSpanEps)) return kWalkDone;  // VolumeHDDA::march: ray.valid()
-  const int w = walk(r, topo, true, t, steps, [&](const Span&) {});
+  const int w = walk(r, topo, true, t, steps, [&](const Span&) {}, track);
   if (w == kWalkBound) return w;
   out   = t;
   found = span_valid(t, 0.0);
   return kWalkDone;
 }
+template <class Topo>
+VDBG_HD int march_first(const Ray& r, const Topo& topo, Span& out, bool& found, uint32_t& steps)
+{
+  NoTrack none;
+  return march_first(r, topo, out, found, steps, none);
+}
 
 // VolumeRayIntersector::hits after setIndexRay: every span, the last open one
 // included when valid.
-template <class Topo, class OnSpan>
-VDBG_HD int all_spans(const Ray& r, const Topo& topo, uint32_t& steps, OnSpan&& on_span)
+template <class Topo, class OnSpan, class Track>
+VDBG_HD int all_spans(const Ray& r, const Topo& topo, uint32_t& steps, OnSpan&& on_span, Track& track)
 {
   Span t{-1.0, -1.0};
-  const int w = walk(r, topo, false, t, steps, on_span);
+  const int w = walk(r, topo, false, t, steps, on_span, track);
   if (w == kWalkBound) return w;
   if (span_valid(t, kSpanEps)) on_span(t);
   return kWalkDone;
+}
+template <class Topo, class OnSpan>
+VDBG_HD int all_spans(const Ray& r, const Topo& topo, uint32_t& steps, OnSpan&& on_span)
+{
+  NoTrack none;
+  return all_spans(r, topo, steps, on_span, none);
+}
+
+// One axis of a voxel walk from its next time t on: the first time >= tau, and
+// how many times lie before it. FP64 addition is linear within a binade (from
+// the second time on, see march.cuh), so a binade takes three additions.
+VDBG_HD uint32_t jump_axis(long long& t, double d, long long tau)
+{
+  constexpr long long kBinade = 1ll << 52;
+  uint32_t k                  = 0;
+  while (t < tau)
+  {
+    const long long top = (t & ~(kBinade - 1)) + kBinade;  // the next binade
+    const long long lim = tau < top ? tau : top;
+    const long long t2  = dbits(add(bits_double(t), d));
+    k += 1;
+    t = t2;
+    if (t2 >= lim) continue;
+    const long long t3 = dbits(add(bits_double(t2), d));
+    k += 1;
+    t = t3;
+    if (t3 >= lim) continue;
+    // `more` further times stay below lim; the next addition is made.
+    const long long step = t3 - t2, room = lim - 1 - t3;
+    uint32_t more        = static_cast<uint32_t>(static_cast<float>(room) / static_cast<float>(step));
+    while (static_cast<long long>(more) * step > room) --more;
+    while (static_cast<long long>(more + 1u) * step <= room) ++more;
+    k += more + 1u;
+    t = dbits(add(bits_double(t3 + static_cast<long long>(more) * step), d));
+  }
+  return k;
+}
+
+// Steps f past every time < tau.
+VDBG_HD void jump(FineDda& f, long long tau)
+{
+  for (int a = 0; a < 3; ++a) f.voxel[a] += f.step[a] * static_cast<int>(jump_axis(f.next[a], f.delta[a], tau));
+}
+
+// Walks f over the voxels entered at times in (lo, hi], `visit(voxel)` for each
+// until it returns false (then false). f stands at the span's start t0 or after
+// an earlier window; hi <= the span's end.
+template <class Visit>
+VDBG_HD bool walk_window(FineDda& f, double t0, double lo, long long hi, Visit&& visit)
+{
+  if (lo > t0) jump(f, tkey(lo) + 1);
+  for (;;)
+  {
+    const long long m = f.next[1] < f.next[2] ? f.next[1] : f.next[2];
+    if ((f.next[0] < m ? f.next[0] : m) > hi) return true;
+    fine_step(f);
+    if (!visit(f.voxel)) return false;
+  }
 }
 
 // Bounding box of the intersector (leaves holding an active voxel): lo and
@@ -532,16 +725,23 @@ VDBG_HD bool trace_ray(const double o[3], const double dir[3], double len, doubl
 }
 
 // The first span of the query's ray clipped by the box (march).
-template <class Topo>
+template <class Topo, class Track>
 VDBG_HD int trace_span(const double oi[3], const double di[3], const Box& box, const Topo& topo, Span& sp,
-                       bool& found, uint32_t& steps)
+                       bool& found, uint32_t& steps, Track& track)
 {
   Ray r = make_ray(oi, di, 0.0, 1.0);
   clip(r, box.lo, box.hi_excl);
   sp    = Span{-1.0, -1.0};
   found = false;
-  if (march_first(r, topo, sp, found, steps) == kWalkBound) return kTraceBound;
+  if (march_first(r, topo, sp, found, steps, track) == kWalkBound) return kTraceBound;
   return kTraceOk;
+}
+template <class Topo>
+VDBG_HD int trace_span(const double oi[3], const double di[3], const Box& box, const Topo& topo, Span& sp,
+                       bool& found, uint32_t& steps)
+{
+  NoTrack none;
+  return trace_span(oi, di, box, topo, sp, found, steps, none);
 }
 
 // The voxel walk over span `sp`: end = the first active voxel after the
@@ -560,6 +760,69 @@ VDBG_HD int trace_walk(const double oi[3], const double di[3], const Span& sp, d
   }
   for (int a = 0; a < 3; ++a) end[a] = mul(static_cast<double>(f.voxel[a]), res);
   return kTraceOk;
+}
+
+// The same from the span's windows (RunTrack).
+template <class Active>
+VDBG_HD void trace_walk_runs(const double oi[3], const double di[3], const Span& sp, const float* lo, const float* hi,
+                             int n, double res, Active&& active, double end[3])
+{
+  const Ray fine = make_ray(oi, di, sp.t0, sp.t1);
+  Dda dda;
+  dda_init(dda, fine, sp.t0, sp.t1, 0);
+  FineDda f = fine_from(dda);
+  bool hit  = false;
+  for (int i = 0; i < n && !hit; ++i)
+  {
+    const long long stop = tkey(static_cast<double>(hi[i]));
+    hit = !walk_window(f, sp.t0, static_cast<double>(lo[i]), stop < f.t1 ? stop : f.t1,
+                       [&](const int v[3]) { return !active(v); });
+  }
+  if (!hit)
+  {
+    // Past the last time <= t1, and one step more.
+    jump(f, f.t1 + 1);
+    fine_step(f);
+  }
+  for (int a = 0; a < 3; ++a) end[a] = mul(static_cast<double>(f.voxel[a]), res);
+}
+
+// castRayIntoGridFast's voxel walk (VDBMapping.hpp:593-600) of the span from t0,
+// as far as the voxels entered at times in (lo, hi], and the span's first voxel
+// when lo <= t0.
+template <class Visit>
+VDBG_HD void fast_walk_window(const double eye[3], const double dir[3], double t0, double lo, double hi, Visit&& visit)
+{
+  const Ray fine = make_ray(eye, dir, t0, hi);
+  Dda dda;
+  dda_init(dda, fine, t0, hi, 0);
+  FineDda f = fine_from(dda);
+  if (!(lo > t0)) visit(f.voxel);
+  walk_window(f, t0, lo, tkey(hi), [&](const int v[3]) {
+    visit(v);
+    return true;
+  });
+}
+
+// The pieces of a window (lo, hi] of fast mode's walk, about kPieceVoxels voxel
+// steps each (l1 = |dir|_1): `item(lo, hi)` for each, in order and adjoining; the
+// first one of a span starts at -1. hi <= the span's end.
+constexpr float kPieceVoxels = 48.0f;
+template <class Item>
+VDBG_HD void window_pieces(double t0, float lo, double hi, float l1, Item&& item)
+{
+  const float a = lo > static_cast<float>(t0) ? lo : static_cast<float>(t0);
+  const float b = static_cast<float>(hi);
+  const float k = (b - a) * l1 * (1.0f / kPieceVoxels);
+  const int n   = k > 1.5f ? static_cast<int>(k + 0.5f < 1.0e6f ? k + 0.5f : 1.0e6f) : 1;
+  const float w = (b - a) / static_cast<float>(n);
+  double from   = static_cast<double>(lo) > t0 ? static_cast<double>(lo) : -1.0;
+  for (int i = 1; i <= n; ++i)
+  {
+    const double to = i < n ? static_cast<double>(a + w * static_cast<float>(i)) : hi;
+    item(from, to);
+    from = to;
+  }
 }
 
 // The end point of a query without a span: the ray's end.

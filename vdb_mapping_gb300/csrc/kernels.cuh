@@ -374,35 +374,6 @@ __device__ __forceinline__ uint32_t lanemask_lt()
   return m;
 }
 
-// OpenVDB's DDA<Ray<double>,0> on integer-keyed state: tMax is kept as the bit
-// pattern of a non-negative double, so the argmin is an integer compare (fast
-// mode's span walk; the insertion's walk is march.cuh).
-struct DdaRay
-{
-  int vx, vy, vz;        // current voxel
-  int sx, sy, sz;        // steps
-  long long nx, ny, nz;  // tMax (bits)
-  double dx, dy, dz;     // tDelta
-};
-
-// DDA::step(): argmin of tMax with ties to the higher axis, branch-free; the
-// sequential tMax += tDelta in FP64. Returns the bits of the t it stepped at.
-__device__ __forceinline__ long long dda_advance(DdaRay& r)
-{
-  const bool ax      = (r.nx < r.ny) && (r.nx < r.nz);
-  const bool ay      = !ax && (r.ny < r.nz);
-  const long long t0 = ax ? r.nx : (ay ? r.ny : r.nz);
-  const double d     = ax ? r.dx : (ay ? r.dy : r.dz);
-  const long long tn = __double_as_longlong(__dadd_rn(__longlong_as_double(t0), d));
-  r.nx               = ax ? tn : r.nx;
-  r.ny               = ay ? tn : r.ny;
-  r.nz               = (!ax && !ay) ? tn : r.nz;
-  r.vx += ax ? r.sx : 0;
-  r.vy += ay ? r.sy : 0;
-  r.vz += (!ax && !ay) ? r.sz : 0;
-  return t0;
-}
-
 // ---------------------------------------------------------------------------
 // k_march: castRayIntoGrid for every ray (VDBMapping.hpp:550-566) into the
 // update grid's visited masks.
@@ -1697,12 +1668,13 @@ struct TopoView
 {
   unsigned long long* key1;  // 128^3-voxel nodes: pack_leaf_key(map, v >> 7)
   unsigned long long* key2;  // 4096^3-voxel nodes: pack_leaf_key(map, v >> 12)
-  uint32_t mask;             // set capacity - 1 (both sets)
+  uint32_t mask;             // set capacity - 1 (both sets; >= 2x the map's blocks)
   int* box;                  // [6] min xyz, max xyz (inclusive) of the leaves with an active voxel
-  uint32_t* count;           // [0] the map's leaves, [1] nonzero when an insert failed
+  uint32_t* count;           // [0] nonzero when the map has a leaf, [1] when an insert failed
   int map;
-  // [blocks][16]: words 0-7, bit `cell` set when the leaf in that cell of the
-  // block is in the map; words 8-15, when it also holds an active voxel.
+  // [blocks][8][2]: of word w, bit `cell & 63` of the first part is set when the
+  // leaf in that cell of the block (cell >> 6 = w) is in the map; of the second
+  // part, when it also holds an active voxel.
   unsigned long long* leafbits;
 };
 
@@ -1745,61 +1717,80 @@ __global__ void k_topo_init(TopoView tv)
   if (threadIdx.x < 2) tv.count[threadIdx.x] = 0u;
 }
 
-__device__ __forceinline__ int find_block(const MapView& m, int map, int bx, int by, int bz);
+// One warp per block of 8^3 leaf cells: the bitmaps of its integrated leaves and
+// of those with an active voxel; the block's nodes enter the node sets, and its
+// active leaves widen the box. The bitmaps are written whole (no clearing, no
+// atomics), a node is looked up once per block instead of once per leaf, and
+// the box and the count take an atomic only from a warp that still changes
+// them. Bound by the reads of every leaf's flag and active words: 70 us for a map of 3.3M leaves (150 us
+// with a thread, two node lookups and up to three atomics per leaf, and 128 MB of
+// node keys to clear).
+constexpr int kTopoWarps = 8;
 
-// One thread per leaf slot: the integrated leaves of map tv.map enter the node
-// sets and their block's leaf bitmap; those with an active voxel widen the
-// box.
-__global__ void __launch_bounds__(256) k_topo_build(const int4* __restrict__ origin,
-                                                    const uint32_t* __restrict__ flags,
-                                                    const unsigned long long* __restrict__ active, uint32_t n,
-                                                    MapView m, TopoView tv)
+__global__ void __launch_bounds__(kTopoWarps * 32) k_topo_build(const uint32_t* __restrict__ flags,
+                                                                const unsigned long long* __restrict__ active,
+                                                                uint32_t blocks, MapView m, TopoView tv)
 {
-  // Whole warps run to the end: the count and the box are reduced over the
-  // warp first, so each warp makes one atomic per counter instead of one per
-  // leaf (the same few words take them from every leaf of the map).
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane   = static_cast<int>(threadIdx.x & 31);
-  int4 o           = make_int4(0, 0, 0, -1);
-  bool in          = i < n && flags[i] != 0u;
-  if (in)
+  const uint32_t b = blockIdx.x * kTopoWarps + (threadIdx.x >> 5);
+  if (b >= blocks) return;
+  const int4 o = m.borigin[b];
+  if (o.w != tv.map) return;  // (another map's block is never looked up)
+  const int* cells = m.bleaf + static_cast<size_t>(b) * 512;
+  unsigned long long mine_in = 0ull, mine_act = 0ull;  // lane w < 8: word w
+  uint32_t xs = 0u, ys = 0u, zs = 0u;  // leaf coordinates of the block with an active leaf
+#pragma unroll
+  for (int half = 0; half < 2; ++half)
   {
-    o  = origin[i];
-    in = o.w == tv.map;
+    int slot[8];
+    uint32_t in[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) slot[k] = __ldg(cells + half * 256 + k * 32 + lane);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) in[k] = slot[k] >= 0 ? __ldg(flags + slot[k]) : 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+    {
+      unsigned long long any = 0ull;
+      if (in[k])
+      {
+        const ulonglong2* a = reinterpret_cast<const ulonglong2*>(active + static_cast<size_t>(slot[k]) * 8);
+        const ulonglong2 a0 = __ldg(a), a1 = __ldg(a + 1), a2 = __ldg(a + 2), a3 = __ldg(a + 3);
+        any = a0.x | a0.y | a1.x | a1.y | a2.x | a2.y | a3.x | a3.y;
+      }
+      const unsigned iw = __ballot_sync(0xffffffffu, in[k] != 0u);
+      const unsigned aw = __ballot_sync(0xffffffffu, any != 0ull);
+      // cell = x * 64 + y * 8 + z: lanes 0-31 of step k hold x = word, y = (k & 1) * 4 + lane / 8
+      const int word = half * 4 + (k >> 1);
+      if (lane == word)
+      {
+        mine_in |= static_cast<unsigned long long>(iw) << (32 * (k & 1));
+        mine_act |= static_cast<unsigned long long>(aw) << (32 * (k & 1));
+      }
+      if (aw) xs |= 1u << word;
+      for (int q = 0; q < 4; ++q)
+      {
+        const uint32_t row = (aw >> (8 * q)) & 0xffu;
+        zs |= row;
+        if (row) ys |= 1u << ((k & 1) * 4 + q);
+      }
+    }
   }
-  bool act = false;
-  if (in)
+  if (lane < 8) reinterpret_cast<ulonglong2*>(tv.leafbits)[static_cast<size_t>(b) * 8 + lane] = make_ulonglong2(mine_in, mine_act);
+  const bool present = __any_sync(0xffffffffu, mine_in != 0ull);
+  if (!present || lane != 0) return;
+  if (*reinterpret_cast<volatile uint32_t*>(tv.count) == 0u) atomicOr(tv.count, 1u);
+  const bool ok = topo_insert(tv.key1, tv.mask, pack_leaf_key(tv.map, o.x >> 1, o.y >> 1, o.z >> 1)) &&
+                  topo_insert(tv.key2, tv.mask, pack_leaf_key(tv.map, o.x >> 6, o.y >> 6, o.z >> 6));
+  if (!ok) atomicOr(tv.count + 1, 1u);
+  if (!xs) return;
+  const int lo[3] = {o.x * 64 + 8 * (__ffs(xs) - 1), o.y * 64 + 8 * (__ffs(ys) - 1), o.z * 64 + 8 * (__ffs(zs) - 1)};
+  const int hi[3] = {o.x * 64 + 8 * (31 - __clz(xs)) + 7, o.y * 64 + 8 * (31 - __clz(ys)) + 7,
+                     o.z * 64 + 8 * (31 - __clz(zs)) + 7};
+  for (int a = 0; a < 3; ++a)
   {
-    const bool ok = topo_insert(tv.key1, tv.mask, pack_leaf_key(tv.map, o.x >> 7, o.y >> 7, o.z >> 7)) &&
-                    topo_insert(tv.key2, tv.mask, pack_leaf_key(tv.map, o.x >> 12, o.y >> 12, o.z >> 12));
-    const int b = find_block(m, tv.map, o.x >> 6, o.y >> 6, o.z >> 6);
-    if (!ok || b < 0) atomicOr(tv.count + 1, 1u);
-    const int cell = (((o.x >> 3) & 7) << 6) | (((o.y >> 3) & 7) << 3) | ((o.z >> 3) & 7);
-    if (b >= 0) atomicOr(tv.leafbits + static_cast<size_t>(b) * 16 + (cell >> 6), 1ull << (cell & 63));
-    unsigned long long any = 0ull;
-    for (int w = 0; w < 8; ++w) any |= active[static_cast<size_t>(i) * 8 + w];
-    act = any != 0ull;
-    if (act && b >= 0) atomicOr(tv.leafbits + static_cast<size_t>(b) * 16 + 8 + (cell >> 6), 1ull << (cell & 63));
-  }
-  const unsigned in_w = __ballot_sync(0xffffffffu, in);
-  if (lane == 0 && in_w) atomicAdd(tv.count, static_cast<uint32_t>(__popc(in_w)));
-  const unsigned act_w = __ballot_sync(0xffffffffu, act);
-  if (!act_w) return;
-  const int big = 0x7fffffff, small = static_cast<int>(0x80000000u);
-  const int x0 = __reduce_min_sync(0xffffffffu, act ? o.x : big);
-  const int y0 = __reduce_min_sync(0xffffffffu, act ? o.y : big);
-  const int z0 = __reduce_min_sync(0xffffffffu, act ? o.z : big);
-  const int x1 = __reduce_max_sync(0xffffffffu, act ? o.x + 7 : small);
-  const int y1 = __reduce_max_sync(0xffffffffu, act ? o.y + 7 : small);
-  const int z1 = __reduce_max_sync(0xffffffffu, act ? o.z + 7 : small);
-  if (lane == 0)
-  {
-    atomicMin(tv.box + 0, x0);
-    atomicMin(tv.box + 1, y0);
-    atomicMin(tv.box + 2, z0);
-    atomicMax(tv.box + 3, x1);
-    atomicMax(tv.box + 4, y1);
-    atomicMax(tv.box + 5, z1);
+    if (lo[a] < *reinterpret_cast<volatile int*>(tv.box + a)) atomicMin(tv.box + a, lo[a]);
+    if (hi[a] > *reinterpret_cast<volatile int*>(tv.box + 3 + a)) atomicMax(tv.box + 3 + a, hi[a]);
   }
 }
 
@@ -1839,7 +1830,8 @@ struct DevTopo
   MapView m;
   mutable int cbx, cby, cbz, cb;  // last block coordinate and its index (-1: none)
   mutable int cw = -1;            // word of cb's leaf bitmap held in `bits` (-1: none)
-  mutable unsigned long long bits = 0ull;
+  mutable ulonglong2 bits = {0ull, 0ull};
+  mutable int at = 0;             // bit of the last cell found
   __device__ __forceinline__ bool has2(const int v[3]) const
   {
     return voxel_in_map_range(v) && topo_find(tv.key2, tv.mask, pack_leaf_key(tv.map, v[0] >> 12, v[1] >> 12, v[2] >> 12));
@@ -1850,14 +1842,13 @@ struct DevTopo
   }
   __device__ __forceinline__ bool has0(const int v[3]) const
   {
-    if (!voxel_in_map_range(v)) return false;
     const int bx = v[0] >> 6, by = v[1] >> 6, bz = v[2] >> 6;
     if (bx != cbx || by != cby || bz != cbz)
     {
       cbx = bx;
       cby = by;
       cbz = bz;
-      cb  = find_block(m, tv.map, bx, by, bz);
+      cb  = voxel_in_map_range(v) ? find_block(m, tv.map, bx, by, bz) : -1;
       cw  = -1;
     }
     if (cb < 0) return false;
@@ -1865,20 +1856,21 @@ struct DevTopo
     if ((cell >> 6) != cw)
     {
       cw   = cell >> 6;
-      bits = tv.leafbits[static_cast<size_t>(cb) * 16 + cw];
+      bits = __ldg(reinterpret_cast<const ulonglong2*>(tv.leafbits) + static_cast<size_t>(cb) * 8 + cw);
     }
-    return (bits >> (cell & 63)) & 1ull;
+    at = cell & 63;
+    return (bits.x >> at) & 1ull;
   }
+  // The leaf has0 has just found holds an active voxel.
+  __device__ __forceinline__ bool active0() const { return (bits.y >> at) & 1ull; }
 };
 
 // isValueOn of the map for voxels along one ray, remembering the last leaf
 // (its block and slot, -1 when absent) and the active word of the z-plane
 // last read (a near-horizontal ray stays in one plane of a leaf for many
-// voxels). With the intersector's per-block bitmaps (`bits`, TopoView
-// leafbits), a leaf without an active voxel is known from one cached bitmap
-// word, and its slot and active words are not read: a walk through free
-// space does one load per 8 x 8 leaves of a block instead of two dependent
-// ones per leaf.
+// voxels). A leaf without an active voxel is known from the intersector's
+// bitmaps (`bits`, TopoView leafbits), and its slot and active words are not
+// read.
 struct ActiveCache
 {
   const MapView* m;
@@ -1889,7 +1881,7 @@ struct ActiveCache
   int wz;                   // plane (z & 7) held in `word`, -1 none
   unsigned long long word;  // active bits of plane wz of leaf `slot`
   int bx = 0x7fffffff, by = 0, bz = 0;  // block coordinate `b` was found for
-  const unsigned long long* bits = nullptr;  // TopoView leafbits, or none
+  const unsigned long long* bits = nullptr;  // TopoView leafbits
   int aw = -1;                               // word of b's active-leaf bitmap held in `abits`
   unsigned long long abits = 0ull;
   __device__ __forceinline__ bool operator()(const int v[3])
@@ -1912,12 +1904,12 @@ struct ActiveCache
       }
       const int cell = ((x & 7) << 6) | ((y & 7) << 3) | (z & 7);
       bool maybe     = b >= 0;
-      if (maybe && bits)
+      if (maybe)
       {
         if ((cell >> 6) != aw)
         {
           aw    = cell >> 6;
-          abits = bits[static_cast<size_t>(b) * 16 + 8 + aw];
+          abits = __ldg(bits + static_cast<size_t>(b) * 16 + 2 * aw + 1);
         }
         maybe = (abits >> (cell & 63)) & 1ull;
       }
@@ -1954,26 +1946,139 @@ __device__ __forceinline__ hdda::Box topo_box(const TopoView& tv)
 // allocated. The prep stage counted the castRayIntoGrid visits of the rays;
 // they are replaced by the marks made here (k_fast_visits).
 // Two phases, so that the lanes of a warp run the same loop: k_fast_spans
-// walks the intersector's three coarse levels for every ray and writes its
-// spans; k_fast_walk then walks the voxel DDA over one span per thread, in
-// the order the spans were written (neighbouring rays' spans together). The
-// spans and their fine walks are those of hdda::fast_cast_one.
-struct SpanRec
+// walks the intersector's three coarse levels for every ray and writes the
+// windows of its spans in which the voxel walk can meet an active voxel
+// (hdda::RunTrack), in pieces of about hdda::kPieceVoxels voxel steps;
+// k_fast_walk then walks the voxel DDA over one piece per thread. The spans and
+// their marks are those of hdda::fast_cast_one. The span walk is bound by
+// the FP64 pipe (74% busy; most of it the DDA start in each 128^3 node), the voxel
+// walk by the latency of its loads: 262144 rays of 60 m at 0.05 m take 0.50 +
+// 0.15 ms, where a walk of every voxel of every span took 0.61 after the span walk
+// of 0.38 (the windows cost that one a quarter), its longest thread 841 voxels.
+struct alignas(16) FastPiece
+{
+  double t0;      // the span's start, where its voxel walk starts
+  double lo, hi;  // the piece: voxels entered in (lo, hi] (and the first one, lo <= t0)
+  int ray;        // index into the ray records
+  int pad;
+};
+// One span of a raytrace query, with the windows in which it can meet an active
+// voxel.
+struct alignas(16) SpanRec
 {
   double t0, t1;
-  int ray;         // index into the ray records (raytrace: the query)
-  int cls;         // length class: floor(log2) of the span's estimated voxel steps
-  uint32_t steps;  // raytrace: the steps its coarse walk took (one bound for the query)
-  uint32_t pad;
+  int ray;  // the query
+  int n;    // windows
+  float lo[hdda::Runs::kMax], hi[hdda::Runs::kMax];
+  int cls;  // length class: floor(log2) of the voxel steps over the windows, estimated
+  int pad;
 };
 constexpr int kSpanClasses = 32;
 
+// Item of a thread when each warp takes `lanes` of the items (threads past them
+// take none: the value is >= n).
+__device__ __forceinline__ uint32_t lane_item(uint32_t lanes, uint32_t n)
+{
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  return lane < lanes ? warp * lanes + lane : n;
+}
+
+// Records written by a span kernel.
+template <class Rec>
 struct SpanBuf
 {
-  SpanRec* rec;
+  Rec* rec;
   uint32_t cap;
-  uint32_t* count;                 // spans written (may exceed cap: the host grows and repeats)
+  uint32_t* count;                 // written (may exceed cap: the host grows and repeats)
   unsigned long long* dda_visits;  // castRayIntoGrid visits the prep counted for these rays
+};
+
+// A slot of `count` for each active thread, one atomic for them together.
+__device__ __forceinline__ uint32_t take_slot(uint32_t* count)
+{
+  const unsigned mask = __activemask();
+  const int leader    = __ffs(mask) - 1;
+  uint32_t base       = 0;
+  if (static_cast<int>(threadIdx.x & 31) == leader) base = atomicAdd(count, static_cast<uint32_t>(__popc(mask)));
+  return __shfl_sync(mask, base, leader) + static_cast<uint32_t>(__popc(mask & lanemask_lt()));
+}
+
+// A ray's windows during its coarse walk, in shared memory (thread's column of a
+// block's arrays): those of all its spans are written out as pieces when the ray
+// is done, the warp's lanes together. Written where a span ends, at a different
+// step in each lane, the records took longer than the walk.
+constexpr int kSpanThreads = 32;  // (blocks of one warp: the rays of a block take very different times)
+constexpr int kFastWindows = 12;
+struct FastWindows
+{
+  double t0[kFastWindows][kSpanThreads], hi[kFastWindows][kSpanThreads];
+  float lo[kFastWindows][kSpanThreads];
+};
+
+// All 32 lanes: the pieces of each lane's n windows, one atomic for the warp.
+__device__ __forceinline__ void write_pieces(const FastWindows& w, int n, float l1, int ray,
+                                             const SpanBuf<FastPiece>& sb)
+{
+  const int x   = static_cast<int>(threadIdx.x);
+  uint32_t mine = 0u;
+  for (int k = 0; k < n; ++k)
+    hdda::window_pieces(w.t0[k][x], w.lo[k][x], w.hi[k][x], l1, [&](double, double) { ++mine; });
+  uint32_t total = 0u;
+  uint32_t slot  = warp_scan_exclusive(mine, static_cast<int>(threadIdx.x & 31u), &total);
+  uint32_t base  = 0u;
+  if ((threadIdx.x & 31u) == 0u && total) base = atomicAdd(sb.count, total);
+  slot += __shfl_sync(0xffffffffu, base, 0);
+  for (int k = 0; k < n; ++k)
+  {
+    const double t0 = w.t0[k][x];
+    hdda::window_pieces(t0, w.lo[k][x], w.hi[k][x], l1, [&](double from, double to) {
+      if (slot < sb.cap) sb.rec[slot] = FastPiece{t0, from, to, ray, 0};
+      ++slot;
+    });
+  }
+}
+
+// Sink of hdda::RunTrack: [0, base) belong to spans that ended, [base, n) to the
+// open one. Further windows join the open span's last; a span that finds no room
+// writes the last window before it, whole.
+struct FastSink
+{
+  FastWindows& w;
+  const SpanBuf<FastPiece>& sb;
+  int ray = 0;
+  int n = 0, base = 0;
+  double t0 = 0.0;
+  __device__ __forceinline__ void open(double t)
+  {
+    t0 = t;
+    n  = base;
+  }
+  __device__ __forceinline__ void window(float lo, float hi)
+  {
+    const int x = static_cast<int>(threadIdx.x);
+    if (base == kFastWindows)
+    {
+      n = --base;
+      const double at = w.t0[n][x], from = w.lo[n][x];
+      const uint32_t slot = atomicAdd(sb.count, 1u);
+      if (slot < sb.cap) sb.rec[slot] = FastPiece{at, from > at ? from : -1.0, w.hi[n][x], ray, 0};
+    }
+    if (n < kFastWindows)
+    {
+      w.t0[n][x] = t0;
+      w.lo[n][x] = lo;
+      ++n;
+    }
+    w.hi[n - 1][x] = static_cast<double>(hi);
+  }
+  // The span ends (its last window may lie past its end).
+  __device__ __forceinline__ void span(const hdda::Span& sp)
+  {
+    const int x = static_cast<int>(threadIdx.x);
+    if (n > base) w.hi[n - 1][x] = fmin(w.hi[n - 1][x], sp.t1);
+    base = n;
+  }
 };
 
 __device__ __forceinline__ void fast_ray(const int4& r, const ScanGeom& g, double eye[3], double dir[3])
@@ -1987,100 +2092,88 @@ __device__ __forceinline__ void fast_ray(const int4& r, const ScanGeom& g, doubl
   }
 }
 
-__global__ void __launch_bounds__(128) k_fast_spans(const int4* __restrict__ rays, const int* __restrict__ order,
-                                                    ScanTable t, MapView m, TopoView tv, SpanBuf sb)
+// (12 warps an SM: 16, with 128 registers, spilled and took 16% longer)
+__global__ void __launch_bounds__(kSpanThreads, 12) k_fast_spans(const int4* __restrict__ rays,
+                                                                 const int* __restrict__ order, ScanTable t,
+                                                                 MapView m, TopoView tv, SpanBuf<FastPiece> sb,
+                                                                 uint32_t lanes)
 {
+  __shared__ FastWindows windows;
   // (read once per warp: the warp reduces below)
   const int lane = static_cast<int>(threadIdx.x & 31);
   if (__shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed_u32(&m.st->error) : 0u, 0) != 0u) return;
   const uint32_t nv = m.st->n_valid;
-  const uint32_t j  = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t j  = lane_item(lanes, nv);
   unsigned long long dv = 0;
+  double eye[3], dir[3];
+  hdda::Ray ray;
+  float l1f = 0.0f;
+  int ri    = 0;
+  bool todo = false;
   if (j < nv && tv.count[1] == 0u)
   {
-    const int ri      = order[j];
+    ri                = order[j];
     const int4 r      = rays[ri];
     const uint32_t l1 = static_cast<uint32_t>(r.w) & kMetaL1Mask;
     dv                = l1 > 0u ? l1 + 1ull : 0ull;
-    if (tv.count[0] != 0u)
-    {
-      const ScanGeom& g = scan_geom(t, scan_of_ray(t, static_cast<uint32_t>(ri)));
-      double eye[3], dir[3];
-      fast_ray(r, g, eye, dir);
-      hdda::Ray ray = hdda::make_ray(eye, dir, 0.0, 1.0);
-      hdda::clip(ray, topo_box(tv).lo, topo_box(tv).hi_excl);
-      DevTopo topo{tv, m, 0x7fffffff, 0, 0, -1};
-      uint32_t steps = 0;
-      const double l1 = fabs(dir[0]) + fabs(dir[1]) + fabs(dir[2]);  // voxels per unit t
-      const int w     = hdda::all_spans(ray, topo, steps, [&](const hdda::Span& sp) {
-        const uint32_t k = atomicAdd(sb.count, 1u);
-        // (an estimate, for ordering only)
-        const double est = fmin((sp.t1 - sp.t0) * l1 + 2.0, 2147483647.0);
-        const int cls    = 31 - __clz(max(1, static_cast<int>(est)));
-        if (k < sb.cap) sb.rec[k] = SpanRec{sp.t0, sp.t1, ri, cls};
-      });
-      if (w == hdda::kWalkBound) atomicOr(&m.st->error, kErrStepBound);
-    }
+    todo              = tv.count[0] != 0u;
+    const ScanGeom& g = scan_geom(t, scan_of_ray(t, static_cast<uint32_t>(ri)));
+    fast_ray(r, g, eye, dir);
+    l1f = static_cast<float>(fabs(dir[0]) + fabs(dir[1]) + fabs(dir[2]));
+    ray = hdda::make_ray(eye, dir, 0.0, 1.0);
+    hdda::clip(ray, topo_box(tv).lo, topo_box(tv).hi_excl);
   }
   else if (j < nv)
   {
     atomicOr(&m.st->error, kErrTopoFull);
   }
+  FastSink sink{windows, sb, ri};
+  if (todo)
+  {
+    DevTopo topo{tv, m, 0x7fffffff, 0, 0, -1};
+    uint32_t steps = 0;
+    hdda::RunTrack<FastSink> track(sink);
+    const int w = hdda::all_spans(ray, topo, steps, [&](const hdda::Span& sp) { sink.span(sp); }, track);
+    if (w == hdda::kWalkBound) atomicOr(&m.st->error, kErrStepBound);
+  }
+  __syncwarp();
+  write_pieces(windows, sink.base, l1f, ri, sb);
   for (int off = 16; off > 0; off >>= 1) dv += __shfl_xor_sync(0xffffffffu, dv, off);
   if ((threadIdx.x & 31) == 0 && dv) atomicAdd(sb.dda_visits, dv);
 }
 
 __global__ void __launch_bounds__(128) k_fast_walk(const int4* __restrict__ rays, ScanTable t, MapView m,
                                                    ChannelView c, TopoView tv,
-                                                   const unsigned long long* __restrict__ active, SpanBuf sb,
-                                                   uint32_t n)
+                                                   const unsigned long long* __restrict__ active,
+                                                   SpanBuf<FastPiece> sb)
 {
   const int lane = static_cast<int>(threadIdx.x & 31);
   if (__shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed_u32(&m.st->error) : 0u, 0) != 0u) return;
-  c.cur_epoch       = *c.epoch;
-  const uint32_t i  = blockIdx.x * blockDim.x + threadIdx.x;
+  c.cur_epoch      = *c.epoch;
+  const uint32_t n = *sb.count;
+  if (n > sb.cap) return;  // (the host repeats the spans with more room)
   unsigned long long marks = 0ull;
-  if (i < n)
+  ActiveCache act{&m, active, tv.map, 0x7fffffff, 0, 0, -1, -1, -1, 0ull};
+  act.bits = tv.leafbits;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
   {
-    const SpanRec sp  = sb.rec[i];
-    const int4 r      = rays[sp.ray];
-    const ScanGeom& g = scan_geom(t, scan_of_ray(t, static_cast<uint32_t>(sp.ray)));
+    const FastPiece p = sb.rec[i];
+    const int4 r      = rays[p.ray];
+    const ScanGeom& g = scan_geom(t, scan_of_ray(t, static_cast<uint32_t>(p.ray)));
     double eye[3], dir[3];
     fast_ray(r, g, eye, dir);
-    const hdda::Ray fine = hdda::make_ray(eye, dir, sp.t0, sp.t1);
-    hdda::Dda dda;
-    hdda::dda_init(dda, fine, sp.t0, sp.t1, 0);
-    // The voxel steps of hdda::dda_step on the insertion DDA's state: the
-    // times held as their order keys (hdda::tkey), the argmin and the FP64
-    // tMax += tDelta as dda_advance does them (same tie rule, same sums).
-    DdaRay d{dda.voxel[0], dda.voxel[1], dda.voxel[2], dda.step[0], dda.step[1], dda.step[2],
-             hdda::tkey(dda.next[0]), hdda::tkey(dda.next[1]), hdda::tkey(dda.next[2]),
-             dda.delta[0], dda.delta[1], dda.delta[2]};
-    const long long t1 = hdda::tkey(sp.t1);
-    ActiveCache act{&m, active, tv.map, 0x7fffffff, 0, 0, -1, -1, -1, 0ull};
-    act.bits = tv.leafbits;
-    uint32_t steps = 0;
-    do
-    {
-      if (++steps > hdda::kStepLimit)
-      {
-        atomicOr(&m.st->error, kErrStepBound);
-        break;
-      }
-      const int v[3] = {d.vx, d.vy, d.vz};
-      if (act(v))
-      {
-        // act holds the voxel's leaf: mark it visited in the update grid.
-        const int b    = act.b;
-        const int cell = ((act.lx & 7) << 6) | ((act.ly & 7) << 3) | (act.lz & 7);
-        touch_block(c, b);
-        unsigned long long* bt = c.btouched + static_cast<size_t>(b) * 8 + (cell >> 6);
-        if (!((*bt >> (cell & 63)) & 1ull)) atomicOr(bt, 1ull << (cell & 63));
-        const int off = ((v[2] & 7) << 6) | ((v[1] & 7) << 3) | (v[0] & 7);
-        atomicOr(c.upd + static_cast<size_t>(act.slot) * 16 + (off >> 6), 1ull << (off & 63));
-        ++marks;
-      }
-    } while (dda_advance(d) <= t1);
+    hdda::fast_walk_window(eye, dir, p.t0, p.lo, p.hi, [&](const int v[3]) {
+      if (!act(v)) return;
+      // act holds the voxel's leaf: mark it visited in the update grid.
+      const int b    = act.b;
+      const int cell = ((act.lx & 7) << 6) | ((act.ly & 7) << 3) | (act.lz & 7);
+      touch_block(c, b);
+      unsigned long long* bt = c.btouched + static_cast<size_t>(b) * 8 + (cell >> 6);
+      if (!((*bt >> (cell & 63)) & 1ull)) atomicOr(bt, 1ull << (cell & 63));
+      const int off = ((v[2] & 7) << 6) | ((v[1] & 7) << 3) | (v[0] & 7);
+      atomicOr(c.upd + static_cast<size_t>(act.slot) * 16 + (off >> 6), 1ull << (off & 63));
+      ++marks;
+    });
   }
   for (int off = 16; off > 0; off >>= 1) marks += __shfl_xor_sync(0xffffffffu, marks, off);
   if ((threadIdx.x & 31) == 0 && marks) atomicAdd(&m.st->visits, marks);
@@ -2117,7 +2210,7 @@ __global__ void k_span_offsets(uint32_t* hist)
 }
 
 __global__ void __launch_bounds__(256) k_span_scatter(const SpanRec* __restrict__ rec, uint32_t n,
-                                                      uint32_t* __restrict__ cursor, SpanRec* __restrict__ out)
+                                                      uint32_t* __restrict__ cursor, uint32_t* __restrict__ out)
 {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool in    = i < n;
@@ -2128,18 +2221,23 @@ __global__ void __launch_bounds__(256) k_span_scatter(const SpanRec* __restrict_
   uint32_t base        = 0;
   if (in && static_cast<int>(threadIdx.x & 31) == leader) base = atomicAdd(cursor + cls, static_cast<uint32_t>(__popc(peers)));
   base = __shfl_sync(0xffffffffu, base, leader);
-  if (in) out[base + static_cast<uint32_t>(__popc(peers & lanemask_lt()))] = rec[i];
+  if (in) out[base + static_cast<uint32_t>(__popc(peers & lanemask_lt()))] = i;
 }
 
 // The fast marking's visits replace the castRayIntoGrid visits the prep
 // counted (one thread).
-__global__ void k_fast_visits(DevStatus* st, const unsigned long long* dda_visits) { st->visits -= *dda_visits; }
+__global__ void k_fast_visits(DevStatus* st, SpanBuf<FastPiece> sb)
+{
+  if (*sb.count <= sb.cap) st->visits -= *sb.dda_visits;
+}
 
 // raytrace (VDBMapping.hpp:675-721) in two phases, as fast mode walks its
 // spans: k_trace_spans finds every query's first span (hdda::trace_span) and
 // answers the queries without one; the spans are sorted by length (longest
 // first, k_span_hist / k_span_scatter), and k_trace_walk walks one span per
-// thread to its first active voxel (hdda::trace_walk). The coarse walk needs
+// thread to its first active voxel, in the windows that can hold one
+// (hdda::trace_walk_runs): 0.58 ms for a million spans of 420 voxels, where
+// every voxel of them took 2.0. The coarse walk needs
 // many registers and the voxel walk few, so apart each runs at its own
 // occupancy, and the walks of a warp take about as many steps each. q holds
 // the origins [n][3], then the directions [n][3], then the lengths [n]; ok[n]
@@ -2256,13 +2354,14 @@ __global__ void __launch_bounds__(256) k_trace_scatter(const unsigned short* __r
   order[atomicAdd(cursor + bin[i], 1u)] = i;
 }
 
-__global__ void __launch_bounds__(128) k_trace_spans(const double* __restrict__ q, uint32_t n, double res,
+// (20 warps an SM, which costs some spills: 16 took 3% longer, 12 without spills as much)
+__global__ void __launch_bounds__(kSpanThreads, 20) k_trace_spans(const double* __restrict__ q, uint32_t n, double res,
                                                      double inv_res, MapView m, TopoView tv,
                                                      const uint32_t* __restrict__ order,
                                                      unsigned char* __restrict__ ok, double* __restrict__ end,
-                                                     SpanBuf sb)
+                                                     SpanBuf<SpanRec> sb, uint32_t lanes)
 {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t j = lane_item(lanes, n);
   if (j >= n) return;
   const uint32_t i = order[j];
   if (tv.count[1] != 0u)
@@ -2284,7 +2383,9 @@ __global__ void __launch_bounds__(128) k_trace_spans(const double* __restrict__ 
   hdda::Span sp{-1.0, -1.0};
   bool found     = false;
   uint32_t steps = 0;
-  if (hdda::trace_span(oi, di, topo_box(tv), topo, sp, found, steps) == hdda::kTraceBound)
+  hdda::Runs runs;
+  hdda::RunTrack<hdda::Runs> track(runs);
+  if (hdda::trace_span(oi, di, topo_box(tv), topo, sp, found, steps, track) == hdda::kTraceBound)
   {
     atomicOr(&m.st->error, kErrStepBound);
     trace_answer(ok, end, i, false, zero);
@@ -2297,23 +2398,37 @@ __global__ void __launch_bounds__(128) k_trace_spans(const double* __restrict__ 
     trace_answer(ok, end, i, false, e);
     return;
   }
-  // (an estimate, for ordering only)
-  const double l1  = fabs(di[0]) + fabs(di[1]) + fabs(di[2]);
-  const double est = fmin((sp.t1 - sp.t0) * l1 + 2.0, 2147483647.0);
-  const int cls    = 31 - __clz(max(1, static_cast<int>(est)));
-  const uint32_t k = atomicAdd(sb.count, 1u);
-  if (k < sb.cap) sb.rec[k] = SpanRec{sp.t0, sp.t1, static_cast<int>(i), cls, steps, 0u};
+  SpanRec r;
+  r.t0        = sp.t0;
+  r.t1        = sp.t1;
+  r.ray       = static_cast<int>(i);
+  r.n         = runs.n;
+  float total = 0.0f;
+  for (int k = 0; k < hdda::Runs::kMax; ++k)
+  {
+    const bool in = k < runs.n;
+    r.lo[k]       = in ? runs.lo[k] : 0.0f;
+    r.hi[k]       = in ? runs.hi[k] : 0.0f;
+    total += r.hi[k] - r.lo[k];
+  }
+  const float l1 = fabsf(static_cast<float>(di[0])) + fabsf(static_cast<float>(di[1])) + fabsf(static_cast<float>(di[2]));
+  r.cls          = 31 - __clz(static_cast<int>(fminf(total * l1 + 1.0f, 1.0e9f)));  // (for ordering only)
+  r.pad          = 0;
+  const uint32_t k = take_slot(sb.count);
+  if (k < sb.cap) sb.rec[k] = r;
 }
 
 __global__ void __launch_bounds__(128) k_trace_walk(const double* __restrict__ q, uint32_t n, double res,
                                                     double inv_res, MapView m, TopoView tv,
                                                     const unsigned long long* __restrict__ active,
                                                     unsigned char* __restrict__ ok, double* __restrict__ end,
-                                                    const SpanRec* __restrict__ rec, uint32_t n_spans)
+                                                    const SpanRec* __restrict__ rec,
+                                                    const uint32_t* __restrict__ by_class, uint32_t n_spans,
+                                                    uint32_t lanes)
 {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t j = lane_item(lanes, n_spans);
   if (j >= n_spans) return;
-  const SpanRec r  = rec[j];
+  const SpanRec& r = rec[by_class[j]];
   const uint32_t i = static_cast<uint32_t>(r.ray);
   double o[3], d[3], len;
   trace_query(q, n, i, o, d, len);
@@ -2321,15 +2436,9 @@ __global__ void __launch_bounds__(128) k_trace_walk(const double* __restrict__ q
   hdda::trace_ray(o, d, len, inv_res, oi, di);  // in range: its span was found
   ActiveCache act{&m, active, tv.map, 0x7fffffff, 0, 0, -1, -1, -1, 0ull};
   act.bits = tv.leafbits;
-  uint32_t steps = r.steps;
-  double e[3]    = {0.0, 0.0, 0.0};
-  const bool done = hdda::trace_walk(oi, di, hdda::Span{r.t0, r.t1}, res, act, e, steps) == hdda::kTraceOk;
-  if (!done)
-  {
-    atomicOr(&m.st->error, kErrStepBound);
-    e[0] = e[1] = e[2] = 0.0;
-  }
-  trace_answer(ok, end, i, done, e);
+  double e[3];
+  hdda::trace_walk_runs(oi, di, hdda::Span{r.t0, r.t1}, r.lo, r.hi, r.n, res, act, e);
+  trace_answer(ok, end, i, true, e);
 }
 
 // ---------------------------------------------------------------------------

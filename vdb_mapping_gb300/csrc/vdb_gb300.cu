@@ -189,9 +189,12 @@ struct vdbg_map
   int* topo_box                    = nullptr;  // [8]: box[6], then two counts
   char* d_trace                    = nullptr;
   size_t trace_bytes               = 0;
-  // Fast mode's span records (k_fast_spans -> k_fast_walk) and their counters.
-  SpanRec* fast_spans              = nullptr;  // [fast_cap] as written, then
-  SpanRec* fast_sorted             = nullptr;  // [fast_cap] by length class
+  // Fast mode's pieces (k_fast_spans -> k_fast_walk), raytrace's span records
+  // (k_trace_spans -> k_trace_walk) and their counters.
+  FastPiece* fast_pieces           = nullptr;  // [piece_cap]
+  uint32_t piece_cap               = 0;
+  SpanRec* fast_spans              = nullptr;  // [fast_cap] as written, and
+  uint32_t* fast_sorted            = nullptr;  // [fast_cap] their order by length class
   uint32_t* fast_hist              = nullptr;  // [kSpanClasses]
   uint32_t fast_cap                = 0;
   unsigned long long* fast_ctr     = nullptr;  // [2]: span count (low 32 bits), castRayIntoGrid visits
@@ -1237,9 +1240,9 @@ int discard_marking(vdbg_map* m, Channel& c, cudaStream_t s)
 // map stands: node sets and box from its integrated leaves.
 int build_topology(vdbg_map* m, int map, cudaStream_t s, TopoView* tv)
 {
-  const uint32_t n = std::min(m->n_leaves, m->capacity);
-  uint32_t need    = 1024;
-  while (static_cast<uint64_t>(need) < 2ull * n && need < (1u << 31)) need <<= 1;
+  const uint32_t blocks = static_cast<uint32_t>(std::min<size_t>(m->n_blocks, m->bcapacity));
+  uint32_t need         = 1024;
+  while (static_cast<uint64_t>(need) < 2ull * blocks && need < (1u << 31)) need <<= 1;
   if (need > m->topo_cap)
   {
     dev_free(m, m->topo_keys, 2 * static_cast<size_t>(m->topo_cap));
@@ -1248,9 +1251,7 @@ int build_topology(vdbg_map* m, int map, cudaStream_t s, TopoView* tv)
     m->topo_cap = need;
   }
   if (!m->topo_box) VDBG_TRY(dev_alloc(m, &m->topo_box, 8));
-  const size_t blocks = std::min(m->n_blocks, m->bcapacity);
-  tv->leafbits        = reinterpret_cast<unsigned long long*>(m->vm_tbits.base);
-  if (blocks > 0) VDBG_CUDA(cudaMemsetAsync(tv->leafbits, 0, blocks * 16 * sizeof(unsigned long long), s));
+  tv->leafbits = reinterpret_cast<unsigned long long*>(m->vm_tbits.base);
   tv->key1  = m->topo_keys;
   tv->key2  = m->topo_keys + m->topo_cap;
   tv->mask  = m->topo_cap - 1;
@@ -1259,14 +1260,50 @@ int build_topology(vdbg_map* m, int map, cudaStream_t s, TopoView* tv)
   tv->map   = map;
   VDBG_CUDA(cudaMemsetAsync(m->topo_keys, 0xff, 2 * static_cast<size_t>(m->topo_cap) * sizeof(unsigned long long), s));
   k_topo_init<<<1, 32, 0, s>>>(*tv);
-  if (n > 0) k_topo_build<<<(n + 255) / 256, 256, 0, s>>>(m->origin, m->flags, m->active, n, map_view(m), *tv);
+  if (blocks > 0)
+    k_topo_build<<<(blocks + kTopoWarps - 1) / kTopoWarps, kTopoWarps * 32, 0, s>>>(m->flags, m->active, blocks,
+                                                                                  map_view(m), *tv);
   VDBG_CUDA(cudaGetLastError());
-  m->timings.launches += n > 0 ? 2 : 1;
+  m->timings.launches += blocks > 0 ? 2 : 1;
   return VDBG_OK;
 }
 
-// Span records of fast mode and raytrace (with their sort's histogram and
-// the two counters) for at least `want` spans.
+// Launch shape of the span and walk kernels for n rays: how many of a warp's
+// lanes take a ray each, and the block size. A thread's walk is a chain of
+// dependent loads whose length differs from ray to ray, and the lanes of a warp
+// take each other's time; with few rays there are warps enough to give each
+// ray fewer neighbours. 32 warps an SM: 1000 queries took 0.19 ms at 4, 0.18 at 8
+// to 128 (0.33 with whole warps), 50000 queries 0.70 at 8, 0.54 at 32, 0.63 at 64.
+struct RayShape
+{
+  uint32_t lanes;
+  unsigned threads, blocks;
+};
+RayShape ray_shape(const vdbg_map* m, uint32_t n, unsigned threads)
+{
+  const uint32_t warps = static_cast<uint32_t>(m->num_sms) * 32u;
+  RayShape r;
+  r.lanes            = std::min<uint32_t>(32, std::max<uint32_t>(1, (n + warps - 1) / warps));
+  r.threads          = r.lanes < 32 ? 32 : threads;
+  const uint32_t per = r.lanes * (r.threads / 32);
+  r.blocks           = (n + per - 1) / per;
+  return r;
+}
+
+// Room for `want` piece records of fast mode.
+int ensure_piece_buffer(vdbg_map* m, uint32_t want)
+{
+  if (!m->fast_ctr) VDBG_TRY(dev_alloc(m, &m->fast_ctr, 2));
+  if (want <= m->piece_cap) return VDBG_OK;
+  dev_free(m, m->fast_pieces, m->piece_cap);
+  m->piece_cap = 0;
+  VDBG_TRY(dev_alloc(m, &m->fast_pieces, want));
+  m->piece_cap = want;
+  return VDBG_OK;
+}
+
+// Span records of raytrace (with their sort's histogram and the two counters)
+// for at least `want` spans.
 int ensure_span_buffers(vdbg_map* m, uint32_t want)
 {
   if (!m->fast_ctr) VDBG_TRY(dev_alloc(m, &m->fast_ctr, 2));
@@ -1289,51 +1326,44 @@ int ensure_span_buffers(vdbg_map* m, uint32_t want)
 int run_fast_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, int64_t n, const ScanTable& t,
                      cudaStream_t s)
 {
-  TopoView tv;
-  VDBG_TRY(build_topology(m, 0, s, &tv));
+  // Spans, walk and hits in one go. The piece records' room is a guess: when it
+  // was too small, nothing was walked, and spans and walk run again with more.
+  // Hits that run out of pool or hash run again alone.
+  const RayShape shape      = ray_shape(m, static_cast<uint32_t>(n), kSpanThreads);
   const unsigned hit_blocks = static_cast<unsigned>((n + 255) / 256);
-  k_mark_hits<<<hit_blocks, 256, 0, s>>>(rays, order, t, map_view(m), channel_view(c));
-  VDBG_CUDA(cudaGetLastError());
-  m->timings.launches += 1;
-  // Phase 1: the spans of every ray (repeated with a larger buffer if they
-  // did not fit; the walk writes nothing but the records and counters).
-  uint32_t want = std::max<uint32_t>(m->fast_cap, static_cast<uint32_t>(std::min<int64_t>(4 * n, 1 << 30)));
-  uint32_t spans = 0;
-  for (int round = 0; round < 3; ++round)
+  uint32_t want = std::max<uint32_t>(m->piece_cap, static_cast<uint32_t>(std::min<int64_t>(2 * n + 4096, 1 << 30)));
+  bool marked   = false;
+  for (int attempt = 0;; ++attempt)
   {
-    VDBG_TRY(ensure_span_buffers(m, want));
-    VDBG_CUDA(cudaMemsetAsync(m->fast_ctr, 0, 2 * sizeof(unsigned long long), s));
-    SpanBuf sb{m->fast_spans, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
-    k_fast_spans<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(rays, order, t, map_view(m), tv, sb);
+    uint32_t pieces = 0;
+    if (!marked)
+    {
+      TopoView tv;
+      VDBG_TRY(build_topology(m, 0, s, &tv));
+      VDBG_TRY(ensure_piece_buffer(m, want));
+      VDBG_CUDA(cudaMemsetAsync(m->fast_ctr, 0, 2 * sizeof(unsigned long long), s));
+      const SpanBuf<FastPiece> sb{m->fast_pieces, m->piece_cap, reinterpret_cast<uint32_t*>(m->fast_ctr),
+                                  m->fast_ctr + 1};
+      k_fast_spans<<<shape.blocks, shape.threads, 0, s>>>(rays, order, t, map_view(m), tv, sb, shape.lanes);
+      k_fast_walk<<<static_cast<unsigned>(m->num_sms) * 12u, 128, 0, s>>>(rays, t, map_view(m), channel_view(c), tv,
+                                                                         m->active, sb);
+      k_fast_visits<<<1, 1, 0, s>>>(m->d_status, sb);
+      VDBG_CUDA(cudaGetLastError());
+      m->timings.launches += 3;
+      VDBG_CUDA(cudaMemcpyAsync(&pieces, m->fast_ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    }
+    // The hits come last: they alone allocate, and what they add (blocks, or the
+    // error of a pool that is full) must not be seen by the phases before.
+    k_mark_hits<<<hit_blocks, 256, 0, s>>>(rays, order, t, map_view(m), channel_view(c));
     VDBG_CUDA(cudaGetLastError());
     m->timings.launches += 1;
-    VDBG_CUDA(cudaMemcpyAsync(&spans, m->fast_ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    VDBG_CUDA(cudaStreamSynchronize(s));
-    if (spans <= m->fast_cap) break;
-    want = spans + spans / 4;
-  }
-  if (spans > m->fast_cap) return oom("fast spans", spans, m->fast_cap);
-  // Phase 2: the voxel walks over the spans, longest first.
-  if (spans > 0)
-  {
-    VDBG_CUDA(cudaMemsetAsync(m->fast_hist, 0, kSpanClasses * sizeof(uint32_t), s));
-    const unsigned sblocks = (spans + 255) / 256;
-    k_span_hist<<<std::min<unsigned>(sblocks, static_cast<unsigned>(m->num_sms) * 4u), 256, 0, s>>>(
-      m->fast_spans, spans, m->fast_hist);
-    k_span_offsets<<<1, 32, 0, s>>>(m->fast_hist);
-    k_span_scatter<<<sblocks, 256, 0, s>>>(m->fast_spans, spans, m->fast_hist, m->fast_sorted);
-    m->timings.launches += 3;
-    SpanBuf sb{m->fast_sorted, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
-    k_fast_walk<<<(spans + 127) / 128, 128, 0, s>>>(rays, t, map_view(m), channel_view(c), tv, m->active, sb,
-                                                    spans);
-    m->timings.launches += 1;
-  }
-  k_fast_visits<<<1, 1, 0, s>>>(m->d_status, m->fast_ctr + 1);
-  VDBG_CUDA(cudaGetLastError());
-  m->timings.launches += 1;
-  VDBG_TRY(fetch_status(m, s));
-  for (int attempt = 0; m->h_status->error != 0u; ++attempt)
-  {
+    m->timings.retries += attempt > 0 ? 1 : 0;
+    VDBG_TRY(fetch_status(m, s));
+    if (pieces > m->piece_cap)
+      want = pieces + pieces / 4;
+    else
+      marked = true;
+    if (m->h_status->error == 0u && marked) break;
     const uint32_t err = m->h_status->error;
     m->n_leaves        = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
     m->n_blocks        = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
@@ -1348,6 +1378,7 @@ int run_fast_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order
     }
     if (err & (kErrSpin | kErrStepBound | kErrTopoFull)) return map_error(err);
     if (attempt >= 40) return oom("fast marking", attempt, err);
+    if (err == 0u) continue;
     if (err & kErrPoolFull) VDBG_TRY(grow_for(m, m->h_status->n_leaves));
     if (err & kErrBlockFull) VDBG_TRY(grow_blocks_for(m, m->h_status->n_blocks));
     if ((err & kErrHashFull) && !(err & kErrBlockFull)) VDBG_TRY(rebuild_hash(m, m->bhash_size * 2, m->n_blocks));
@@ -1359,11 +1390,6 @@ int run_fast_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order
     VDBG_CUDA(cudaStreamSynchronize(m->stream));
     clear_error_keep_counters(m);
     VDBG_CUDA(cudaMemcpyAsync(m->d_status, m->h_status, sizeof(DevStatus), cudaMemcpyHostToDevice, s));
-    k_mark_hits<<<hit_blocks, 256, 0, s>>>(rays, order, t, map_view(m), channel_view(c));
-    VDBG_CUDA(cudaGetLastError());
-    m->timings.launches += 1;
-    m->timings.retries += 1;
-    VDBG_TRY(fetch_status(m, s));
   }
   m->n_leaves = std::min<uint32_t>(m->h_status->n_leaves, m->capacity);
   m->n_blocks = std::min<uint32_t>(m->h_status->n_blocks, m->bcapacity);
@@ -1958,6 +1984,7 @@ int vdbg_destroy(vdbg_map* m)
   dev_free(m, m->topo_keys, 2 * static_cast<size_t>(m->topo_cap));
   dev_free(m, m->topo_box, 8);
   dev_free(m, m->d_trace, m->trace_bytes);
+  dev_free(m, m->fast_pieces, m->piece_cap);
   dev_free(m, m->fast_spans, m->fast_cap);
   dev_free(m, m->fast_sorted, m->fast_cap);
   dev_free(m, m->fast_hist, kSpanClasses);
@@ -3005,9 +3032,10 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   k_trace_bin<<<(n32 + 255) / 256, 256, 0, s>>>(q, n32, mc.inv_res, bins, bin_hist);
   k_trace_offsets<<<1, 1024, 0, s>>>(bin_hist);
   k_trace_scatter<<<(n32 + 255) / 256, 256, 0, s>>>(bins, n32, bin_hist, order);
-  const SpanBuf sb{m->fast_spans, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
-  k_trace_spans<<<(n32 + 127) / 128, 128, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, order, ok,
-                                                 end, sb);
+  const SpanBuf<SpanRec> sb{m->fast_spans, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
+  const RayShape all = ray_shape(m, n32, kSpanThreads);
+  k_trace_spans<<<all.blocks, all.threads, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, order, ok, end,
+                                                   sb, all.lanes);
   VDBG_CUDA(cudaGetLastError());
   uint32_t spans = 0;
   VDBG_CUDA(cudaMemcpyAsync(&spans, m->fast_ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -3022,8 +3050,9 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
       m->fast_spans, spans, m->fast_hist);
     k_span_offsets<<<1, 32, 0, s>>>(m->fast_hist);
     k_span_scatter<<<sblocks, 256, 0, s>>>(m->fast_spans, spans, m->fast_hist, m->fast_sorted);
-    k_trace_walk<<<(spans + 127) / 128, 128, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, m->active,
-                                                    ok, end, m->fast_sorted, spans);
+    const RayShape some = ray_shape(m, spans, 128);
+    k_trace_walk<<<some.blocks, some.threads, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, m->active,
+                                                      ok, end, m->fast_spans, m->fast_sorted, spans, some.lanes);
     VDBG_CUDA(cudaGetLastError());
     m->timings.launches += 4;
   }
