@@ -2531,6 +2531,107 @@ __global__ void k_morph_load(const int4* __restrict__ origin, const unsigned lon
   for (int w = 0; w < 8; ++w) out.mask[static_cast<size_t>(j) * 8 + w] = mask[static_cast<size_t>(i) * 8 + w];
 }
 
+// The same over a dense grid of leaf cells, for a set whose cells (with room for
+// what its dilations reach) are few: no hash, no list between the steps, and the
+// cells' order is that of the origins. @MORPH@
+struct MorphGrid
+{
+  int3 first, dims;            // leaf coordinate of the first cell; cells x, y, z (z fastest)
+  uint32_t cells;
+  unsigned char* present;      // [cells] a leaf of the kept topology
+};
+
+__device__ __forceinline__ void morph_cell(const MorphGrid& g, uint32_t i, int& x, int& y, int& z)
+{
+  const uint32_t xy = i / static_cast<uint32_t>(g.dims.z);
+  z                 = static_cast<int>(i - xy * static_cast<uint32_t>(g.dims.z));
+  x                 = static_cast<int>(xy / static_cast<uint32_t>(g.dims.y));
+  y                 = static_cast<int>(xy - static_cast<uint32_t>(x) * static_cast<uint32_t>(g.dims.y));
+}
+
+// One thread per (leaf, word) of the input; a repeated origin's masks merge.
+__global__ void __launch_bounds__(256) k_morph_place(MorphGrid g, const int* __restrict__ origin,
+                                                     const unsigned long long* __restrict__ mask, uint32_t n,
+                                                     unsigned long long* __restrict__ out)
+{
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = t >> 3;
+  if (i >= n) return;
+  const int x = (origin[3 * static_cast<size_t>(i)] >> 3) - g.first.x,
+            y = (origin[3 * static_cast<size_t>(i) + 1] >> 3) - g.first.y,
+            z = (origin[3 * static_cast<size_t>(i) + 2] >> 3) - g.first.z;
+  const uint32_t c = (static_cast<uint32_t>(x) * static_cast<uint32_t>(g.dims.y) + static_cast<uint32_t>(y)) *
+                       static_cast<uint32_t>(g.dims.z) + static_cast<uint32_t>(z);
+  const unsigned long long m = mask[t];
+  if (m) atomicOr(out + static_cast<size_t>(c) * 8 + (t & 7u), m);
+  if ((t & 7u) == 0u) g.present[c] = 1;
+}
+
+// The 27 neighbour cells of a cell (none outside the grid).
+struct MorphCells
+{
+  const unsigned long long* in;
+  const MorphGrid* g;
+  int x, y, z;
+  __device__ __forceinline__ const uint64_t* operator()(int d) const
+  {
+    const int nx = x + d / 9 - 1, ny = y + (d / 3) % 3 - 1, nz = z + d % 3 - 1;
+    if (nx < 0 || ny < 0 || nz < 0 || nx >= g->dims.x || ny >= g->dims.y || nz >= g->dims.z) return nullptr;
+    return reinterpret_cast<const uint64_t*>(
+      in + (static_cast<size_t>(nx * g->dims.y + ny) * static_cast<size_t>(g->dims.z) + static_cast<size_t>(nz)) * 8);
+  }
+};
+
+// One step, one thread per (cell, word). A leaf that a dilation reaches (its word
+// is not empty) joins the kept topology.
+__global__ void __launch_bounds__(256) k_morph_step(MorphGrid g, const unsigned long long* __restrict__ in,
+                                                    unsigned long long* __restrict__ out, int dilate)
+{
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = t >> 3;
+  if (i >= g.cells) return;
+  const int a = static_cast<int>(t & 7u);
+  unsigned long long w = 0ull;
+  if (dilate || in[t])  // (an erosion leaves nothing where nothing was)
+  {
+    MorphCells nb{in, &g, 0, 0, 0};
+    morph_cell(g, i, nb.x, nb.y, nb.z);
+    w = dilate ? morph::dilate_word(nb, a) : morph::erode_word(nb, a);
+  }
+  out[t] = w;
+  if (dilate && w) g.present[i] = 1;
+}
+
+// Which cells are leaves of the result.
+__global__ void __launch_bounds__(256) k_morph_keep(MorphGrid g, const unsigned long long* __restrict__ in, int keep,
+                                                    uint32_t* __restrict__ out)
+{
+  const uint32_t t     = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i     = t >> 3;
+  const bool any       = i < g.cells && in[t] != 0ull;
+  const unsigned votes = __ballot_sync(0xffffffffu, any);
+  if (i >= g.cells || (t & 7u) != 0u) return;
+  out[i] = ((votes >> (threadIdx.x & 24u)) & 0xffu) != 0u || (keep && g.present[i]) ? 1u : 0u;
+}
+
+__global__ void __launch_bounds__(256) k_morph_write(MorphGrid g, const unsigned long long* __restrict__ in,
+                                                     const uint32_t* __restrict__ keep,
+                                                     const uint32_t* __restrict__ pos, int* __restrict__ out_o,
+                                                     unsigned long long* __restrict__ out_m)
+{
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = t >> 3, a = t & 7u;
+  if (i >= g.cells || !keep[i]) return;
+  const size_t at    = pos[i];
+  out_m[at * 8 + a] = in[t];
+  if (a < 3u)
+  {
+    int x, y, z;
+    morph_cell(g, i, x, y, z);
+    out_o[at * 3 + a] = 8 * (a == 0u ? g.first.x + x : a == 1u ? g.first.y + y : g.first.z + z);
+  }
+}
+
 // Dilation: one thread per (leaf of `in`, direction); the neighbours that
 // receive bits become the leaves of `out` (deduplicated by its hash).
 // Erosion (dilate == 0): the leaves of `in` themselves. `keep`: every leaf of

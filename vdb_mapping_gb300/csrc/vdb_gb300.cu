@@ -224,6 +224,7 @@ namespace {
 constexpr uint32_t kDefaultCapacity = 1u << 16;
 constexpr uint32_t kMinBlocks       = 1u << 10;
 constexpr size_t kWorkKept          = size_t(64) << 20;
+constexpr int64_t kMorphCells       = int64_t(1) << 18;  // leaf cells of a set taken as a dense grid (37 MB)
 constexpr int64_t kSectionCells     = int64_t(1) << 20;  // boxes of more leaf cells list the map's leaves
 
 uint32_t next_pow2(uint64_t v)
@@ -2842,6 +2843,56 @@ int morph_run(vdbg_map* m, int op, int iterations, bool keep, const std::vector<
   return st;
 }
 
+// The same for a set within `g` (see k_morph_step), whose leaves need not be unique;
+// the results come back in the order of their origins.
+int morph_grid(vdbg_map* m, int op, int iterations, bool keep, MorphGrid g, int64_t n, const int32_t* origins,
+               const uint64_t* masks, int64_t capacity, int32_t* out_origins, uint64_t* out_masks, int64_t* n_out)
+{
+  cudaStream_t s     = m->stream;
+  const size_t cells = g.cells, rows = static_cast<size_t>(n);
+  const size_t words = cells * 8;
+  VDBG_TRY(work_ensure(m, 1, (2 * words + rows * 8) * sizeof(uint64_t) +
+                               (2 * cells + 3 * cells + 3 * rows + 64) * sizeof(uint32_t) + cells));
+  unsigned long long* a    = reinterpret_cast<unsigned long long*>(m->work[1]);
+  unsigned long long* b    = a + words;
+  unsigned long long* in_m = b + words;
+  uint32_t* kept           = reinterpret_cast<uint32_t*>(in_m + rows * 8);
+  uint32_t* pos            = kept + cells;
+  uint32_t* total          = pos + cells;
+  int* out_o               = reinterpret_cast<int*>(total + 64);
+  int* in_o                = out_o + 3 * cells;
+  g.present                = reinterpret_cast<unsigned char*>(in_o + 3 * rows);
+  VDBG_CUDA(cudaMemcpyAsync(in_o, origins, 3 * rows * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+  VDBG_CUDA(cudaMemcpyAsync(in_m, masks, 8 * rows * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
+  VDBG_CUDA(cudaMemsetAsync(a, 0, words * sizeof(uint64_t), s));
+  VDBG_CUDA(cudaMemsetAsync(g.present, 0, cells, s));
+  const unsigned blocks = static_cast<unsigned>((words + 255) / 256);
+  k_morph_place<<<static_cast<unsigned>((rows * 8 + 255) / 256), 256, 0, s>>>(g, in_o, in_m, static_cast<uint32_t>(n),
+                                                                             a);
+  const int steps = op >= 2 ? 2 * iterations : iterations;
+  for (int i = 0; i < steps; ++i)
+  {
+    const bool first = i < iterations;
+    k_morph_step<<<blocks, 256, 0, s>>>(g, a, b, (op == 0 || (op == 2 && first) || (op == 3 && !first)) ? 1 : 0);
+    std::swap(a, b);
+  }
+  k_morph_keep<<<blocks, 256, 0, s>>>(g, a, keep ? 1 : 0, kept);
+  k_section_scan<<<1, 1024, 0, s>>>(kept, g.cells, pos, total);
+  k_morph_write<<<blocks, 256, 0, s>>>(g, a, kept, pos, out_o, b);
+  VDBG_CUDA(cudaGetLastError());
+  m->timings.launches += 4 + steps;
+  uint32_t k = 0;
+  VDBG_CUDA(cudaMemcpyAsync(&k, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaStreamSynchronize(s));
+  *n_out = k;
+  if (static_cast<int64_t>(k) > capacity) return VDBG_ERR_BUFFER_TOO_SMALL;
+  if (k == 0) return VDBG_OK;
+  VDBG_CUDA(cudaMemcpyAsync(out_origins, out_o, 3 * size_t(k) * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaMemcpyAsync(out_masks, b, 8 * size_t(k) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  VDBG_CUDA(cudaStreamSynchronize(s));
+  return VDBG_OK;
+}
+
 // Replaces the device copy of the artificial leaves with the host's.
 int upload_artificial(vdbg_map* m)
 {
@@ -3076,19 +3127,49 @@ int vdbg_section_morphology(vdbg_map* m, int op, int iterations, int64_t n, cons
     return VDBG_ERR_INVALID_ARGUMENT;
   *n_out = 0;
   if (n > (int64_t(1) << 24)) return VDBG_ERR_SIZE_LIMIT;
-  // Unique leaves (masks of a repeated origin are merged); origins within
-  // +-2^20, so the steps' leaves stay inside the key range.
+  // Origins within +-2^20, so the steps' leaves stay inside the key range.
+  int32_t lo[3] = {1 << 20, 1 << 20, 1 << 20}, hi[3] = {-(1 << 20), -(1 << 20), -(1 << 20)};
+  for (int64_t i = 0; i < n; ++i)
+    for (int a = 0; a < 3; ++a)
+    {
+      const int32_t o = origins[3 * i + a];
+      if ((o & 7) != 0) return VDBG_ERR_INVALID_ARGUMENT;
+      if (!(o >= -(1 << 20) && o < (1 << 20))) return VDBG_ERR_COORD_RANGE;
+      lo[a] = std::min(lo[a], o);
+      hi[a] = std::max(hi[a], o);
+    }
+  if (n > 0)
+  {
+    // The grid of leaf cells the steps stay in (a dilation goes one voxel further).
+    const int room = op == 1 ? 0 : (iterations + 7) / 8;
+    int64_t dims[3], cells = 1;
+    for (int a = 0; a < 3; ++a)
+    {
+      dims[a] = ((hi[a] - lo[a]) >> 3) + 1 + 2 * room;
+      cells   = cells > kMorphCells ? cells : cells * dims[a];
+    }
+    if (cells <= kMorphCells)
+    {
+      MorphGrid g;
+      g.first   = make_int3((lo[0] >> 3) - room, (lo[1] >> 3) - room, (lo[2] >> 3) - room);
+      g.dims    = make_int3(static_cast<int>(dims[0]), static_cast<int>(dims[1]), static_cast<int>(dims[2]));
+      g.cells   = static_cast<uint32_t>(cells);
+      g.present = nullptr;
+      VDBG_TRY(set_device(m));
+      std::lock_guard<std::mutex> lock(m->work_mutex);
+      const int st =
+        morph_grid(m, op, iterations, keep, g, n, origins, masks, capacity, out_origins, out_masks, n_out);
+      work_done(m);
+      return st;
+    }
+  }
+  // Unique leaves (masks of a repeated origin are merged).
   std::map<std::tuple<int32_t, int32_t, int32_t>, size_t> index;
   std::vector<int32_t> uo;
   std::vector<uint64_t> um;
   for (int64_t i = 0; i < n; ++i)
   {
     const int32_t* o = origins + 3 * i;
-    for (int a = 0; a < 3; ++a)
-    {
-      if ((o[a] & 7) != 0) return VDBG_ERR_INVALID_ARGUMENT;
-      if (!(o[a] >= -(1 << 20) && o[a] < (1 << 20))) return VDBG_ERR_COORD_RANGE;
-    }
     const auto key = std::make_tuple(o[0], o[1], o[2]);
     auto it        = index.find(key);
     if (it == index.end())

@@ -231,10 +231,12 @@ def _morphology(lib, h, origins, masks, op, iterations, check, keep_leaves=False
     mk = np.ascontiguousarray(np.asarray(masks, np.uint64).reshape(-1, 8))
     code = MORPH_OPS[op] | (MORPH_KEEP_LEAVES if keep_leaves else 0)
     n = C.c_int64()
-    cap = 0
+    # Room for what a few steps give, so that they run once (only the rows
+    # returned are ever written).
+    cap = 2 * len(o) + 4096
     while True:
-        oo = np.zeros((cap, 3), np.int32)
-        om = np.zeros((cap, 8), np.uint64)
+        oo = np.empty((cap, 3), np.int32)
+        om = np.empty((cap, 8), np.uint64)
         s = lib.vdbg_section_morphology(h, code, int(iterations), len(o), o.ctypes.data, mk.ctypes.data, cap,
                                         oo.ctypes.data, om.ctypes.data, C.byref(n))
         if s == _lib.STATUS_CODE["VDBG_ERR_BUFFER_TOO_SMALL"]:
