@@ -1439,9 +1439,61 @@ __device__ __forceinline__ unsigned long long swap_mask_word(Word&& word, int a)
   return out;
 }
 
-// Which candidates give a leaf of the section (getMapSection: an inside voxel
-// is active or, full, holds a value other than the background 0). Eight lanes
-// per candidate, one z-plane each.
+// Does a plane (w) of leaf `slot` hold a voxel of the section (getMapSection: an
+// inside voxel is active or, full, holds a value other than the background 0)?
+__device__ __forceinline__ bool section_plane(int slot, int w, const int4* __restrict__ origin,
+                                              const float* __restrict__ values,
+                                              const unsigned long long* __restrict__ active, int3 lo, int3 hi, int full)
+{
+  const unsigned long long inbox = box_plane_mask(origin[slot], w, lo, hi);
+  bool any                       = (active[static_cast<size_t>(slot) * 8 + w] & inbox) != 0ull;
+  if (full && !any && inbox)
+  {
+    const float4* vp = reinterpret_cast<const float4*>(values + static_cast<size_t>(slot) * 512 + w * 64);
+    for (int q0 = 0; q0 < 16 && !any; q0 += 4)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+      {
+        const int qd      = q0 + k;
+        const uint32_t in = static_cast<uint32_t>(inbox >> (4 * qd)) & 0xfu;
+        const float4 v    = vp[plane_quad(qd)];
+        any = any || ((in & 1u) && v.x != 0.0f) || ((in & 2u) && v.y != 0.0f) || ((in & 4u) && v.z != 0.0f) ||
+              ((in & 8u) && v.w != 0.0f);
+      }
+  }
+  return any;
+}
+
+// Candidates of the leaf cells first + [0, dims) in the order of their origins
+// (k_section_cells) and which of them give a leaf of the section, eight lanes per
+// cell.
+__global__ void __launch_bounds__(256) k_section_find(MapView m, int map, const uint32_t* __restrict__ flags, int3 first,
+                                                      int3 dims, uint32_t n, const float* __restrict__ values,
+                                                      const unsigned long long* __restrict__ active, int3 lo, int3 hi,
+                                                      int full, int* __restrict__ cand, uint32_t* __restrict__ keep)
+{
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = t >> 3;
+  const int w      = static_cast<int>(t & 7u);
+  int slot         = -1;
+  if (w == 0 && i < n)
+  {
+    const uint32_t z = i % static_cast<uint32_t>(dims.z), xy = i / static_cast<uint32_t>(dims.z);
+    const int lx = first.x + static_cast<int>(xy / static_cast<uint32_t>(dims.y)),
+              ly = first.y + static_cast<int>(xy % static_cast<uint32_t>(dims.y)), lz = first.z + static_cast<int>(z);
+    slot = find_leaf(m, map, lx, ly, lz);
+    if (slot >= 0 && flags[slot] == 0u) slot = -1;
+  }
+  slot                 = __shfl_sync(0xffffffffu, slot, static_cast<int>(threadIdx.x & 24u));
+  const bool any       = slot >= 0 && section_plane(slot, w, m.origin, values, active, lo, hi, full);
+  const unsigned votes = __ballot_sync(0xffffffffu, any);
+  if (w != 0 || i >= n) return;
+  cand[i] = slot;
+  keep[i] = ((votes >> (threadIdx.x & 24u)) & 0xffu) ? 1u : 0u;
+}
+
+// Which candidates give a leaf of the section, eight lanes per candidate, one
+// z-plane each.
 __global__ void __launch_bounds__(256) k_section_keep(const int* __restrict__ cand, uint32_t n,
                                                       const int4* __restrict__ origin,
                                                       const float* __restrict__ values,
@@ -1452,26 +1504,7 @@ __global__ void __launch_bounds__(256) k_section_keep(const int* __restrict__ ca
   const uint32_t j = t >> 3;
   const int w      = static_cast<int>(t & 7u);
   const int slot   = j < n ? cand[j] : -1;
-  bool any         = false;
-  if (slot >= 0)
-  {
-    const unsigned long long inbox = box_plane_mask(origin[slot], w, lo, hi);
-    any                            = (active[static_cast<size_t>(slot) * 8 + w] & inbox) != 0ull;
-    if (full && !any && inbox)
-    {
-      const float4* vp = reinterpret_cast<const float4*>(values + static_cast<size_t>(slot) * 512 + w * 64);
-      for (int q0 = 0; q0 < 16 && !any; q0 += 4)
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-        {
-          const int qd      = q0 + k;
-          const uint32_t in = static_cast<uint32_t>(inbox >> (4 * qd)) & 0xfu;
-          const float4 v    = vp[plane_quad(qd)];
-          any = any || ((in & 1u) && v.x != 0.0f) || ((in & 2u) && v.y != 0.0f) || ((in & 4u) && v.z != 0.0f) ||
-                ((in & 8u) && v.w != 0.0f);
-        }
-    }
-  }
+  const bool any   = slot >= 0 && section_plane(slot, w, origin, values, active, lo, hi, full);
   const unsigned votes = __ballot_sync(0xffffffffu, any);
   if (w == 0 && j < n) keep[j] = ((votes >> (threadIdx.x & 24u)) & 0xffu) ? 1u : 0u;
 }

@@ -157,6 +157,8 @@ struct vdbg_map
   std::mutex work_mutex;
   char* work[2]         = {nullptr, nullptr};
   size_t work_bytes[2]  = {0, 0};
+  char* sec_host        = nullptr;  // pinned: a small section's count, masks and origins
+  size_t sec_bytes      = 0;
 
   int64_t bytes         = 0;
   int num_sms           = 152;
@@ -224,6 +226,8 @@ namespace {
 constexpr uint32_t kDefaultCapacity = 1u << 16;
 constexpr uint32_t kMinBlocks       = 1u << 10;
 constexpr size_t kWorkKept          = size_t(64) << 20;
+constexpr uint32_t kSectionPinned   = 1u << 15;  // boxes of at most this many leaf cells are written at once
+constexpr size_t kSectionRow        = 8 * sizeof(uint64_t) + 3 * sizeof(int32_t);
 constexpr int64_t kMorphCells       = int64_t(1) << 18;  // leaf cells of a set taken as a dense grid (37 MB)
 constexpr int64_t kSectionCells     = int64_t(1) << 20;  // boxes of more leaf cells list the map's leaves
 
@@ -1982,6 +1986,7 @@ int vdbg_destroy(vdbg_map* m)
   dev_free(m, m->d_order, m->ray_cap);
   dev_free(m, m->axis_mem, kAxisTableBytes);
   work_done(m, 0);
+  if (m->sec_host) cudaFreeHost(m->sec_host);
   dev_free(m, m->topo_keys, 2 * static_cast<size_t>(m->topo_cap));
   dev_free(m, m->topo_box, 8);
   dev_free(m, m->d_trace, m->trace_bytes);
@@ -2544,6 +2549,22 @@ int3 box_corner(const int32_t v[3])
   return make_int3(c(v[0]), c(v[1]), c(v[2]));
 }
 
+// Leaf cells of the box [lo, hi] within the map's range; their number (a box of more
+// than kSectionCells: that + 1).
+uint32_t section_cells(int3 lo, int3 hi, int3* first, int3* dims)
+{
+  if (lo.x > hi.x || lo.y > hi.y || lo.z > hi.z) return 0;
+  const int kLo = static_cast<int>(kVoxelMin) >> 3, kHi = (static_cast<int>(kVoxelMaxExcl) >> 3) - 1;
+  *first          = make_int3(std::max(lo.x >> 3, kLo), std::max(lo.y >> 3, kLo), std::max(lo.z >> 3, kLo));
+  const int3 last = make_int3(std::min(hi.x >> 3, kHi), std::min(hi.y >> 3, kHi), std::min(hi.z >> 3, kHi));
+  if (first->x > last.x || first->y > last.y || first->z > last.z) return 0;
+  *dims = make_int3(last.x - first->x + 1, last.y - first->y + 1, last.z - first->z + 1);
+  // (each at most 2^19)
+  const int64_t plane = static_cast<int64_t>(dims->x) * dims->y;
+  if (plane > kSectionCells || plane * dims->z > kSectionCells) return static_cast<uint32_t>(kSectionCells) + 1u;
+  return static_cast<uint32_t>(plane * dims->z);
+}
+
 // Candidate slots of the box [lo, hi] of map `mp` in the order of their
 // origins, into workspace 0 (from its start). *cand null: none.
 int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, int** cand, uint32_t* n_out)
@@ -2552,18 +2573,11 @@ int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, int** cand, uint32
   *n_out = 0;
   cudaStream_t s   = m->stream;
   const uint32_t n = std::min(m->n_leaves, m->capacity);
-  if (n == 0 || lo.x > hi.x || lo.y > hi.y || lo.z > hi.z) return VDBG_OK;
-  // Leaf cells of the box within the map's range.
-  const int kLo = static_cast<int>(kVoxelMin) >> 3, kHi = (static_cast<int>(kVoxelMaxExcl) >> 3) - 1;
-  const int3 first = make_int3(std::max(lo.x >> 3, kLo), std::max(lo.y >> 3, kLo), std::max(lo.z >> 3, kLo));
-  const int3 last  = make_int3(std::min(hi.x >> 3, kHi), std::min(hi.y >> 3, kHi), std::min(hi.z >> 3, kHi));
-  if (first.x > last.x || first.y > last.y || first.z > last.z) return VDBG_OK;
-  const int3 dims = make_int3(last.x - first.x + 1, last.y - first.y + 1, last.z - first.z + 1);
-  // (each at most 2^19)
-  const int64_t plane = static_cast<int64_t>(dims.x) * dims.y;
-  if (plane <= kSectionCells && plane * dims.z <= kSectionCells)
+  int3 first, dims;
+  const uint32_t cells = n > 0 ? section_cells(lo, hi, &first, &dims) : 0u;
+  if (cells == 0) return VDBG_OK;
+  if (cells <= kSectionCells)
   {
-    const uint32_t cells = static_cast<uint32_t>(plane * dims.z);
     VDBG_TRY(work_ensure(m, 0, static_cast<size_t>(cells) * 3 * sizeof(uint32_t) + 256));
     *cand  = reinterpret_cast<int*>(m->work[0]);
     *n_out = cells;
@@ -2604,12 +2618,63 @@ int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, int** cand, uint32
   return VDBG_OK;
 }
 
+// getMapSection of a box of few leaf cells: room for every cell, so that the leaves
+// are written without waiting for their number; origins and masks go straight to
+// pinned memory, from which the host copies them while the values' copy runs.
+// (With the count fetched first and three copies, a section of 936 cells took 90 to
+// 117 us a call, of 5408 as much; this 58 to 60.)
+int section_export_small(vdbg_map* m, int mp, int3 lo, int3 hi, int3 first, int3 dims, uint32_t n, int full,
+                         int64_t capacity, int32_t* origins, float* values, uint64_t* masks, int64_t* n_out)
+{
+  cudaStream_t s = m->stream;
+  const size_t pinned = (n * kSectionRow + 64 + 0xffff) & ~size_t(0xffff);
+  if (pinned > m->sec_bytes)
+  {
+    if (m->sec_host) cudaFreeHost(m->sec_host);
+    m->sec_host  = nullptr;
+    m->sec_bytes = 0;
+    VDBG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->sec_host), pinned));
+    m->sec_bytes = pinned;
+  }
+  VDBG_TRY(work_ensure(m, 0, static_cast<size_t>(n) * 3 * sizeof(uint32_t) + 256));
+  if (values) VDBG_TRY(work_ensure(m, 1, static_cast<size_t>(n) * 512 * sizeof(float)));
+  int* cand                  = reinterpret_cast<int*>(m->work[0]);
+  uint32_t* keep             = reinterpret_cast<uint32_t*>(cand) + n;
+  uint32_t* pos              = keep + n;
+  volatile uint32_t* kept_at = reinterpret_cast<uint32_t*>(m->sec_host);
+  unsigned long long* h_m    = reinterpret_cast<unsigned long long*>(m->sec_host + 64);
+  int* h_o                   = reinterpret_cast<int*>(h_m + 8 * static_cast<size_t>(n));
+  k_section_find<<<static_cast<unsigned>((static_cast<uint64_t>(n) * 8 + 255) / 256), 256, 0, s>>>(
+    map_view(m), mp, m->flags, first, dims, n, m->values, m->active, lo, hi, full, cand, keep);
+  k_section_scan<<<1, 1024, 0, s>>>(keep, n, pos, reinterpret_cast<uint32_t*>(m->sec_host));
+  k_section_write<<<static_cast<unsigned>((static_cast<uint64_t>(n) * 32 + 255) / 256), 256, 0, s>>>(
+    cand, n, keep, pos, m->origin, m->values, m->active, lo, hi, full, h_o,
+    values ? reinterpret_cast<float*>(m->work[1]) : nullptr, h_m);
+  VDBG_CUDA(cudaGetLastError());
+  VDBG_CUDA(cudaStreamSynchronize(s));
+  const uint32_t kept = *kept_at;
+  *n_out              = kept;
+  if (static_cast<int64_t>(kept) > capacity) return VDBG_ERR_BUFFER_TOO_SMALL;
+  if (kept == 0) return VDBG_OK;
+  const size_t k = kept;
+  if (values) VDBG_CUDA(cudaMemcpyAsync(values, m->work[1], k * 512 * sizeof(float), cudaMemcpyDeviceToHost, s));
+  if (masks) std::memcpy(masks, h_m, k * 8 * sizeof(uint64_t));
+  if (origins) std::memcpy(origins, h_o, k * 3 * sizeof(int32_t));
+  if (values) VDBG_CUDA(cudaStreamSynchronize(s));
+  return VDBG_OK;
+}
+
 // getMapSection into host arrays (any of them may be null).
 int section_export(vdbg_map* m, int mp, int3 lo, int3 hi, int full, int64_t capacity, int32_t* origins, float* values,
                    uint64_t* masks, int64_t* n_out)
 {
   cudaStream_t s = m->stream;
-  int* cand      = nullptr;
+  int3 first, dims;
+  const uint32_t cells = m->n_leaves > 0 ? section_cells(lo, hi, &first, &dims) : 0u;
+  if (cells == 0) return VDBG_OK;
+  if (cells <= kSectionPinned)
+    return section_export_small(m, mp, lo, hi, first, dims, cells, full, capacity, origins, values, masks, n_out);
+  int* cand  = nullptr;
   uint32_t n = 0, kept = 0;
   VDBG_TRY(section_candidates(m, mp, lo, hi, &cand, &n));
   if (n == 0) return VDBG_OK;
