@@ -97,8 +97,8 @@ struct DevStatus
   unsigned long long nonfinite;
   uint32_t max_l1;      // longest ray, when in the first length class (else 0)
   uint32_t n_blocks;    // block bump allocator
-  uint32_t windows;     // update-grid windows closed by k_finish_window
-  uint32_t pad;
+  uint32_t windows;     // update-grid windows closed (finish_window)
+  uint32_t sweep_blocks;  // blocks of a gated k_sweep that are done
   unsigned long long runs;         // plane runs merged by k_march
   unsigned long long item_cursor;  // next work item of k_march
 };
@@ -316,12 +316,22 @@ __device__ __forceinline__ unsigned long long pack_leaf_key(int map, int lx, int
          (static_cast<unsigned long long>(lz) & m);
 }
 
-// Appends block `b` to the channel's touched-block list the first time it is
-// seen in the current integration window.
 // True when this call's marking is free of errors (k_march casts every ray),
 // so its update grids may be integrated.
 __device__ __forceinline__ bool marking_complete(const DevStatus* st) { return ld_relaxed_u32(&st->error) == 0u; }
 
+// After a sweep: a fresh update grid for the channel (one thread).
+__device__ __forceinline__ void finish_window(const ChannelView& c, DevStatus* st)
+{
+  st->windows += 1u;
+  c.n_touched[0]   = 0u;
+  *c.n_blist       = 0u;
+  const uint32_t e = c.n_touched[2] + 1u;
+  c.n_touched[2]   = e == 0u ? 1u : e;  // 0 marks blocks never touched
+}
+
+// Appends block `b` to the channel's touched-block list the first time it is
+// seen in the current integration window.
 __device__ __forceinline__ void touch_block(const ChannelView& c, int b)
 {
   uint32_t* e = c.bepoch + b;

@@ -317,8 +317,8 @@ int queue_prep(vdbg_map* m, PrepSet& p, const std::vector<ServerRequest>& step, 
   }
   VDBG_CUDA(cudaMemsetAsync(p.st, 0, sizeof(DevStatus), ps));
   const unsigned blocks = static_cast<unsigned>((p.total + 255) / 256);
-  k_prep<<<blocks, 256, 0, ps>>>(p.pts, nullptr, p.total, 16, t, p.rays, nm > 1 ? p.ray_scan : nullptr, p.hist,
-                                 p.st);
+  k_prep<<<prep_blocks(p.total), kPrepThreads, 0, ps>>>(p.pts, nullptr, p.total, 16, t, p.rays,
+                                                        nm > 1 ? p.ray_scan : nullptr, p.hist, p.st);
   launch_scan(p.hist, p.cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), p.st, ps);
   k_scatter<<<blocks, 256, 0, ps>>>(p.rays, p.total, t, p.cursor, p.order);
   VDBG_CUDA(cudaGetLastError());

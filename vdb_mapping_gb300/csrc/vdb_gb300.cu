@@ -799,6 +799,8 @@ void launch_scan(uint32_t* hist, uint32_t* cursor, uint32_t nb, DevStatus* st, c
   k_scan_tiles<<<tiles, 1024, 0, s>>>(hist, cursor, nb, cursor + nb);
 }
 
+unsigned prep_blocks(int64_t n) { return static_cast<unsigned>((n + kPrepThreads - 1) / kPrepThreads); }
+
 // Queues the per-point stage of raycastPointCloud (VDBMapping.hpp:499-519)
 // for the scans of table `t` (n points in all, in scan order): clip,
 // quantise, sort rays into the DDA order.
@@ -814,7 +816,7 @@ int launch_prep(vdbg_map* m, Channel& c, const float* xyz, int64_t n, int64_t st
     pts = pts_scratch;
   }
   const unsigned blocks = static_cast<unsigned>((n + 255) / 256);
-  k_prep<<<blocks, 256, 0, s>>>(pts, nullptr, n, stride, t, rays, ray_scan, hist, m->d_status);
+  k_prep<<<prep_blocks(n), kPrepThreads, 0, s>>>(pts, nullptr, n, stride, t, rays, ray_scan, hist, m->d_status);
   launch_scan(hist, cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), m->d_status, s);
   k_scatter<<<blocks, 256, 0, s>>>(rays, n, t, cursor, order);
   VDBG_CUDA(cudaGetLastError());
@@ -945,9 +947,6 @@ int run_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, con
     VDBG_CUDA(cudaEventRecord(m->ev_dda, s));
     VDBG_TRY(reset_changes(m, s));
     VDBG_TRY(launch_sweep(m, c, s, true));
-    k_finish_window<<<1, 1, 0, s>>>(channel_view(c), m->d_status, 1);
-    VDBG_CUDA(cudaGetLastError());
-    m->timings.launches += 1;
   }
   VDBG_TRY(fetch_status(m, s));
   if (eager && m->h_status->windows > 0u)
@@ -1014,8 +1013,8 @@ int reset_changes(vdbg_map* m, cudaStream_t s)
   return VDBG_OK;
 }
 
-// `gated`: a captured step, in which the sweep skips itself on the device
-// unless the marking completed.
+// `gated`: the sweep follows its marking without a host round trip: it skips itself
+// unless the marking completed, and closes the window.
 int launch_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated = false)
 {
   const int g = gated ? 1 : 0;
@@ -1046,9 +1045,9 @@ int launch_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated = false)
 }
 
 // After a sweep (or a dropped marking): fresh update grid for the channel.
-int finish_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated = false)
+int finish_sweep(vdbg_map* m, Channel& c, cudaStream_t s)
 {
-  k_finish_window<<<1, 1, 0, s>>>(channel_view(c), m->d_status, gated ? 1 : 0);
+  k_finish_window<<<1, 1, 0, s>>>(channel_view(c), m->d_status);
   VDBG_CUDA(cudaGetLastError());
   c.pending = false;
   return VDBG_OK;
@@ -1430,7 +1429,7 @@ CastPlan plan_single(const vdbg_map* m, int64_t n, const double origin[3], doubl
 }
 
 // Kernel launches of one captured step (memsets excluded).
-constexpr uint32_t kGraphKernels = 7;
+constexpr uint32_t kGraphKernels = 6;
 
 // Queues one batched step for capture: the point count is read on the device
 // from t.first[t.n], the grids cover the scratch capacity `cap`, and every
@@ -1438,15 +1437,14 @@ constexpr uint32_t kGraphKernels = 7;
 int queue_step(vdbg_map* m, Channel& c, int64_t cap, int64_t stride, const ScanTable& t, cudaStream_t s)
 {
   const unsigned blocks = static_cast<unsigned>((cap + 255) / 256);
-  k_prep<<<blocks, 256, 0, s>>>(nullptr, m->d_pts_ref, cap, stride, t, m->d_rays, m->d_ray_scan, m->d_hist,
-                                m->d_status);
+  k_prep<<<prep_blocks(cap), kPrepThreads, 0, s>>>(nullptr, m->d_pts_ref, cap, stride, t, m->d_rays, m->d_ray_scan,
+                                                   m->d_hist, m->d_status);
   launch_scan(m->d_hist, m->d_cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), m->d_status, s);
   k_scatter<<<blocks, 256, 0, s>>>(m->d_rays, cap, t, m->d_cursor, m->d_order);
   VDBG_CUDA(cudaEventRecordWithFlags(m->ev_prep, s, cudaEventRecordExternal));
   VDBG_TRY(launch_marking(m, c, m->d_rays, m->d_order, m->d_cursor, cap, t, s));
   VDBG_CUDA(cudaEventRecordWithFlags(m->ev_dda, s, cudaEventRecordExternal));
   VDBG_TRY(launch_sweep(m, c, s, true));
-  k_finish_window<<<1, 1, 0, s>>>(channel_view(c), m->d_status, 1);
   VDBG_CUDA(cudaGetLastError());
   return VDBG_OK;
 }
@@ -2204,7 +2202,8 @@ int vdbg_ray_digests(vdbg_map* m, const float* xyz, int64_t n, int64_t stride, c
   unsigned long long* d_out = nullptr;
   VDBG_TRY(dev_alloc(m, &d_out, static_cast<size_t>(n) * 2));
   const unsigned blocks = static_cast<unsigned>((n + 255) / 256);
-  k_prep<<<blocks, 256, 0, s>>>(pts, nullptr, n, stride, plan.table, m->d_rays, nullptr, m->d_hist, m->d_status);
+  k_prep<<<prep_blocks(n), kPrepThreads, 0, s>>>(pts, nullptr, n, stride, plan.table, m->d_rays, nullptr, m->d_hist,
+                                                 m->d_status);
   k_ray_digest<<<blocks, 256, 0, s>>>(m->d_rays, n, plan.table, m->axis, d_out, m->d_status);
   int st = cudaGetLastError() == cudaSuccess ? VDBG_OK : VDBG_ERR_CUDA;
   // (k_prep counted the rays into the sort histogram, which must start the
