@@ -3114,10 +3114,12 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   VDBG_TRY(begin_call(m, s));
   const size_t nn    = static_cast<size_t>(n);
   // queries (7 doubles) and end points (3), then the order (u32), the bins
-  // (u16), the bin offsets and the success flags
+  // (u16), the bins' offsets, the sort blocks' counts and the success flags
   const size_t n16   = (nn + 15) & ~static_cast<size_t>(15);
+  const uint32_t sort_blocks =
+    std::min<uint32_t>(static_cast<uint32_t>(m->num_sms), static_cast<uint32_t>((nn + 4095) / 4096));
   const size_t bytes = nn * 10 * sizeof(double) + n16 * (sizeof(uint32_t) + sizeof(unsigned short)) +
-                       kTraceBins * sizeof(uint32_t) + n16;
+                       (static_cast<size_t>(sort_blocks) + 1) * kTraceBins * sizeof(uint32_t) + n16;
   if (bytes > m->trace_bytes)
   {
     dev_free(m, m->d_trace, m->trace_bytes);
@@ -3132,7 +3134,8 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   uint32_t* order        = reinterpret_cast<uint32_t*>(q + 10 * nn);
   unsigned short* bins   = reinterpret_cast<unsigned short*>(order + n16);
   uint32_t* bin_hist     = reinterpret_cast<uint32_t*>(bins + n16);
-  unsigned char* ok      = reinterpret_cast<unsigned char*>(bin_hist + kTraceBins);
+  uint32_t* bin_counts   = bin_hist + kTraceBins;
+  unsigned char* ok      = reinterpret_cast<unsigned char*>(bin_counts + static_cast<size_t>(sort_blocks) * kTraceBins);
   VDBG_CUDA(cudaMemcpyAsync(q, origins, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, s));
   VDBG_CUDA(cudaMemcpyAsync(q + 3 * nn, directions, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, s));
   VDBG_CUDA(cudaMemcpyAsync(q + 6 * nn, max_lengths, nn * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -3143,34 +3146,35 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   const MapConf& mc = m->conf[mp];
   const uint32_t n32 = static_cast<uint32_t>(nn);
   VDBG_CUDA(cudaMemsetAsync(m->fast_ctr, 0, 2 * sizeof(unsigned long long), s));
-  VDBG_CUDA(cudaMemsetAsync(bin_hist, 0, kTraceBins * sizeof(uint32_t), s));
-  k_trace_bin<<<(n32 + 255) / 256, 256, 0, s>>>(q, n32, mc.inv_res, bins, bin_hist);
-  k_trace_offsets<<<1, 1024, 0, s>>>(bin_hist);
-  k_trace_scatter<<<(n32 + 255) / 256, 256, 0, s>>>(bins, n32, bin_hist, order);
   const SpanBuf<SpanRec> sb{m->fast_spans, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
-  const RayShape all = ray_shape(m, n32, kSpanThreads);
-  k_trace_spans<<<all.blocks, all.threads, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, order, ok, end,
-                                                   sb, all.lanes);
-  VDBG_CUDA(cudaGetLastError());
-  uint32_t spans = 0;
-  VDBG_CUDA(cudaMemcpyAsync(&spans, m->fast_ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  VDBG_CUDA(cudaStreamSynchronize(s));
-  m->timings.launches += 4;
-  if (spans > 0)
+  const RayShape all = ray_shape(m, n32, kSpanThreads), some = ray_shape(m, n32, 128);
+  // The orders pay where a warp's lanes wait for one another: a warp with a single
+  // query needs none (1000 queries 157 us on the device, 198 with both sorts).
+  const bool sort = all.lanes > 1;
+  if (sort)
   {
-    spans = std::min(spans, m->fast_cap);
-    VDBG_CUDA(cudaMemsetAsync(m->fast_hist, 0, kSpanClasses * sizeof(uint32_t), s));
-    const unsigned sblocks = (spans + 255) / 256;
-    k_span_hist<<<std::min<unsigned>(sblocks, static_cast<unsigned>(m->num_sms) * 4u), 256, 0, s>>>(
-      m->fast_spans, spans, m->fast_hist);
-    k_span_offsets<<<1, 32, 0, s>>>(m->fast_hist);
-    k_span_scatter<<<sblocks, 256, 0, s>>>(m->fast_spans, spans, m->fast_hist, m->fast_sorted);
-    const RayShape some = ray_shape(m, spans, 128);
-    k_trace_walk<<<some.blocks, some.threads, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, m->active,
-                                                      ok, end, m->fast_spans, m->fast_sorted, spans, some.lanes);
-    VDBG_CUDA(cudaGetLastError());
-    m->timings.launches += 4;
+    const uint32_t per = (n32 + sort_blocks - 1) / sort_blocks;
+    k_trace_bin<<<sort_blocks, kTraceSortThreads, 0, s>>>(q, n32, per, mc.inv_res, bins, bin_counts);
+    k_trace_sums<<<(kTraceBins + 63) / 64, 64, 0, s>>>(bin_counts, sort_blocks, bin_hist);
+    k_trace_offsets<<<1, 1024, 0, s>>>(bin_hist);
+    k_trace_scatter<<<sort_blocks, kTraceSortThreads, 0, s>>>(bins, n32, per, bin_counts, bin_hist, order);
   }
+  k_trace_spans<<<all.blocks, all.threads, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv,
+                                                   sort ? order : nullptr, ok, end, sb, all.lanes);
+  if (sort)
+  {
+    VDBG_CUDA(cudaMemsetAsync(m->fast_hist, 0, kSpanClasses * sizeof(uint32_t), s));
+    const unsigned sblocks = (n32 + 255) / 256;
+    k_span_hist<<<std::min<unsigned>(sblocks, static_cast<unsigned>(m->num_sms) * 4u), 256, 0, s>>>(
+      m->fast_spans, sb.count, m->fast_hist);
+    k_span_offsets<<<1, 32, 0, s>>>(m->fast_hist);
+    k_span_scatter<<<sblocks, 256, 0, s>>>(m->fast_spans, sb.count, m->fast_hist, m->fast_sorted);
+  }
+  k_trace_walk<<<some.blocks, some.threads, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, m->active, ok,
+                                                    end, m->fast_spans, sort ? m->fast_sorted : nullptr, sb.count,
+                                                    some.lanes);
+  VDBG_CUDA(cudaGetLastError());
+  m->timings.launches += sort ? 9 : 2;
   VDBG_CUDA(cudaEventRecord(m->ev_dda, s));
   VDBG_CUDA(cudaMemcpyAsync(end_points, end, 3 * nn * sizeof(double), cudaMemcpyDeviceToHost, s));
   VDBG_CUDA(cudaMemcpyAsync(successes, ok, nn, cudaMemcpyDeviceToHost, s));
