@@ -1205,8 +1205,86 @@ __global__ void __launch_bounds__(kSweepWarps * 32, kSweepBlocks)
     if (threadIdx.x == 0)
     {
       __threadfence();
-      if (atomicAdd(&st->sweep_blocks, 1u) == gridDim.x - 1u) finish_window(c, st);
+      if (atomicAdd(&st->sweep_blocks, 1u) == gridDim.x - 1u)
+      {
+        st->sweep_blocks = 0u;
+        finish_window(c, st);
+      }
     }
+  }
+}
+
+// Word of the plane of x (`a`, 0-7) of a leaf in OpenVDB's order, bit
+// (y << 3) | z, from the z-plane words (bit (y << 3) | x): an 8 x 8 x 8
+// transposition of x and z, the same both ways.
+template <class Word>
+__device__ __forceinline__ unsigned long long swap_mask_word(Word&& word, int a)
+{
+  unsigned long long out = 0ull;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) out |= ((word(b) >> a) & 0x0101010101010101ull) << b;
+  return out;
+}
+
+// A short change list in the order of its origins, in two kernels. Keys first: the
+// leaves of map `map` (-1: all) as their origins' order, with the map's own order
+// after it; head[0] counts them (0 at the start), head[1] is the length of the
+// list (above `rows` nothing is done).
+__global__ void __launch_bounds__(256) k_change_keys(ChangeView ch, const int4* __restrict__ origin, int map,
+                                                     uint32_t rows, ulonglong2* __restrict__ keys,
+                                                     uint32_t* __restrict__ head)
+{
+  const uint32_t n = *ch.count;
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0u) head[1] = n;
+  if (n > rows || k >= n) return;
+  const int slot = ch.list[k];
+  const int4 o   = origin[slot];
+  if (map >= 0 && o.w != map) return;
+  constexpr int kBias = 1 << 22;
+  const unsigned long long x = static_cast<unsigned long long>((o.x + kBias) >> 3),
+                           y = static_cast<unsigned long long>((o.y + kBias) >> 3),
+                           z = static_cast<unsigned long long>((o.z + kBias) >> 3);
+  keys[atomicAdd(head, 1u)] = make_ulonglong2((x << 42) | (y << 21) | z, static_cast<unsigned long long>(slot));
+}
+
+// One warp per leaf: its place is the number of smaller keys (equal origins, of
+// different maps, by slot); its origin and its words in OpenVDB's order go to row
+// `place` of pinned memory. Quadratic, but of 2,000 leaves a warp compares 63 keys
+// a lane. An export of 2,110 leaves takes 54 us, of 10,079 236 (gathered, fetched
+// and sorted on the host 560 and 2,100).
+__global__ void __launch_bounds__(256) k_change_rows(ChangeView ch, const ulonglong2* __restrict__ keys,
+                                                     const uint32_t* __restrict__ head, uint32_t rows,
+                                                     int* __restrict__ out_o, unsigned long long* __restrict__ out_a,
+                                                     unsigned long long* __restrict__ out_v, uint32_t* __restrict__ out_n)
+{
+  const uint32_t listed = head[1], n = head[0];
+  if (blockIdx.x == 0u && threadIdx.x == 0u)
+  {
+    out_n[0] = n;
+    out_n[1] = listed;
+  }
+  const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane   = static_cast<int>(threadIdx.x & 31);
+  if (listed > rows || j >= n) return;
+  const ulonglong2 mine = keys[j];
+  uint32_t place        = 0;
+  for (uint32_t k = static_cast<uint32_t>(lane); k < n; k += 32u)
+  {
+    const ulonglong2 other = keys[k];
+    place += other.x < mine.x || (other.x == mine.x && other.y < mine.y) ? 1u : 0u;
+  }
+  place = __reduce_add_sync(0xffffffffu, place);
+  // Lanes 0-7 hold the words flipped, 8-15 those flipped on.
+  const unsigned long long w = lane < 16 ? ch.words[mine.y * 16ull + static_cast<unsigned long long>(lane)] : 0ull;
+  const unsigned long long v = swap_mask_word([&](int b) { return __shfl_sync(0xffffffffu, w, (lane & 8) | b); }, lane & 7);
+  if (lane < 8) out_a[static_cast<size_t>(place) * 8 + lane] = v;
+  if (lane >= 8 && lane < 16) out_v[static_cast<size_t>(place) * 8 + (lane & 7)] = v;
+  if (lane >= 16 && lane < 19)
+  {
+    const int shift = lane == 16 ? 42 : lane == 17 ? 21 : 0;
+    out_o[static_cast<size_t>(place) * 3 + (lane - 16)] =
+      static_cast<int>(((mine.x >> shift) & 0x1fffffull) << 3) - (1 << 22);
   }
 }
 
@@ -1456,18 +1534,6 @@ __global__ void k_section_origins(const uint32_t* __restrict__ list, uint32_t n,
 {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = origin[list[i]];
-}
-
-// Word of the plane of x (`a`, 0-7) of a leaf in OpenVDB's order, bit
-// (y << 3) | z, from the z-plane words (bit (y << 3) | x): an 8 x 8 x 8
-// transposition of x and z, the same both ways.
-template <class Word>
-__device__ __forceinline__ unsigned long long swap_mask_word(Word&& word, int a)
-{
-  unsigned long long out = 0ull;
-#pragma unroll
-  for (int b = 0; b < 8; ++b) out |= ((word(b) >> a) & 0x0101010101010101ull) << b;
-  return out;
 }
 
 // Does a plane (w) of leaf `slot` hold a voxel of the section (getMapSection: an

@@ -157,8 +157,9 @@ struct vdbg_map
   std::mutex work_mutex;
   char* work[2]         = {nullptr, nullptr};
   size_t work_bytes[2]  = {0, 0};
-  char* sec_host        = nullptr;  // pinned: a small section's count, masks and origins
-  size_t sec_bytes      = 0;
+  char* pin             = nullptr;  // pinned: a small result's count and rows
+  size_t pin_bytes      = 0;
+  uint32_t chg_rows     = 0;  // rows of the longest change list fetched in one go
 
   int64_t bytes         = 0;
   int num_sms           = 152;
@@ -228,6 +229,8 @@ constexpr uint32_t kMinBlocks       = 1u << 10;
 constexpr size_t kWorkKept          = size_t(64) << 20;
 constexpr uint32_t kSectionPinned   = 1u << 15;  // boxes of at most this many leaf cells are written at once
 constexpr size_t kSectionRow        = 8 * sizeof(uint64_t) + 3 * sizeof(int32_t);
+constexpr size_t kPinnedAtStart      = size_t(320) << 10;  // (2,048 rows of a change list, 4,300 of a section)
+constexpr uint32_t kChangeRows      = 1u << 14;  // change lists of at most this many leaves are ordered on the device
 constexpr int64_t kMorphCells       = int64_t(1) << 18;  // leaf cells of a set taken as a dense grid (37 MB)
 constexpr int64_t kSectionCells     = int64_t(1) << 20;  // boxes of more leaf cells list the map's leaves
 
@@ -834,6 +837,7 @@ void clear_error_keep_counters(vdbg_map* m)
   m->h_status->n_blocks = m->n_blocks;
 }
 
+int pinned_ensure(vdbg_map* m, size_t bytes);
 int map_error(uint32_t err);
 int grow_for(vdbg_map* m, uint64_t requested);
 int grow_blocks_for(vdbg_map* m, uint64_t requested);
@@ -931,6 +935,8 @@ int settle_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, 
 // hits (VDBMapping.hpp:533-536), into channel `c`, with one status fetch
 // (more after a pool or hash that ran out).
 int reset_changes(vdbg_map* m, cudaStream_t s);
+int export_changes_short(vdbg_map* m, int map, int64_t capacity, int32_t* origins, uint64_t* active, uint64_t* value,
+                         int64_t* n_out, uint32_t* listed, bool* done);
 int launch_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated);
 
 // `eager`: the channel's window is the only one the call integrates, so its
@@ -1641,14 +1647,22 @@ int accumulate_and_integrate(vdbg_map* m, const float* xyz, int64_t n, int64_t s
   if (integrate_all || only) VDBG_TRY(reset_changes(m, s));
   for (Channel* c : todo)
   {
-    VDBG_TRY(launch_sweep(m, *c, s));
+    VDBG_TRY(launch_sweep(m, *c, s, m->art_n == 0));
     if (m->art_n > 0) VDBG_TRY(reactivate_artificial(m, *c, s));
   }
   VDBG_TRY(fetch_status(m, s));
   if (m->h_status->error != 0u) return map_error(m->h_status->error);
   record_timings(m);
-  for (Channel* c : todo) VDBG_TRY(finish_sweep(m, *c, s));
-  if (!todo.empty()) VDBG_CUDA(cudaStreamSynchronize(s));
+  // (artificial voxels are set from the window's block list after its sweep, so
+  // their windows are closed here, the others by the sweep)
+  for (Channel* c : todo)
+  {
+    if (m->art_n > 0)
+      VDBG_TRY(finish_sweep(m, *c, s));
+    else
+      c->pending = false;
+  }
+  if (!todo.empty() && m->art_n > 0) VDBG_CUDA(cudaStreamSynchronize(s));
   fill_stats(m, leaves_before, stats);
   VDBG_TRY(end_call(m, s));
   return call_status;
@@ -1799,6 +1813,7 @@ int create_impl(int n_maps, const double* resolutions, const vdbg_options* optio
     return fail(VDBG_ERR_OUT_OF_MEMORY);
   clear_status(m->h_status);
   int s = dev_alloc(m, &m->d_status, 1);
+  if (s == VDBG_OK) s = pinned_ensure(m, kPinnedAtStart);
   if (s != VDBG_OK) return fail(s);
   m->buckets = static_cast<uint32_t>(kBucketsPerScan) * static_cast<uint32_t>(n_maps);
   s          = dev_alloc(m, &m->d_hist, m->buckets);
@@ -1984,7 +1999,7 @@ int vdbg_destroy(vdbg_map* m)
   dev_free(m, m->d_order, m->ray_cap);
   dev_free(m, m->axis_mem, kAxisTableBytes);
   work_done(m, 0);
-  if (m->sec_host) cudaFreeHost(m->sec_host);
+  if (m->pin) cudaFreeHost(m->pin);
   dev_free(m, m->topo_keys, 2 * static_cast<size_t>(m->topo_cap));
   dev_free(m, m->topo_box, 8);
   dev_free(m, m->d_trace, m->trace_bytes);
@@ -2393,8 +2408,12 @@ int vdbg_export_changes(vdbg_map* m, int map, int64_t capacity, int32_t* origins
   VDBG_TRY(set_device(m));
   cudaStream_t s = m->stream;
   uint32_t n     = 0;
-  VDBG_CUDA(cudaMemcpyAsync(&n, m->chg_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  VDBG_CUDA(cudaStreamSynchronize(s));
+  {
+    bool done = false;
+    std::lock_guard<std::mutex> lock(m->work_mutex);
+    const int st = export_changes_short(m, map, capacity, origins, active, value, n_out, &n, &done);
+    if (st != VDBG_OK || done) return st;
+  }
   std::vector<int4> o;
   std::vector<unsigned long long> w;
   uint32_t kept = 0;
@@ -2543,6 +2562,65 @@ bool leaf_origin_ok(const int32_t* o)
   return true;
 }
 
+// Pinned memory of the calls that fetch small results (with the workspaces).
+int pinned_ensure(vdbg_map* m, size_t bytes)
+{
+  if (bytes <= m->pin_bytes) return VDBG_OK;
+  if (m->pin) cudaFreeHost(m->pin);
+  m->pin       = nullptr;
+  m->pin_bytes = 0;
+  bytes        = (bytes + 0xffff) & ~size_t(0xffff);
+  VDBG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->pin), bytes));
+  m->pin_bytes = bytes;
+  return VDBG_OK;
+}
+
+// vdbg_export_changes for a list of at most kChangeRows leaves, ordered on the
+// device and fetched in one go. *listed: the list's length; *done: this was it.
+int export_changes_short(vdbg_map* m, int map, int64_t capacity, int32_t* origins, uint64_t* active, uint64_t* value,
+                         int64_t* n_out, uint32_t* listed, bool* done)
+{
+  cudaStream_t s = m->stream;
+  ChangeView ch{};
+  ch.words = m->chg_words;
+  ch.list  = m->chg_list;
+  ch.count = m->chg_count;
+  // (room for the usual list; a longer one says how long it is and goes again)
+  for (uint32_t rows = std::max(2048u, m->chg_rows);;)
+  {
+    constexpr size_t kRow = 16 * sizeof(uint64_t) + 3 * sizeof(int32_t);
+    VDBG_TRY(pinned_ensure(m, 64 + rows * kRow));
+    VDBG_TRY(work_ensure(m, 0, rows * sizeof(ulonglong2) + 64));
+    uint32_t* head          = reinterpret_cast<uint32_t*>(m->work[0]);
+    ulonglong2* keys        = reinterpret_cast<ulonglong2*>(m->work[0] + 64);
+    volatile uint32_t* h_n  = reinterpret_cast<uint32_t*>(m->pin);
+    unsigned long long* h_a = reinterpret_cast<unsigned long long*>(m->pin + 64);
+    unsigned long long* h_v = h_a + 8 * static_cast<size_t>(rows);
+    int* h_o                = reinterpret_cast<int*>(h_v + 8 * static_cast<size_t>(rows));
+    VDBG_CUDA(cudaMemsetAsync(head, 0, 2 * sizeof(uint32_t), s));
+    k_change_keys<<<rows / 256, 256, 0, s>>>(ch, m->origin, map, rows, keys, head);
+    k_change_rows<<<rows / 8, 256, 0, s>>>(ch, keys, head, rows, h_o, h_a, h_v, reinterpret_cast<uint32_t*>(m->pin));
+    VDBG_CUDA(cudaGetLastError());
+    VDBG_CUDA(cudaStreamSynchronize(s));
+    const uint32_t kept = h_n[0];
+    *listed             = h_n[1];
+    if (*listed > kChangeRows) return VDBG_OK;
+    if (*listed > rows)
+    {
+      rows        = (*listed + 2047u) & ~2047u;
+      m->chg_rows = rows;
+      continue;
+    }
+    *done  = true;
+    *n_out = kept;
+    if (static_cast<int64_t>(kept) > capacity) return VDBG_ERR_BUFFER_TOO_SMALL;
+    if (origins) std::memcpy(origins, h_o, kept * 3 * sizeof(int32_t));
+    if (active) std::memcpy(active, h_a, kept * 8 * sizeof(uint64_t));
+    if (value) std::memcpy(value, h_v, kept * 8 * sizeof(uint64_t));
+    return VDBG_OK;
+  }
+}
+
 // A section box's corner, brought to just outside the index range (differences
 // with voxel indices stay within int).
 int3 box_corner(const int32_t v[3])
@@ -2629,26 +2707,18 @@ int section_export_small(vdbg_map* m, int mp, int3 lo, int3 hi, int3 first, int3
                          int64_t capacity, int32_t* origins, float* values, uint64_t* masks, int64_t* n_out)
 {
   cudaStream_t s = m->stream;
-  const size_t pinned = (n * kSectionRow + 64 + 0xffff) & ~size_t(0xffff);
-  if (pinned > m->sec_bytes)
-  {
-    if (m->sec_host) cudaFreeHost(m->sec_host);
-    m->sec_host  = nullptr;
-    m->sec_bytes = 0;
-    VDBG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->sec_host), pinned));
-    m->sec_bytes = pinned;
-  }
+  VDBG_TRY(pinned_ensure(m, n * kSectionRow + 64));
   VDBG_TRY(work_ensure(m, 0, static_cast<size_t>(n) * 3 * sizeof(uint32_t) + 256));
   if (values) VDBG_TRY(work_ensure(m, 1, static_cast<size_t>(n) * 512 * sizeof(float)));
   int* cand                  = reinterpret_cast<int*>(m->work[0]);
   uint32_t* keep             = reinterpret_cast<uint32_t*>(cand) + n;
   uint32_t* pos              = keep + n;
-  volatile uint32_t* kept_at = reinterpret_cast<uint32_t*>(m->sec_host);
-  unsigned long long* h_m    = reinterpret_cast<unsigned long long*>(m->sec_host + 64);
+  volatile uint32_t* kept_at = reinterpret_cast<uint32_t*>(m->pin);
+  unsigned long long* h_m    = reinterpret_cast<unsigned long long*>(m->pin + 64);
   int* h_o                   = reinterpret_cast<int*>(h_m + 8 * static_cast<size_t>(n));
   k_section_find<<<static_cast<unsigned>((static_cast<uint64_t>(n) * 8 + 255) / 256), 256, 0, s>>>(
     map_view(m), mp, m->flags, first, dims, n, m->values, m->active, lo, hi, full, cand, keep);
-  k_section_scan<<<1, 1024, 0, s>>>(keep, n, pos, reinterpret_cast<uint32_t*>(m->sec_host));
+  k_section_scan<<<1, 1024, 0, s>>>(keep, n, pos, reinterpret_cast<uint32_t*>(m->pin));
   k_section_write<<<static_cast<unsigned>((static_cast<uint64_t>(n) * 32 + 255) / 256), 256, 0, s>>>(
     cand, n, keep, pos, m->origin, m->values, m->active, lo, hi, full, h_o,
     values ? reinterpret_cast<float*>(m->work[1]) : nullptr, h_m);

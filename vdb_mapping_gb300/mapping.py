@@ -67,11 +67,11 @@ def _export_changes(lib, h, map_index, check):
     """(origins (L,3) int32, active (L,8) uint64, value (L,8) uint64) of the
     last integration's change set."""
     n = C.c_int64()
-    cap = 1024
+    cap = 16384  # (only the rows returned are ever written)
     while True:
-        origins = np.zeros((cap, 3), np.int32)
-        active = np.zeros((cap, 8), np.uint64)
-        value = np.zeros((cap, 8), np.uint64)
+        origins = np.empty((cap, 3), np.int32)
+        active = np.empty((cap, 8), np.uint64)
+        value = np.empty((cap, 8), np.uint64)
         s = lib.vdbg_export_changes(h, int(map_index), cap, origins.ctypes.data, active.ctypes.data,
                                     value.ctypes.data, C.byref(n))
         if s == _lib.STATUS_CODE["VDBG_ERR_BUFFER_TOO_SMALL"]:
