@@ -268,11 +268,12 @@ def _raytrace(lib, h, map_index, origins, directions, max_lengths, check):
     if d.shape[0] != n:
         raise ValueError("origins and directions differ in length")
     ln = np.ascontiguousarray(np.broadcast_to(np.asarray(max_lengths, np.float64), (n,)))
-    ok = np.zeros(n, np.uint8)
-    ends = np.zeros((n, 3), np.float64)
+    # (every query is answered; empty arrays take no pass of zeros first)
+    ok = np.empty(n, np.uint8)
+    ends = np.empty((n, 3), np.float64)
     check(lib.vdbg_raytrace(h, int(map_index), n, o.ctypes.data, d.ctypes.data, ln.ctypes.data, ok.ctypes.data,
                             ends.ctypes.data), "vdbg_raytrace")
-    return ok.astype(bool), ends
+    return ok.view(bool), ends
 
 
 class OccupancyVDBMapping:
