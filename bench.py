@@ -43,10 +43,13 @@ STATUS_BYTES = 88  # device status block (DevStatus) read back by every call
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch of
 # each kernel on a steady-state dense scan, from one ncu capture of the
-# default workload's launch list (the last of three inserts; prep = k_prep +
-# k_scatter). Only meaningful for the dense workload; other workloads report
+# default workload's launch list (the last of three inserts). Only meaningful for the dense workload; other workloads report
 # None.
-NCU_TRAFFIC_BYTES = {}
+NCU_TRAFFIC_BYTES = {
+    "prep (k_prep+k_scan+k_scatter)": 8_498_688,
+    "k_march": 330_307_072,  # with k_mark_hits
+    "k_sweep": 1_991_856_384,
+}
 
 
 def parse_args():
@@ -516,9 +519,9 @@ def run_ours(args):
         "marking (k_mark_hits+k_march)": {
             "ms": dda, "algorithmic_atomics": mean_v,
             "traffic": traffic.get("k_march")},
-        "sweep (k_compact+k_sweep)": {"ms": sweep, "algorithmic_bytes": 8.25 * mean_u + 128.0 * mean_lt,
-                                      "GBps": (8.25 * mean_u + 128.0 * mean_lt) / (sweep / 1000.0) / 1e9,
-                                      "traffic": traffic.get("k_sweep")},
+        "sweep (k_sweep)": {"ms": sweep, "algorithmic_bytes": 8.25 * mean_u + 128.0 * mean_lt,
+                            "GBps": (8.25 * mean_u + 128.0 * mean_lt) / (sweep / 1000.0) / 1e9,
+                            "traffic": traffic.get("k_sweep")},
     }
 
     line = {
@@ -531,7 +534,7 @@ def run_ours(args):
         "latency_ms": {"p50": float(np.percentile(step_ms, 50)), "p99": float(np.percentile(step_ms, 99)),
                        "max": max(step_ms)},
         "phases_ms": {"prep": prep, "marking (k_mark_hits+k_march)": dda,
-                      "sweep (k_compact+k_sweep)": sweep, "kernels_total": mean_total_ms},
+                      "sweep (k_sweep)": sweep, "kernels_total": mean_total_ms},
         "per_scan": {"rays": n_pts, "visits": statistics.mean(s["visits"] for s in stats),
                      "runs": mean_runs, "updates": mean_u, "touched_leaves": mean_lt,
                      "new_leaves": statistics.mean(s["new_leaves"] for s in stats),

@@ -12,17 +12,19 @@
 //   k_mark_hits VDBMapping.hpp:533-536  hit bits of unclipped endpoints
 //   k_compact  (none)                   touched blocks -> flat touched-leaf list
 //                                       (a dropped marking)
-//   k_sweep    VDBMapping.hpp:731-792 + per touched leaf: FP32 log-odds update,
-//              OccupancyVDBMapping.hpp:92-117  thresholds, clamp, active mask;
-//                                       clears the update masks
+//   k_sweep    VDBMapping.hpp:731-792 + finds the touched leaves; per leaf the FP32
+//              OccupancyVDBMapping.hpp:92-117  log-odds update, thresholds, clamp,
+//                                       active mask; clears the update masks
+//   k_change_* VDBMapping.hpp:733-781   the change set in order
+//   k_section_* VDBMapping.hpp:883-1085 map sections out of and into the map
 //   k_rehash   (none)                   rebuilds the block hash after growth
 //   k_topo_build VDBMapping.hpp:1436-1449  the volume ray intersector's view of
 //                                       the map: node sets and active-leaf box
 //   k_fast_spans, k_fast_walk VDBMapping.hpp:577-602  fast mode: the
 //                                       intersector's spans of each ray, then
 //                                       the active map voxels along each span
-//   k_trace_spans, k_trace_walk VDBMapping.hpp:675-721  raytrace queries:
-//                                       first spans, then the voxel walks
+//   k_trace_*  VDBMapping.hpp:675-721   raytrace queries: their order, the first
+//                                       spans, then the voxel walks
 //   k_morph_*  VDBMapping.hpp:1094-1147 dilation / erosion of section leaves
 //   k_wall_voxels VDBMapping.hpp:1210-1236  artificial walls, castRayIntoGrid per layer
 //   k_artificial_restore VDBMapping.hpp:1153-1166  restoreMapIntegrity
