@@ -303,15 +303,23 @@ int work_ensure(vdbg_map* m, int k, size_t bytes)
   if (bytes <= m->work_bytes[k]) return VDBG_OK;
   dev_free(m, m->work[k], m->work_bytes[k]);
   m->work_bytes[k] = 0;
-  const size_t want = (bytes + bytes / 4 + 0xfffff) & ~size_t(0xfffff);
-  VDBG_TRY(dev_alloc(m, &m->work[k], want));
-  m->work_bytes[k] = want;
-  return VDBG_OK;
+  size_t want = (bytes + bytes / 4 + 0xfffff) & ~size_t(0xfffff);
+  int st      = dev_alloc(m, &m->work[k], want);
+  if (st != VDBG_OK)
+  {
+    // (a tight budget: without the room to spare)
+    want = bytes;
+    st   = dev_alloc(m, &m->work[k], want);
+  }
+  if (st == VDBG_OK) m->work_bytes[k] = want;
+  return st;
 }
 
-// The end of a call that used the workspaces: large ones are given back.
+// The end of a call that used the workspaces: large ones are given back, and all of
+// them under a budget, which they would take from the pools.
 void work_done(vdbg_map* m, size_t keep = kWorkKept)
 {
+  if (m->max_bytes > 0) keep = 0;
   for (int k = 0; k < 2; ++k)
     if (m->work_bytes[k] > keep)
     {
@@ -1813,8 +1821,8 @@ int create_impl(int n_maps, const double* resolutions, const vdbg_options* optio
     return fail(VDBG_ERR_OUT_OF_MEMORY);
   clear_status(m->h_status);
   int s = dev_alloc(m, &m->d_status, 1);
-  if (s == VDBG_OK) s = pinned_ensure(m, kPinnedAtStart);
   if (s != VDBG_OK) return fail(s);
+  pinned_ensure(m, kPinnedAtStart);  // (calls ask again for what they need)
   m->buckets = static_cast<uint32_t>(kBucketsPerScan) * static_cast<uint32_t>(n_maps);
   s          = dev_alloc(m, &m->d_hist, m->buckets);
   if (s != VDBG_OK) return fail(s);
@@ -2411,7 +2419,14 @@ int vdbg_export_changes(vdbg_map* m, int map, int64_t capacity, int32_t* origins
   {
     bool done = false;
     std::lock_guard<std::mutex> lock(m->work_mutex);
-    const int st = export_changes_short(m, map, capacity, origins, active, value, n_out, &n, &done);
+    int st = export_changes_short(m, map, capacity, origins, active, value, n_out, &n, &done);
+    work_done(m, st == VDBG_ERR_OUT_OF_MEMORY ? 0 : kWorkKept);
+    if (st == VDBG_ERR_OUT_OF_MEMORY)
+    {
+      VDBG_CUDA(cudaMemcpyAsync(&n, m->chg_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      VDBG_CUDA(cudaStreamSynchronize(s));
+      st = VDBG_OK;
+    }
     if (st != VDBG_OK || done) return st;
   }
   std::vector<int4> o;
@@ -2570,7 +2585,12 @@ int pinned_ensure(vdbg_map* m, size_t bytes)
   m->pin       = nullptr;
   m->pin_bytes = 0;
   bytes        = (bytes + 0xffff) & ~size_t(0xffff);
-  VDBG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->pin), bytes));
+  if (cudaMallocHost(reinterpret_cast<void**>(&m->pin), bytes) != cudaSuccess)
+  {
+    cudaGetLastError();
+    m->pin = nullptr;
+    return VDBG_ERR_OUT_OF_MEMORY;
+  }
   m->pin_bytes = bytes;
   return VDBG_OK;
 }
@@ -2745,7 +2765,11 @@ int section_export(vdbg_map* m, int mp, int3 lo, int3 hi, int full, int64_t capa
   const uint32_t cells = m->n_leaves > 0 ? section_cells(lo, hi, &first, &dims) : 0u;
   if (cells == 0) return VDBG_OK;
   if (cells <= kSectionPinned)
-    return section_export_small(m, mp, lo, hi, first, dims, cells, full, capacity, origins, values, masks, n_out);
+  {
+    // (its room for every cell may not fit a budget that the leaves fit)
+    const int st = section_export_small(m, mp, lo, hi, first, dims, cells, full, capacity, origins, values, masks, n_out);
+    if (st != VDBG_ERR_OUT_OF_MEMORY) return st;
+  }
   int* cand  = nullptr;
   uint32_t n = 0, kept = 0;
   VDBG_TRY(section_candidates(m, mp, lo, hi, &cand, &n));
@@ -3187,12 +3211,12 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   VDBG_TRY(begin_call(m, s));
   const size_t nn    = static_cast<size_t>(n);
   // queries (7 doubles) and end points (3), then the order (u32), the bins
-  // (u16), the bins' offsets, the sort blocks' counts and the success flags
+  // (u16), the bins' offsets and the success flags
   const size_t n16   = (nn + 15) & ~static_cast<size_t>(15);
   const uint32_t sort_blocks =
     std::min<uint32_t>(static_cast<uint32_t>(m->num_sms), static_cast<uint32_t>((nn + 4095) / 4096));
   const size_t bytes = nn * 10 * sizeof(double) + n16 * (sizeof(uint32_t) + sizeof(unsigned short)) +
-                       (static_cast<size_t>(sort_blocks) + 1) * kTraceBins * sizeof(uint32_t) + n16;
+                       kTraceBins * sizeof(uint32_t) + n16;
   if (bytes > m->trace_bytes)
   {
     dev_free(m, m->d_trace, m->trace_bytes);
@@ -3207,8 +3231,10 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   uint32_t* order        = reinterpret_cast<uint32_t*>(q + 10 * nn);
   unsigned short* bins   = reinterpret_cast<unsigned short*>(order + n16);
   uint32_t* bin_hist     = reinterpret_cast<uint32_t*>(bins + n16);
-  uint32_t* bin_counts   = bin_hist + kTraceBins;
-  unsigned char* ok      = reinterpret_cast<unsigned char*>(bin_counts + static_cast<size_t>(sort_blocks) * kTraceBins);
+  // (the blocks' counts lie where the end points will: 8 bytes a query of their 24,
+  // where queries are sorted)
+  uint32_t* bin_counts   = reinterpret_cast<uint32_t*>(end);
+  unsigned char* ok      = reinterpret_cast<unsigned char*>(bin_hist + kTraceBins);
   VDBG_CUDA(cudaMemcpyAsync(q, origins, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, s));
   VDBG_CUDA(cudaMemcpyAsync(q + 3 * nn, directions, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, s));
   VDBG_CUDA(cudaMemcpyAsync(q + 6 * nn, max_lengths, nn * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -3223,7 +3249,7 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   const RayShape all = ray_shape(m, n32, kSpanThreads), some = ray_shape(m, n32, 128);
   // The orders pay where a warp's lanes wait for one another: a warp with a single
   // query needs none (1000 queries 157 us on the device, 198 with both sorts).
-  const bool sort = all.lanes > 1;
+  const bool sort = all.lanes > 1 && static_cast<size_t>(sort_blocks) * kTraceBins * sizeof(uint32_t) <= nn * 24;
   if (sort)
   {
     const uint32_t per = (n32 + sort_blocks - 1) / sort_blocks;
@@ -3300,8 +3326,8 @@ int vdbg_section_morphology(vdbg_map* m, int op, int iterations, int64_t n, cons
       std::lock_guard<std::mutex> lock(m->work_mutex);
       const int st =
         morph_grid(m, op, iterations, keep, g, n, origins, masks, capacity, out_origins, out_masks, n_out);
-      work_done(m);
-      return st;
+      work_done(m, st == VDBG_ERR_OUT_OF_MEMORY ? 0 : kWorkKept);
+      if (st != VDBG_ERR_OUT_OF_MEMORY) return st;
     }
   }
   // Unique leaves (masks of a repeated origin are merged).
