@@ -788,7 +788,7 @@ def measure_serving(local, seconds, budget_gb, use_graph=True, drift=None):
     batch.useGraph(use_graph)
     for i, c in enumerate(wl.configs):
         batch.setConfig(i, c)
-    # Warm the scratch and run buffers with one scan per map (not timed).
+    # Warm the scratch buffers with one scan per map (not timed).
     batch.insert([scans[(i, 0)][0] for i in range(len(wl.streams))],
                  [scans[(i, 0)][1] for i in range(len(wl.streams))])
     budget = int(budget_gb * (1 << 30))
