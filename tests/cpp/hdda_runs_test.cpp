@@ -188,7 +188,7 @@ int main()
         {
           double e0[3], e1[3];
           H::trace_walk(eye, dir, sp, 0.05, active, e0, steps);
-          H::trace_walk_runs(eye, dir, sp, runs.lo, runs.hi, runs.n, 0.05, active, e1);
+          H::trace_walk_runs(H::make_ray(eye, dir, sp.t0, sp.t1), sp, runs.lo, runs.hi, runs.n, 0.05, active, e1);
           if (std::memcmp(e0, e1, sizeof(e0)) != 0 && bad++ < 20) std::printf("trace case %d kind %d\n", cases, kind);
           ++hits;
           runs0 += runs.n == 0;

@@ -762,12 +762,11 @@ VDBG_HD int trace_walk(const double oi[3], const double di[3], const Span& sp, d
   return kTraceOk;
 }
 
-// The same from the span's windows (RunTrack).
+// The same from the span's windows (RunTrack); `fine` is the query's ray (make_ray).
 template <class Active>
-VDBG_HD void trace_walk_runs(const double oi[3], const double di[3], const Span& sp, const float* lo, const float* hi,
-                             int n, double res, Active&& active, double end[3])
+VDBG_HD void trace_walk_runs(const Ray& fine, const Span& sp, const float* lo, const float* hi, int n, double res,
+                             Active&& active, double end[3])
 {
-  const Ray fine = make_ray(oi, di, sp.t0, sp.t1);
   Dda dda;
   dda_init(dda, fine, sp.t0, sp.t1, 0);
   FineDda f = fine_from(dda);

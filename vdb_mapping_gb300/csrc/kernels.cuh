@@ -2371,7 +2371,7 @@ __global__ void k_fast_visits(DevStatus* st, SpanBuf<FastPiece> sb)
 // answers the queries without one; the spans are sorted by length (longest
 // first, k_span_hist / k_span_scatter), and k_trace_walk walks one span per
 // thread to its first active voxel, in the windows that can hold one
-// (hdda::trace_walk_runs): 0.58 ms for a million spans of 420 voxels, where
+// (hdda::trace_walk_runs): 0.53 ms for a million spans of 420 voxels, where
 // every voxel of them took 2.0. The coarse walk needs
 // many registers and the voxel walk few, so apart each runs at its own
 // occupancy, and the walks of a warp take about as many steps each. q holds
@@ -2540,7 +2540,7 @@ __global__ void __launch_bounds__(kTraceSortThreads) k_trace_scatter(const unsig
 }
 
 // (20 warps an SM, which costs some spills: 16 took 3% longer, 12 without spills as much)
-__global__ void __launch_bounds__(kSpanThreads, 20) k_trace_spans(const double* __restrict__ q, uint32_t n, double res,
+__global__ void __launch_bounds__(kSpanThreads, 20) k_trace_spans(double* q, uint32_t n, double res,
                                                      double inv_res, MapView m, TopoView tv,
                                                      const uint32_t* __restrict__ order,
                                                      unsigned char* __restrict__ ok, double* __restrict__ end,
@@ -2599,6 +2599,15 @@ __global__ void __launch_bounds__(kSpanThreads, 20) k_trace_spans(const double* 
   const float l1 = fabsf(static_cast<float>(di[0])) + fabsf(static_cast<float>(di[1])) + fabsf(static_cast<float>(di[2]));
   r.cls          = 31 - __clz(static_cast<int>(fminf(total * l1 + 1.0f, 1.0e9f)));  // (for ordering only)
   r.pad          = 0;
+  // The walk takes the ray from here: its direction in the query's place, its
+  // inverse where the end point will be. (A root and four divisions it would make
+  // again: a million queries' walks 571 to 528 us, the spans 20 more.)
+  double* dq = q + 3 * static_cast<size_t>(n);
+  for (int a = 0; a < 3; ++a)
+  {
+    dq[3 * static_cast<size_t>(i) + a]  = di[a];
+    end[3 * static_cast<size_t>(i) + a] = hdda::dvd(1.0, di[a]);
+  }
   const uint32_t k = take_slot(sb.count);
   if (k < sb.cap) sb.rec[k] = r;
 }
@@ -2616,14 +2625,21 @@ __global__ void __launch_bounds__(128) k_trace_walk(const double* __restrict__ q
   if (j >= n_spans) return;
   const SpanRec& r = rec[by_class ? by_class[j] : j];
   const uint32_t i = static_cast<uint32_t>(r.ray);
-  double o[3], d[3], len;
-  trace_query(q, n, i, o, d, len);
-  double oi[3], di[3];
-  hdda::trace_ray(o, d, len, inv_res, oi, di);  // in range: its span was found
+  // (k_trace_spans left the direction and its inverse)
+  const double* dq = q + 3 * static_cast<size_t>(n);
+  hdda::Ray ray;
+  for (int a = 0; a < 3; ++a)
+  {
+    ray.eye[a] = hdda::mul(q[3 * static_cast<size_t>(i) + a], inv_res);
+    ray.dir[a] = dq[3 * static_cast<size_t>(i) + a];
+    ray.inv[a] = end[3 * static_cast<size_t>(i) + a];
+  }
+  ray.t0 = r.t0;
+  ray.t1 = r.t1;
   ActiveCache act{&m, active, tv.map, 0x7fffffff, 0, 0, -1, -1, -1, 0ull};
   act.bits = tv.leafbits;
   double e[3];
-  hdda::trace_walk_runs(oi, di, hdda::Span{r.t0, r.t1}, r.lo, r.hi, r.n, res, act, e);
+  hdda::trace_walk_runs(ray, hdda::Span{r.t0, r.t1}, r.lo, r.hi, r.n, res, act, e);
   trace_answer(ok, end, i, true, e);
 }
 
