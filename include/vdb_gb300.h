@@ -363,6 +363,12 @@ int vdbg_restore_map_integrity(vdbg_map* map);
  * VDBG_ERR_INVALID_ARGUMENT when the leaf exists. */
 int vdbg_test_stall_leaf(vdbg_map* map, int map_index, int32_t lx, int32_t ly, int32_t lz);
 
+/* Test hook for a device short of memory (no counterpart in the reference).
+ * Of the map's coming device allocations (workspaces, scratch; not the pools),
+ * `skip` go through and the `count` after them are refused by the CUDA driver,
+ * as on a full device; then all go through again. */
+int vdbg_test_fail_allocs(vdbg_map* map, int64_t skip, int64_t count);
+
 /* Morphology of a map section's active voxels with the 26-neighbourhood:
  * openvdb::tools::dilateActiveValues / erodeActiveValues with
  * NN_FACE_EDGE_VERTEX as VDBMapping.hpp:1094-1147 calls them

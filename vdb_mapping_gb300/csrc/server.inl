@@ -73,7 +73,11 @@ public:
     size_t c = 4096;
     while (c < bytes) c <<= 1;
     void* p = nullptr;
-    if (cudaMallocHost(&p, c) != cudaSuccess) return nullptr;
+    if (cudaMallocHost(&p, c) != cudaSuccess)
+    {
+      cudaGetLastError();
+      return nullptr;
+    }
     *cap = c;
     return static_cast<float*>(p);
   }
@@ -228,7 +232,10 @@ int ensure_prep(vdbg_map* m, PrepSet& p, int64_t total)
     VDBG_CUDA(cudaMemset(p.hist, 0, m->buckets * sizeof(uint32_t)));
     if (cudaMallocHost(reinterpret_cast<void**>(&p.h_geom), sizeof(ScanGeom) * nm) != cudaSuccess ||
         cudaMallocHost(reinterpret_cast<void**>(&p.h_first), sizeof(uint32_t) * (nm + 1)) != cudaSuccess)
+    {
+      cudaGetLastError();
       return VDBG_ERR_OUT_OF_MEMORY;
+    }
     VDBG_CUDA(cudaEventCreateWithFlags(&p.ready, cudaEventDisableTiming));
   }
   const size_t need_pts = static_cast<size_t>(total) * 16;

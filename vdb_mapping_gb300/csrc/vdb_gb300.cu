@@ -209,16 +209,23 @@ struct vdbg_map
   int4* d_art_o                    = nullptr;
   unsigned long long* d_art_m      = nullptr;
   uint32_t art_n                   = 0;  // leaves in the device copy
+
+  // Allocations the test hook refuses (vdbg_test_fail_allocs).
+  int64_t fail_skip                = 0;
+  int64_t fail_count               = 0;
 };
 
 namespace {
 
+// (A failed call also leaves its error as the thread's last one, where the next
+// launch's check would take it for its own; it is reported here, so it ends here.)
 #define VDBG_CUDA(call)                                                                    \
   do                                                                                       \
   {                                                                                        \
     cudaError_t e_ = (call);                                                               \
     if (e_ != cudaSuccess)                                                                 \
     {                                                                                      \
+      cudaGetLastError();                                                                  \
       std::fprintf(stderr, "vdb_gb300: %s failed: %s\n", #call, cudaGetErrorString(e_));   \
       return e_ == cudaErrorMemoryAllocation ? VDBG_ERR_OUT_OF_MEMORY : VDBG_ERR_CUDA;     \
     }                                                                                      \
@@ -272,7 +279,18 @@ int dev_alloc(vdbg_map* m, T** p, size_t count)
   if (count == 0) return VDBG_OK;
   const size_t b = count * sizeof(T);
   if (m->max_bytes > 0 && m->bytes + static_cast<int64_t>(b) > m->max_bytes) return oom("dev_alloc budget", b);
-  VDBG_CUDA(cudaMalloc(reinterpret_cast<void**>(p), b));
+  size_t ask = b;
+  if (m->fail_count > 0)
+  {
+    if (m->fail_skip > 0)
+      m->fail_skip -= 1;
+    else
+    {
+      m->fail_count -= 1;
+      ask = size_t(1) << 50;  // (no device has it: refused by the driver)
+    }
+  }
+  VDBG_CUDA(cudaMalloc(reinterpret_cast<void**>(p), ask));
   m->bytes += static_cast<int64_t>(b);
   m->layout += 1;
   return VDBG_OK;
@@ -1802,6 +1820,7 @@ int create_impl(int n_maps, const double* resolutions, const vdbg_options* optio
   }
   auto fail = [&](int s) {
     vdbg_destroy(m);
+    cudaGetLastError();
     return s;
   };
   if (cudaSetDevice(m->device) != cudaSuccess) return fail(VDBG_ERR_CUDA);
@@ -2307,6 +2326,7 @@ int vdbg_l2_atomic_rate(int device, int pattern, double* ops_per_s)
   }
   if (st == VDBG_OK && best > 0.f)
     *ops_per_s = static_cast<double>(grid) * 256.0 * iters / (static_cast<double>(best) * 1e-3);
+  if (st != VDBG_OK) cudaGetLastError();
   if (buf) cudaFree(buf);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
@@ -3382,6 +3402,14 @@ int vdbg_export_section(vdbg_map* m, int map, const int32_t lo[3], const int32_t
                                 masks, n_out);
   work_done(m);
   return st;
+}
+
+int vdbg_test_fail_allocs(vdbg_map* m, int64_t skip, int64_t count)
+{
+  if (!m || skip < 0 || count < 0) return VDBG_ERR_INVALID_ARGUMENT;
+  m->fail_skip  = skip;
+  m->fail_count = count;
+  return VDBG_OK;
 }
 
 int vdbg_test_stall_leaf(vdbg_map* m, int map, int32_t lx, int32_t ly, int32_t lz)
