@@ -65,3 +65,12 @@ def test_time_of_states_over_a_large_box(vdbg):
     small = best(lambda: g.applyMapSectionStates(*box((60, 60, 60)), *empty))
     large = best(lambda: g.applyMapSectionStates(*box((160, 160, 160)), *empty))
     assert large < 20.0 * small, (small, large)
+
+
+@pytest.mark.parametrize("cells", [(64, 64, 64), (100, 100, 100)])
+def test_time_of_reads_with_few_leaves(vdbg, cells):
+    g, _ = blob(vdbg, None, 300, (1.0, 1.0, 0.4))
+    for at in ((0, 0, 0), (3000, 3000, 3000)):
+        small = best(lambda: g.getMapSection(*box((8, 8, 8), at), full=True))
+        large = best(lambda: g.getMapSection(*box(cells, at), full=True))
+        assert large < 10.0 * small, (at, small, large)
