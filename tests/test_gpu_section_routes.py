@@ -67,7 +67,7 @@ def test_time_of_states_over_a_large_box(vdbg):
     assert large < 20.0 * small, (small, large)
 
 
-@pytest.mark.parametrize("cells", [(64, 64, 64), (100, 100, 100)])
+@pytest.mark.parametrize("cells", [(40, 40, 20), (64, 64, 64), (100, 100, 100)])
 def test_time_of_reads_with_few_leaves(vdbg, cells):
     g, _ = blob(vdbg, None, 300, (1.0, 1.0, 0.4))
     for at in ((0, 0, 0), (3000, 3000, 3000)):
