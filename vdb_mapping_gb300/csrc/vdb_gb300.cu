@@ -341,11 +341,12 @@ int work_ensure(vdbg_map* m, int k, size_t bytes)
   if (bytes <= m->work_bytes[k]) return VDBG_OK;
   dev_free(m, m->work[k], m->work_bytes[k]);
   m->work_bytes[k] = 0;
-  size_t want = (bytes + bytes / 4 + 0xfffff) & ~size_t(0xfffff);
+  // (under a budget without room to spare: it would be given back after the call, and
+  // may be what the other workspace needs)
+  size_t want = m->max_bytes > 0 ? bytes : (bytes + bytes / 4 + 0xfffff) & ~size_t(0xfffff);
   int st      = dev_alloc(m, &m->work[k], want);
-  if (st != VDBG_OK)
+  if (st != VDBG_OK && want > bytes)
   {
-    // (a tight budget: without the room to spare)
     want = bytes;
     st   = dev_alloc(m, &m->work[k], want);
   }
@@ -2726,8 +2727,9 @@ int section_list(vdbg_map* m, int mp, int3 lo, int3 hi, int k, uint32_t** list, 
 
 // Candidate slots of the box [lo, hi] of map `mp`, in the order of their origins
 // where `ordered` (a read; states are applied in any order), into workspace 0.
-// *cand null: none.
-int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, bool ordered, int** cand, uint32_t* n_out)
+// `lean`: by the list in any case, whose room is that of the map's leaves. *cand null:
+// none.
+int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, bool ordered, bool lean, int** cand, uint32_t* n_out)
 {
   *cand  = nullptr;
   *n_out = 0;
@@ -2738,11 +2740,14 @@ int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, bool ordered, int*
   uint32_t* list = nullptr;
   uint32_t c     = 0;
   bool listed    = false;
-  if (cells > (ordered ? kSectionPinned : kSectionUnordered))
+  if (lean || cells > (ordered ? kSectionPinned : kSectionUnordered))
   {
-    VDBG_TRY(section_list(m, mp, lo, hi, ordered ? 1 : 0, &list, &c));
-    if (c == 0) return VDBG_OK;
-    listed = !ordered || cells > kSectionCells || cells > kListedFrom + kCellsPerLeaf * c;
+    const int st = section_list(m, mp, lo, hi, ordered ? 1 : 0, &list, &c);
+    // (without room for the list, the cells' table may still fit)
+    if (st != VDBG_OK && (st != VDBG_ERR_OUT_OF_MEMORY || lean || cells > kSectionCells)) return st;
+    if (st == VDBG_OK && c == 0) return VDBG_OK;
+    listed =
+      st == VDBG_OK && (lean || !ordered || cells > kSectionCells || cells > kListedFrom + kCellsPerLeaf * c);
   }
   if (!listed)
   {
@@ -2775,6 +2780,12 @@ int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, bool ordered, int*
     return ho[a].z < ho[b].z;
   });
   for (uint32_t& i : idx) i = hl[i];
+  if (lean)
+  {
+    // (what the sort took goes to the values)
+    work_done(m, 0);
+    VDBG_TRY(work_ensure(m, 0, static_cast<size_t>(c) * 3 * sizeof(uint32_t) + 256));
+  }
   VDBG_CUDA(cudaMemcpyAsync(m->work[0], idx.data(), c * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   VDBG_CUDA(cudaStreamSynchronize(s));  // (idx goes out of scope)
   *cand = reinterpret_cast<int*>(m->work[0]);
@@ -2819,30 +2830,14 @@ int section_export_small(vdbg_map* m, int mp, int3 lo, int3 hi, int3 first, int3
   return VDBG_OK;
 }
 
-// getMapSection into host arrays (any of them may be null).
-int section_export(vdbg_map* m, int mp, int3 lo, int3 hi, int full, int64_t capacity, int32_t* origins, float* values,
-                   uint64_t* masks, int64_t* n_out)
+// getMapSection into host arrays (any of them may be null), through the candidates.
+int section_export_counted(vdbg_map* m, int mp, int3 lo, int3 hi, int full, bool lean, int64_t capacity,
+                           int32_t* origins, float* values, uint64_t* masks, int64_t* n_out)
 {
   cudaStream_t s = m->stream;
-  int3 first, dims;
-  const uint32_t cells = m->n_leaves > 0 ? section_cells(lo, hi, &first, &dims) : 0u;
-  if (cells == 0) return VDBG_OK;
-  if (cells <= kSectionPinned)
-  {
-    if (cells > kSectionUnasked)
-    {
-      uint32_t* list = nullptr;
-      uint32_t c     = 0;
-      VDBG_TRY(section_list(m, mp, lo, hi, 1, &list, &c));
-      if (c == 0) return VDBG_OK;
-    }
-    // (its room for every cell may not fit a budget that the leaves fit)
-    const int st = section_export_small(m, mp, lo, hi, first, dims, cells, full, capacity, origins, values, masks, n_out);
-    if (st != VDBG_ERR_OUT_OF_MEMORY) return st;
-  }
   int* cand  = nullptr;
   uint32_t n = 0, kept = 0;
-  VDBG_TRY(section_candidates(m, mp, lo, hi, true, &cand, &n));
+  VDBG_TRY(section_candidates(m, mp, lo, hi, true, lean, &cand, &n));
   if (n == 0) return VDBG_OK;
   uint32_t* keep  = reinterpret_cast<uint32_t*>(cand) + n;
   uint32_t* pos   = keep + n;
@@ -2869,6 +2864,39 @@ int section_export(vdbg_map* m, int mp, int3 lo, int3 hi, int full, int64_t capa
   if (origins) VDBG_CUDA(cudaMemcpyAsync(origins, d_o, k * 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   VDBG_CUDA(cudaStreamSynchronize(s));
   return VDBG_OK;
+}
+
+// getMapSection: small boxes at once, others by their candidates. The room for every
+// cell of a box (2 KB, or 12 bytes) may not fit a device or a budget that the leaves in
+// it fit: then by the list of the leaves.
+int section_export(vdbg_map* m, int mp, int3 lo, int3 hi, int full, int64_t capacity, int32_t* origins, float* values,
+                   uint64_t* masks, int64_t* n_out)
+{
+  int3 first, dims;
+  const uint32_t cells = m->n_leaves > 0 ? section_cells(lo, hi, &first, &dims) : 0u;
+  if (cells == 0) return VDBG_OK;
+  int st = VDBG_ERR_OUT_OF_MEMORY;
+  if (cells <= kSectionPinned)
+  {
+    if (cells > kSectionUnasked)
+    {
+      uint32_t* list = nullptr;
+      uint32_t c     = 0;
+      st             = section_list(m, mp, lo, hi, 1, &list, &c);
+      if (st == VDBG_OK && c == 0) return VDBG_OK;
+      if (st != VDBG_OK && st != VDBG_ERR_OUT_OF_MEMORY) return st;
+    }
+    st = section_export_small(m, mp, lo, hi, first, dims, cells, full, capacity, origins, values, masks, n_out);
+    if (st != VDBG_ERR_OUT_OF_MEMORY) return st;
+    work_done(m, 0);
+  }
+  for (bool lean : {false, true})
+  {
+    st = section_export_counted(m, mp, lo, hi, full, lean, capacity, origins, values, masks, n_out);
+    if (st != VDBG_ERR_OUT_OF_MEMORY) return st;
+    work_done(m, 0);
+  }
+  return st;
 }
 
 // Runs `launch` (which allocates leaves through the map's status counters)
@@ -3510,11 +3538,18 @@ int vdbg_apply_section_states(vdbg_map* m, int map, const int32_t lo[3], const i
   std::vector<int4> ho(static_cast<size_t>(n));
   for (int64_t i = 0; i < n; ++i) ho[i] = make_int4(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2], mp);
   std::lock_guard<std::mutex> lock(m->work_mutex);
-  int* cand  = nullptr;
-  uint32_t c = 0;
+  int* cand      = nullptr;
+  uint32_t c     = 0;
   const size_t k = static_cast<size_t>(n);
-  int st         = section_candidates(m, mp, blo, bhi, false, &cand, &c);
-  if (st == VDBG_OK) st = work_ensure(m, 1, k * (sizeof(int4) + 8 * sizeof(uint64_t)) + 16);
+  int st         = VDBG_OK;
+  // (as in section_export: by the list where the cells' table leaves no room)
+  for (bool lean : {false, true})
+  {
+    st = section_candidates(m, mp, blo, bhi, false, lean, &cand, &c);
+    if (st == VDBG_OK) st = work_ensure(m, 1, k * (sizeof(int4) + 8 * sizeof(uint64_t)) + 16);
+    if (st != VDBG_ERR_OUT_OF_MEMORY) break;
+    work_done(m, 0);
+  }
   int4* d_o               = reinterpret_cast<int4*>(m->work[1]);
   unsigned long long* d_m = reinterpret_cast<unsigned long long*>(d_o + k);
   if (st == VDBG_OK && n > 0 &&
