@@ -1329,21 +1329,48 @@ int build_topology(vdbg_map* m, int map, cudaStream_t s, TopoView* tv)
 // lanes take a ray each, and the block size. A thread's walk is a chain of
 // dependent loads whose length differs from ray to ray, and the lanes of a warp
 // take each other's time; with few rays there are warps enough to give each
-// ray fewer neighbours. 32 warps an SM: 1000 queries took 0.19 ms at 4, 0.18 at 8
-// to 128 (0.33 with whole warps), 50000 queries 0.70 at 8, 0.54 at 32, 0.63 at 64.
+// ray fewer neighbours: as many as keep `warps` of them on each SM.
 struct RayShape
 {
   uint32_t lanes;
   unsigned threads, blocks;
 };
-RayShape ray_shape(const vdbg_map* m, uint32_t n, unsigned threads)
+RayShape ray_shape(const vdbg_map* m, uint32_t n, unsigned threads, uint32_t per_sm)
 {
-  const uint32_t warps = static_cast<uint32_t>(m->num_sms) * 32u;
+  const uint32_t warps = static_cast<uint32_t>(m->num_sms) * per_sm;
   RayShape r;
   r.lanes            = std::min<uint32_t>(32, std::max<uint32_t>(1, (n + warps - 1) / warps));
   r.threads          = r.lanes < 32 ? 32 : threads;
   const uint32_t per = r.lanes * (r.threads / 32);
   r.blocks           = (n + per - 1) / per;
+  return r;
+}
+
+// Warps an SM for the walks of few rays. The voxel walks, fast mode's spans and
+// raytrace's spans in a map of many leaves take 32. Elsewhere raytrace's span walk
+// takes eight, but for up to 16 queries an SM one query a warp: it is bound by the FP64
+// pipe, which a warp holds as long for one lane as for 32, and only the long spans of a
+// large map make up for that. 10,000 queries in a room of 3,400 leaves take 133 us
+// with 8 warps an SM, 153 with 16, 213 with 32, and 141 with whole warps; 50,000 in a
+// room of 81,000 leaves 354 with 8, 425 with 32; 80,000 in a street of 3.6M leaves 737
+// with 8, 640 with 32; 50,000 in a room of 454,000 leaves 417 and 431. One query a
+// warp: 2,000 queries in the street 194 us, two a warp 233.
+constexpr uint32_t kWalkWarps  = 32;
+constexpr uint32_t kSpanWarps  = 8;
+constexpr uint32_t kSpanAlone  = 16;
+constexpr uint32_t kLongSpans  = 1u << 20;  // leaves
+
+// Raytrace's span walk, and whether its queries and spans are sorted. The orders pay
+// where many lanes of a warp wait for one another: seven launches, 40 us (10,000 and
+// 30,000 queries without and with them: room 133 and 149, 163 and 161 us; street of
+// 452,000 leaves 198 and 206, 295 and 235). In a map of many leaves from two on (10,000
+// queries 403 and 387).
+RayShape trace_span_shape(const vdbg_map* m, uint32_t n, bool* sort)
+{
+  const bool longer = m->n_leaves > kLongSpans;
+  const bool alone  = n <= static_cast<uint32_t>(m->num_sms) * kSpanAlone;
+  const RayShape r  = ray_shape(m, n, kSpanThreads, longer ? kWalkWarps : alone ? kSpanAlone : kSpanWarps);
+  *sort             = r.lanes > (longer ? 1u : 16u);
   return r;
 }
 
@@ -1386,7 +1413,7 @@ int run_fast_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order
   // Spans, walk and hits in one go. The piece records' room is a guess: when it
   // was too small, nothing was walked, and spans and walk run again with more.
   // Hits that run out of pool or hash run again alone.
-  const RayShape shape      = ray_shape(m, static_cast<uint32_t>(n), kSpanThreads);
+  const RayShape shape      = ray_shape(m, static_cast<uint32_t>(n), kSpanThreads, kWalkWarps);
   const unsigned hit_blocks = static_cast<unsigned>((n + 255) / 256);
   uint32_t want = std::max<uint32_t>(m->piece_cap, static_cast<uint32_t>(std::min<int64_t>(2 * n + 4096, 1 << 30)));
   bool marked   = false;
@@ -3344,10 +3371,9 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   const uint32_t n32 = static_cast<uint32_t>(nn);
   VDBG_CUDA(cudaMemsetAsync(m->fast_ctr, 0, 2 * sizeof(unsigned long long), s));
   const SpanBuf<SpanRec> sb{m->fast_spans, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
-  const RayShape all = ray_shape(m, n32, kSpanThreads), some = ray_shape(m, n32, 128);
-  // The orders pay where a warp's lanes wait for one another: a warp with a single
-  // query needs none (1000 queries 157 us on the device, 198 with both sorts).
-  const bool sort = all.lanes > 1 && static_cast<size_t>(sort_blocks) * kTraceBins * sizeof(uint32_t) <= nn * 24;
+  bool sort = false;
+  const RayShape all = trace_span_shape(m, n32, &sort), some = ray_shape(m, n32, 128, kWalkWarps);
+  sort = sort && static_cast<size_t>(sort_blocks) * kTraceBins * sizeof(uint32_t) <= nn * 24;
   if (sort)
   {
     const uint32_t per = (n32 + sort_blocks - 1) / sort_blocks;
