@@ -119,6 +119,7 @@ struct PrepSet
   cudaEvent_t ready  = nullptr;  // the preparation is complete
   ScanTable table{};
   int64_t total      = 0;
+  uint64_t launches  = 0;        // kernels of the preparation
   int status         = VDBG_OK;  // a step that cannot be cast (an origin out of range)
 };
 
@@ -326,7 +327,7 @@ int queue_prep(vdbg_map* m, PrepSet& p, const std::vector<ServerRequest>& step, 
   const unsigned blocks = static_cast<unsigned>((p.total + 255) / 256);
   k_prep<<<prep_blocks(p.total), kPrepThreads, 0, ps>>>(p.pts, nullptr, p.total, 16, t, p.rays,
                                                         nm > 1 ? p.ray_scan : nullptr, p.hist, p.st);
-  launch_scan(p.hist, p.cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), p.st, ps);
+  p.launches = 2 + launch_scan(p.hist, p.cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), p.st, ps);
   k_scatter<<<blocks, 256, 0, ps>>>(p.rays, p.total, t, p.cursor, p.order);
   VDBG_CUDA(cudaGetLastError());
   VDBG_CUDA(cudaEventRecord(p.ready, ps));
@@ -347,6 +348,7 @@ int run_prepped(vdbg_map* m, PrepSet& p, vdbg_scan_stats* stats)
   VDBG_CUDA(cudaStreamWaitEvent(s, p.ready, 0));
   k_absorb_prep<<<1, 1, 0, s>>>(m->d_status, p.st);
   VDBG_CUDA(cudaGetLastError());
+  m->timings.launches += p.launches + 1;
   c.pending  = true;
   bool swept = false;
   int d = run_marking(m, c, p.rays, p.order, p.cursor, p.total, p.table, true, s, true, &swept);

@@ -179,6 +179,7 @@ struct vdbg_map
   bool use_graph                   = true;
   cudaGraphExec_t graph            = nullptr;
   uint64_t graph_layout            = 0;
+  uint64_t graph_kernels           = 0;  // kernels of the captured step
   const char** d_pts_ref           = nullptr;  // the step's points address (batch), read by k_prep
   const char** h_pts_ref           = nullptr;  // pinned staging
   int64_t graph_stride             = 0;
@@ -538,6 +539,7 @@ int rebuild_hash(vdbg_map* m, uint32_t hsize, uint32_t n, cudaStream_t s)
   {
     k_rehash<<<(n + 255) / 256, 256, 0, s>>>(map_view(m), n);
     VDBG_CUDA(cudaGetLastError());
+    m->timings.launches += 1;
   }
   return VDBG_OK;
 }
@@ -835,18 +837,19 @@ ScanTable single_table(const ScanGeom& g)
 
 // Exclusive scan of nb bucket counts into cursor (total to the status):
 // one block for up to four tiles, else the multi-block form with its tile
-// sums in cursor[nb, nb + tiles).
-void launch_scan(uint32_t* hist, uint32_t* cursor, uint32_t nb, DevStatus* st, cudaStream_t s)
+// sums in cursor[nb, nb + tiles). Returns the kernels launched.
+uint64_t launch_scan(uint32_t* hist, uint32_t* cursor, uint32_t nb, DevStatus* st, cudaStream_t s)
 {
   if (nb <= 4 * kScanTile)
   {
     k_scan<<<1, 1024, 0, s>>>(hist, cursor, nb, st);
-    return;
+    return 1;
   }
   const uint32_t tiles = (nb + kScanTile - 1) / kScanTile;
   k_scan_sums<<<tiles, 1024, 0, s>>>(hist, nb, cursor + nb);
   k_scan_tops<<<1, 1024, 0, s>>>(cursor + nb, tiles, st);
   k_scan_tiles<<<tiles, 1024, 0, s>>>(hist, cursor, nb, cursor + nb);
+  return 3;
 }
 
 unsigned prep_blocks(int64_t n) { return static_cast<unsigned>((n + kPrepThreads - 1) / kPrepThreads); }
@@ -867,12 +870,12 @@ int launch_prep(vdbg_map* m, Channel& c, const float* xyz, int64_t n, int64_t st
   }
   const unsigned blocks = static_cast<unsigned>((n + 255) / 256);
   k_prep<<<prep_blocks(n), kPrepThreads, 0, s>>>(pts, nullptr, n, stride, t, rays, ray_scan, hist, m->d_status);
-  launch_scan(hist, cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), m->d_status, s);
+  const uint64_t scans = launch_scan(hist, cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), m->d_status, s);
   k_scatter<<<blocks, 256, 0, s>>>(rays, n, t, cursor, order);
   VDBG_CUDA(cudaGetLastError());
   VDBG_CUDA(cudaEventRecord(m->ev_prep, s));
   m->timed_prep = true;
-  m->timings.launches += 3;
+  m->timings.launches += 2 + scans;  // k_prep, the scan, k_scatter
   c.pending = true;
   return VDBG_OK;
 }
@@ -961,6 +964,7 @@ int settle_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, 
       k_reset_failed_leaves<<<m->num_sms * 4, 256, 0, m->stream>>>(m->bleaf,
                                                                    static_cast<size_t>(m->n_blocks) * 512);
       VDBG_CUDA(cudaGetLastError());
+      m->timings.launches += 1;
     }
     VDBG_CUDA(cudaStreamSynchronize(m->stream));
     clear_error_keep_counters(m);
@@ -1102,6 +1106,7 @@ int finish_sweep(vdbg_map* m, Channel& c, cudaStream_t s)
 {
   k_finish_window<<<1, 1, 0, s>>>(channel_view(c), m->d_status);
   VDBG_CUDA(cudaGetLastError());
+  m->timings.launches += 1;
   c.pending = false;
   return VDBG_OK;
 }
@@ -1253,6 +1258,7 @@ int discard_marking(vdbg_map* m, Channel& c, cudaStream_t s)
   k_compact<<<m->num_sms * 4, 256, 0, s>>>(map_view(m), channel_view(c));
   k_clear_touched<<<m->num_sms * 4, 256, 0, s>>>(channel_view(c));
   VDBG_CUDA(cudaGetLastError());
+  m->timings.launches += 2;
   VDBG_TRY(finish_sweep(m, c, s));
   const uint32_t keep_leaves = std::min(m->call_leaves, m->n_leaves);
   const uint32_t keep_blocks = std::min(m->call_blocks, m->n_blocks);
@@ -1261,6 +1267,7 @@ int discard_marking(vdbg_map* m, Channel& c, cudaStream_t s)
     const uint32_t n = m->n_leaves - keep_leaves;
     k_release_leaves<<<(n + 255) / 256, 256, 0, s>>>(map_view(m), keep_leaves, m->n_leaves, keep_blocks);
     VDBG_CUDA(cudaGetLastError());
+    m->timings.launches += 1;
   }
   if (m->n_blocks > keep_blocks)
   {
@@ -1273,6 +1280,7 @@ int discard_marking(vdbg_map* m, Channel& c, cudaStream_t s)
   {
     k_reset_failed_leaves<<<m->num_sms * 4, 256, 0, s>>>(m->bleaf, static_cast<size_t>(m->n_blocks) * 512);
     VDBG_CUDA(cudaGetLastError());
+    m->timings.launches += 1;
   }
   VDBG_CUDA(cudaMemsetAsync(m->bkeys, 0xff, static_cast<size_t>(m->bhash_size) * sizeof(unsigned long long), s));
   VDBG_CUDA(cudaMemsetAsync(m->bslots, 0xff, static_cast<size_t>(m->bhash_size) * sizeof(int), s));
@@ -1280,6 +1288,7 @@ int discard_marking(vdbg_map* m, Channel& c, cudaStream_t s)
   {
     k_rehash<<<(m->n_blocks + 255) / 256, 256, 0, s>>>(map_view(m), m->n_blocks);
     VDBG_CUDA(cudaGetLastError());
+    m->timings.launches += 1;
   }
   DevStatus clean;
   clear_status(&clean);
@@ -1470,6 +1479,7 @@ int run_fast_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order
     {
       k_reset_failed_leaves<<<m->num_sms * 4, 256, 0, m->stream>>>(m->bleaf, static_cast<size_t>(m->n_blocks) * 512);
       VDBG_CUDA(cudaGetLastError());
+      m->timings.launches += 1;
     }
     VDBG_CUDA(cudaStreamSynchronize(m->stream));
     clear_error_keep_counters(m);
@@ -1508,9 +1518,6 @@ CastPlan plan_single(const vdbg_map* m, int64_t n, const double origin[3], doubl
   return p;
 }
 
-// Kernel launches of one captured step (memsets excluded).
-constexpr uint32_t kGraphKernels = 6;
-
 // Queues one batched step for capture: the point count is read on the device
 // from t.first[t.n], the grids cover the scratch capacity `cap`, and every
 // kernel after the marking skips itself unless it completed.
@@ -1519,7 +1526,8 @@ int queue_step(vdbg_map* m, Channel& c, int64_t cap, int64_t stride, const ScanT
   const unsigned blocks = static_cast<unsigned>((cap + 255) / 256);
   k_prep<<<prep_blocks(cap), kPrepThreads, 0, s>>>(nullptr, m->d_pts_ref, cap, stride, t, m->d_rays, m->d_ray_scan,
                                                    m->d_hist, m->d_status);
-  launch_scan(m->d_hist, m->d_cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), m->d_status, s);
+  m->timings.launches +=
+    2 + launch_scan(m->d_hist, m->d_cursor, static_cast<uint32_t>(kBucketsPerScan * t.n), m->d_status, s);
   k_scatter<<<blocks, 256, 0, s>>>(m->d_rays, cap, t, m->d_cursor, m->d_order);
   VDBG_CUDA(cudaEventRecordWithFlags(m->ev_prep, s, cudaEventRecordExternal));
   VDBG_TRY(launch_marking(m, c, m->d_rays, m->d_order, m->d_cursor, cap, t, s));
@@ -1533,11 +1541,12 @@ int queue_step(vdbg_map* m, Channel& c, int64_t cap, int64_t stride, const ScanT
 // executable graph in place when its topology allows).
 int capture_step(vdbg_map* m, Channel& c, int64_t stride, const ScanTable& t, cudaStream_t s)
 {
-  const uint32_t launches = m->timings.launches;
+  const uint64_t launches = m->timings.launches;
   cudaGraph_t g           = nullptr;
   VDBG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   const int q          = queue_step(m, c, static_cast<int64_t>(m->ray_cap), stride, t, s);
   const cudaError_t ec = cudaStreamEndCapture(s, &g);
+  m->graph_kernels     = m->timings.launches - launches;
   m->timings.launches  = launches;
   if (q != VDBG_OK || ec != cudaSuccess)
   {
@@ -1594,7 +1603,7 @@ int graph_step(vdbg_map* m, Channel& c, const float* xyz, int64_t n, int64_t str
   VDBG_CUDA(cudaGraphLaunch(m->graph, s));
   m->graph_replays += 1;
   m->timed_prep = true;
-  m->timings.launches += kGraphKernels;
+  m->timings.launches += m->graph_kernels;
   VDBG_TRY(fetch_status(m, s));
   if (m->h_status->windows > 0u)
   {
@@ -2950,6 +2959,7 @@ int run_allocating(vdbg_map* m, F&& launch)
     {
       k_reset_failed_leaves<<<m->num_sms * 4, 256, 0, s>>>(m->bleaf, static_cast<size_t>(m->n_blocks) * 512);
       VDBG_CUDA(cudaGetLastError());
+      m->timings.launches += 1;
     }
     VDBG_CUDA(cudaStreamSynchronize(s));
     clear_error_keep_counters(m);
