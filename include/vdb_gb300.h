@@ -275,7 +275,7 @@ int vdbg_get_tuning(const vdbg_map* map, vdbg_tuning* out);
 /* Sizes of a run buffer that the call no longer has: for sources that name them. */
 #define VDBG_NOALLOC_DDA_WARPS 256
 #define VDBG_NOALLOC_RUN_SEGMENT 4096
-#define VDBG_NOALLOC_SCRATCH_BYTES (28u << 20)
+#define VDBG_NOALLOC_SCRATCH_BYTES (10u << 20)
 int vdbg_insert_point_cloud_noalloc(vdbg_map* map, const float* xyz, int64_t n, int64_t stride_bytes,
                                     const double origin[3], const char* source_id, uint32_t flags,
                                     void* stream, vdbg_scan_stats* stats);

@@ -31,3 +31,11 @@ def test_binding_agrees(tmp_path):
     v = values(tmp_path)
     assert v["VDBG_NOALLOC_MAX_POINTS"] == _lib.VDBG_NOALLOC_MAX_POINTS
     assert v["VDBG_NOALLOC_SCRATCH_BYTES"] == _lib.VDBG_NOALLOC_SCRATCH_BYTES
+
+
+def test_scratch_is_what_the_call_uses(tmp_path):
+    """Staged points, ray records and ray order per point, two histograms of the 11,154
+    sort buckets, and at most 1 MiB to spare (every GPU that loads the library holds it)."""
+    v = values(tmp_path)
+    used = v["VDBG_NOALLOC_MAX_POINTS"] * (16 + 16 + 4) + 2 * 11154 * 4
+    assert used <= v["VDBG_NOALLOC_SCRATCH_BYTES"] <= used + (1 << 20)

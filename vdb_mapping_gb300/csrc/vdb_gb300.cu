@@ -3737,7 +3737,9 @@ constexpr size_t kNoAllocRaysBytes  = align256(static_cast<size_t>(kNoAllocMaxPo
 constexpr size_t kNoAllocOrderBytes = align256(static_cast<size_t>(kNoAllocMaxPoints) * sizeof(int));
 constexpr size_t kNoAllocHistBytes  = align256(static_cast<size_t>(kBucketsPerScan) * sizeof(uint32_t));
 constexpr size_t kNoAllocBytes = kNoAllocPtsBytes + kNoAllocRaysBytes + kNoAllocOrderBytes + 2 * kNoAllocHistBytes;
-static_assert(kNoAllocBytes <= static_cast<size_t>(VDBG_NOALLOC_SCRATCH_BYTES), "scratch size and header disagree");
+static_assert(kNoAllocBytes <= static_cast<size_t>(VDBG_NOALLOC_SCRATCH_BYTES) &&
+                static_cast<size_t>(VDBG_NOALLOC_SCRATCH_BYTES) <= kNoAllocBytes + (size_t(1) << 20),
+              "scratch size and header disagree");
 
 constexpr int kNoAllocMaxDevices = 64;
 
