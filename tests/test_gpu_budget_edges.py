@@ -1,0 +1,51 @@
+"""Budgets that leave no room for what only speeds a call up."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import assert_same_map, pair, ref_config
+
+pytestmark = pytest.mark.gpu
+
+TABLE = 16384 * 10 * 24 + 16384 * 8  # the walk's table of crossing times
+
+
+def test_a_map_without_room_for_the_table(vdbg, oracle):
+    """The pools fit and the table does not: the map is made, and inserts as any other."""
+    g = vdbg.OccupancyVDBMapping(0.1, initial_leaf_capacity=1024, initial_block_capacity=1024)
+    g.addInputSource("s", 5000.0, 0)
+    held = g.deviceBytes()
+    g.close()
+    rng = np.random.default_rng(4)
+    pts = (rng.normal(size=(500, 3)) * [4.0, 4.0, 1.0]).astype(np.float32)
+    far = np.concatenate([pts, pts * np.float32(40.0)])
+    cfg = ref_config(max_range=5000.0)
+    g, o = pair(vdbg, oracle, 0.1, cfg, max_device_bytes=held - TABLE + (64 << 10), initial_leaf_capacity=1024,
+                initial_block_capacity=1024)
+    assert g.deviceBytes() <= held - TABLE + (64 << 10)
+    for m in (g, o):
+        m.insertPointCloud(pts[:40] * np.float32(0.2), (0.1, 0.2, 0.3), "s")
+    assert_same_map(g.exportLeaves(), o.exportLeaves(), "tight")
+    g, o = pair(vdbg, oracle, 0.1, cfg, max_device_bytes=1 << 30)
+    for k in range(2):
+        for m in (g, o):
+            m.insertPointCloud(far, (0.1, 0.2 + k, 0.3), "s")
+    assert_same_map(g.exportLeaves(), o.exportLeaves(), "roomy")
+
+
+def test_the_call_that_allocates_nothing(vdbg, oracle):
+    """With a budget the table is made by the first regular insert: before it the walk
+    computes what the table holds, for short rays and for rays beyond its range."""
+    from vdb_mapping_gb300 import _lib
+
+    cfg = ref_config(max_range=5000.0)
+    g, o = pair(vdbg, oracle, 0.1, cfg, max_device_bytes=4 << 30, initial_leaf_capacity=1 << 19,
+                initial_block_capacity=1 << 17)
+    lib = _lib.load()
+    rng = np.random.default_rng(6)
+    for n, spread in ((300, 3.0), (12000, 3.0), (40, 900.0)):
+        pts = np.zeros((n, 4), np.float32)
+        pts[:, :3] = rng.normal(size=(n, 3)) * spread
+        assert lib.vdbg_insert_point_cloud_noalloc(g._h, pts.ctypes.data, n, 16, (_lib.C.c_double * 3)(0.1, 0.2, 0.3),
+                                                   b"s", 0, None, None) == 0
+        o.insertPointCloud(np.ascontiguousarray(pts[:, :3]), (0.1, 0.2, 0.3), "s")
+        assert_same_map(g.exportLeaves(), o.exportLeaves(), f"{n}")

@@ -451,7 +451,7 @@ constexpr uint32_t kMarchMaxRounds = 96;   // far above a chunk's rounds (one mo
 // The axis entries of march.cuh for all n below kAxisTableN in the binades
 // [2^-(j + 1), 2^-j), j < kAxisTableJ, n fastest: with chunks of 64 steps all
 // that rays with L1 up to 65,536 need. Other entries are computed when a chunk
-// begins.
+// begins, and all of them for a map whose budget has no room for the table.
 constexpr uint32_t kAxisTableN   = 16384;
 constexpr int kAxisTableJ        = 10;
 constexpr size_t kAxisTableBytes = size_t(kAxisTableN) * kAxisTableJ * (sizeof(ulonglong2) + sizeof(int2)) +
@@ -462,13 +462,14 @@ struct AxisTable
   ulonglong2* td;  // [kAxisTableJ][kAxisTableN] t1, d
   int2* kf;        // [kAxisTableJ][kAxisTableN] k1, df
   double* delta;   // [kAxisTableN] 1 / n (DBL_MAX for 0)
+  uint32_t n;      // kAxisTableN, or 0: no table
 };
 
 __device__ __noinline__ march::Axis axis_entry_far(uint32_t n, int j) { return march::axis_entry(n, j); }
 
 __device__ __forceinline__ march::Axis axis_at(const AxisTable& at, uint32_t n, int j)
 {
-  if (n < kAxisTableN && j < kAxisTableJ)
+  if (n < at.n && j < kAxisTableJ)
   {
     const ulonglong2 td = __ldg(at.td + static_cast<size_t>(j) * kAxisTableN + n);
     const int2 kf       = __ldg(at.kf + static_cast<size_t>(j) * kAxisTableN + n);
@@ -479,10 +480,11 @@ __device__ __forceinline__ march::Axis axis_at(const AxisTable& at, uint32_t n, 
 
 __device__ __forceinline__ double axis_delta_at(const AxisTable& at, uint32_t n)
 {
-  return n < kAxisTableN ? __ldg(at.delta + n) : march::axis_delta(n);
+  if (n < at.n) return __ldg(at.delta + n);
+  return n == 0u ? hdda::kDblMax : march::axis_delta(n);
 }
 
-// One thread per entry (a new map).
+// One thread per entry.
 __global__ void __launch_bounds__(256) k_axis_table(AxisTable at)
 {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;

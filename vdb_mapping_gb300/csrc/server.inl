@@ -345,6 +345,7 @@ int run_prepped(vdbg_map* m, PrepSet& p, vdbg_scan_stats* stats)
   VDBG_TRY(begin_call(m, s));
   const uint32_t leaves_before = m->n_leaves;
   if (p.total == 0) return VDBG_OK;
+  VDBG_TRY(ensure_axis(m, s));
   VDBG_CUDA(cudaStreamWaitEvent(s, p.ready, 0));
   k_absorb_prep<<<1, 1, 0, s>>>(m->d_status, p.st);
   VDBG_CUDA(cudaGetLastError());
