@@ -49,3 +49,19 @@ def test_the_call_that_allocates_nothing(vdbg, oracle):
                                                    b"s", 0, None, None) == 0
         o.insertPointCloud(np.ascontiguousarray(pts[:, :3]), (0.1, 0.2, 0.3), "s")
         assert_same_map(g.exportLeaves(), o.exportLeaves(), f"{n}")
+
+
+def test_room_of_a_raytrace(vdbg, oracle):
+    """A query takes 87 bytes of inputs, answers and order and 64 of span record."""
+    from test_gpu_raytrace import same_trace
+
+    g, o = pair(vdbg, oracle, 0.1, ref_config(max_range=8.0))
+    for m in (g, o):
+        m.insertPointCloud(np.ones((10, 3), np.float32), (0.1, 0.2, 0.3), "s")
+    n = 100000
+    held = g.deviceBytes()
+    d = np.random.default_rng(1).normal(size=(n, 3))
+    ln = np.full(n, 5.0)
+    same_trace(g.raytrace(np.zeros((n, 3)), d, ln), o.raytrace(np.zeros((n, 3)), d, ln))
+    nodes = 2 * 1024 * 16
+    assert g.deviceBytes() - held <= n * (87 + 64) + nodes + (64 << 10)

@@ -197,8 +197,7 @@ struct vdbg_map
   // (k_trace_spans -> k_trace_walk) and their counters.
   FastPiece* fast_pieces           = nullptr;  // [piece_cap]
   uint32_t piece_cap               = 0;
-  SpanRec* fast_spans              = nullptr;  // [fast_cap] as written, and
-  uint32_t* fast_sorted            = nullptr;  // [fast_cap] their order by length class
+  SpanRec* fast_spans              = nullptr;  // [fast_cap]
   uint32_t* fast_hist              = nullptr;  // [kSpanClasses]
   uint32_t fast_cap                = 0;
   unsigned long long* fast_ctr     = nullptr;  // [2]: span count (low 32 bits), castRayIntoGrid visits
@@ -1424,10 +1423,8 @@ int ensure_span_buffers(vdbg_map* m, uint32_t want)
   if (!m->fast_hist) VDBG_TRY(dev_alloc(m, &m->fast_hist, kSpanClasses));
   if (want <= m->fast_cap) return VDBG_OK;
   dev_free(m, m->fast_spans, m->fast_cap);
-  dev_free(m, m->fast_sorted, m->fast_cap);
   m->fast_cap = 0;
   VDBG_TRY(dev_alloc(m, &m->fast_spans, want));
-  VDBG_TRY(dev_alloc(m, &m->fast_sorted, want));
   m->fast_cap = want;
   return VDBG_OK;
 }
@@ -2109,7 +2106,6 @@ int vdbg_destroy(vdbg_map* m)
   dev_free(m, m->d_trace, m->trace_bytes);
   dev_free(m, m->fast_pieces, m->piece_cap);
   dev_free(m, m->fast_spans, m->fast_cap);
-  dev_free(m, m->fast_sorted, m->fast_cap);
   dev_free(m, m->fast_hist, kSpanClasses);
   dev_free(m, m->fast_ctr, 2);
   dev_free(m, m->d_art_o, m->art_n);
@@ -3421,10 +3417,11 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
     k_span_hist<<<std::min<unsigned>(sblocks, static_cast<unsigned>(m->num_sms) * 4u), 256, 0, s>>>(
       m->fast_spans, sb.count, m->fast_hist);
     k_span_offsets<<<1, 32, 0, s>>>(m->fast_hist);
-    k_span_scatter<<<sblocks, 256, 0, s>>>(m->fast_spans, sb.count, m->fast_hist, m->fast_sorted);
+    // (the spans' order takes the place of the queries', which has been read)
+    k_span_scatter<<<sblocks, 256, 0, s>>>(m->fast_spans, sb.count, m->fast_hist, order);
   }
   k_trace_walk<<<some.blocks, some.threads, 0, s>>>(q, n32, mc.resolution, mc.inv_res, map_view(m), tv, m->active, ok,
-                                                    end, m->fast_spans, sort ? m->fast_sorted : nullptr, sb.count,
+                                                    end, m->fast_spans, sort ? order : nullptr, sb.count,
                                                     some.lanes);
   VDBG_CUDA(cudaGetLastError());
   m->timings.launches += sort ? 9 : 2;
