@@ -65,3 +65,38 @@ def test_room_of_a_raytrace(vdbg, oracle):
     same_trace(g.raytrace(np.zeros((n, 3)), d, ln), o.raytrace(np.zeros((n, 3)), d, ln))
     nodes = 2 * 1024 * 16
     assert g.deviceBytes() - held <= n * (87 + 64) + nodes + (64 << 10)
+
+
+@pytest.mark.parametrize("count", [0, 1])
+def test_fast_mode_without_room_for_its_pieces(vdbg, oracle, count):
+    """The room for the pieces of every ray's windows is refused: the scan goes on with a
+    piece a span."""
+    from test_gpu_raytrace import active_pair
+
+    vox = [(x, y, z) for x in range(0, 4000, 24) for y in (-4, 3) for z in (1, 9)]
+    g, o = active_pair(vdbg, oracle, vox)
+    n = 2000
+    rng = np.random.default_rng(8)
+    far = np.stack([rng.uniform(3000.0, 4100.0, n), rng.uniform(-3.9, 3.9, n), rng.uniform(0.0, 12.0, n)], 1)
+    near = np.tile(np.array([[-3.2, 0.6, 4.6]]), (n, 1))
+    cfg = ref_config(max_range=5000.0)
+    for fast in (False, True):  # (leaves all along the rays, so that their spans are long)
+        cfg.fast_mode = fast
+        for m in (g, o):
+            m.setConfig(cfg)
+            if not fast:
+                m.addInputSource("s", 5000.0, 0)
+                m.insertPointCloud(far.astype(np.float32), (-3.5, 0.5, 4.5), "s")
+    # (the first scan has a fast scan's other buffers made)
+    for k, pts in enumerate((near, far, far + [0.0, 0.7, 0.2])):
+        if k == 1:
+            held = g.deviceBytes()
+            assert g._lib.vdbg_test_fail_allocs(g._h, 0, count) == 0
+        for m in (g, o):
+            m.insertPointCloud(pts.astype(np.float32), (-3.5, 0.5, 4.5), "s")
+        if k == 1:
+            # more pieces than the first guess has room for, or the refusal did not matter
+            assert (g.deviceBytes() > held + 32 * (2 * n + 4096)) == (count == 0)
+        for key in ("rays", "visits", "hits", "updates"):
+            assert g.last_stats[key] == o.last_stats[key], (k, key)
+        assert_same_map(g.exportLeaves(), o.exportLeaves(), f"fast {k}")

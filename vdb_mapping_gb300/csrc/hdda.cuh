@@ -368,13 +368,15 @@ enum Walk : int
 // voxel the walk stands on at its start need not be looked at either.
 // `sink`: open(t0) at a span's first cell; window(lo, hi) in ascending order, without
 // overlap (the last one's hi may lie past the span's end).
-// A window that starts within kGapVoxels of the last one's end joins it: walking
-// the gap costs less than the jump over it, or a piece of its own.
+// A window that starts within gap_voxels of the last one's end joins it: walking
+// the gap costs less than the jump over it, or a piece of its own. (Infinite: a span
+// has one window, from its first active leaf to its last.)
 template <class Sink>
 struct RunTrack
 {
   static constexpr float kGapVoxels = 24.0f;
   Sink& sink;
+  float gap_voxels = kGapVoxels;
   float margin = 0.0f, gap = 0.0f, lo = 0.0f, hi = 0.0f;
   int floor_hi = 0;
   bool all = false, has = false, running = false, near = false;
@@ -393,7 +395,7 @@ struct RunTrack
     }
     all    = !(e < 1.4901161e-8f);  // 2^-26
     margin = 3.0f / l1 + 4.7683716e-7f;
-    gap    = kGapVoxels / l1;
+    gap    = gap_voxels / l1;
     // Upper word of 2^23 e as a double, rounded up.
     const float f = all ? 2.0f : e * 8388608.0f;
     int b;

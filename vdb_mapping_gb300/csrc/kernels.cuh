@@ -2118,15 +2118,18 @@ __device__ __forceinline__ uint32_t lane_item(uint32_t lanes, uint32_t n)
   return lane < lanes ? warp * lanes + lane : n;
 }
 
-// Records written by a span kernel.
-template <class Rec>
+// Records written by a span kernel. `Count`: 64 bits for pieces, of which a ray may have
+// any number.
+template <class Rec, class Count>
 struct SpanBuf
 {
   Rec* rec;
   uint32_t cap;
-  uint32_t* count;                 // written (may exceed cap: the host grows and repeats)
+  Count* count;                    // written (may exceed cap: the host grows and repeats)
   unsigned long long* dda_visits;  // castRayIntoGrid visits the prep counted for these rays
 };
+using PieceBuf = SpanBuf<FastPiece, unsigned long long>;
+using TraceBuf = SpanBuf<SpanRec, uint32_t>;
 
 // A slot of `count` for each active thread, one atomic for them together.
 __device__ __forceinline__ uint32_t take_slot(uint32_t* count)
@@ -2152,7 +2155,7 @@ struct FastWindows
 
 // All 32 lanes: the pieces of each lane's n windows, one atomic for the warp.
 __device__ __forceinline__ void write_pieces(const FastWindows& w, int n, float l1, int ray,
-                                             const SpanBuf<FastPiece>& sb)
+                                             const PieceBuf& sb)
 {
   const int x   = static_cast<int>(threadIdx.x);
   uint32_t mine = 0u;
@@ -2160,14 +2163,16 @@ __device__ __forceinline__ void write_pieces(const FastWindows& w, int n, float 
     hdda::window_pieces(w.t0[k][x], w.lo[k][x], w.hi[k][x], l1, [&](double, double) { ++mine; });
   uint32_t total = 0u;
   uint32_t slot  = warp_scan_exclusive(mine, static_cast<int>(threadIdx.x & 31u), &total);
-  uint32_t base  = 0u;
-  if ((threadIdx.x & 31u) == 0u && total) base = atomicAdd(sb.count, total);
-  slot += __shfl_sync(0xffffffffu, base, 0);
+  unsigned long long base = 0ull;
+  if ((threadIdx.x & 31u) == 0u && total) base = atomicAdd(sb.count, static_cast<unsigned long long>(total));
+  base                = __shfl_sync(0xffffffffu, base, 0);
+  const uint32_t room = base < sb.cap ? sb.cap - static_cast<uint32_t>(base) : 0u;
+  FastPiece* rec      = sb.rec + base;
   for (int k = 0; k < n; ++k)
   {
     const double t0 = w.t0[k][x];
     hdda::window_pieces(t0, w.lo[k][x], w.hi[k][x], l1, [&](double from, double to) {
-      if (slot < sb.cap) sb.rec[slot] = FastPiece{t0, from, to, ray, 0};
+      if (slot < room) rec[slot] = FastPiece{t0, from, to, ray, 0};
       ++slot;
     });
   }
@@ -2179,7 +2184,7 @@ __device__ __forceinline__ void write_pieces(const FastWindows& w, int n, float 
 struct FastSink
 {
   FastWindows& w;
-  const SpanBuf<FastPiece>& sb;
+  const PieceBuf& sb;
   int ray = 0;
   int n = 0, base = 0;
   double t0 = 0.0;
@@ -2195,7 +2200,7 @@ struct FastSink
     {
       n = --base;
       const double at = w.t0[n][x], from = w.lo[n][x];
-      const uint32_t slot = atomicAdd(sb.count, 1u);
+      const unsigned long long slot = atomicAdd(sb.count, 1ull);
       if (slot < sb.cap) sb.rec[slot] = FastPiece{at, from > at ? from : -1.0, w.hi[n][x], ray, 0};
     }
     if (n < kFastWindows)
@@ -2226,11 +2231,12 @@ __device__ __forceinline__ void fast_ray(const int4& r, const ScanGeom& g, doubl
   }
 }
 
+// `coarse`: one piece a span, for when there is no room for more.
 // (12 warps an SM: 16, with 128 registers, spilled and took 16% longer)
 __global__ void __launch_bounds__(kSpanThreads, 12) k_fast_spans(const int4* __restrict__ rays,
                                                                  const int* __restrict__ order, ScanTable t,
-                                                                 MapView m, TopoView tv, SpanBuf<FastPiece> sb,
-                                                                 uint32_t lanes)
+                                                                 MapView m, TopoView tv, PieceBuf sb,
+                                                                 uint32_t lanes, int coarse)
 {
   __shared__ FastWindows windows;
   // (read once per warp: the warp reduces below)
@@ -2267,6 +2273,11 @@ __global__ void __launch_bounds__(kSpanThreads, 12) k_fast_spans(const int4* __r
     DevTopo topo{tv, m, 0x7fffffff, 0, 0, -1};
     uint32_t steps = 0;
     hdda::RunTrack<FastSink> track(sink);
+    if (coarse)
+    {
+      track.gap_voxels = INFINITY;
+      l1f              = 0.0f;
+    }
     const int w = hdda::all_spans(ray, topo, steps, [&](const hdda::Span& sp) { sink.span(sp); }, track);
     if (w == hdda::kWalkBound) atomicOr(&m.st->error, kErrStepBound);
   }
@@ -2279,13 +2290,14 @@ __global__ void __launch_bounds__(kSpanThreads, 12) k_fast_spans(const int4* __r
 __global__ void __launch_bounds__(128) k_fast_walk(const int4* __restrict__ rays, ScanTable t, MapView m,
                                                    ChannelView c, TopoView tv,
                                                    const unsigned long long* __restrict__ active,
-                                                   SpanBuf<FastPiece> sb)
+                                                   PieceBuf sb)
 {
   const int lane = static_cast<int>(threadIdx.x & 31);
   if (__shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed_u32(&m.st->error) : 0u, 0) != 0u) return;
   c.cur_epoch      = *c.epoch;
-  const uint32_t n = *sb.count;
-  if (n > sb.cap) return;  // (the host repeats the spans with more room)
+  const unsigned long long pieces = *sb.count;
+  if (pieces > sb.cap) return;  // (the host repeats the spans with more room)
+  const uint32_t n = static_cast<uint32_t>(pieces);
   unsigned long long marks = 0ull;
   ActiveCache act{&m, active, tv.map, 0x7fffffff, 0, 0, -1, -1, -1, 0ull};
   act.bits = tv.leafbits;
@@ -2363,7 +2375,7 @@ __global__ void __launch_bounds__(256) k_span_scatter(const SpanRec* __restrict_
 
 // The fast marking's visits replace the castRayIntoGrid visits the prep
 // counted (one thread).
-__global__ void k_fast_visits(DevStatus* st, SpanBuf<FastPiece> sb)
+__global__ void k_fast_visits(DevStatus* st, PieceBuf sb)
 {
   if (*sb.count <= sb.cap) st->visits -= *sb.dda_visits;
 }
@@ -2546,7 +2558,7 @@ __global__ void __launch_bounds__(kSpanThreads, 20) k_trace_spans(double* q, uin
                                                      double inv_res, MapView m, TopoView tv,
                                                      const uint32_t* __restrict__ order,
                                                      unsigned char* __restrict__ ok, double* __restrict__ end,
-                                                     SpanBuf<SpanRec> sb, uint32_t lanes)
+                                                     TraceBuf sb, uint32_t lanes)
 {
   const uint32_t j = lane_item(lanes, n);
   if (j >= n) return;

@@ -200,7 +200,7 @@ struct vdbg_map
   SpanRec* fast_spans              = nullptr;  // [fast_cap]
   uint32_t* fast_hist              = nullptr;  // [kSpanClasses]
   uint32_t fast_cap                = 0;
-  unsigned long long* fast_ctr     = nullptr;  // [2]: span count (low 32 bits), castRayIntoGrid visits
+  unsigned long long* fast_ctr     = nullptr;  // [2]: pieces (or spans, 32 bits), castRayIntoGrid visits
   // Artificial areas (VDBMapping.hpp:1152-1236): their voxels as leaves
   // (origins, device-order masks) on the host, and the device copy that
   // k_section_set_states re-activates after every update of the map.
@@ -1438,30 +1438,39 @@ int run_fast_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order
                      cudaStream_t s)
 {
   // Spans, walk and hits in one go. The piece records' room is a guess: when it
-  // was too small, nothing was walked, and spans and walk run again with more.
+  // was too small, nothing was walked, and spans and walk run again with more, or,
+  // where that does not fit, with one piece a span (32 bytes a span).
   // Hits that run out of pool or hash run again alone.
   const RayShape shape      = ray_shape(m, static_cast<uint32_t>(n), kSpanThreads, kWalkWarps);
   const unsigned hit_blocks = static_cast<unsigned>((n + 255) / 256);
-  uint32_t want = std::max<uint32_t>(m->piece_cap, static_cast<uint32_t>(std::min<int64_t>(2 * n + 4096, 1 << 30)));
+  const uint32_t guess      = static_cast<uint32_t>(std::min<int64_t>(2 * n + 4096, 1 << 30));
+  uint32_t want = std::max<uint32_t>(m->piece_cap, guess);
   bool marked   = false;
+  bool coarse   = false;
   for (int attempt = 0;; ++attempt)
   {
-    uint32_t pieces = 0;
+    unsigned long long pieces = 0;
     if (!marked)
     {
       TopoView tv;
       VDBG_TRY(build_topology(m, 0, s, &tv));
-      VDBG_TRY(ensure_piece_buffer(m, want));
+      int st = ensure_piece_buffer(m, want);
+      if (st == VDBG_ERR_OUT_OF_MEMORY && !coarse && want > guess)
+      {
+        coarse = true;
+        st     = ensure_piece_buffer(m, guess);
+      }
+      VDBG_TRY(st);
       VDBG_CUDA(cudaMemsetAsync(m->fast_ctr, 0, 2 * sizeof(unsigned long long), s));
-      const SpanBuf<FastPiece> sb{m->fast_pieces, m->piece_cap, reinterpret_cast<uint32_t*>(m->fast_ctr),
-                                  m->fast_ctr + 1};
-      k_fast_spans<<<shape.blocks, shape.threads, 0, s>>>(rays, order, t, map_view(m), tv, sb, shape.lanes);
+      const PieceBuf sb{m->fast_pieces, m->piece_cap, m->fast_ctr, m->fast_ctr + 1};
+      k_fast_spans<<<shape.blocks, shape.threads, 0, s>>>(rays, order, t, map_view(m), tv, sb, shape.lanes,
+                                                          coarse ? 1 : 0);
       k_fast_walk<<<static_cast<unsigned>(m->num_sms) * 12u, 128, 0, s>>>(rays, t, map_view(m), channel_view(c), tv,
                                                                          m->active, sb);
       k_fast_visits<<<1, 1, 0, s>>>(m->d_status, sb);
       VDBG_CUDA(cudaGetLastError());
       m->timings.launches += 3;
-      VDBG_CUDA(cudaMemcpyAsync(&pieces, m->fast_ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      VDBG_CUDA(cudaMemcpyAsync(&pieces, m->fast_ctr, sizeof(pieces), cudaMemcpyDeviceToHost, s));
     }
     // The hits come last: they alone allocate, and what they add (blocks, or the
     // error of a pool that is full) must not be seen by the phases before.
@@ -1471,7 +1480,16 @@ int run_fast_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order
     m->timings.retries += attempt > 0 ? 1 : 0;
     VDBG_TRY(fetch_status(m, s));
     if (pieces > m->piece_cap)
-      want = pieces + pieces / 4;
+    {
+      // (records of more than 2^31 pieces are not tried)
+      want = static_cast<uint32_t>(std::min<unsigned long long>(pieces + pieces / 4, 1ull << 31));
+      if (pieces > (1ull << 31))
+      {
+        if (coarse) return oom("fast pieces", pieces, m->piece_cap);
+        coarse = true;
+        want   = std::max(m->piece_cap, guess);
+      }
+    }
     else
       marked = true;
     if (m->h_status->error == 0u && marked) break;
@@ -3396,7 +3414,7 @@ int vdbg_raytrace(vdbg_map* m, int map, int64_t n, const double* origins, const 
   const MapConf& mc = m->conf[mp];
   const uint32_t n32 = static_cast<uint32_t>(nn);
   VDBG_CUDA(cudaMemsetAsync(m->fast_ctr, 0, 2 * sizeof(unsigned long long), s));
-  const SpanBuf<SpanRec> sb{m->fast_spans, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
+  const TraceBuf sb{m->fast_spans, m->fast_cap, reinterpret_cast<uint32_t*>(m->fast_ctr), m->fast_ctr + 1};
   bool sort = false;
   const RayShape all = trace_span_shape(m, n32, &sort), some = ray_shape(m, n32, 128, kWalkWarps);
   sort = sort && static_cast<size_t>(sort_blocks) * kTraceBins * sizeof(uint32_t) <= nn * 24;
