@@ -84,3 +84,39 @@ def test_the_next_call(vdbg, oracle):
     for m in (g, o):
         m.insertPointCloud(pts, (0.1, 0.2, 0.3), "s")
     assert_same_map(g.exportLeaves(), o.exportLeaves(), "after a refused call")
+
+
+@pytest.mark.parametrize("skip", [0, 1, 2])
+def test_bytes_after_a_refused_insert(vdbg, skip):
+    """device bytes count what a refused call gave back."""
+    pts = np.full((200000, 3), 1.0, np.float32)
+    held = []
+    for refused in (False, True):
+        g = vdbg.OccupancyVDBMapping(0.1)
+        g.setConfig(Config(max_range=30.0, **FLIPPY))
+        g.addInputSource("s", 30.0, 0)
+        if refused:
+            refuse(g, skip, 1)
+            with pytest.raises(VdbgError):
+                g.insertPointCloud(pts, (0.1, 0.2, 0.3), "s")
+        g.insertPointCloud(pts, (0.1, 0.2, 0.3), "s")
+        held.append(g.deviceBytes())
+    assert held[0] == held[1]
+
+
+@pytest.mark.parametrize("skip", range(12))
+def test_bytes_after_a_refused_morphology(vdbg, oracle, skip):
+    """Leaves too far apart for one grid: the hashed sets, one allocation of which is
+    refused (the others go back, at their size)."""
+    g, _ = inserted(vdbg, oracle)
+    so = np.array([[0, 0, 0], [8 * 900, 8 * 900, 8 * 900]], np.int32)
+    sm = np.full((2, 8), 0x00FF00FF00FF00FF, np.uint64)
+    held = g.deviceBytes()
+    refuse(g, skip, 1)
+    with pytest.raises(VdbgError) as e:
+        g.sectionMorphology(so, sm, "close", 2)
+    assert "OUT_OF_MEMORY" in str(e.value)
+    assert g.deviceBytes() == held
+    for a, b in zip(g.sectionMorphology(so, sm, "close", 2), oracle.morphology(so, sm, "close", 2)):
+        assert np.array_equal(a, b)
+    assert g.deviceBytes() == held

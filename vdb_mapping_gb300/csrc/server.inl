@@ -255,9 +255,16 @@ int ensure_prep(vdbg_map* m, PrepSet& p, int64_t total)
     dev_free(m, p.ray_scan, p.ray_cap);
     p.ray_cap        = 0;
     const size_t cap = static_cast<size_t>(total) + static_cast<size_t>(total) / 2;
-    VDBG_TRY(dev_alloc(m, &p.rays, cap));
-    VDBG_TRY(dev_alloc(m, &p.order, cap));
-    VDBG_TRY(dev_alloc(m, &p.ray_scan, cap));
+    int st = dev_alloc(m, &p.rays, cap);
+    if (st == VDBG_OK) st = dev_alloc(m, &p.order, cap);
+    if (st == VDBG_OK) st = dev_alloc(m, &p.ray_scan, cap);
+    if (st != VDBG_OK)
+    {
+      dev_free(m, p.rays, cap);
+      dev_free(m, p.order, cap);
+      dev_free(m, p.ray_scan, cap);
+      return st;
+    }
     p.ray_cap = cap;
   }
   return VDBG_OK;

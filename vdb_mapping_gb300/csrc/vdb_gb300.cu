@@ -676,9 +676,17 @@ int ensure_scratch(vdbg_map* m, int64_t n, int64_t stride, bool host_input)
     const size_t cap = std::max(static_cast<size_t>(n), m->ray_cap * 3 / 2);
     dev_free(m, m->d_ray_scan, m->ray_cap);
     m->ray_cap       = 0;
-    VDBG_TRY(dev_alloc(m, &m->d_rays, cap));
-    VDBG_TRY(dev_alloc(m, &m->d_order, cap));
-    if (m->batch) VDBG_TRY(dev_alloc(m, &m->d_ray_scan, cap));
+    int st = dev_alloc(m, &m->d_rays, cap);
+    if (st == VDBG_OK) st = dev_alloc(m, &m->d_order, cap);
+    if (st == VDBG_OK && m->batch) st = dev_alloc(m, &m->d_ray_scan, cap);
+    if (st != VDBG_OK)
+    {
+      // (what was had goes back, at the size it has)
+      dev_free(m, m->d_rays, cap);
+      dev_free(m, m->d_order, cap);
+      dev_free(m, m->d_ray_scan, cap);
+      return st;
+    }
     m->ray_cap = cap;
   }
   return VDBG_OK;
@@ -3038,12 +3046,13 @@ int morph_alloc(vdbg_map* m, MorphBuf& b, uint32_t cap, uint32_t* count, cudaStr
   cap = std::max<uint32_t>(cap, 1u);
   uint32_t hs = 1024;
   while (hs < 2ull * cap) hs <<= 1;
+  // (the sizes that morph_free counts, also where one of the four is refused)
+  b.cap   = cap;
+  b.hsize = hs;
   VDBG_TRY(dev_alloc(m, &b.origin, cap));
-  b.cap = cap;
   VDBG_TRY(dev_alloc(m, &b.mask, static_cast<size_t>(cap) * 8));
   VDBG_TRY(dev_alloc(m, &b.keys, hs));
   VDBG_TRY(dev_alloc(m, &b.vals, hs));
-  b.hsize = hs;
   VDBG_CUDA(cudaMemsetAsync(b.keys, 0xff, static_cast<size_t>(hs) * sizeof(unsigned long long), s));
   VDBG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
   return VDBG_OK;
