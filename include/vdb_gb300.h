@@ -246,7 +246,8 @@ typedef struct vdbg_tuning
   int32_t apply_chunk_runs;  /* checked (256-4096, a multiple of 256; 2048), steers nothing */
   int32_t length_edges[3];   /* checked (positive, descending; 2048, 1024, 512), steers nothing */
   float hash_load;           /* block-hash load factor (0.05-0.9; 0.5); a change rebuilds the hash */
-  int32_t dda_warps_per_sm;  /* resident traversal warps per SM in sixteenths of what fits (2-20, even; 16) */
+  int32_t dda_warps_per_sm;  /* resident traversal warps per SM in sixteenths of what fits (2-20, even; 16, and all
+                                that fits above it) */
   int32_t sweep_kernel;      /* checked (0-2; 0), steers nothing */
 } vdbg_tuning;
 
@@ -413,12 +414,11 @@ int vdbg_raytrace(vdbg_map* map, int map_index, int64_t n, const double* origins
 
 /* CUDA-graph replay of vdbg_batch_insert (batches of two or more maps; on by
  * default). The step is captured once per buffer layout and replayed as one
- * graph launch: prep, endpoint hits beside the traversal, compact, sweep. It
- * is captured again after a pool or scratch reallocation or a tuning change
+ * graph launch: prep, endpoint hits beside the traversal, the sweep, whose last
+ * block ends the window. It is captured again after a pool or scratch reallocation or a tuning change
  * (the input's address and point counts reach the graph through device
- * memory). When a step needs a pool to grow, the graph's compact and sweep
- * skip themselves on the device and the call finishes the step with separate
- * launches. Off, or with change tracking on, every step uses separate
+ * memory). When a step needs a pool to grow, the graph's sweep skips itself on
+ * the device and the call finishes the step with separate launches. Off, or with change tracking on, every step uses separate
  * launches; the results are the same either way. vdbg_graph_stats reports
  * the captures and replays so far. */
 int vdbg_batch_use_graph(vdbg_map* batch, int enable);

@@ -71,7 +71,6 @@ constexpr uint32_t kErrSpin       = 4u;
 constexpr uint32_t kErrCoordRange = 8u;
 constexpr uint32_t kErrStepBound  = 16u;
 constexpr uint32_t kErrBlockFull  = 32u;
-constexpr uint32_t kErrRunsFull   = 64u;
 
 // Ray record meta word: bits 0-28 L1 length, bit 29 clipped, bit 30 valid.
 constexpr uint32_t kMetaL1Mask   = (1u << 29) - 1;

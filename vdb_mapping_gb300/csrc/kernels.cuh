@@ -432,8 +432,8 @@ __device__ __forceinline__ uint32_t lanemask_lt()
 // (the ORs are idempotent).
 //
 // It is bound by the ALU pipe and instruction issue: a step of a warp takes
-// about 48 instructions, 28 of them on the ALU pipe, which takes one every two
-// cycles; applying 32 runs takes about 120. Measured on one GB300 against one
+// about 51 instructions, more than half of them on the ALU pipe, which takes one every
+// two cycles; applying 32 runs takes about 120. Measured on one GB300 against one
 // FP64 walk per ray with a run buffer and a merging kernel behind it (marking
 // alone, hits included): 262,144-point street scan 0.55 ms (1.10), 307,200-point
 // depth image 0.45 (0.78), 65,536-point room scan 0.097 (0.23), 16,381 random
@@ -445,7 +445,7 @@ __device__ __forceinline__ uint32_t lanemask_lt()
 constexpr int kMarchWarps          = 2;    // per block (each works by itself)
 constexpr int kMarchBlocks         = 14;   // per SM (72 registers; 12 and 16 were 1-4% slower)
 constexpr int kMarchSteps          = 4;    // steps between looks at the ends and the record list
-constexpr uint32_t kMarchRecords   = 32u * (kMarchSteps + 2);  // a remainder below 32, 8 steps, the last runs
+constexpr uint32_t kMarchRecords   = 32u * (kMarchSteps + 2);  // a remainder below 32, kMarchSteps steps, the last runs
 constexpr uint32_t kMarchMaxRounds = 96;   // far above a chunk's rounds (one more per cut)
 
 // The axis entries of march.cuh for all n below kAxisTableN in the binades
@@ -897,12 +897,13 @@ __global__ void __launch_bounds__(256) k_mark_hits(const int4* __restrict__ rays
 // do). So every lane has a group whatever the planes hold, and neighbouring
 // lanes take neighbouring groups of a plane.
 //
-// It is bound by the latency of its loads (DRAM is about half busy). Measured
-// on one GB300 against a compaction kernel and a sweep of one plane per lane
-// (eight lanes per plane for batches): street scan, 1.48M leaves with 42
-// updates each, 0.46 ms (0.53); 32 maps, 6.3M leaves with 51, 1.9 ms (2.8);
-// random long rays, 4.5M leaves with 9, 1.23 ms (1.46); 2,048 points, 3,400
-// leaves, 0.016 ms (0.030).
+// It is bound by its 32-byte sectors at random places (2.6 times the bytes of the
+// updated voxels on a street scan): its warps wait for their loads, and neither more
+// groups ahead nor more leaves a batch make it faster. Measured on one GB300 against a
+// compaction kernel and a sweep of one plane per lane (eight lanes per plane for
+// batches): street scan, 1.48M leaves with 42 updates each, 0.44 ms (0.53); 32 maps,
+// 6.3M leaves with 51, 1.8 ms (2.8); random long rays, 4.5M leaves with 9, 1.22 ms
+// (1.46); 2,048 points, 3,400 leaves, 0.012 ms (0.030).
 //
 // kPerMap: the pool holds a batch of maps, each leaf takes its map's log-odds
 // constants. kChanges: record the change set (every touched word, and the
@@ -1361,9 +1362,6 @@ __global__ void k_window_init(ChannelView c)
   *c.n_blist     = 0u;
 }
 
-// After a sweep (or a dropped marking): a fresh window for the channel.
-// `gated` (a captured step) skips it when the marking did not complete, so
-// the window is left to the host's continuation of the step.
 // A step whose rays were prepared ahead on another stream into their own
 // status block: its counters and the quantiser's error bit join the call's
 // status before the marking reads them.
@@ -1378,6 +1376,7 @@ __global__ void k_absorb_prep(DevStatus* st, const DevStatus* __restrict__ prep)
   st->error |= prep->error;
 }
 
+// After a sweep that does not end its window itself, or a dropped marking.
 __global__ void k_finish_window(ChannelView c, DevStatus* st) { finish_window(c, st); }
 
 // Inserts blocks [0, n) of the block pool into an empty block hash.
@@ -1459,14 +1458,14 @@ __global__ void k_reset_failed_leaves(int* __restrict__ bleaf, size_t cells)
 // outside (x outermost, where the pool has z-planes).
 //
 // A section's candidates are leaf slots in the order of the leaf origins (-1:
-// no leaf). Up to kSectionCells leaf cells the box itself gives that order:
-// one look-up per cell through the block index, however many leaves the map
-// holds; the kernels keep, number and write the leaves, and the copies go
-// straight into the caller's arrays. Larger boxes list the map's leaves and
-// sort them on the host, which costs more than empty cells do. Measured on one
-// GB300 through getMapSection, a box of 936 cells: 0.11 ms (0.73-1.1 ms with
-// the list, per-call allocations, a counting call and the conversion and sort
-// on the host), in a map of 4.2M leaves 0.11 ms (1.5 ms).
+// no leaf). The box itself gives that order, with one look-up per cell through
+// the block index however many leaves the map holds; the kernels keep, number and
+// write the leaves, and the copies go straight into the caller's arrays. Boxes of
+// many cells for the leaves in them, and those of more than kSectionCells, list the
+// map's leaves and sort them on the host (the rule is at section_candidates).
+// Measured on one GB300 through getMapSection, a box of 936 cells: 0.06 ms (0.73-1.1
+// ms with the list, per-call allocations, a counting call and the conversion and sort
+// on the host), in a map of 4.2M leaves as much (1.5 ms).
 // ---------------------------------------------------------------------------
 
 // Slot of the existing leaf (lx, ly, lz) of map `map`, or -1 (no insertion;
@@ -2386,7 +2385,10 @@ __global__ void k_fast_visits(DevStatus* st, PieceBuf sb)
 // first, k_span_hist / k_span_scatter), and k_trace_walk walks one span per
 // thread to its first active voxel, in the windows that can hold one
 // (hdda::trace_walk_runs): 0.53 ms for a million spans of 420 voxels, where
-// every voxel of them took 2.0. The coarse walk needs
+// every voxel of them took 2.0. (In clutter they save little and the windows cost
+// more: 200,000 queries among points scattered through 20% of the leaves take 1.82 ms
+// in both walks, 1.22 without windows; which it is only the device could tell.) The
+// coarse walk needs
 // many registers and the voxel walk few, so apart each runs at its own
 // occupancy, and the walks of a warp take about as many steps each. q holds
 // the origins [n][3], then the directions [n][3], then the lengths [n]; ok[n]

@@ -339,7 +339,6 @@ VDBG_HD Start start_axis(const Axis& a, uint32_t n, uint32_t i, int p, uint64_t 
 struct Cuts
 {
   int8_t f[3];
-  VDBG_HD bool any() const { return f[0] || f[1] || f[2]; }
 };
 
 VDBG_HD uint32_t upper(uint64_t t) { return static_cast<uint32_t>(t >> 32); }
@@ -374,7 +373,7 @@ VDBG_HD void resume(Walk& w, Cuts& c, uint32_t first, uint32_t end)
 }
 
 // The end of chunk i of 2^p, as an upper word (thresholds i * 2^-p with i < 2^20
-// have no lower bits; p <= 18). The walk goes on while t <= 1, and no time
+// have no lower bits; p <= 19: L1 < 3 * 2^22 in chunks of 32). The walk goes on while t <= 1, and no time
 // equals 1: the nearest ideal times are 1 -+ 1 / (2 n), n < 2^23, and the sums
 // are off by at most n * 2^-53.
 VDBG_HD uint32_t chunk_end(uint32_t i, int p) { return upper(threshold_bits(i + 1u, p)); }

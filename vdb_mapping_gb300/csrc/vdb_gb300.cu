@@ -35,7 +35,7 @@ struct Channel
   std::string id;
   double max_range                  = 0.0;
   unsigned long long* upd           = nullptr;  // [P][16]
-  int* touched                      = nullptr;  // [P] compacted touched leaves
+  int* touched                      = nullptr;  // [P] leaves of a marking that is dropped
   uint32_t* n_touched               = nullptr;  // device scalar
   unsigned long long* btouched      = nullptr;  // [PB][8]
   uint32_t* bepoch                  = nullptr;  // [PB]
@@ -174,7 +174,7 @@ struct vdbg_map
   uint32_t* chg_count              = nullptr;
   uint32_t chg_cur                 = 0;
   // Captured batched step: prep, endpoint hits beside the walk,
-  // compact, sweep, window end. Replayed while nothing it names has moved.
+  // sweep (which ends the window). Replayed while nothing it names has moved.
   uint64_t layout                  = 0;  // bumped by every device (re)allocation and tuning change
   bool use_graph                   = true;
   cudaGraphExec_t graph            = nullptr;
@@ -822,7 +822,7 @@ bool scan_geom_for(const vdbg_map* m, int map, const double origin[3], double ra
 }
 
 // log2 of the most steps of k_march's chunks, by the points of the call. A
-// chunk costs about 400 instructions to begin, a step of a warp about 55, so
+// chunk costs about 400 instructions to begin, a step of a warp about 51, so
 // long chunks are cheaper; a small scan needs short ones to keep the device
 // busy. Marking times on one GB300 with chunks of 32 / 64 / 128 steps: 2,048
 // points of a room (99 steps a ray) 27 / 35 / 55 us, 16,381 random rays of
@@ -1019,7 +1019,7 @@ int export_changes_short(vdbg_map* m, int map, int64_t capacity, int32_t* origin
 int launch_sweep(vdbg_map* m, Channel& c, cudaStream_t s, bool gated);
 
 // `eager`: the channel's window is the only one the call integrates, so its
-// compact, sweep and window end go out right behind the marking, gated on
+// sweep, which ends the window, goes out right behind the marking, gated on
 // the device on a marking without errors (no host round trip in between);
 // *swept tells whether they ran. Otherwise the caller sweeps.
 int run_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, const uint32_t* cursor, int64_t n,
@@ -1046,8 +1046,6 @@ int run_marking(vdbg_map* m, Channel& c, const int4* rays, const int* order, con
   return settle_marking(m, c, rays, order, cursor, n, t, may_grow, s);
 }
 
-// Integration of one update grid: compact its touched blocks into the list
-// of touched leaves, then sweep them.
 void free_changes(vdbg_map* m)
 {
   vm_free(m, m->vm_chg_words);
@@ -2806,7 +2804,7 @@ int section_list(vdbg_map* m, int mp, int3 lo, int3 hi, int k, uint32_t** list, 
 // Candidate slots of the box [lo, hi] of map `mp`, in the order of their origins
 // where `ordered` (a read; states are applied in any order), into workspace 0.
 // `lean`: by the list in any case, whose room is that of the map's leaves. *cand null:
-// none.
+// none. (kSectionCells and the constants below it say which way is taken.)
 int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, bool ordered, bool lean, int** cand, uint32_t* n_out)
 {
   *cand  = nullptr;
