@@ -479,12 +479,15 @@ def run_ours(args):
     #   HBM bytes of the window = 12 N (points) + 8.25 U (FP32 read+write and
     #     the active bit per updated voxel) + 128 Lt (visited and hit masks
     #     read once per touched leaf), over the whole insertion's kernels;
-    #   atomics of the marking = V (one visited-bit OR per DDA visit and one
-    #     hit-bit OR per unclipped ray, before any merging), over the marking
-    #     kernels (k_mark_hits, k_march), against the L2
-    #     atomic rate measured on this GPU (vdbg_l2_atomic_rate).
-    # Intermediates this design chose (ray records) are
-    # not algorithmic: they show up in `traffic` (ncu DRAM bytes).
+    # against the measured copy bandwidth. Intermediates this design chose (ray
+    # records) are not algorithmic: they show up in `traffic` (ncu DRAM bytes).
+    # Beside it the rate of the marking's visits V (one visited-bit OR per DDA
+    # visit and one hit-bit OR per unclipped ray, before any merging) and the L2
+    # atomic rate measured on this GPU (vdbg_l2_atomic_rate). That is no bound
+    # of the marking, which merges visits into z-plane runs and leaves words
+    # alone that hold them: k_march is limited by the ALU pipe and issue, the
+    # sweep by 32-byte sectors at random places (`limiters`, from the counters
+    # in profiles/launches_cases.md).
     hbm_peak, peak_kind = measured_peaks()
     mean = lambda key: statistics.mean(p[key] for p in phases)  # noqa: E731
     dda = mean("dda_ms")
@@ -503,16 +506,13 @@ def run_ours(args):
            "scope": "the whole insertion (prep, marking, sweep)",
            "traffic": sum(traffic.values()) if traffic else None}
     atomic_rate = l2_atomic_rates(local)
-    atomic = None
+    visit_rate = None
     if atomic_rate and not args.fast_mode:
-        a_achieved = mean_v / (dda / 1000.0) / 1e9
-        atomic = {"achieved": a_achieved, "peak": atomic_rate["random"] / 1e9, "unit": "G atomics/s",
-                  "frac": a_achieved / (atomic_rate["random"] / 1e9), "peak_kind": "measured (vdbg_l2_atomic_rate)",
-                  "peak_coalesced": atomic_rate["coalesced"] / 1e9, "algorithmic_atomics_per_launch": mean_v,
-                  "launch_ms": dda, "scope": "the marking (k_mark_hits, k_march)",
-                  "note": "the marking merges visits into z-plane runs before its ORs reach L2, so it issues far "
-                          "fewer atomics than V"}
-    top = atomic if atomic and atomic["frac"] > hbm["frac"] else hbm
+        visit_rate = {"visits_per_launch": mean_v, "launch_ms": dda, "visits": mean_v / (dda / 1000.0) / 1e9,
+                      "l2_atomic_rate": atomic_rate["random"] / 1e9,
+                      "l2_atomic_rate_coalesced": atomic_rate["coalesced"] / 1e9, "unit": "G/s",
+                      "scope": "the marking (k_mark_hits, k_march)",
+                      "note": "no bound: the marking issues far fewer atomics than it has visits"}
     per_kernel = {
         "prep (k_prep+k_scan+k_scatter)": {"ms": prep, "algorithmic_bytes": 12.0 * n_pts,
                                            "traffic": traffic.get("prep (k_prep+k_scan+k_scatter)")},
@@ -539,11 +539,11 @@ def run_ours(args):
                      "runs": mean_runs, "updates": mean_u, "touched_leaves": mean_lt,
                      "new_leaves": statistics.mean(s["new_leaves"] for s in stats),
                      "dda_passes": [p["passes"] for p in phases], "warmup_dda_passes": warmup_passes},
-        "roofline": {"bound": "l2_atomic" if top is atomic else "hbm",
-                     "kernel": "marking (k_mark_hits+k_march)" if top is atomic else
-                               "the whole insertion",
-                     "achieved": top["achieved"], "peak": top["peak"], "unit": top["unit"], "frac": top["frac"],
-                     "traffic": hbm["traffic"], "hbm": hbm, "atomic": atomic, "per_kernel": per_kernel},
+        "roofline": {"bound": "hbm", "kernel": "the whole insertion",
+                     "achieved": hbm["achieved"], "peak": hbm["peak"], "unit": hbm["unit"], "frac": hbm["frac"],
+                     "traffic": hbm["traffic"], "hbm": hbm, "visit_rate": visit_rate, "per_kernel": per_kernel,
+                     "limiters": {"marking (k_mark_hits+k_march)": "ALU pipe and instruction issue",
+                                  "sweep (k_sweep)": "32-byte sectors at random places"}},
         "gpu_launches": launches,
         "wall_s_timed_region": wall,
         "map_leaves": m.leafCount(),
