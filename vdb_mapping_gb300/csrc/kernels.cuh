@@ -405,6 +405,16 @@ __device__ __forceinline__ uint32_t lanemask_lt()
   return m;
 }
 
+// A slot of `count` for each active thread, one atomic for them together.
+__device__ __forceinline__ uint32_t take_slot(uint32_t* count)
+{
+  const unsigned mask = __activemask();
+  const int leader    = __ffs(mask) - 1;
+  uint32_t base       = 0;
+  if (static_cast<int>(threadIdx.x & 31) == leader) base = atomicAdd(count, static_cast<uint32_t>(__popc(mask)));
+  return __shfl_sync(mask, base, leader) + static_cast<uint32_t>(__popc(mask & lanemask_lt()));
+}
+
 // ---------------------------------------------------------------------------
 // k_march: castRayIntoGrid for every ray (VDBMapping.hpp:550-566) into the
 // update grid's visited masks.
@@ -1505,16 +1515,19 @@ __device__ __forceinline__ unsigned long long box_plane_mask(const int4& o, int 
 }
 
 // Leaves of map `map` in the map (flags set) whose 8^3 box overlaps [lo, hi]
-// (CoordBBox::hasOverlap): their slots into list[*count].
+// (CoordBBox::hasOverlap): their slots into list, their number into *count (more than
+// `room`: the rest is counted only).
 __global__ void k_section_leaves(const int4* __restrict__ origin, const uint32_t* __restrict__ flags, uint32_t n,
-                                 int map, int3 lo, int3 hi, uint32_t* __restrict__ list, uint32_t* count)
+                                 int map, int3 lo, int3 hi, uint32_t* __restrict__ list, uint32_t room,
+                                 uint32_t* count)
 {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || flags[i] == 0u) return;
   const int4 o = origin[i];
   if (o.w != map) return;
   if (o.x > hi.x || o.x + 7 < lo.x || o.y > hi.y || o.y + 7 < lo.y || o.z > hi.z || o.z + 7 < lo.z) return;
-  list[atomicAdd(count, 1u)] = i;
+  const uint32_t at = take_slot(count);
+  if (at < room) list[at] = i;
 }
 
 // Candidates of the leaf cells first + [0, dims): one thread per cell, in the
@@ -2129,16 +2142,6 @@ struct SpanBuf
 };
 using PieceBuf = SpanBuf<FastPiece, unsigned long long>;
 using TraceBuf = SpanBuf<SpanRec, uint32_t>;
-
-// A slot of `count` for each active thread, one atomic for them together.
-__device__ __forceinline__ uint32_t take_slot(uint32_t* count)
-{
-  const unsigned mask = __activemask();
-  const int leader    = __ffs(mask) - 1;
-  uint32_t base       = 0;
-  if (static_cast<int>(threadIdx.x & 31) == leader) base = atomicAdd(count, static_cast<uint32_t>(__popc(mask)));
-  return __shfl_sync(mask, base, leader) + static_cast<uint32_t>(__popc(mask & lanemask_lt()));
-}
 
 // A ray's windows during its coarse walk, in shared memory (thread's column of a
 // block's arrays): those of all its spans are written out as pieces when the ray

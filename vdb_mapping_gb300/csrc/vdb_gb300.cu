@@ -243,16 +243,18 @@ constexpr size_t kSectionRow        = 8 * sizeof(uint64_t) + 3 * sizeof(int32_t)
 constexpr size_t kPinnedAtStart      = size_t(320) << 10;  // (2,048 rows of a change list, 4,300 of a section)
 constexpr uint32_t kChangeRows      = 1u << 14;  // change lists of at most this many leaves are ordered on the device
 constexpr int64_t kMorphCells       = int64_t(1) << 18;  // leaf cells of a set taken as a dense grid (37 MB)
-// Boxes of more leaf cells than this ask first whether there is a leaf in them: 15 us of
-// a read with leaves, but an empty box of 26,000 cells takes 31 us instead of 51 (one of
-// 8,000, not asked for, 39).
+// Boxes of more leaf cells than this, in a map of fewer than 48 leaves to a cell, ask
+// first how many leaves are in them. Asking takes 15 us and 6.4 a million leaves of the
+// map, looking up a box 25 us and 0.72 a thousand cells: an empty box of 26,000 cells
+// in a small map takes 31 us instead of 51 (one of 8,000, not asked for, 39); in a map
+// of 12.9M leaves one of 26,000 takes 48, asked for 89.
 constexpr uint32_t kSectionUnasked  = 1u << 13;
+constexpr int64_t kLeavesPerCell    = 48;
 constexpr int64_t kSectionCells     = int64_t(1) << 20;  // boxes of more leaf cells list the map's leaves
-// Smaller boxes above kSectionPinned count their leaves by that list first (15 us, and
-// the end where there are none), and stay with it where sorting c leaves costs less
-// than looking up the cells: a read takes about 95 + 0.07 c us by the list, 25 + 0.72
-// a thousand cells by the cells. (262,000 cells with 74 leaves 240 us by the cells, 101
-// by the list; 500,000 cells with 4,600 leaves 430 and 422.)
+// Smaller boxes above kSectionPinned that have asked stay with the leaves where sorting
+// c of them costs less than looking up the cells: a read takes about 95 + 0.07 c us by
+// the list, 25 + 0.72 a thousand cells by the cells. (262,000 cells with 74 leaves 240
+// us by the cells, 101 by the list; 500,000 cells with 4,600 leaves 430 and 422.)
 constexpr int64_t kListedFrom       = int64_t(1) << 16;
 constexpr int64_t kCellsPerLeaf     = 100;
 // The same where their order does not matter (states are applied): looking a cell up
@@ -2782,19 +2784,25 @@ uint32_t section_cells(int3 lo, int3 hi, int3* first, int3* dims)
   return static_cast<uint32_t>(plane * dims->z);
 }
 
+bool section_asks(uint32_t cells, uint32_t leaves)
+{
+  return cells > kSectionUnasked && static_cast<int64_t>(leaves) < kLeavesPerCell * cells;
+}
+
 // The map's leaves overlapping the box [lo, hi] of map `mp`, in no order, into
-// workspace `k`: their slots at *list, *n_out of them.
-int section_list(vdbg_map* m, int mp, int3 lo, int3 hi, int k, uint32_t** list, uint32_t* n_out)
+// workspace `k`: their slots at *list, at most `room` of them; *n_out is their number.
+int section_list(vdbg_map* m, int mp, int3 lo, int3 hi, int k, uint32_t room, uint32_t** list, uint32_t* n_out)
 {
   *list  = nullptr;
   *n_out = 0;
   cudaStream_t s   = m->stream;
   const uint32_t n = std::min(m->n_leaves, m->capacity);
-  VDBG_TRY(work_ensure(m, k, static_cast<size_t>(n) * sizeof(uint32_t) + 256));
+  room             = std::min(room, n);
+  VDBG_TRY(work_ensure(m, k, static_cast<size_t>(room) * sizeof(uint32_t) + 256));
   uint32_t* count = reinterpret_cast<uint32_t*>(m->work[k]);
   *list           = count + 64;
   VDBG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
-  k_section_leaves<<<(n + 255) / 256, 256, 0, s>>>(m->origin, m->flags, n, mp, lo, hi, *list, count);
+  k_section_leaves<<<(n + 255) / 256, 256, 0, s>>>(m->origin, m->flags, n, mp, lo, hi, *list, room, count);
   VDBG_CUDA(cudaGetLastError());
   VDBG_CUDA(cudaMemcpyAsync(n_out, count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   VDBG_CUDA(cudaStreamSynchronize(s));
@@ -2811,19 +2819,30 @@ int section_candidates(vdbg_map* m, int mp, int3 lo, int3 hi, bool ordered, bool
   *n_out = 0;
   cudaStream_t s = m->stream;
   int3 first, dims;
-  const uint32_t cells = std::min(m->n_leaves, m->capacity) > 0 ? section_cells(lo, hi, &first, &dims) : 0u;
+  const uint32_t leaves = std::min(m->n_leaves, m->capacity);
+  const uint32_t cells  = leaves > 0 ? section_cells(lo, hi, &first, &dims) : 0u;
   if (cells == 0) return VDBG_OK;
   uint32_t* list = nullptr;
   uint32_t c     = 0;
   bool listed    = false;
-  if (lean || cells > (ordered ? kSectionPinned : kSectionUnordered))
+  // What is asked of the map's leaves, and the room for it: all that overlap the box, or
+  // (a read of at most kSectionCells) as many as make the list the better way. States
+  // take the way with less room.
+  bool ask      = lean || cells > kSectionCells;
+  uint32_t room = leaves;
+  if (!ask && ordered && section_asks(cells, leaves))
   {
-    const int st = section_list(m, mp, lo, hi, ordered ? 1 : 0, &list, &c);
+    ask  = true;
+    room = cells > kListedFrom ? static_cast<uint32_t>((cells - kListedFrom) / kCellsPerLeaf) : 0u;
+  }
+  if (!ask && !ordered) ask = cells > kSectionUnordered && cells > leaves / 3u;
+  if (ask)
+  {
+    const int st = section_list(m, mp, lo, hi, ordered ? 1 : 0, room, &list, &c);
     // (without room for the list, the cells' table may still fit)
     if (st != VDBG_OK && (st != VDBG_ERR_OUT_OF_MEMORY || lean || cells > kSectionCells)) return st;
     if (st == VDBG_OK && c == 0) return VDBG_OK;
-    listed =
-      st == VDBG_OK && (lean || !ordered || cells > kSectionCells || cells > kListedFrom + kCellsPerLeaf * c);
+    listed = st == VDBG_OK && c <= room;
   }
   if (!listed)
   {
@@ -2954,11 +2973,11 @@ int section_export(vdbg_map* m, int mp, int3 lo, int3 hi, int full, int64_t capa
   int st = VDBG_ERR_OUT_OF_MEMORY;
   if (cells <= kSectionPinned)
   {
-    if (cells > kSectionUnasked)
+    if (section_asks(cells, std::min(m->n_leaves, m->capacity)))
     {
       uint32_t* list = nullptr;
       uint32_t c     = 0;
-      st             = section_list(m, mp, lo, hi, 1, &list, &c);
+      st             = section_list(m, mp, lo, hi, 1, 0u, &list, &c);
       if (st == VDBG_OK && c == 0) return VDBG_OK;
       if (st != VDBG_OK && st != VDBG_ERR_OUT_OF_MEMORY) return st;
     }
