@@ -63,16 +63,6 @@ def _origin(origin):
     return o
 
 
-def _rows(n, *arrays):
-    """The arrays' first n rows. Room of more than eight times that goes back, so that a
-    result that is kept does not keep it (in place: nothing is copied)."""
-    if 8 * n >= len(arrays[0]):
-        return tuple(a[:n] for a in arrays)
-    for a in arrays:
-        a.resize((n, *a.shape[1:]), refcheck=False)
-    return arrays
-
-
 def _export_changes(lib, h, map_index, check):
     """(origins (L,3) int32, active (L,8) uint64, value (L,8) uint64) of the
     last integration's change set."""
@@ -88,7 +78,8 @@ def _export_changes(lib, h, map_index, check):
             cap = n.value
             continue
         check(s, "vdbg_export_changes")
-        return _rows(n.value, origins, active, value)
+        k = n.value
+        return origins[:k], active[:k], value[:k]
 
 
 class Grid:
@@ -208,7 +199,8 @@ def _section_export(lib, h, map_index, lo, hi, full, check):
             cap = n.value
             continue
         check(s, "vdbg_export_section")
-        return _rows(n.value, origins, values, masks)
+        k = n.value
+        return origins[:k], values[:k], masks[:k]
 
 
 def _section_states(lib, h, map_index, lo, hi, origins, masks, check):
@@ -251,7 +243,7 @@ def _morphology(lib, h, origins, masks, op, iterations, check, keep_leaves=False
             cap = n.value
             continue
         check(s, "vdbg_section_morphology")
-        return _rows(n.value, oo, om)
+        return oo[: n.value], om[: n.value]
 
 
 def _close_value_section(lib, h, origins, values, masks, iterations, check):
